@@ -1,0 +1,417 @@
+// Recurrences S <- decay S + weight k v^T, y = S^T q with one decay and one weight a head and
+// row (ssd.cu, mlstm.cu) over the many rows of a prompt, 64 rows at a time and all chunks side by
+// side, as products on the tensor cores of operands split in two (split_mma.cuh).
+//
+//   chunk_state_kernel   what each chunk adds to the memory, from zero: sum_s W_s k_s v_s^T
+//   chunk_carry_kernel   the memory before each chunk, chunk after chunk, element by element; the
+//                        running state's start and end
+//   chunk_out_kernel     a chunk's rows: alpha_t (q_t . S) + sum_{s<=t} w_ts (q_t . k_s) v_s
+//
+// W, alpha and w come from the policy (which recurrence): products of decays as exponentials of
+// differences of their running logarithms.  Those are summed in 64 bits from the chunk's first row
+// and kept as two 32-bit numbers each, so that the difference of neighbours is as exact as 32 bits
+// allow however far the sum has run.
+//
+// A walk through the rows has one chain of dependent steps a head and leaves most SMs without
+// work; chunks cost the memory's way out and back (heads x N x P floats each) and about twice the
+// arithmetic.  A prompt of 2,048 rows: 1.2 ms walking and 0.15 ms in chunks for 32 heads of 64 x 128
+// (36 us the chunks' sums, 19 the carry, 96 the rows), 0.76 and 0.14 ms for 8 of 128 x 256 (36, 27 and
+// 74); the three kernels are bound by the tensor pipe's mma.sync rate and, in the carry, by L2.  64 rows: with 32 that traffic doubles, with 128 the products inside the chunk do and
+// a block no longer shares its SM.
+//
+// A policy `Pol` gives: q, k, v rows (float32, 16-byte aligned, counts in fours), `heads`, `per`
+// (heads per q/k head), N (elements of q and k, at most 128), P (elements of v) and the functions
+// named below.  What depends on a step: sequence `seq`'s rows `first_row` .. in chunks from
+// `seg * seg_rows` on, so that a long step can go through a bounded scratch in several rounds.
+#pragma once
+
+#include "attn_mma.cuh"
+#include "common.cuh"
+#include "split_mma.cuh"
+
+namespace chunk {
+
+using namespace rfx;
+
+constexpr int L = 64;     // rows of a chunk
+constexpr int PT = 64;    // elements of v a block takes at a time
+constexpr int VLD = PT + 4;  // row stride of v's tile: 2 VLD = 8 mod 32, four rows' reads meet all banks
+
+struct Step {
+    const int* seq_slot;
+    const int* seq_row0;
+    int seg_rows, seg, n_segs;
+    float* scratch;  // [place][head][P][N] (+ [N] with a normaliser): a chunk's own sum, then the memory before it
+    float4* aux;     // [place][head]: what the carry needs of a chunk
+    float* before;   // [place][head]: the policy's running number before the chunk
+};
+
+// The place of chunk c (of this segment) of sequence `seq` among all: with one segment at most
+// R / L + sequences of them, with several (seg_rows / L) x sequences.
+__device__ __forceinline__ size_t place_of(const Step& s, int row0, int seq, int c) {
+    return s.n_segs == 1 ? (size_t)row0 / L + seq + c : (size_t)seq * (s.seg_rows / L) + c;
+}
+
+struct Rows {
+    int first, n;  // the chunk's first row and how many it has
+    size_t place;
+};
+__device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
+    const int row0 = s.seq_row0[seq], from = row0 + s.seg * s.seg_rows;
+    const int to = min(s.seq_row0[seq + 1], from + s.seg_rows);
+    const int first = from + c * L;
+    return {first, min(L, to - first), place_of(s, row0, seq, c)};
+}
+
+// A tile of `rows` rows of 4 * c4 floats, rows from n on and columns from n4 (in fours) on zero.
+template <int THREADS>
+__device__ __forceinline__ void load_tile(float* dst, int ld, const float* src, size_t src_ld, int rows, int n, int c4,
+                                          int n4) {
+    for (int e = threadIdx.x; e < rows * c4; e += THREADS) {
+        const int r = e / c4, c = e - r * c4;
+        const bool ok = r < n && c < n4;
+        attn::cp_async_16(dst + r * ld + 4 * c, ok ? src + (size_t)r * src_ld + 4 * c : src, ok);
+    }
+}
+
+// A block a (chunk, head, PT elements of v): the chunk's own sum, [P][N].  Warps: 16 of v's elements
+// by 64 of k's.
+template <class Pol>
+__global__ void __launch_bounds__(256) chunk_state_kernel(Pol pol, Step st) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ __align__(8) float wl[L];
+    rfx::pdl_prologue();
+    const int seq = blockIdx.y;
+    const Rows ch = rows_of(st, seq, blockIdx.x);
+    if (ch.n <= 0) return;
+    const int ptiles = (pol.P + PT - 1) / PT, h = blockIdx.z / ptiles, p0 = (blockIdx.z - h * ptiles) * PT;
+    const int N8 = (pol.N + 7) / 8 * 8, ldk = N8 + 4;
+    float *Vs = sm, *Ks = sm + L * VLD;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+    load_tile<256>(Vs, VLD, pol.v_row(ch.first, h) + p0, pol.ldv, L, ch.n, PT / 4, min(PT, pol.P - p0) / 4);
+    load_tile<256>(Ks, ldk, pol.k_row(ch.first, h), pol.ldk, L, ch.n, N8 / 4, pol.N / 4);
+    attn::cp_async_commit();
+    const size_t at = ch.place * pol.heads + h;
+    if (warp == 0) {
+        const float4 a = pol.state_weights(wl, h, ch.first, ch.n, lane);
+        if (p0 == 0 && lane == 0) st.aux[at] = a;
+    }
+    attn::cp_async_wait<0>();
+    __syncthreads();
+    const int pm = (warp & 3) * 16, n0 = (warp >> 2) * 64;
+    const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
+    float* out = st.scratch + at * E;
+    if (n0 < N8 && p0 + pm < pol.P) {
+        float acc[8][4] = {};
+#pragma unroll 2
+        for (int s = 0; s < L / 8; ++s) {
+            const float2 w = *reinterpret_cast<const float2*>(wl + 8 * s + 2 * j);
+            const float* v = Vs + (8 * s + 2 * j) * VLD + pm + g;
+            const Left a = left_from(v[0] * w.x, v[8] * w.x, v[VLD] * w.y, v[VLD + 8] * w.y);
+            const float* k = Ks + (8 * s + 2 * j) * ldk + g;
+            float2 b[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const int c = n0 + 8 * t < N8 ? n0 + 8 * t : 0;  // a tile beyond N: any column, not stored
+                b[t] = make_float2(k[c], k[ldk + c]);
+            }
+            product3<8>(acc, a, b);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int n = n0 + 8 * t + 2 * j, p = p0 + pm + g;
+            if (n < pol.N) {
+                if (p < pol.P) store2(out + (size_t)p * pol.N + n, acc[t][0], acc[t][1]);
+                if (p + 8 < pol.P) store2(out + (size_t)(p + 8) * pol.N + n, acc[t][2], acc[t][3]);
+            }
+        }
+    }
+    if (Pol::NORMALISER && p0 == 0)
+        for (int n = threadIdx.x; n < pol.N; n += 256) {
+            float a = 0.0f;
+            for (int s = 0; s < ch.n; ++s) a = fmaf(wl[s], Ks[s * ldk + n], a);
+            out[(size_t)pol.P * pol.N + n] = a;
+        }
+}
+
+// Four neighbouring elements of a head's memory a thread; eight chunks' sums are fetched ahead.
+template <class Pol>
+__global__ void __launch_bounds__(128) chunk_carry_kernel(Pol pol, Step st) {
+    constexpr int AHEAD = 8;
+    rfx::pdl_prologue();
+    const int seq = blockIdx.y, h = blockIdx.z;
+    const int e = 4 * (blockIdx.x * 128 + threadIdx.x);
+    const int E = pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
+    if (e >= E) return;
+    const int row0 = st.seq_row0[seq], from = row0 + st.seg * st.seg_rows;
+    const int rows = min(st.seq_row0[seq + 1] - from, st.seg_rows);
+    const int n = (rows + L - 1) / L;
+    if (rows <= 0) return;
+    const int slot = st.seq_slot[seq];
+    float4 S = pol.load_state(slot, h, e);
+    float m = pol.load_number(slot, h);
+    const size_t at = place_of(st, row0, seq, 0) * pol.heads + h;
+    float* sc = st.scratch + at * E + e;
+    const size_t step = (size_t)pol.heads * E;
+    for (int c0 = 0; c0 < n; c0 += AHEAD) {
+        float4 d[AHEAD], a[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (c0 + i < n) {
+                d[i] = *reinterpret_cast<const float4*>(sc + (c0 + i) * step);
+                a[i] = st.aux[at + (size_t)(c0 + i) * pol.heads];
+            }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (c0 + i < n) {
+                *reinterpret_cast<float4*>(sc + (c0 + i) * step) = S;
+                if (e == 0) st.before[at + (size_t)(c0 + i) * pol.heads] = m;
+                const float2 f = pol.carry(a[i], m);
+                S.x = fmaf(f.x, S.x, f.y * d[i].x);
+                S.y = fmaf(f.x, S.y, f.y * d[i].y);
+                S.z = fmaf(f.x, S.z, f.y * d[i].z);
+                S.w = fmaf(f.x, S.w, f.y * d[i].w);
+            }
+    }
+    pol.store_state(slot, h, e, S);
+    if constexpr (Pol::NORMALISER) {
+        if (e == 0) pol.store_number(slot, h, m);
+    }
+}
+
+// Inclusive sums (or maxima) over the chunk's 64 rows, lane i holding rows i and i + 32.
+__device__ __forceinline__ void scan_sum(double& a, double& b, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+        if (lane >= o) {
+            a += x;
+            b += y;
+        }
+    }
+    b += __shfl_sync(0xffffffffu, a, 31);
+}
+__device__ __forceinline__ void scan_max(double& a, double& b, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+        if (lane >= o) {
+            a = fmax(a, x);
+            b = fmax(b, y);
+        }
+    }
+    b = fmax(b, __shfl_sync(0xffffffffu, a, 31));
+}
+__device__ __forceinline__ void two_parts(double v, float* hi, float* lo) {
+    const float h = (float)v;
+    *hi = h;
+    *lo = isinf(h) ? 0.0f : (float)(v - (double)h);
+}
+
+// The rows' weights of a chunk and head: w_ts = exp((g_s + e_t)) * w_s, g and e in two parts.
+struct Weights {
+    float g_hi[L], g_lo[L], e_hi[L], e_lo[L], w[L], alpha[L], extra[L];
+};
+
+// A block a (chunk, q/k head, some of that head's items); an item is a (head, PT elements of v).
+// A warp takes sixteen rows: their products with the chunk's k, once, stay in registers; then item
+// by item the memory's tile and v's replace k's in shared memory.
+template <class Pol>
+__global__ void __launch_bounds__(128) chunk_out_kernel(Pol pol, Step st, int items_a_block) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ Weights wt;
+    __shared__ float nv[128];
+    rfx::pdl_prologue();
+    const int seq = blockIdx.y;
+    const Rows ch = rows_of(st, seq, blockIdx.x);
+    if (ch.n <= 0) return;
+    const int ptiles = (pol.P + PT - 1) / PT, items = pol.per * ptiles;
+    const int sets = (items + items_a_block - 1) / items_a_block;
+    const int kvh = blockIdx.z / sets, i0 = (blockIdx.z - kvh * sets) * items_a_block;
+    const int i1 = min(items, i0 + items_a_block);
+    const int N8 = (pol.N + 7) / 8 * 8, ld = N8 + 8;
+    float *Qs = sm, *Bs = sm + L * ld, *Vs = Bs + L * ld;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+    load_tile<128>(Qs, ld, pol.q_row(ch.first, kvh * pol.per), pol.ldq, L, ch.n, N8 / 4, pol.N / 4);
+    load_tile<128>(Bs, ld, pol.k_row(ch.first, kvh * pol.per), pol.ldk, L, ch.n, N8 / 4, pol.N / 4);
+    attn::cp_async_commit();
+    attn::cp_async_wait<0>();
+    __syncthreads();
+    const float* qa = Qs + (16 * warp + g) * ld + 2 * j;
+    const int tiles = 2 * warp + 2;  // of eight rows s <= the warp's last row
+    float G[8][4] = {};
+    if (warp >= 2) {
+        for (int s = 0; s < N8 / 8; ++s) {
+            const float2 x = *reinterpret_cast<const float2*>(qa + 8 * s);
+            const float2 y = *reinterpret_cast<const float2*>(qa + 8 * ld + 8 * s);
+            const Left a = left_from(x.x, y.x, x.y, y.y);
+            float2 b[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
+            product3<8>(G, a, b);
+        }
+    } else {
+        for (int s = 0; s < N8 / 8; ++s) {
+            const float2 x = *reinterpret_cast<const float2*>(qa + 8 * s);
+            const float2 y = *reinterpret_cast<const float2*>(qa + 8 * ld + 8 * s);
+            const Left a = left_from(x.x, y.x, x.y, y.y);
+            float2 b[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
+            product3<4>(*reinterpret_cast<float(*)[4][4]>(&G), a, b);
+        }
+    }
+    int head = -1;
+    for (int item = i0; item < i1; ++item) {
+        const int h = kvh * pol.per + item / ptiles, p0 = (item % ptiles) * PT;
+        const size_t at = ch.place * pol.heads + h;
+        const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
+        const float* S = st.scratch + at * E;
+        __syncthreads();  // k, or the item before, has been read by every warp
+        load_tile<128>(Bs, ld, S + (size_t)p0 * pol.N, pol.N, PT, min(PT, pol.P - p0), N8 / 4, pol.N / 4);
+        load_tile<128>(Vs, VLD, pol.v_row(ch.first, h) + p0, pol.ldv, L, ch.n, PT / 4, min(PT, pol.P - p0) / 4);
+        attn::cp_async_commit();
+        if (h != head) {
+            if (warp == 0) pol.row_weights(wt, h, ch.first, ch.n, st.before[at], lane);
+            if (Pol::NORMALISER)
+                for (int n = threadIdx.x; n < pol.N; n += 128) nv[n] = S[(size_t)pol.P * pol.N + n];
+            head = h;
+        }
+        attn::cp_async_wait<0>();
+        __syncthreads();
+        const int ra = 16 * warp + g, rb = ra + 8;
+        float acc[8][4] = {};
+        for (int s = 0; s < N8 / 8; ++s) {
+            const float2 x = *reinterpret_cast<const float2*>(qa + 8 * s);
+            const float2 y = *reinterpret_cast<const float2*>(qa + 8 * ld + 8 * s);
+            const Left a = left_from(x.x, y.x, x.y, y.y);
+            float2 b[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
+            product3<8>(acc, a, b);
+        }
+        const float aa = wt.alpha[ra], ab = wt.alpha[rb];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            acc[t][0] *= aa;
+            acc[t][1] *= aa;
+            acc[t][2] *= ab;
+            acc[t][3] *= ab;
+        }
+        const float eah = wt.e_hi[ra], eal = wt.e_lo[ra], ebh = wt.e_hi[rb], ebl = wt.e_lo[rb];
+        float sum_a = 0.0f, sum_b = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            if (t < tiles) {
+                float p[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int s = 8 * t + 2 * j + i;
+                    const float gh = wt.g_hi[s], gl = wt.g_lo[s], w = wt.w[s];
+                    p[i] = s <= ra ? G[t][i] * (w * expf((gh + eah) + (gl + eal))) : 0.0f;
+                    p[2 + i] = s <= rb ? G[t][2 + i] * (w * expf((gh + ebh) + (gl + ebl))) : 0.0f;
+                }
+                if (Pol::NORMALISER) {
+                    sum_a += p[0] + p[1];
+                    sum_b += p[2] + p[3];
+                }
+                const Left a = left_of(p);
+                const float* v = Vs + (8 * t + 2 * j) * VLD + g;
+                float2 b[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) b[c] = make_float2(v[8 * c], v[VLD + 8 * c]);
+                product3<8>(acc, a, b);
+            }
+        }
+        if constexpr (Pol::NORMALISER) {
+            if (p0 == 0) {
+                float qa_n = 0.0f, qb_n = 0.0f;
+                for (int n = j; n < pol.N; n += 4) {
+                    qa_n = fmaf(Qs[ra * ld + n], nv[n], qa_n);
+                    qb_n = fmaf(Qs[rb * ld + n], nv[n], qb_n);
+                }
+                sum_a = fmaf(aa, qa_n, sum_a);
+                sum_b = fmaf(ab, qb_n, sum_b);
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    sum_a += __shfl_xor_sync(0xffffffffu, sum_a, o);
+                    sum_b += __shfl_xor_sync(0xffffffffu, sum_b, o);
+                }
+                if (j == 0) {
+                    if (ra < ch.n) pol.store_sum(ch.first + ra, h, sum_a, wt.extra[ra]);
+                    if (rb < ch.n) pol.store_sum(ch.first + rb, h, sum_b, wt.extra[rb]);
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int p = p0 + 8 * t + 2 * j;
+            if (p < pol.P) {
+                const float* va = Vs + ra * VLD + 8 * t + 2 * j;
+                const float* vb = Vs + rb * VLD + 8 * t + 2 * j;
+                if (ra < ch.n) pol.store_row(ch.first + ra, h, p, acc[t][0], acc[t][1], va[0], va[1]);
+                if (rb < ch.n) pol.store_row(ch.first + rb, h, p, acc[t][2], acc[t][3], vb[0], vb[1]);
+            }
+        }
+    }
+}
+
+inline long long places(int R, int n_seq, int seg_rows, int n_segs) {
+    return n_segs == 1 ? R / L + n_seq : (long long)n_seq * (seg_rows / L);
+}
+
+// Floats of scratch a step needs: the memories of all its chunks, up to about `budget` floats;
+// beyond that the rows go through in rounds of `*seg_rows` rows a sequence.
+inline long long scratch_floats(int R, int n_seq, int max_rows, int heads, long long E, int* seg_rows) {
+    const long long budget = 64LL << 20;  // 256 MB
+    const long long one = heads * (E + 8);
+    const int whole = (max_rows + L - 1) / L * L;
+    int seg = whole;
+    if ((long long)(R / L + n_seq) * one > budget) {
+        seg = (int)((budget / (one * n_seq)) * L);
+        if (seg < 4 * L) seg = 4 * L;
+        if (seg >= whole) seg = whole;
+    }
+    *seg_rows = seg;
+    return places(R, n_seq, seg, (max_rows + seg - 1) / seg) * one;
+}
+
+template <class Pol>
+int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int R, int max_rows, float* scratch,
+        cudaStream_t s) {
+    const long long E = (long long)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
+    int seg_rows = 0;
+    scratch_floats(R, n_seq, max_rows, pol.heads, E, &seg_rows);
+    Step st;
+    st.seq_slot = seq_slot;
+    st.seq_row0 = seq_row0;
+    st.seg_rows = seg_rows;
+    st.n_segs = (max_rows + seg_rows - 1) / seg_rows;
+    const long long n_places = places(R, n_seq, seg_rows, st.n_segs);
+    st.scratch = scratch;
+    st.aux = reinterpret_cast<float4*>(scratch + n_places * pol.heads * E);  // E is a multiple of four
+    st.before = scratch + n_places * pol.heads * (E + 4);
+    const int N8 = (pol.N + 7) / 8 * 8, ptiles = (pol.P + PT - 1) / PT;
+    const int chunks = (min(seg_rows, max_rows) + L - 1) / L;
+    const size_t sm_state = (size_t)L * (VLD + N8 + 4) * sizeof(float);
+    const size_t sm_out = (size_t)L * (VLD + 2 * (N8 + 8)) * sizeof(float);
+    const int qk_heads = pol.heads / pol.per, items = pol.per * ptiles;
+    // as many items a block as leave two blocks an SM: the rows' products with k serve them all
+    int ipb = items;
+    while (ipb > 1 && (long long)chunks * n_seq * qk_heads * ((items + ipb - 1) / ipb) < 2LL * sm_count()) ipb = (ipb + 1) / 2;
+    const int sets = (items + ipb - 1) / ipb;
+    if (n_seq > 65535 || (long long)pol.heads * ptiles > 65535 || (long long)qk_heads * sets > 65535)
+        return RFX_ERR_UNSUPPORTED;
+    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_state);
+    if (e != cudaSuccess) return (int)e;
+    e = cudaFuncSetAttribute(chunk_out_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_out);
+    if (e != cudaSuccess) return (int)e;
+    for (st.seg = 0; st.seg < st.n_segs; ++st.seg) {
+        RFX_LAUNCH(chunk_state_kernel<Pol>, dim3(chunks, n_seq, pol.heads * ptiles), 256, sm_state, s, pol, st);
+        RFX_LAUNCH(chunk_carry_kernel<Pol>, dim3((unsigned)((E / 4 + 127) / 128), n_seq, pol.heads), 128, 0, s, pol, st);
+        RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, n_seq, qk_heads * sets), 128, sm_out, s, pol, st, ipb);
+    }
+    return 0;
+}
+
+}  // namespace chunk

@@ -11,17 +11,15 @@
 // chunk: rfx_gated_delta_chunk_prep does that for all chunks side by side, and
 // rfx_gated_delta_chunk walks the chunks with the products.
 //
-// The memory stays 32-bit (the products' accumulators are the memory itself).  Products run as
-// three tensor-core products of operands split into a leading and a trailing part of 11 bits
-// (x = hi + lo exactly up to 2^-22; hi hi + hi lo + lo hi, 32-bit sums): 32-bit products up
-// to about 2^-21 of their size.  The true 32-bit path takes the row-by-row kernel instead.
+// The memory stays 32-bit (the products' accumulators are the memory itself); products are
+// those of split_mma.cuh.  The true 32-bit path takes the row-by-row kernel instead.
 //
-// S^T [16 columns x channels] of a warp is an accumulator tile row of mma.sync m16n8k8, and,
-// with the channels of every eight taken in the order (0, 2, 4, 6, 1, 3, 5, 7), the same
-// registers are the left operand of the next chunk's products; likewise u^T.
+// S^T [16 columns x channels] of a warp is an accumulator tile row of mma.sync m16n8k8, and the
+// same registers are the left operand of the next chunk's products; likewise u^T.
 #include "attn_mma.cuh"
 #include "common.cuh"
 #include "sm100.cuh"
+#include "split_mma.cuh"
 
 namespace {
 
@@ -31,54 +29,9 @@ constexpr int TLD = 24;           // row stride of T and M: a fragment's 8-byte 
 // per chunk and head: T [16][TLD], M [16][TLD], c [16], r_last [16], c_last and padding
 constexpr int COEF = 2 * CH * TLD + 2 * CH + 4;
 
-struct Split {
-    uint32_t hi, lo;
-};
-__device__ __forceinline__ Split split(float x) {
-    const uint32_t h = __float_as_uint(x) & 0xffffe000u;
-    return {h, __float_as_uint(x - __uint_as_float(h))};
-}
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// The left operand of a k-step from an accumulator tile (columns 2 j and 2 j + 1 are the k
-// places j and j + 4), split.
-struct Left {
-    uint32_t hi[4], lo[4];
-};
-__device__ __forceinline__ Left left_of(const float (&t)[4]) {
-    Left l;
-    const int order[4] = {0, 2, 1, 3};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const Split s = split(t[order[i]]);
-        l.hi[i] = s.hi;
-        l.lo[i] = s.lo;
-    }
-    return l;
-}
-// d[n] += a b[n]^T for N right operands, pass by pass so that the products of different n
-// follow one another, not those of one sum.
-template <int N>
-__device__ __forceinline__ void product3(float (&d)[N][4], const Left& a, const float2 (&b)[N]) {
-    Split x[N], y[N];
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-        x[n] = split(b[n].x);
-        y[n] = split(b[n].y);
-    }
-#pragma unroll
-    for (int n = 0; n < N; ++n) mma_tf32(d[n], a.lo, x[n].hi, y[n].hi);
-#pragma unroll
-    for (int n = 0; n < N; ++n) mma_tf32(d[n], a.hi, x[n].lo, y[n].lo);
-#pragma unroll
-    for (int n = 0; n < N; ++n) mma_tf32(d[n], a.hi, x[n].hi, y[n].hi);
-}
+using rfx::Left;
+using rfx::left_of;
+using rfx::product3;
 
 // `bytes` (a multiple of 16, both addresses 16-byte aligned) into shared memory, counted on `bar`.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {

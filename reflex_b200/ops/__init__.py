@@ -859,17 +859,23 @@ def mlstm_state_floats(dim: int, vdim: int) -> int:
 
 
 MLSTM_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_CHUNK_MIN_ROWS", 48, 1, 1 << 30)
+# from here on the tensor-core chunks: level with the walk at 48 to 64 rows of a sequence (the whole
+# mixer at width 2048: 50 us walking and 53 in chunks at 48 rows, 76 and 54 at 100)
+MLSTM_CHUNKS_MIN_ROWS = 64
 
 
 def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale: float, batch,
-               state: torch.Tensor, heads: int, dim: int, vdim: int, max_rows: Optional[int] = None):
+               state: torch.Tensor, heads: int, dim: int, vdim: int, max_rows: Optional[int] = None,
+               exact: bool = True):
     """The recurrence over the step's rows, sequence by sequence.  `proj`
     float32 [R, ld] holds q, k, v and the two gate pre-activations at the
     column offsets `offsets` = (q, k, v, i, f); `state` [slots, heads, floats].
     Returns the numerators S^T q [R, heads * vdim] and denominators [R, heads].
     `max_rows`: the most rows any sequence brings; from `MLSTM_CHUNK_MIN_ROWS`
     on (and dim up to 256) the chunkwise kernel runs, else the row-by-row walk:
-    the same function, rounded differently."""
+    the same function, rounded differently.  Without `exact`, and for dim up to 128,
+    many rows go through the kernels that take 64 at a time on the tensor cores, products
+    of 32-bit numbers split in two (csrc/mlstm_chunk.cu)."""
     R = proj.shape[0]
     _chk(proj, "proj", torch.float32)
     if state.shape[-1] != mlstm_state_floats(dim, vdim) or state.shape[-2] != heads:
@@ -878,6 +884,19 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale:
     den = _new((R, heads), torch.float32, proj.device)
     q_off, k_off, v_off, i_off, f_off = (int(o) for o in offsets)
     chunked = max_rows is not None and max_rows >= MLSTM_CHUNK_MIN_ROWS and dim <= 256
+    if chunked and not exact and max_rows >= MLSTM_CHUNKS_MIN_ROWS and dim <= 128 and dim % 4 == 0 and vdim % 4 == 0:
+        S, most = batch.seq_slot.numel(), min(int(max_rows), R)
+        scratch = _new((int(native.lib().rfx_mlstm_chunks_floats(R, S, most, heads, dim, vdim)),), torch.float32,
+                       proj.device)
+        st = native.lib().rfx_mlstm_chunks(
+            proj.data_ptr(), proj.shape[1], q_off, k_off, v_off, i_off, f_off, _chk(bias_i, "bias_i", torch.float32),
+            _chk(bias_f, "bias_f", torch.float32), float(cap), float(q_scale),
+            _chk(batch.seq_slot, "seq_slot", torch.int32), _chk(batch.seq_row0, "seq_row0", torch.int32), S, R, most,
+            _chk(state, "state", torch.float32), num.data_ptr(), den.data_ptr(), scratch.data_ptr(), heads, dim, vdim,
+            _stream())
+        if st != native.ERR_UNSUPPORTED:  # rows that are not on 16 bytes
+            native.check(st, f"mlstm_chunks (dim={dim}, vdim={vdim})")
+            return num, den
     fn = native.lib().rfx_mlstm_chunk if chunked else native.lib().rfx_mlstm_scan
     st = fn(
         proj.data_ptr(), proj.shape[1], q_off, k_off, v_off, i_off, f_off,
@@ -1663,14 +1682,24 @@ def attention_sigmoid(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv
 
 
 # ------------------------------------------- recurrences with a matrix state a head
+# Rows of the longest sequence from which the chunked kernels run: their three launches and the
+# memory's way out and back cost about 30 us, the walk 0.5 us a row (one sequence, width 2048, the
+# whole mixer: 71 us walking and 79 in chunks at 48 rows, 106 and 84 at 100; eight sequences of 37
+# rows 117 and 105).
+SSD_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_SSD_CHUNK_MIN_ROWS", 80, 1, 1 << 30)
+
+
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_bias: torch.Tensor, A: torch.Tensor,
              D: Optional[torch.Tensor], state: torch.Tensor, state_off: int, batch, heads: int, vdim: int,
-             states: int, groups: int, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
+             states: int, groups: int, out_dtype: torch.dtype = torch.float32, exact: bool = True) -> torch.Tensor:
     """The state-space recurrence with one decay a head (csrc/ssd.cu): `xbc` float32
     rows [x | B | C], `proj` float32 rows with z at `z_off` and the step sizes'
     pre-activations at `dt_off`; `A` float32 [heads], negative; the running state is
     `state[slot, state_off : state_off + heads * states * vdim]`.  Returns
-    (S^T C + D x) * silu(z), [R, heads * vdim]."""
+    (S^T C + D x) * silu(z), [R, heads * vdim].  Without `exact`, from
+    `SSD_CHUNK_MIN_ROWS` rows of a sequence on the kernels that take 64 rows at a time
+    run (csrc/ssd_chunk.cu: the same function, products of 32-bit numbers split for the
+    tensor cores); else, and for sizes those do not take, the row-by-row walk."""
     R = xbc.shape[0]
     inner = heads * vdim
     if xbc.shape[1] != inner + 2 * groups * states:
@@ -1678,6 +1707,21 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
     if z_off + inner > proj.shape[1] or dt_off + heads > proj.shape[1]:
         raise InvalidInput("ssd_scan: z or dt do not fit into the rows of proj")
     out = _new((R, inner), out_dtype, xbc.device)
+    chunked = batch.max_new >= SSD_CHUNK_MIN_ROWS or (batch.max_new >= 32 and R >= 256 and SSD_CHUNK_MIN_ROWS <= 256)
+    if (not exact and chunked and out_dtype == torch.float32 and vdim % 4 == 0
+            and states % 4 == 0 and states <= 128):
+        S, most = batch.seq_slot.numel(), int(batch.max_new)
+        scratch = _new((int(native.lib().rfx_ssd_chunk_floats(R, S, most, heads, vdim, states)),), torch.float32,
+                       xbc.device)
+        st = native.lib().rfx_ssd_chunk(
+            _chk(xbc, "xbc", torch.float32), xbc.shape[1], _chk(proj, "proj", torch.float32), proj.shape[1], int(z_off),
+            int(dt_off), _chk(dt_bias, "dt_bias", torch.float32), _chk(A, "A", torch.float32),
+            _chk(D, "D", torch.float32), _chk(state, "state", torch.float32), state.stride(0), int(state_off),
+            _chk(batch.seq_slot, "seq_slot", torch.int32), _chk(batch.seq_row0, "seq_row0", torch.int32), S, R, most,
+            out.data_ptr(), scratch.data_ptr(), heads, vdim, states, groups, _stream())
+        if st != native.ERR_UNSUPPORTED:  # rows or state that are not on 16 bytes
+            native.check(st, f"ssd_chunk (heads={heads}, vdim={vdim}, states={states})")
+            return out
     st = native.lib().rfx_ssd_scan(
         _chk(xbc, "xbc", torch.float32), xbc.shape[1], _chk(proj, "proj", torch.float32), proj.shape[1], int(z_off),
         int(dt_off), _chk(dt_bias, "dt_bias", torch.float32), _chk(A, "A", torch.float32), _chk(D, "D", torch.float32),

@@ -101,6 +101,9 @@ _SIGNATURES = {
     "rfx_mlstm_chunk": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                         c_float, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                         c_void_p],
+    "rfx_mlstm_chunks": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
+                         c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                         c_int, c_void_p],
     "rfx_mlstm_out": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int,
                       c_int, c_int, c_void_p],
     "rfx_moe_route": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -165,6 +168,9 @@ _SIGNATURES = {
     "rfx_ssd_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                      c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
                      c_void_p],
+    "rfx_ssd_chunk": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                      c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+                      c_int, c_int, c_void_p],
     "rfx_delta_rule": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float,
                        c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                        c_void_p],
@@ -221,6 +227,10 @@ def lib() -> ctypes.CDLL:
         handle.rfx_mamba_scan_scratch.restype = c_longlong
         handle.rfx_gated_delta_chunk_floats.argtypes = [c_int, c_int, c_int]
         handle.rfx_gated_delta_chunk_floats.restype = c_longlong
+        handle.rfx_ssd_chunk_floats.argtypes = [c_int] * 6
+        handle.rfx_ssd_chunk_floats.restype = c_longlong
+        handle.rfx_mlstm_chunks_floats.argtypes = [c_int] * 6
+        handle.rfx_mlstm_chunks_floats.restype = c_longlong
         handle.rfx_sm_count.argtypes = []
         handle.rfx_sm_count.restype = c_int
         handle.rfx_sample_work_bytes.argtypes = [c_int, c_int]

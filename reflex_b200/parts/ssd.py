@@ -107,7 +107,8 @@ class StateSpaceDuality:
             ops.conv_state_update(proj, col0 + self.inner, cc, None, self.taps, state, batch)
         ops.prof_mark("conv_post")
         y = ops.ssd_scan(xbc, proj, col0, col0 + self.inner + cc, self.dt_bias, self.A, self.D, state,
-                         (self.taps - 1) * cc, batch, self.heads, self.vdim, self.states, self.groups)
+                         (self.taps - 1) * cc, batch, self.heads, self.vdim, self.states, self.groups,
+                         exact=self.dtype == torch.float32)
         ops.prof_mark("scan")
         y = ops.group_norm_gate(y, self.norm, self.eps, self.norm_groups, self.dtype)
         ops.prof_mark("scan_norm")

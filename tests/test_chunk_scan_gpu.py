@@ -1,0 +1,163 @@
+"""The recurrences that take a prompt's rows 64 at a time on the tensor cores (csrc/chunk_scan.cuh)
+against their row-by-row rules in 64 bits, at the edges of chunks and tiles.
+
+Tolerance, of the largest result: products of numbers split in two are exact to 2^-21 each; sums of
+up to N + 64 <= 192 terms in 32 bits add at most 192 * 2^-24 = 1.2e-5."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TOL = 2e-5
+
+
+def ops():
+    from reflex_b200 import ops as o
+
+    return o
+
+
+def i32(v):
+    return torch.tensor(list(v), dtype=torch.int32, device=DEV)
+
+
+class Batch:
+    def __init__(self, counts, slots):
+        self.row0 = [0]
+        for c in counts:
+            self.row0.append(self.row0[-1] + c)
+        self.seq_slot, self.seq_new, self.seq_row0 = i32(slots), i32(counts), i32(self.row0)
+        self.max_new = max(counts)
+
+
+def off(got, ref):
+    got = got.double().cpu().numpy()
+    return np.abs(got - ref).max() / np.abs(ref).max()
+
+
+def ssd_rule(x, B, C, dt, A, D, S):
+    """x [T, H, P], B, C [T, H, N], dt [T, H], S [H, P, N]."""
+    ys = []
+    for t in range(x.shape[0]):
+        S = np.exp(A * dt[t])[:, None, None] * S + (dt[t][:, None] * x[t])[:, :, None] * B[t][:, None, :]
+        ys.append((S * C[t][:, None, :]).sum(-1) + D[:, None] * x[t])
+    return np.stack(ys), S
+
+
+@pytest.mark.parametrize("heads,groups,P,N", [(4, 2, 64, 128), (2, 1, 12, 20), (3, 3, 68, 8), (2, 2, 132, 100)])
+@pytest.mark.parametrize("counts", [(64,), (65, 1, 63), (128, 0, 129), (200,)])
+def test_ssd_in_chunks(heads, groups, P, N, counts, monkeypatch):
+    monkeypatch.setattr(ops(), "SSD_CHUNK_MIN_ROWS", 1)
+    rng = np.random.default_rng(heads * 100 + N + sum(counts))
+    inner, R = heads * P, sum(counts)
+    xbc = rng.standard_normal((R, inner + 2 * groups * N)).astype(np.float32)
+    proj = rng.standard_normal((R, inner + heads + (-heads) % 4)).astype(np.float32)
+    proj[:, inner:inner + heads] *= 3.0  # steps from near nothing to several
+    A, D = -np.exp(rng.uniform(-2, 1, heads)).astype(np.float32), rng.standard_normal(heads).astype(np.float32)
+    bias = rng.uniform(-0.5, 0.5, heads).astype(np.float32)
+    slots = [3, 0, 5][:len(counts)]
+    state = rng.standard_normal((6, 8 + heads * P * N)).astype(np.float32)
+    dev = torch.from_numpy(state).to(DEV)
+    to = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
+    b = Batch(counts, slots)
+    out = ops().ssd_scan(to(xbc), to(proj), 0, inner, to(bias), to(A), to(D), dev, 8, b, heads, P, N, groups, exact=False)
+    for i, (n, slot) in enumerate(zip(counts, slots)):
+        rows = slice(b.row0[i], b.row0[i + 1])
+        if not n:
+            assert torch.equal(dev[slot].cpu(), torch.from_numpy(state[slot]))
+            continue
+        xd, pd = xbc[rows].astype(np.float64), proj[rows].astype(np.float64)
+        x = xd[:, :inner].reshape(n, heads, P)
+        rep = heads // groups
+        Bm, Cm = (xd[:, inner + k * groups * N:inner + (k + 1) * groups * N].reshape(n, groups, N).repeat(rep, 1)
+                  for k in (0, 1))
+        dt = np.logaddexp(0.0, pd[:, inner:inner + heads] + bias)
+        y, S = ssd_rule(x, Bm, Cm, dt, A.astype(np.float64), D.astype(np.float64),
+                        state[slot, 8:].astype(np.float64).reshape(heads, P, N))
+        z = pd[:, :inner]
+        assert off(out[rows], y.reshape(n, inner) * z / (1 + np.exp(-z))) < TOL
+        assert off(dev[slot, 8:], S.ravel()) < TOL
+        assert torch.equal(dev[slot, :8].cpu(), torch.from_numpy(state[slot, :8]))
+    untouched = [s for s in range(6) if s not in slots]
+    assert torch.equal(dev[untouched].cpu(), torch.from_numpy(state[untouched]))
+
+
+def mlstm_rule(q, k, v, i, f, S, n, m):
+    num, den = [], []
+    for t in range(q.shape[0]):
+        m2 = np.maximum(f[t] + m, i[t])
+        a, b = np.exp(f[t] + m - m2), np.exp(i[t] - m2)
+        S = a[:, None, None] * S + (b[:, None] * k[t])[:, :, None] * v[t][:, None, :]
+        n = a[:, None] * n + b[:, None] * k[t]
+        m = m2
+        num.append((S * q[t][:, :, None]).sum(1))
+        den.append(np.maximum(np.abs((n * q[t]).sum(-1)), np.exp(-m)) + 1e-6)
+    return np.stack(num), np.stack(den), S, n, m
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 256), (3, 20, 12), (2, 64, 68), (4, 100, 130 - 2)])
+@pytest.mark.parametrize("counts", [(64,), (65, 1, 127), (193,)])
+def test_mlstm_in_chunks(heads, dim, vdim, counts):
+    rng = np.random.default_rng(heads + dim + sum(counts))
+    R, cap = sum(counts), 12.0
+    q_off, k_off, v_off = 0, heads * dim, 2 * heads * dim
+    i_off = v_off + heads * vdim
+    f_off = i_off + heads
+    ld = f_off + heads + (-(f_off + heads)) % 4
+    proj = rng.standard_normal((R, ld)).astype(np.float32)
+    proj[:, i_off:f_off + heads] *= 4.0  # gates that swing
+    bi, bf = rng.standard_normal(heads).astype(np.float32), (rng.standard_normal(heads) + 2).astype(np.float32)
+    floats = ops().mlstm_state_floats(dim, vdim)
+    state = np.zeros((6, heads, floats), dtype=np.float32)
+    state[3, :, :dim * vdim + dim] = rng.standard_normal((heads, dim * vdim + dim))
+    state[3, :, dim * vdim + dim:] = rng.standard_normal(heads)[:, None]  # a sequence that goes on
+    slots = [3, 0, 5][:len(counts)]
+    dev = torch.from_numpy(state.copy()).to(DEV)
+    to = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
+    b = Batch(counts, slots)
+    num, den = ops().mlstm_scan(to(proj), (q_off, k_off, v_off, i_off, f_off), to(bi), to(bf), cap, 0.25, b, dev, heads,
+                                dim, vdim, max_rows=b.max_new, exact=False)
+    for j, (n, slot) in enumerate(zip(counts, slots)):
+        rows = slice(b.row0[j], b.row0[j + 1])
+        p = proj[rows].astype(np.float64)
+        cut = lambda o, w: p[:, o:o + heads * w].reshape(n, heads, w)  # noqa: E731
+        i = cap * np.tanh((p[:, i_off:i_off + heads] + bi) / cap)
+        f = -np.logaddexp(0.0, -cap * np.tanh((p[:, f_off:f_off + heads] + bf) / cap))
+        old = state[slot].astype(np.float64)
+        rn, rd, S, nn, m = mlstm_rule(cut(q_off, dim) * 0.25, cut(k_off, dim), cut(v_off, vdim), i, f,
+                                      old[:, :dim * vdim].reshape(heads, dim, vdim),
+                                      old[:, dim * vdim:dim * vdim + dim], old[:, -1])
+        assert off(num[rows], rn.reshape(n, -1)) < TOL
+        assert off(den[rows], rd) < TOL
+        new = dev[slot].double().cpu().numpy()
+        scale = np.exp(new[:, -1] - m)  # the memory is relative to the number beside it
+        assert np.abs(new[:, -1] - m).max() < 1e-5 * (1 + np.abs(m).max())
+        assert off(torch.from_numpy(new[:, :dim * vdim] * scale[:, None]), S.reshape(heads, -1)) < TOL
+        assert off(torch.from_numpy(new[:, dim * vdim:dim * vdim + dim] * scale[:, None]), nn) < TOL
+
+
+def test_a_long_step_goes_through_a_bounded_scratch():
+    """Memories of 64 heads of 256 x 128 for 37 chunks (310 MB) do not fit the scratch: two rounds,
+    the second going on from the state that the first one left; beside it a short sequence.  With
+    decays near one a result is a sum over all rows; the walk it is compared with rounds 2,300 times,
+    2300 * 2^-24 = 1.4e-4."""
+    heads, groups, P, N, counts = 64, 2, 256, 128, (2300, 70)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    R, inner = sum(counts), heads * P
+    xbc = torch.randn((R, inner + 2 * groups * N), generator=g, device=DEV)
+    proj = torch.randn((R, inner + heads), generator=g, device=DEV)
+    A = -torch.rand(heads, generator=g, device=DEV) * 0.05  # slow decays: the first round's rows count in the second
+    D, bias = torch.randn(heads, generator=g, device=DEV), torch.zeros(heads, device=DEV)
+    assert ops().native.lib().rfx_ssd_chunk_floats(R, 2, 2300, heads, P, N) < 100 << 20
+    got = []
+    for exact in (True, False):
+        state = torch.zeros((2, heads * P * N), device=DEV)
+        y = ops().ssd_scan(xbc, proj, 0, inner, bias, A, D, state, 0, Batch(counts, [1, 0]), heads, P, N, groups, exact=exact)
+        got.append((y, state))
+    for a, b in zip(*got):
+        assert ((a - b).abs().max() / a.abs().max()).item() < 1.4e-4
+    assert math.isfinite(got[1][0].sum().item())
