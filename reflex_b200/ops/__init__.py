@@ -1732,19 +1732,40 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
     return out
 
 
+# rows of the longest sequence from which the chunked kernels run (one sequence, width 2048, the whole
+# mixer: 47 us walking and 48 in chunks at 48 rows, 57 and 40 at 100)
+DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_DELTA_CHUNK_MIN_ROWS", 64, 1, 1 << 30)
+
+
 def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: int, wpre: torch.Tensor,
                w_bias: torch.Tensor, a_bias: torch.Tensor, rate: float, unit_eps: float, state: torch.Tensor,
-               state_off: int, batch, heads: int, dim: int) -> torch.Tensor:
+               state_off: int, batch, heads: int, dim: int, exact: bool = True) -> torch.Tensor:
     """The generalized delta rule (csrc/delta_rule.cu): `proj` float32 rows with r, k,
     v and the removal rate's pre-activation at their column offsets (heads * dim
     each), `wpre` float32 [R, heads * dim] the decay's; the running state is
     `state[slot, state_off : state_off + heads * dim * dim]`.  Returns S^T r,
-    float32 [R, heads * dim]."""
+    float32 [R, heads * dim].  Without `exact`, from `DELTA_CHUNK_MIN_ROWS` rows of a
+    sequence on and for heads of 64, the kernels that take 32 rows at a time run
+    (csrc/delta_rule_chunk.cu: the same function, products of 32-bit numbers split for
+    the tensor cores)."""
     R = proj.shape[0]
     hd = heads * dim
     if max(r_off, k_off, v_off, a_off) + hd > proj.shape[1] or tuple(wpre.shape) != (R, hd):
         raise InvalidInput("delta_rule: the columns do not fit into the rows")
     out = _new((R, hd), torch.float32, proj.device)
+    if not exact and dim == 64 and batch.max_new >= DELTA_CHUNK_MIN_ROWS:
+        S, most = batch.seq_slot.numel(), int(batch.max_new)
+        scratch = _new((int(native.lib().rfx_delta_rule_chunk_floats(R, S, most, heads)),), torch.float32, proj.device)
+        st = native.lib().rfx_delta_rule_chunk(
+            _chk(proj, "proj", torch.float32), proj.shape[1], int(r_off), int(k_off), int(v_off), int(a_off),
+            _chk(wpre, "wpre", torch.float32), _chk(w_bias, "w_bias", torch.float32),
+            _chk(a_bias, "a_bias", torch.float32), float(rate), float(unit_eps), _chk(state, "state", torch.float32),
+            state.stride(0), int(state_off), _chk(batch.seq_slot, "seq_slot", torch.int32),
+            _chk(batch.seq_row0, "seq_row0", torch.int32), S, R, most, out.data_ptr(), scratch.data_ptr(), heads, dim,
+            _stream())
+        if st != native.ERR_UNSUPPORTED:  # rows that are not on 16 bytes, a rate beyond 2
+            native.check(st, f"delta_rule_chunk (heads={heads}, dim={dim})")
+            return out
     st = native.lib().rfx_delta_rule(
         _chk(proj, "proj", torch.float32), proj.shape[1], int(r_off), int(k_off), int(v_off), int(a_off),
         _chk(wpre, "wpre", torch.float32), _chk(w_bias, "w_bias", torch.float32), _chk(a_bias, "a_bias", torch.float32),
@@ -1784,7 +1805,9 @@ def gated_delta_prep(proj: torch.Tensor, b_off: int, a_off: int, filters_t: torc
 
 
 # from so many rows of a sequence on, the recurrence takes them sixteen at a time as products
-GATED_DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_GATED_DELTA_CHUNK_MIN_ROWS", 8, 1, 1 << 30)
+GATED_# rows of the longest sequence from which the chunked kernels run (one sequence, width 2048, the whole
+# mixer: 47 us walking and 48 in chunks at 48 rows, 57 and 40 at 100)
+DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_GATED_DELTA_CHUNK_MIN_ROWS", 8, 1, 1 << 30)
 
 
 def gated_delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor, state_off: int, batch, heads: int,

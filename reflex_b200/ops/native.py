@@ -174,6 +174,9 @@ _SIGNATURES = {
     "rfx_delta_rule": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float,
                        c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                        c_void_p],
+    "rfx_delta_rule_chunk": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float,
+                             c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
+                             c_void_p, c_int, c_int, c_void_p],
     "rfx_short_conv": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong,
                        c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "rfx_conv_qkv_post": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_void_p,
@@ -231,6 +234,8 @@ def lib() -> ctypes.CDLL:
         handle.rfx_ssd_chunk_floats.restype = c_longlong
         handle.rfx_mlstm_chunks_floats.argtypes = [c_int] * 6
         handle.rfx_mlstm_chunks_floats.restype = c_longlong
+        handle.rfx_delta_rule_chunk_floats.argtypes = [c_int] * 4
+        handle.rfx_delta_rule_chunk_floats.restype = c_longlong
         handle.rfx_sm_count.argtypes = []
         handle.rfx_sm_count.restype = c_int
         handle.rfx_sample_work_bytes.argtypes = [c_int, c_int]

@@ -93,7 +93,7 @@ class DeltaRule:
         wpre = ops.linear(low, self.w2, out_dtype=torch.float32)
         ops.prof_mark("scan_proj")
         o = ops.delta_rule(proj, 0, hd, 2 * hd, 4 * hd, wpre, self.w0, self.a_bias, self.rate, self.unit_eps,
-                           ctx.state, 0, batch, self.heads, self.dim)
+                           ctx.state, 0, batch, self.heads, self.dim, exact=self.dtype == torch.float32)
         ops.prof_mark("scan")
         o = ops.group_norm_gate(o, self.norm, self.eps, self.heads, self.dtype, gate=proj, gate_col=3 * hd)
         ops.prof_mark("scan_norm")

@@ -161,3 +161,66 @@ def test_a_long_step_goes_through_a_bounded_scratch():
     for a, b in zip(*got):
         assert ((a - b).abs().max() / a.abs().max()).item() < 1.4e-4
     assert math.isfinite(got[1][0].sum().item())
+
+
+def delta_rule_rows(r, k, v, w, a, S, eps):
+    """All [T, H, d]; S [H, value, key].  Both terms read the old S."""
+    out = []
+    for t in range(r.shape[0]):
+        u = k[t] / np.sqrt((k[t] ** 2).sum(-1, keepdims=True) + eps)
+        seen = (S * u[:, None, :]).sum(-1)
+        S = S * w[t][:, None, :] - seen[:, :, None] * (a[t] * u)[:, None, :] + v[t][:, :, None] * k[t][:, None, :]
+        out.append((S * r[t][:, None, :]).sum(-1))
+    return np.stack(out), S
+
+
+@pytest.mark.parametrize("rate", [math.exp(-0.5), 2.0, 0.0, 2.5])  # 2.5: beyond the chunks' range, the walk
+@pytest.mark.parametrize("counts", [(32,), (33, 1, 31), (64, 0, 97), (160,)])
+def test_delta_rule_in_chunks(counts, rate, monkeypatch):
+    monkeypatch.setattr(ops(), "DELTA_CHUNK_MIN_ROWS", 1)
+    heads, d = 3, 64
+    hd, R = heads * d, sum(counts)
+    rng = np.random.default_rng(sum(counts))
+    proj = rng.standard_normal((R, 4 * hd)).astype(np.float32)
+    wpre = (3 * rng.standard_normal((R, hd))).astype(np.float32)
+    wb, ab = rng.standard_normal(hd).astype(np.float32), rng.standard_normal(hd).astype(np.float32)
+    slots = [3, 0, 5][:len(counts)]
+    state = rng.standard_normal((6, 4 + hd * d)).astype(np.float32)
+    dev = torch.from_numpy(state.copy()).to(DEV)
+    to = lambda x: torch.from_numpy(x).to(DEV)  # noqa: E731
+    b = Batch(counts, slots)
+    out = ops().delta_rule(to(proj), 0, hd, 2 * hd, 3 * hd, to(wpre), to(wb), to(ab), rate, 1e-6, dev, 4, b, heads, d,
+                           exact=False)
+    for i, (n, slot) in enumerate(zip(counts, slots)):
+        if not n:
+            assert torch.equal(dev[slot].cpu(), torch.from_numpy(state[slot]))
+            continue
+        rows = slice(b.row0[i], b.row0[i + 1])
+        r, k, v, a = (proj[rows, o * hd:(o + 1) * hd].astype(np.float64).reshape(n, heads, d) for o in range(4))
+        sig = lambda x: 1 / (1 + np.exp(-x))  # noqa: E731
+        w = np.exp(-rate * sig((wpre[rows].astype(np.float64) + wb).reshape(n, heads, d)))
+        ref, S = delta_rule_rows(r, k, v, w, sig(a + ab.astype(np.float64).reshape(heads, d)),
+                                 state[slot, 4:].astype(np.float64).reshape(heads, d, d), 1e-6)
+        assert off(out[rows], ref.reshape(n, hd)) < TOL
+        assert off(dev[slot, 4:], S.ravel()) < TOL
+        assert torch.equal(dev[slot, :4].cpu(), torch.from_numpy(state[slot, :4]))
+    untouched = [s for s in range(6) if s not in slots]
+    assert torch.equal(dev[untouched].cpu(), torch.from_numpy(state[untouched]))
+
+
+def test_a_long_delta_step_goes_through_a_bounded_scratch():
+    heads, d, counts = 64, 64, (5000, 70)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    R, hd = sum(counts), heads * d
+    proj = torch.randn((R, 4 * hd), generator=g, device=DEV)
+    wpre = torch.randn((R, hd), generator=g, device=DEV) - 6.0  # slow decays
+    zero = torch.zeros(hd, device=DEV)
+    assert ops().native.lib().rfx_delta_rule_chunk_floats(R, 2, 5000, heads) < 80 << 20
+    got = []
+    for exact in (True, False):
+        state = torch.zeros((2, hd * d), device=DEV)
+        y = ops().delta_rule(proj, 0, hd, 2 * hd, 3 * hd, wpre, zero, zero, math.exp(-0.5), 1e-6, state, 0,
+                             Batch(counts, [1, 0]), heads, d, exact=exact)
+        got.append((y, state))
+    for a, b in zip(*got):  # the removal forgets what 32 rows back added: no sum over all rows here
+        assert ((a - b).abs().max() / a.abs().max()).item() < TOL
