@@ -1805,9 +1805,7 @@ def gated_delta_prep(proj: torch.Tensor, b_off: int, a_off: int, filters_t: torc
 
 
 # from so many rows of a sequence on, the recurrence takes them sixteen at a time as products
-GATED_# rows of the longest sequence from which the chunked kernels run (one sequence, width 2048, the whole
-# mixer: 47 us walking and 48 in chunks at 48 rows, 57 and 40 at 100)
-DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_GATED_DELTA_CHUNK_MIN_ROWS", 8, 1, 1 << 30)
+GATED_DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_GATED_DELTA_CHUNK_MIN_ROWS", 8, 1, 1 << 30)
 
 
 def gated_delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor, state_off: int, batch, heads: int,
