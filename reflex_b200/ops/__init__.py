@@ -1682,6 +1682,11 @@ def attention_sigmoid(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv
 
 
 # ------------------------------------------- recurrences with a matrix state a head
+def _most_rows(batch) -> int:
+    """The most rows a sequence of the step brings; 0 where the caller's batch does not say."""
+    return int(getattr(batch, "max_new", 0))
+
+
 # Rows of the longest sequence from which the chunked kernels run: their three launches and the
 # memory's way out and back cost about 30 us, the walk 0.5 us a row (one sequence, width 2048, the
 # whole mixer: 71 us walking and 79 in chunks at 48 rows, 106 and 84 at 100; eight sequences of 37
@@ -1707,10 +1712,11 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
     if z_off + inner > proj.shape[1] or dt_off + heads > proj.shape[1]:
         raise InvalidInput("ssd_scan: z or dt do not fit into the rows of proj")
     out = _new((R, inner), out_dtype, xbc.device)
-    chunked = batch.max_new >= SSD_CHUNK_MIN_ROWS or (batch.max_new >= 32 and R >= 256 and SSD_CHUNK_MIN_ROWS <= 256)
+    most = _most_rows(batch)
+    chunked = most >= SSD_CHUNK_MIN_ROWS or (most >= 32 and R >= 256 and SSD_CHUNK_MIN_ROWS <= 256)
     if (not exact and chunked and out_dtype == torch.float32 and vdim % 4 == 0
             and states % 4 == 0 and states <= 128):
-        S, most = batch.seq_slot.numel(), int(batch.max_new)
+        S = batch.seq_slot.numel()
         scratch = _new((int(native.lib().rfx_ssd_chunk_floats(R, S, most, heads, vdim, states)),), torch.float32,
                        xbc.device)
         st = native.lib().rfx_ssd_chunk(
@@ -1753,8 +1759,9 @@ def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: in
     if max(r_off, k_off, v_off, a_off) + hd > proj.shape[1] or tuple(wpre.shape) != (R, hd):
         raise InvalidInput("delta_rule: the columns do not fit into the rows")
     out = _new((R, hd), torch.float32, proj.device)
-    if not exact and dim == 64 and batch.max_new >= DELTA_CHUNK_MIN_ROWS:
-        S, most = batch.seq_slot.numel(), int(batch.max_new)
+    most = _most_rows(batch)
+    if not exact and dim == 64 and most >= DELTA_CHUNK_MIN_ROWS:
+        S = batch.seq_slot.numel()
         scratch = _new((int(native.lib().rfx_delta_rule_chunk_floats(R, S, most, heads)),), torch.float32, proj.device)
         st = native.lib().rfx_delta_rule_chunk(
             _chk(proj, "proj", torch.float32), proj.shape[1], int(r_off), int(k_off), int(v_off), int(a_off),
