@@ -4,7 +4,7 @@
 //  * rfx_gemm_f32: the true 32-bit product.  CUDA-core fused multiply-adds
 //    only; each output element is reduced over k = 0..K-1 in index order by one
 //    thread, so its value does not depend on how many rows the call has or on
-//    where the row sits in the batch.
+//    where the row sits in the batch, nor on which of the three forms runs.
 //  * rfx_gemv_bf16: bfloat16 weights and activations for a few rows (decode),
 //    32-bit accumulation; a pure weight-streaming kernel with 16-byte loads.
 #include "common.cuh"
@@ -64,6 +64,183 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ W, float*
             if (n < N) y[(size_t)r * N + n] = acc[i][j];
         }
     }
+}
+
+// The forms below read both operands 16 bytes an access through rings of asynchronous copies (K a
+// multiple of four, both matrices on 16 bytes; other products take the form above).
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(valid ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void wait_copies() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Up to 64 rows: the weights are streamed once.  A block owns 32 columns, a lane a column, a warp RPW
+// rows; what bounds it is one element's chain of K dependent multiply-adds (four cycles each), beside
+// which the weights of a square matrix arrive at about the memory's rate, so the chains of different
+// rows run in different warps, few to a warp.
+constexpr int KT = 64, WLD = KT + 4;  // columns of a stage; row stride: eight lanes' 16-byte reads meet all banks
+
+template <int RPW>
+__global__ void __launch_bounds__(512)
+gemm_f32_rows_kernel(const float* __restrict__ x, const float* __restrict__ W, float* __restrict__ y, int R, int N,
+                     int K, int stages) {
+    extern __shared__ __align__(16) float sm[];
+    pdl_prologue();
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rows = warps * RPW, r0 = blockIdx.y * rows, n0 = blockIdx.x * 32;
+    const int stage = 32 * WLD + rows * KT;  // [32][WLD] of W, [rows][KT] of x
+    const int tiles = (K + KT - 1) / KT;
+    auto fetch = [&](int t) {
+        if (t < tiles) {
+            float* to = sm + (t % stages) * stage;
+            for (int e = threadIdx.x; e < (32 + rows) * (KT / 4); e += blockDim.x) {
+                const int i = e / (KT / 4), c = 4 * (e % (KT / 4)), k = t * KT + c;
+                if (i < 32) copy16(to + i * WLD + c, W + (size_t)(n0 + i < N ? n0 + i : 0) * K + (k < K ? k : 0), n0 + i < N && k < K);
+                else {
+                    const int r = r0 + i - 32;
+                    copy16(to + 32 * WLD + (i - 32) * KT + c, x + (size_t)(r < R ? r : 0) * K + (k < K ? k : 0), r < R && k < K);
+                }
+            }
+        }
+        copies_done();
+    };
+    for (int t = 0; t < stages - 1; ++t) fetch(t);
+    float acc[RPW];
+#pragma unroll
+    for (int i = 0; i < RPW; ++i) acc[i] = 0.0f;
+    for (int t = 0; t < tiles; ++t) {
+        switch (stages) {  // the group of tile t is the oldest of stages - 1 in flight
+            case 8: wait_copies<6>(); break;
+            case 6: wait_copies<4>(); break;
+            default: wait_copies<2>(); break;
+        }
+        __syncthreads();  // tile t has landed, and every warp is done with the tile before
+        fetch(t + stages - 1);
+        const float* w = sm + (t % stages) * stage + lane * WLD;
+        const float* xs = sm + (t % stages) * stage + 32 * WLD + warp * RPW * KT;
+#pragma unroll
+        for (int k = 0; k < KT; k += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(w + k);
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(xs + i * KT + k);
+                acc[i] = fmaf(a.x, b.x, acc[i]);
+                acc[i] = fmaf(a.y, b.y, acc[i]);
+                acc[i] = fmaf(a.z, b.z, acc[i]);
+                acc[i] = fmaf(a.w, b.w, acc[i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RPW; ++i) {
+        const int r = r0 + warp * RPW + i;
+        if (r < R && n0 + lane < N) y[(size_t)r * N + n0 + lane] = acc[i];
+    }
+}
+
+// More rows: BM x BN tiles, a thread 8 rows by TN columns (rows ty + BM / 8 i, columns tx + 16 j: the
+// reads of a quarter warp then meet all banks), both operands as they lie, sixteen k a stage.
+constexpr int BK = 16, BLD = BK + 4, BSTAGES = 4;
+
+template <int BM, int BN>
+__global__ void __launch_bounds__(BM * 2)
+gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ W, float* __restrict__ y, int R, int N,
+                     int K) {
+    constexpr int THREADS = BM * 2, TN = BN / 16, STAGE = (BM + BN) * BLD;
+    extern __shared__ __align__(16) float sm[];
+    pdl_prologue();
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int r0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int tiles = (K + BK - 1) / BK;
+    auto fetch = [&](int t) {
+        if (t < tiles) {
+            float* to = sm + (t % BSTAGES) * STAGE;
+#pragma unroll
+            for (int e = threadIdx.x; e < (BM + BN) * (BK / 4); e += THREADS) {
+                const int i = e / (BK / 4), c = 4 * (e % (BK / 4)), k = t * BK + c;
+                const int row = i < BM ? r0 + i : n0 + i - BM;
+                const bool ok = row < (i < BM ? R : N) && k < K;
+                const float* src = i < BM ? x : W;
+                copy16(to + i * BLD + c, ok ? src + (size_t)row * K + k : src, ok);
+            }
+        }
+        copies_done();
+    };
+#pragma unroll
+    for (int t = 0; t < BSTAGES - 1; ++t) fetch(t);
+    float acc[8][TN];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+    for (int t = 0; t < tiles; ++t) {
+        wait_copies<BSTAGES - 2>();
+        __syncthreads();
+        fetch(t + BSTAGES - 1);
+        const float* a = sm + (t % BSTAGES) * STAGE + ty * BLD;
+        const float* b = sm + (t % BSTAGES) * STAGE + (BM + tx) * BLD;
+#pragma unroll
+        for (int k = 0; k < BK; k += 4) {
+            float4 av[8], bv[TN];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const float4*>(a + i * (BM / 8) * BLD + k);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) bv[j] = *reinterpret_cast<const float4*>(b + j * 16 * BLD + k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].x, bv[j].x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].y, bv[j].y, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].z, bv[j].z, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].w, bv[j].w, acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = r0 + ty + (BM / 8) * i;
+        if (r >= R) continue;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx + 16 * j;
+            if (n < N) y[(size_t)r * N + n] = acc[i][j];
+        }
+    }
+}
+
+template <int RPW>
+int launch_rows(const float* x, const float* W, float* y, int R, int N, int K, cudaStream_t s) {
+    int warps = (R + RPW - 1) / RPW;
+    if (warps < 4) warps = 4;  // enough threads to issue the copies
+    const size_t stage = (size_t)(32 * WLD + warps * RPW * KT) * sizeof(float);
+    const int stages = stage * 8 <= 100 * 1024 ? 8 : stage * 6 <= 110 * 1024 ? 6 : 4;
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(stage * stages));
+    if (e != cudaSuccess) return (int)e;
+    RFX_LAUNCH(gemm_f32_rows_kernel<RPW>, dim3((N + 31) / 32, 1), warps * 32, stage * stages, s, x, W, y, R, N, K, stages);
+    return 0;
+}
+
+template <int BM, int BN>
+int launch_tiles(const float* x, const float* W, float* y, int R, int N, int K, cudaStream_t s) {
+    constexpr size_t smem = (size_t)BSTAGES * (BM + BN) * BLD * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    RFX_LAUNCH((gemm_f32_tile_kernel<BM, BN>), dim3((N + BN - 1) / BN, (R + BM - 1) / BM), BM * 2, smem, s, x, W, y, R, N, K);
+    return 0;
 }
 
 // One warp per output column n; RT rows of x per pass.  K must be a multiple
@@ -226,6 +403,16 @@ extern "C" int rfx_gemm_f32(const float* x, const float* W, float* y, int R, int
     if (K <= 0) return RFX_ERR_BAD_ARG;
     dim3 grid((N + TN - 1) / TN, (R + TM - 1) / TM);
     if (grid.y > 65535) return RFX_ERR_UNSUPPORTED;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (K % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) == 0) {
+        if (R <= 8) return launch_rows<1>(x, W, y, R, N, K, st);
+        if (R <= 32) return launch_rows<2>(x, W, y, R, N, K, st);
+        if (R <= 64) return launch_rows<4>(x, W, y, R, N, K, st);
+        // the larger tile reads shared memory half as often a multiply-add; it needs two tiles an SM
+        if ((long long)((R + 127) / 128) * ((N + 127) / 128) >= 2LL * sm_count())
+            return launch_tiles<128, 128>(x, W, y, R, N, K, st);
+        return launch_tiles<64, 64>(x, W, y, R, N, K, st);
+    }
     RFX_LAUNCH(gemm_f32_kernel, grid, 256, 0, (cudaStream_t)stream, x, W, y, R, N, K);
     return 0;
 }

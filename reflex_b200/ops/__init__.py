@@ -524,6 +524,29 @@ def attention_plain(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     return out
 
 
+def attention_f32(q, k_pages, v_pages, page_table, page_size, batch, nq: int, nkv: int, head_dim: int, window, scale,
+                  sink=None, slopes=None, keep_first: int = 0, softcap: float = 0.0) -> Optional[torch.Tensor]:
+    """`attention_plain`'s 32-bit results, bit for bit, from a kernel that takes 32 keys and
+    several queries at a time (csrc/attention_f32.cu); None for head sizes other than 32,
+    64, 128 and 256 or pages that are not on 16 bytes."""
+    most = int(getattr(batch, "max_new", 0))
+    if head_dim not in (32, 64, 128, 256) or not most:
+        return None
+    out = _new(q.shape, q.dtype, q.device)
+    st = native.lib().rfx_attention_f32(
+        _chk(q, "q", torch.float32), _chk(k_pages, "k_pages", torch.float32), _chk(v_pages, "v_pages", torch.float32),
+        _chk(page_table, "page_table", torch.int32), page_table.shape[1], page_size,
+        _chk(batch.seq_slot, "seq_slot", torch.int32), _chk(batch.seq_start, "seq_start", torch.int32),
+        _chk(batch.seq_new, "seq_new", torch.int32), _chk(batch.seq_row0, "seq_row0", torch.int32), out.data_ptr(),
+        batch.seq_slot.numel(), most, nq, nkv, head_dim, int(window or 0),
+        int(keep_first if window else 0), float(scale), _chk(sink, "sink", torch.float32),
+        _chk(slopes, "slopes", torch.float32), float(softcap), _stream())
+    if st == native.ERR_UNSUPPORTED:
+        return None
+    native.check(st, f"attention_f32 (head_dim={head_dim})")
+    return out
+
+
 def gemv_simple(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """The plain CUDA-core bfloat16 product (one warp per output column); kept
     as the readable counterpart of `gemm_tc` for tests."""
@@ -722,8 +745,11 @@ def attention(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv, head_d
                                  batch.seq_start, batch.seq_new, batch.seq_row0, batch.max_new, nq,
                                  nkv, head_dim, window, scale, sink, slopes, keep_first, softcap)
     else:
-        out = attention_plain(q, k_pages, v_pages, page_table, page_size, batch.row_pos,
-                              batch.row_slot, nq, nkv, head_dim, window, scale, sink, slopes, keep_first, softcap)
+        out = attention_f32(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv, head_dim, window, scale, sink,
+                            slopes, keep_first, softcap) if q.dtype == torch.float32 else None
+        if out is None:
+            out = attention_plain(q, k_pages, v_pages, page_table, page_size, batch.row_pos,
+                                  batch.row_slot, nq, nkv, head_dim, window, scale, sink, slopes, keep_first, softcap)
     return out if gate is None else sigmoid_gate_mul_(out, gate[0], gate[1], heads=nq)
 
 
