@@ -73,6 +73,11 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
           "r"(x), "r"(y), "r"(z)
         : "memory");
 }
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 // 2^x, hardware approximation (about 2 ulp; the result is rounded to bfloat16)
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -155,6 +160,10 @@ __device__ __forceinline__ void load_logits16(const rfx::RowGate& gate, size_t a
 // takes the raw score's place and `scale_log2` is cap * log2(e), so the rest of the page's code
 // is the same.  MODE 2 takes any argument; MODE 3 the polynomial for |s in_scale| <= 1/2, which
 // leaves the special-function unit to the softmax's exponentials.
+// MODE 4: no softmax, every visible key's weight is sigmoid(score + bias of the head), `slopes`
+// holding the biases: no maximum, no denominator, O never rescaled.  2,048 rows of 16 heads of 128,
+// window 1,024: 38 us; 137 us on mma.sync (sigmoid_attention_mma.cu, which keeps decode rows and the
+// other head sizes).
 // CONTIG: keys and values are not pages but the rows of one matrix (a latent's keys and
 // values made for this step): position p of sequence i is row seq_base[i] + p, head h's key its
 // columns h DK .., its value its columns v_col + h DV .. (map_k and map_v then are the same
@@ -171,7 +180,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                             float scale_log2, float in_scale, const float* __restrict__ sink,
                             const float* __restrict__ slopes, const int* __restrict__ seq_base, int v_col, int dv,
                             rfx::RowGate gate, int* __restrict__ err) {
-    constexpr bool SLOPES = MODE == 1;
+    constexpr bool SLOPES = MODE == 1, SIGMOID = MODE == 4;
     static_assert(DK % 64 == 0 && DK <= 192 && (DV == 64 || DV == 128), "keys up to 192, values 64 or 128");
     constexpr int KB = DK / 64, VB = DV / 64;  // 64-column blocks of a row
     constexpr int K_BYTES = PAGE * DK * 2, V_BYTES = PAGE * DV * 2;
@@ -379,6 +388,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         // the row's head's slope in units of the raw score (a weight: read before any wait)
         float slope_raw = 0.0f;
         if constexpr (SLOPES) slope_raw = slopes[kvh * g + min(row_h, g - 1)] * 1.4426950408889634f / scale_log2;
+        float bias2 = 0.0f;
+        if constexpr (SIGMOID) bias2 = slopes ? slopes[kvh * g + min(row_h, g - 1)] * 1.4426950408889634f : 0.0f;
         constexpr float RAISE = 8.0f;  // raise the reference maximum only past 2^8
         float m = -INFINITY, l = 0.0f;
         bool ok = true;
@@ -403,81 +414,98 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
             // every key of the page visible to every valid row of the tile: no compares
             const bool all_visible = basej + PAGE - 1 <= pos_first && (basej >= lo_last || basej + PAGE <= keep_first) &&
                                      n_rows == ROWS;
-            // four independent chains each for the maximum and the sum: one warp per
-            // scheduler has nothing else to hide a dependent chain's latency with
-            float s[PAGE];  // raw scores; the scale (positive) goes into the exponent's multiply-add
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            if constexpr (SLOPES) {
-                const float d0 = (float)(row_pos - basej);  // distance of the page's first key
-#pragma unroll
-                for (int c = 0; c < PAGE; ++c)
-                    sr[c] = __float_as_uint(fmaf(-slope_raw, d0 - (float)c, __uint_as_float(sr[c])));
-            }
-            if constexpr (MODE == 2) {
-#pragma unroll
-                for (int c = 0; c < PAGE; ++c)
-                    sr[c] = __float_as_uint(
-                        attn::capped_log2(__uint_as_float(sr[c]), 2.0f * 1.4426950408889634f * in_scale, 1.0f));
-            }
-            if constexpr (MODE == 3) {
-#pragma unroll
-                for (int c = 0; c < PAGE; ++c)
-                    sr[c] = __float_as_uint(attn::tanh_small(__uint_as_float(sr[c]) * in_scale));
-            }
-            if (all_visible) {
-#pragma unroll
-                for (int c = 0; c < PAGE; ++c) s[c] = __uint_as_float(sr[c]);
-#pragma unroll
-                for (int c = 0; c < PAGE; c += 8)  // two new values per maximum: a three-input instruction
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(fmaxf(mx4[k], s[c + 2 * k]), s[c + 2 * k + 1]);
-            } else {
-#pragma unroll
-                for (int c = 0; c < PAGE; ++c) {
-                    const int key = basej + c;
-                    s[c] = (key <= row_pos && (key >= row_lo || key < keep_first)) ? __uint_as_float(sr[c]) : -INFINITY;
-                    mx4[c & 3] = fmaxf(mx4[c & 3], s[c]);
-                }
-            }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
-            // the reference maximum moves only when it must
-            float corr = 1.0f;
-            const bool raise = mx > m + RAISE || (m == -INFINITY && mx != -INFINITY);
-            if (raise) {
-                corr = (m == -INFINITY) ? 0.0f : ex2(m - mx);
-                m = mx;
-                l *= corr;
-            }
-            // rows that have seen no key yet: every s is -inf, shift by 0 gives p = 0
-            const float shift = (m == -INFINITY) ? 0.0f : m;
-            float rs4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             uint32_t packed[PAGE / 2];
+            if constexpr (SIGMOID) {
+                // sigmoid(x) = 1 / (1 + 2^(-x log2 e)); the hardware's exponential and reciprocal are a few
+                // units in the last place of 32 bits off, the weight is rounded to bfloat16
 #pragma unroll
-            for (int c = 0; c < PAGE; c += 2) {
-                const float e0 = ex2(fmaf(s[c], scale_log2, -shift));
-                const float e1 = ex2(fmaf(s[c + 1], scale_log2, -shift));
-                rs4[(c >> 1) & 3] += e0 + e1;
-                __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
-                packed[c / 2] = *reinterpret_cast<uint32_t*>(&h);
-            }
-            l += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
-
-            // rescale this row of O if its reference moved (whole warp together:
-            // the TMEM accesses are warp-wide; lanes that did not move scale by 1)
-            if (j > 0 && __any_sync(0xffffffffu, raise)) {
-                if (!mbar_wait(&o_full, (uint32_t)((j - 1) & 1))) { atomicExch(err, 21); ok = false; break; }
-                tc_fence_after_sync();
+                for (int c = 0; c < PAGE; c += 2) {
+                    float e[2];
 #pragma unroll
-                for (int c = 0; c < DV / 16; ++c) {
-                    uint32_t o[16];
-                    tmem_ld_16_nowait(tmem + lane_addr + O_COL + c * 16, o);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
-                    tmem_st_16(tmem + lane_addr + O_COL + c * 16, o);
+                    for (int k = 0; k < 2; ++k) {
+                        e[k] = rcp(1.0f + ex2(fmaf(__uint_as_float(sr[c + k]), -scale_log2, -bias2)));
+                        const int key = basej + c + k;
+                        if (!all_visible && !(key <= row_pos && key >= row_lo)) e[k] = 0.0f;
+                    }
+                    __nv_bfloat162 h = __floats2bfloat162_rn(e[0], e[1]);
+                    packed[c / 2] = *reinterpret_cast<uint32_t*>(&h);
                 }
-                tmem_st_wait();
-                tc_fence_before_sync();
+            } else {
+                // four independent chains each for the maximum and the sum: one warp per
+                // scheduler has nothing else to hide a dependent chain's latency with
+                float s[PAGE];  // raw scores; the scale (positive) goes into the exponent's multiply-add
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                if constexpr (SLOPES) {
+                    const float d0 = (float)(row_pos - basej);  // distance of the page's first key
+#pragma unroll
+                    for (int c = 0; c < PAGE; ++c)
+                        sr[c] = __float_as_uint(fmaf(-slope_raw, d0 - (float)c, __uint_as_float(sr[c])));
+                }
+                if constexpr (MODE == 2) {
+#pragma unroll
+                    for (int c = 0; c < PAGE; ++c)
+                        sr[c] = __float_as_uint(
+                            attn::capped_log2(__uint_as_float(sr[c]), 2.0f * 1.4426950408889634f * in_scale, 1.0f));
+                }
+                if constexpr (MODE == 3) {
+#pragma unroll
+                    for (int c = 0; c < PAGE; ++c)
+                        sr[c] = __float_as_uint(attn::tanh_small(__uint_as_float(sr[c]) * in_scale));
+                }
+                if (all_visible) {
+#pragma unroll
+                    for (int c = 0; c < PAGE; ++c) s[c] = __uint_as_float(sr[c]);
+#pragma unroll
+                    for (int c = 0; c < PAGE; c += 8)  // two new values per maximum: a three-input instruction
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(fmaxf(mx4[k], s[c + 2 * k]), s[c + 2 * k + 1]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < PAGE; ++c) {
+                        const int key = basej + c;
+                        s[c] = (key <= row_pos && (key >= row_lo || key < keep_first)) ? __uint_as_float(sr[c]) : -INFINITY;
+                        mx4[c & 3] = fmaxf(mx4[c & 3], s[c]);
+                    }
+                }
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+                // the reference maximum moves only when it must
+                float corr = 1.0f;
+                const bool raise = mx > m + RAISE || (m == -INFINITY && mx != -INFINITY);
+                if (raise) {
+                    corr = (m == -INFINITY) ? 0.0f : ex2(m - mx);
+                    m = mx;
+                    l *= corr;
+                }
+                // rows that have seen no key yet: every s is -inf, shift by 0 gives p = 0
+                const float shift = (m == -INFINITY) ? 0.0f : m;
+                float rs4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int c = 0; c < PAGE; c += 2) {
+                    const float e0 = ex2(fmaf(s[c], scale_log2, -shift));
+                    const float e1 = ex2(fmaf(s[c + 1], scale_log2, -shift));
+                    rs4[(c >> 1) & 3] += e0 + e1;
+                    __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
+                    packed[c / 2] = *reinterpret_cast<uint32_t*>(&h);
+                }
+                l += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
+
+                // rescale this row of O if its reference moved (whole warp together:
+                // the TMEM accesses are warp-wide; lanes that did not move scale by 1)
+                if (j > 0 && __any_sync(0xffffffffu, raise)) {
+                    if (!mbar_wait(&o_full, (uint32_t)((j - 1) & 1))) { atomicExch(err, 21); ok = false; break; }
+                    tc_fence_after_sync();
+#pragma unroll
+                    for (int c = 0; c < DV / 16; ++c) {
+                        uint32_t o[16];
+                        tmem_ld_16_nowait(tmem + lane_addr + O_COL + c * 16, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+                        tmem_st_16(tmem + lane_addr + O_COL + c * 16, o);
+                    }
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                }
             }
 
             // row t of P into TMEM, over the columns its S came from
@@ -511,7 +539,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         if (ok && n_pages > 0) {
             tc_fence_after_sync();
             // a sink adds exp(sink - reference) to the denominator, once, with no value
-            float inv = 1.0f / (sink ? l + ex2(fmaf(sink[kvh * g + row_h], 1.4426950408889634f, -m)) : l);
+            float inv = SIGMOID ? 1.0f : 1.0f / (sink ? l + ex2(fmaf(sink[kvh * g + row_h], 1.4426950408889634f, -m)) : l);
             if (!CONTIG && gate.z && row_valid) inv *= gate.factor(row0 + q0 + row_p, kvh * g + row_h);
             const int ow = CONTIG ? dv : DV;  // columns of an output head
             __nv_bfloat16* o = out + ((size_t)(row0 + q0 + row_p) * nq + kvh * g + row_h) * ow;
@@ -597,7 +625,8 @@ int launch_tc(const void* q, const void* k_pages, const void* v_pages, long long
     if (grid.y > 65535 || grid.z > 65535) return RFX_ERR_UNSUPPORTED;
     RFX_LAUNCH(kernel, grid, THREADS, smem, s, mq, mk, mv, cache, seq_slot, seq_start, seq_new, seq_row0,
                (__nv_bfloat16*)out, nq, bq, window, keep_first,
-               (MODE >= 2 ? softcap : scale) * 1.4426950408889634f, MODE >= 2 ? scale / softcap : 1.0f, sink, slopes,
+               (MODE == 2 || MODE == 3 ? softcap : scale) * 1.4426950408889634f,
+               MODE == 2 || MODE == 3 ? scale / softcap : 1.0f, sink, slopes,
                (const int*)nullptr, 0, D, gate, err);
     return 0;
 }
@@ -691,6 +720,31 @@ extern "C" int rfx_attention_prefill_tc_kf(const void* q, const void* k_pages, c
     RFX_D(64)
     RFX_D(128)
 #undef RFX_D
+#undef RFX_GO
+    return RFX_ERR_UNSUPPORTED;
+}
+
+// Attention with sigmoid weights (rfx_attention_sigmoid_mma) for keys and values of 64 or 128: `bias` one float
+// per query head or null.
+extern "C" int rfx_attention_sigmoid_tc(const void* q, const void* k_pages, const void* v_pages,
+                                        long long n_pages_total, const int* page_table, int max_pages, int page_size,
+                                        const int* seq_slot, const int* seq_start, const int* seq_new,
+                                        const int* seq_row0, void* out, int S, int max_new, int R, int nq, int nkv,
+                                        int head_dim, int window, float scale, const float* bias, int* err,
+                                        void* stream) {
+    if (S <= 0 || max_new <= 0 || R <= 0) return 0;
+    if (page_size != PAGE || nkv <= 0 || nq % nkv != 0) return RFX_ERR_BAD_ARG;
+    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_pages) |
+         reinterpret_cast<uintptr_t>(v_pages) | reinterpret_cast<uintptr_t>(out)) & 15)
+        return RFX_ERR_UNSUPPORTED;
+    rfx::RowGate gate;
+    rfx::row_gate(&gate, nullptr, RFX_DT_F32, 0, 0, 0);
+    PagedKV cache{page_table, max_pages, page_size, nkv, head_dim};
+#define RFX_GO(DD)                                                                                              \
+    launch_tc<DD, 4>(q, k_pages, v_pages, n_pages_total, cache, seq_slot, seq_start, seq_new, seq_row0, out, S, \
+                     max_new, R, nq, window, 0, scale, nullptr, bias, 0.0f, gate, err, (cudaStream_t)stream)
+    if (head_dim == 64) return RFX_GO(64);
+    if (head_dim == 128) return RFX_GO(128);
 #undef RFX_GO
     return RFX_ERR_UNSUPPORTED;
 }

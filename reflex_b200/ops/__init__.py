@@ -1696,10 +1696,35 @@ def attention_sigmoid_mma(q, k_pages, v_pages, page_table, page_size, seq_slot, 
     return out
 
 
+def attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, seq_slot, seq_start, seq_new, seq_row0,
+                         max_new: int, nq, nkv, dim, window, scale, bias) -> torch.Tensor:
+    """The tcgen05/TMEM form of `attention_sigmoid_mma` for keys and values of one size, 64
+    or 128 (csrc/attention_prefill_tc.cu)."""
+    out = _new(q.shape, q.dtype, q.device)
+    st = native.lib().rfx_attention_sigmoid_tc(
+        _chk(q, "q", torch.bfloat16), _chk(k_pages, "k_pages", torch.bfloat16), _chk(v_pages, "v_pages", torch.bfloat16),
+        k_pages.shape[0], _chk(page_table, "page_table", torch.int32), page_table.shape[1], page_size,
+        _chk(seq_slot, "seq_slot", torch.int32), _chk(seq_start, "seq_start", torch.int32),
+        _chk(seq_new, "seq_new", torch.int32), _chk(seq_row0, "seq_row0", torch.int32), out.data_ptr(),
+        seq_slot.numel(), int(max_new), q.shape[0], nq, nkv, dim, int(window or 0), float(scale),
+        _chk(bias, "bias", torch.float32), device_error_word(q.device).data_ptr(), _stream())
+    native.check(st, f"attention_sigmoid_tc (dim={dim})")
+    return out
+
+
+# level with the mma.sync form at 24 rows of a sequence (the whole pair at width 2048: 52 us either way),
+# ahead from there on (100 rows 85 -> 80, 2,048 rows 419 -> 322)
+SIGMOID_TC_MIN_ROWS = _env_int("REFLEX_B200_SIGMOID_TC_MIN_ROWS", 2, 1, 1 << 30)
+
+
 def attention_sigmoid(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv, dim, vdim, window, scale, bias):
     """Attention with sigmoid weights for the step's rows; picks the kernel."""
     if (q.dtype == torch.bfloat16 and dim % 8 == 0 and vdim % 8 == 0 and dim <= 256 and vdim <= 128
             and nq // nkv <= 128 and page_size == 64):
+        if (dim == vdim and dim in (64, 128) and batch.max_new >= SIGMOID_TC_MIN_ROWS and k_pages.dim() == 4
+                and (q.data_ptr() | k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0):
+            return attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, batch.seq_slot, batch.seq_start,
+                                        batch.seq_new, batch.seq_row0, batch.max_new, nq, nkv, dim, window, scale, bias)
         return attention_sigmoid_mma(q, k_pages, v_pages, page_table, page_size, batch.seq_slot, batch.seq_start,
                                      batch.seq_new, batch.seq_row0, batch.max_new, nq, nkv, dim, vdim, window,
                                      scale, bias)
