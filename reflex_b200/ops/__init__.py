@@ -1026,8 +1026,9 @@ def moe_experts(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, ids: torc
     top = ids.shape[1]
     in_scale, out_wts = (wts, None) if weight_input else (None, wts)
     if moe_grouped(x):
-        # captured steps too, as long as the library's grouped product (no wait for the host) is there
-        if not torch.cuda.is_current_stream_capturing() or (_GROUPED_MM[0] and width % 8 == 0 and ff % 8 == 0):
+        # captured steps too, as long as a grouped product that needs no wait for the host is there
+        if not torch.cuda.is_current_stream_capturing() or (width % 8 == 0 and ff % 8 == 0
+                                                            and (_GROUPED_MM[0] or R <= MOE_GEMM_MAX_ROWS)):
             rows = moe_experts_grouped(x, up, down, ids, wts, activation, weight_input, alpha, limit, placed)
             return rows if leave_sum else rows.summed()
     act = _new((R * top, ff), x.dtype, x.device)
@@ -1058,9 +1059,10 @@ def moe_grouped(x: torch.Tensor) -> bool:
 def moe_experts_grouped(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, ids: torch.Tensor,
                         wts: torch.Tensor, activation: str = "relu2", weight_input: bool = False,
                         alpha: float = 1.0, limit: float = 0.0, placed=None) -> ExpertRows:
-    """The same for many bfloat16 rows (prefill), up to the sum: the (row, choice) pairs are
-    placed expert by expert on the device, each expert's block of rows goes
-    through its two matrices as library products (where the dense layers use
+    """The same for several bfloat16 rows, up to the sum: the (row, choice) pairs are
+    placed expert by expert on the device, and each expert's block of rows goes
+    through its two matrices: for up to MOE_GEMM_MAX_ROWS rows by this library's kernel
+    (csrc/moe_gemm.cu), beyond that as library products (where the dense layers use
     them too: the library's grouped product, or one product an expert where it
     has none, for which the host reads the experts' offsets once); a row's results
     are to be summed in the order of their rank."""
@@ -1094,6 +1096,16 @@ def moe_experts_grouped(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, i
     xg = _new((n, width), x.dtype, x.device)
     native.check(lib.rfx_moe_gather(_chk(x, "x"), place.data_ptr(), _chk(in_scale, "wts", torch.float32),
                                     xg.data_ptr(), dt_code(x.dtype), n, top, width, _stream()), "moe_gather")
+    if R <= MOE_GEMM_MAX_ROWS and width % 8 == 0 and ff % 8 == 0 and (up.data_ptr() | down.data_ptr()) % 16 == 0:
+        # a few rows: this library's kernel streams each chosen expert's weights once
+        act = _new((n, ff), x.dtype, x.device)
+        yg = _new((n, width), torch.float32, x.device)
+        err = device_error_word(x.device).data_ptr()
+        code = {"relu2": 1, "silu": 2, "glu_clamped": 3, "swiglu": 4}[activation]
+        for a, w, out, rows, cols, kind in ((xg, up, act, ff, width, code), (act, down, yg, width, ff, 0)):
+            native.check(lib.rfx_moe_gemm(a.data_ptr(), _chk(w, "experts", x.dtype), offsets.data_ptr(), out.data_ptr(), n,
+                                          R, E, rows, cols, kind, float(alpha), float(limit), err, _stream()), "moe_gemm")
+        return ExpertRows(yg, place, out_wts, R, top)
     grouped = getattr(torch, "_grouped_mm", None) if _GROUPED_MM[0] else None
     if grouped is not None and width % 8 == 0 and ff % 8 == 0:
         # the library's grouped product reads the experts' offsets on the device: no wait for the host
@@ -1125,6 +1137,7 @@ def moe_experts_grouped(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, i
     return ExpertRows(yg, place, out_wts, R, top)
 
 
+MOE_GEMM_MAX_ROWS = _env_int("REFLEX_B200_MOE_GEMM_MAX_ROWS", 64, 0, 64)
 _GROUPED_MM = [True, True]  # whether the library's grouped product is tried, and its 32-bit output
 
 

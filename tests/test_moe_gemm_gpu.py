@@ -1,0 +1,56 @@
+"""The experts' products for a few rows (csrc/moe_gemm.cu) against 64-bit formulas.
+
+Inputs are bfloat16 exactly; sums are 32-bit (K 2^-24 of the terms' size at worst), the activation is
+rounded to bfloat16 once before the second product (2^-9 each, averaged over the sum)."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from reflex_b200 import ops as o
+
+    return o
+
+
+def act64(kind, g, u):
+    if kind == "relu2":
+        return g.clamp(min=0) ** 2
+    if kind == "silu":
+        return g * torch.sigmoid(g)
+    if kind == "swiglu":
+        return g * torch.sigmoid(g) * u
+    g, u = g.clamp(max=0.7), u.clamp(-0.7, 0.7)
+    return g * torch.sigmoid(1.5 * g) * (u + 1)
+
+
+@pytest.mark.parametrize("kind", ["relu2", "silu", "glu_clamped", "swiglu"])
+@pytest.mark.parametrize("R,E,top,width,ff", [(2, 8, 1, 64, 8), (5, 3, 2, 40, 72), (16, 16, 4, 136, 200),
+                                              (17, 4, 3, 264, 128), (33, 40, 2, 128, 64), (64, 2, 2, 512, 136)])
+def test_a_few_rows_through_their_experts(R, E, top, width, ff, kind):
+    g = torch.Generator(device=DEV).manual_seed(R + E)
+    gated = kind in ("glu_clamped", "swiglu")
+    x = torch.randn((R, width), generator=g, device=DEV).bfloat16()
+    up = (torch.randn((E, ff * (2 if gated else 1), width), generator=g, device=DEV) * 0.1).bfloat16()
+    down = (torch.randn((E, width, ff), generator=g, device=DEV) * 0.1).bfloat16()
+    # the first expert is never chosen where there are others enough
+    scores = torch.randn((R, E), generator=g, device=DEV)
+    if E > top:
+        scores[:, 0] = -100.0
+    ids, wts, placed = ops().moe_route(scores, None, top, place=True)
+    for by_input in (False, True):
+        got = ops().moe_experts(x, up, down, ids, wts, activation=kind, weight_input=by_input, alpha=1.5, limit=0.7,
+                                placed=placed)
+        ref = torch.zeros((R, width), dtype=torch.float64, device=DEV)
+        for r in range(R):
+            for k in range(top):
+                e, w = int(ids[r, k]), wts[r, k].double()
+                row = (x[r].float() * wts[r, k]).bfloat16().double() if by_input else x[r].double()
+                h = up[e].double() @ row
+                y = down[e].double() @ act64(kind, h[:ff], h[ff:] if gated else None)
+                ref[r] += y if by_input else w * y
+        assert ((got - ref).norm() / ref.norm()).item() < 3e-3  # 2^-9 = 2e-3 an activation, uniform: 1.1e-3 rms
+    ops().check_device_errors(DEV)
