@@ -10,6 +10,7 @@
 //    [heads, N, K]; optionally times a per-(row, head) factor, or an element's
 //    sigmoid gate.  32-bit
 //    accumulation, each output reduced over k in index order by one thread.
+#include "attn_mma.cuh"
 #include "common.cuh"
 #include "paged.cuh"
 
@@ -179,6 +180,100 @@ heads_gemv_kernel(const T* __restrict__ x, int ldx, int xh, const T* __restrict_
     }
 }
 
+// The bfloat16 product for a decode step's rows on mma.sync: a block takes 16 of one head's columns a
+// warp.  The weights are the left operand, so few rows still fill the instruction; they come to shared
+// memory before the wait on the kernel before (they do not depend on it), which hides their latency:
+// what is left after it is the rows' load, K / 16 products and the store.  A tcgen05 tile would be 128
+// columns of a head that has 128 or 256, and set-up would cost more than the product.  (Eight rows of 16
+// heads of 128 x 256, both products of a latent attention's step: the step 63 us with a warp a column on
+// CUDA cores, 48 with this.)
+template <int RT>  // row tiles of eight
+__global__ void __launch_bounds__(128)
+heads_mma_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int xh, const __nv_bfloat16* __restrict__ W,
+                 __nv_bfloat16* __restrict__ y, int ldy, int yh, const float* __restrict__ scale, RowGate gate, int R,
+                 int N, int K, int heads) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.x, n0 = blockIdx.y * 16 * warps;
+    const int K16 = (K + 15) / 16 * 16, LD = K16 + 8, k8 = K16 / 8;
+    __nv_bfloat16* Ws = reinterpret_cast<__nv_bfloat16*>(smem_raw);  // [16 warps][LD]
+    __nv_bfloat16* Xs = Ws + 16 * warps * LD;                          // [8 RT][LD]
+    pdl_launch_dependents();
+    const __nv_bfloat16* wb = W + (size_t)b * N * K;
+    for (int e = threadIdx.x; e < 16 * warps * k8; e += blockDim.x) {
+        const int i = e / k8, c = 8 * (e - i * k8);
+        const bool ok = n0 + i < N && c < K;
+        attn::cp_async_16(Ws + i * LD + c, ok ? wb + (size_t)(n0 + i) * K + c : wb, ok);
+    }
+    attn::cp_async_commit();
+    pdl_wait();
+    for (int e = threadIdx.x; e < 8 * RT * k8; e += blockDim.x) {
+        const int r = e / k8, c = 8 * (e - r * k8);
+        const bool ok = r < R && c < K;
+        attn::cp_async_16(Xs + r * LD + c, ok ? x + (size_t)r * ldx + (size_t)b * xh + c : x, ok);
+    }
+    attn::cp_async_commit();
+    // factors of this lane's results, on their way meanwhile: columns g and g + 8, rows 8 t + 2 j and + 1
+    const int g = lane >> 2, j = lane & 3, n = n0 + 16 * warp + g;
+    float f[RT][4];
+#pragma unroll
+    for (int t = 0; t < RT; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 8 * t + 2 * j + (i & 1), nn = n + (i & 2 ? 8 : 0);
+            f[t][i] = r >= R || nn >= N ? 0.0f
+                      : gate.z          ? gate.factor(r, b * N + nn)
+                      : scale           ? scale[(size_t)r * heads + b]
+                                        : 1.0f;
+        }
+    attn::cp_async_wait<0>();
+    __syncthreads();
+    float acc[RT][4] = {};
+    const __nv_bfloat16* wa = Ws + (16 * warp + (lane & 7) + 8 * ((lane >> 3) & 1)) * LD + 8 * (lane >> 4);
+    for (int k = 0; k < K16; k += 16) {
+        uint32_t a[4];
+        attn::ldmatrix_x4(a, wa + k);
+#pragma unroll
+        for (int t = 0; t < RT; t += 2) {
+            if (t + 1 < RT) {
+                uint32_t u[4];
+                attn::ldmatrix_x4(u, Xs + (8 * t + (lane & 7) + 8 * (lane >> 4)) * LD + k + 8 * ((lane >> 3) & 1));
+                attn::mma_bf16(acc[t], a, u[0], u[1]);
+                attn::mma_bf16(acc[t + 1], a, u[2], u[3]);
+            } else {
+                uint32_t u[2];
+                attn::ldmatrix_x2(u, Xs + (8 * t + (lane & 7)) * LD + k + 8 * ((lane >> 3) & 1));
+                attn::mma_bf16(acc[t], a, u[0], u[1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < RT; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 8 * t + 2 * j + (i & 1), nn = n + (i & 2 ? 8 : 0);
+            if (r < R && nn < N) y[(size_t)r * ldy + (size_t)b * yh + nn] = __float2bfloat16_rn(acc[t][i] * f[t][i]);
+        }
+}
+
+template <int RT>
+int launch_heads_mma(const void* x, int ldx, int xh, const void* W, void* y, int ldy, int yh, const float* scale,
+                     const RowGate& gate, int R, int N, int K, int heads, cudaStream_t s) {
+    // four warps a block, fewer while that leaves SMs without a block
+    int warps = 4;
+    while (warps > 1 && (long long)heads * ((N + 16 * warps - 1) / (16 * warps)) < sm_count()) warps /= 2;
+    const size_t smem = (size_t)(16 * warps + 8 * RT) * ((K + 15) / 16 * 16 + 8) * 2;
+    if (smem > 200 * 1024) return RFX_ERR_UNSUPPORTED;
+    auto kernel = heads_mma_kernel<RT>;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    RFX_LAUNCH(kernel, dim3(heads, (N + 16 * warps - 1) / (16 * warps)), 32 * warps, smem, s, (const __nv_bfloat16*)x, ldx,
+               xh, (const __nv_bfloat16*)W, (__nv_bfloat16*)y, ldy, yh, scale, gate, R, N, K, heads);
+    return 0;
+}
+
 // y[r, b, :] *= scale[r, b]
 template <typename T>
 __global__ void scale_heads_kernel(T* __restrict__ y, const float* __restrict__ scale, size_t total,
@@ -220,6 +315,17 @@ extern "C" int rfx_heads_linear(const void* x, int ldx, int xh, const void* W, v
     if (K <= 0 || xh < K || yh < N || (scale && gate_z) || !row_gate(&gate, gate_z, gate_dt, gate_ld, gate_col, heads * N))
         return RFX_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    if (dt == RFX_DT_BF16 && R <= 64 && ((ldx | xh | K) & 7) == 0 && (N + 15) / 16 <= 65535 &&
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) == 0) {
+        int st;
+#define RFX_GO(T) st = launch_heads_mma<T>(x, ldx, xh, W, y, ldy, yh, scale, gate, R, N, K, heads, s)
+        if (R <= 8) RFX_GO(1);
+        else if (R <= 16) RFX_GO(2);
+        else if (R <= 32) RFX_GO(4);
+        else RFX_GO(8);
+#undef RFX_GO
+        if (st != RFX_ERR_UNSUPPORTED) return st;  // rows too wide for shared memory
+    }
     if (R <= GV_ROWS && (size_t)R * K * sizeof(float) <= 48 * 1024) {
         // a few rows: every weight is read once and meets all rows
         int gy = (N + 7) / 8;
