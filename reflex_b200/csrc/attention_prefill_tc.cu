@@ -106,7 +106,7 @@ __host__ __device__ constexpr uint32_t idesc_b_mn(int M, int N) {
 
 struct Bars {
     uint64_t q_full, k_full[KV_STAGES], k_empty[KV_STAGES], v_full[KV_STAGES], v_empty[KV_STAGES], s_full[2], p_full[2],
-        o_full;
+        o_full, o_done;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -204,7 +204,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         __shared__ __align__(8) Bars bars_static;
         bars = &bars_static;
     }
-    uint64_t &q_full = bars->q_full, &o_full = bars->o_full;
+    uint64_t &q_full = bars->q_full, &o_full = bars->o_full, &o_done = bars->o_done;
     uint64_t *k_full = bars->k_full, *k_empty = bars->k_empty, *v_full = bars->v_full, *v_empty = bars->v_empty,
              *s_full = bars->s_full, *p_full = bars->p_full;
     uint32_t& tmem_base_smem = bars->tmem_base;
@@ -248,6 +248,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
             mbar_init(&p_full[i], 4);
         }
         mbar_init(&o_full, 1);
+        mbar_init(&o_done, 1);
         abort_flag = 0;
         fence_barrier_init();
     }
@@ -342,6 +343,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                 }
                 umma_commit(&v_empty[s]);
                 umma_commit(&o_full);
+                if (i == n_pages - 1) umma_commit(&o_done);
                 return true;
             };
             for (int j = 0; j < n_pages && ok; ++j) {
@@ -534,7 +536,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         if (t == 0) trace_mark(3);
         if (tracing) trace_value(11, wait_s);
         if (ok && n_pages > 0) {
-            if (!mbar_wait(&o_full, (uint32_t)((n_pages - 1) & 1))) { atomicExch(err, 25); ok = false; }
+            // A barrier of its own: a warp ahead of the others gets here while the product before last still
+            // waits for their rows, and o_full, two pages behind, would read as complete (one phase bit).
+            if (!mbar_wait(&o_done, 0)) { atomicExch(err, 25); ok = false; }
         }
         if (ok && n_pages > 0) {
             tc_fence_after_sync();
