@@ -4,7 +4,7 @@
 //  * rfx_gemm_f32: the true 32-bit product.  CUDA-core fused multiply-adds
 //    only; each output element is reduced over k = 0..K-1 in index order by one
 //    thread, so its value does not depend on how many rows the call has or on
-//    where the row sits in the batch, nor on which of the three forms runs.
+//    where the row sits in the batch, nor on which form (tile) runs.
 //  * rfx_gemv_bf16: bfloat16 weights and activations for a few rows (decode),
 //    32-bit accumulation; a pure weight-streaming kernel with 16-byte loads.
 #include "common.cuh"
@@ -79,167 +79,118 @@ __device__ __forceinline__ void wait_copies() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Up to 64 rows: the weights are streamed once.  A block owns 32 columns, a lane a column, a warp RPW
-// rows; what bounds it is one element's chain of K dependent multiply-adds (four cycles each), beside
-// which the weights of a square matrix arrive at about the memory's rate, so the chains of different
-// rows run in different warps, few to a warp.
-constexpr int KT = 64, WLD = KT + 4;  // columns of a stage; row stride: eight lanes' 16-byte reads meet all banks
+// A block owns BM rows by BN columns, a thread TM rows (BM / TM apart) by TN columns (BN / TN apart:
+// the reads of eight neighbours then meet all banks).  An element's sum is one chain over k, so neither
+// tensor cores nor a split of k may serve, and the chip is filled by elements alone.  What bounds it:
+// with one or two rows the weights (4,096 x 4,096: 3.3 TB/s, 24,576 x 4,096: 5.9); with few rows the
+// chain of K dependent multiply-adds beside the reads of shared memory, so threads have few elements and
+// stages are long (one barrier for 128 steps of the chain); with many rows the registers' banks, as a
+// multiply-add whose sum and weight share one takes two cycles, and columns side by side in K alternate
+// with it: 48 of 72 TFLOP/s at most, 47 reached (24,576 columns, 1,024 rows).  Packed pairs of columns (one
+// instruction, no such meeting) were slower, the pairs' x being read twice from shared memory.
+template <int BM, int BN, int TM, int TN, int BK, int STAGES_>
+struct Tile {
+    static constexpr int ACROSS = BN / TN, THREADS = BM / TM * ACROSS, LD = BK + 4, STAGE = (BM + BN) * LD;
+    static constexpr int STAGES = STAGES_, RS = THREADS / (BK / 4);  // rows a pass of the block's copies covers
+    static constexpr int XC = (BM + RS - 1) / RS, WC = (BN + RS - 1) / RS;
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(float);
+    static_assert(THREADS % (BK / 4) == 0 && BN % RS == 0, "whole passes");
+};
 
-template <int RPW>
-__global__ void __launch_bounds__(512)
-gemm_f32_rows_kernel(const float* __restrict__ x, const float* __restrict__ W, float* __restrict__ y, int R, int N,
-                     int K, int stages) {
-    extern __shared__ __align__(16) float sm[];
-    pdl_prologue();
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rows = warps * RPW, r0 = blockIdx.y * rows, n0 = blockIdx.x * 32;
-    const int stage = 32 * WLD + rows * KT;  // [32][WLD] of W, [rows][KT] of x
-    const int tiles = (K + KT - 1) / KT;
-    auto fetch = [&](int t) {
-        if (t < tiles) {
-            float* to = sm + (t % stages) * stage;
-            for (int e = threadIdx.x; e < (32 + rows) * (KT / 4); e += blockDim.x) {
-                const int i = e / (KT / 4), c = 4 * (e % (KT / 4)), k = t * KT + c;
-                if (i < 32) copy16(to + i * WLD + c, W + (size_t)(n0 + i < N ? n0 + i : 0) * K + (k < K ? k : 0), n0 + i < N && k < K);
-                else {
-                    const int r = r0 + i - 32;
-                    copy16(to + 32 * WLD + (i - 32) * KT + c, x + (size_t)(r < R ? r : 0) * K + (k < K ? k : 0), r < R && k < K);
-                }
-            }
-        }
-        copies_done();
-    };
-    for (int t = 0; t < stages - 1; ++t) fetch(t);
-    float acc[RPW];
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) acc[i] = 0.0f;
-    for (int t = 0; t < tiles; ++t) {
-        switch (stages) {  // the group of tile t is the oldest of stages - 1 in flight
-            case 8: wait_copies<6>(); break;
-            case 6: wait_copies<4>(); break;
-            default: wait_copies<2>(); break;
-        }
-        __syncthreads();  // tile t has landed, and every warp is done with the tile before
-        fetch(t + stages - 1);
-        const float* w = sm + (t % stages) * stage + lane * WLD;
-        const float* xs = sm + (t % stages) * stage + 32 * WLD + warp * RPW * KT;
-#pragma unroll
-        for (int k = 0; k < KT; k += 4) {
-            const float4 b = *reinterpret_cast<const float4*>(w + k);
-#pragma unroll
-            for (int i = 0; i < RPW; ++i) {
-                const float4 a = *reinterpret_cast<const float4*>(xs + i * KT + k);
-                acc[i] = fmaf(a.x, b.x, acc[i]);
-                acc[i] = fmaf(a.y, b.y, acc[i]);
-                acc[i] = fmaf(a.z, b.z, acc[i]);
-                acc[i] = fmaf(a.w, b.w, acc[i]);
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-        const int r = r0 + warp * RPW + i;
-        if (r < R && n0 + lane < N) y[(size_t)r * N + n0 + lane] = acc[i];
-    }
-}
-
-// More rows: BM x BN tiles, a thread 8 rows by TN columns (rows ty + BM / 8 i, columns tx + 16 j: the
-// reads of a quarter warp then meet all banks), both operands as they lie, sixteen k a stage.
-constexpr int BK = 16, BLD = BK + 4, BSTAGES = 4;
-
-template <int BM, int BN>
-__global__ void __launch_bounds__(BM * 2)
+template <class T, int BM, int BN, int TM, int TN, int BK>
+__global__ void __launch_bounds__(T::THREADS)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ W, float* __restrict__ y, int R, int N,
                      int K) {
-    constexpr int THREADS = BM * 2, TN = BN / 16, STAGE = (BM + BN) * BLD;
+    constexpr int STAGES = T::STAGES, LD = T::LD, RS = T::RS;
     extern __shared__ __align__(16) float sm[];
     pdl_prologue();
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int tx = threadIdx.x % T::ACROSS, ty = threadIdx.x / T::ACROSS;
     const int r0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tiles = (K + BK - 1) / BK;
+    const int crow = threadIdx.x / (BK / 4), cc = 4 * (threadIdx.x % (BK / 4));
+    const float* xsrc = x + (size_t)(r0 + crow) * K + cc;
+    const float* wsrc = W + (size_t)(n0 + crow) * K + cc;
+    int to = 0;  // the stage the next tile goes to
     auto fetch = [&](int t) {
         if (t < tiles) {
-            float* to = sm + (t % BSTAGES) * STAGE;
+            const bool in = t * BK + cc < K;
+            float* d = sm + to * T::STAGE + crow * LD + cc;
 #pragma unroll
-            for (int e = threadIdx.x; e < (BM + BN) * (BK / 4); e += THREADS) {
-                const int i = e / (BK / 4), c = 4 * (e % (BK / 4)), k = t * BK + c;
-                const int row = i < BM ? r0 + i : n0 + i - BM;
-                const bool ok = row < (i < BM ? R : N) && k < K;
-                const float* src = i < BM ? x : W;
-                copy16(to + i * BLD + c, ok ? src + (size_t)row * K + k : src, ok);
+            for (int i = 0; i < T::WC; ++i) {
+                const bool ok = in && n0 + crow + i * RS < N;
+                copy16(d + (BM + i * RS) * LD, ok ? wsrc + (size_t)(i * RS) * K : W, ok);
             }
+#pragma unroll
+            for (int i = 0; i < T::XC; ++i) {
+                if (BM % RS && crow + i * RS >= BM) continue;
+                const bool ok = in && r0 + crow + i * RS < R;
+                copy16(d + i * RS * LD, ok ? xsrc + (size_t)(i * RS) * K : x, ok);
+            }
+            xsrc += BK;
+            wsrc += BK;
         }
         copies_done();
+        to = to + 1 == STAGES ? 0 : to + 1;
     };
 #pragma unroll
-    for (int t = 0; t < BSTAGES - 1; ++t) fetch(t);
-    float acc[8][TN];
+    for (int t = 0; t < STAGES - 1; ++t) fetch(t);
+    float acc[TM][TN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+    int at = 0;
     for (int t = 0; t < tiles; ++t) {
-        wait_copies<BSTAGES - 2>();
-        __syncthreads();
-        fetch(t + BSTAGES - 1);
-        const float* a = sm + (t % BSTAGES) * STAGE + ty * BLD;
-        const float* b = sm + (t % BSTAGES) * STAGE + (BM + tx) * BLD;
+        wait_copies<STAGES - 2>();
+        __syncthreads();  // tile t has landed, and every warp is done with the tile before
+        fetch(t + STAGES - 1);
+        const float* a = sm + at * T::STAGE + ty * LD;
+        const float* b = sm + at * T::STAGE + (BM + tx) * LD;
+        at = at + 1 == STAGES ? 0 : at + 1;
 #pragma unroll
         for (int k = 0; k < BK; k += 4) {
-            float4 av[8], bv[TN];
+            float4 av[TM], bv[TN];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const float4*>(a + i * (BM / 8) * BLD + k);
+            for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const float4*>(a + i * (BM / TM) * LD + k);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) bv[j] = *reinterpret_cast<const float4*>(b + j * 16 * BLD + k);
+            for (int j = 0; j < TN; ++j) bv[j] = *reinterpret_cast<const float4*>(b + j * T::ACROSS * LD + k);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].x, bv[j].x, acc[i][j]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].y, bv[j].y, acc[i][j]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].z, bv[j].z, acc[i][j]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i].w, bv[j].w, acc[i][j]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = r0 + ty + (BM / 8) * i;
+    for (int i = 0; i < TM; ++i) {
+        const int r = r0 + ty + BM / TM * i;
         if (r >= R) continue;
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tx + 16 * j;
+            const int n = n0 + tx + T::ACROSS * j;
             if (n < N) y[(size_t)r * N + n] = acc[i][j];
         }
     }
 }
 
-template <int RPW>
-int launch_rows(const float* x, const float* W, float* y, int R, int N, int K, cudaStream_t s) {
-    int warps = (R + RPW - 1) / RPW;
-    if (warps < 4) warps = 4;  // enough threads to issue the copies
-    const size_t stage = (size_t)(32 * WLD + warps * RPW * KT) * sizeof(float);
-    const int stages = stage * 8 <= 100 * 1024 ? 8 : stage * 6 <= 110 * 1024 ? 6 : 4;
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(stage * stages));
-    if (e != cudaSuccess) return (int)e;
-    RFX_LAUNCH(gemm_f32_rows_kernel<RPW>, dim3((N + 31) / 32, 1), warps * 32, stage * stages, s, x, W, y, R, N, K, stages);
-    return 0;
-}
-
-template <int BM, int BN>
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
 int launch_tiles(const float* x, const float* W, float* y, int R, int N, int K, cudaStream_t s) {
-    constexpr size_t smem = (size_t)BSTAGES * (BM + BN) * BLD * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    using T = Tile<BM, BN, TM, TN, BK, STAGES>;
+    auto kernel = gemm_f32_tile_kernel<T, BM, BN, TM, TN, BK>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
     if (e != cudaSuccess) return (int)e;
-    RFX_LAUNCH((gemm_f32_tile_kernel<BM, BN>), dim3((N + BN - 1) / BN, (R + BM - 1) / BM), BM * 2, smem, s, x, W, y, R, N, K);
+    RFX_LAUNCH(kernel, dim3((N + BN - 1) / BN, (R + BM - 1) / BM), T::THREADS, T::SMEM, s, x, W, y, R, N, K);
     return 0;
 }
 
@@ -405,13 +356,30 @@ extern "C" int rfx_gemm_f32(const float* x, const float* W, float* y, int R, int
     if (grid.y > 65535) return RFX_ERR_UNSUPPORTED;
     cudaStream_t st = (cudaStream_t)stream;
     if (K % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) == 0) {
-        if (R <= 8) return launch_rows<1>(x, W, y, R, N, K, st);
-        if (R <= 32) return launch_rows<2>(x, W, y, R, N, K, st);
-        if (R <= 64) return launch_rows<4>(x, W, y, R, N, K, st);
-        // the larger tile reads shared memory half as often a multiply-add; it needs two tiles an SM
-        if ((long long)((R + 127) / 128) * ((N + 127) / 128) >= 2LL * sm_count())
-            return launch_tiles<128, 128>(x, W, y, R, N, K, st);
-        return launch_tiles<64, 64>(x, W, y, R, N, K, st);
+        // measured for N = K = 4,096 (and N = 24,576) against the 32-column form next to it in the list
+        const bool few = N <= 32 * sm_count();  // 32 columns a block do not fill the chip
+        if (R <= 1) return launch_tiles<1, 32, 1, 1, 128, 6>(x, W, y, R, N, K, st);  // 20 (69) us
+        if (R <= 2) return launch_tiles<2, 32, 2, 1, 128, 6>(x, W, y, R, N, K, st);  // 25 (74)
+        if (R <= 4) return launch_tiles<4, 16, 2, 1, 128, 6>(x, W, y, R, N, K, st);  // 28 (99), by 32 columns 33 (102)
+        if (R <= 8) return launch_tiles<8, 16, 2, 1, 128, 5>(x, W, y, R, N, K, st);  // 37 (128), by 32: 43 (130)
+        if (R <= 16)  // 44 (240) and 62 (147)
+            return few ? launch_tiles<16, 16, 2, 2, 128, 5>(x, W, y, R, N, K, st)
+                       : launch_tiles<16, 32, 4, 2, 64, 5>(x, W, y, R, N, K, st);
+        if (R <= 32)  // 61 (347) and 94 (229)
+            return few ? launch_tiles<32, 32, 4, 2, 128, 4>(x, W, y, R, N, K, st)
+                       : launch_tiles<32, 32, 4, 4, 64, 4>(x, W, y, R, N, K, st);
+        if (R <= 64 && few) return launch_tiles<64, 32, 4, 2, 128, 3>(x, W, y, R, N, K, st);  // 92 (533), below 127 (376)
+        // Waves of blocks times a tile's work; small tiles do 6 % less a cycle, large ones a third less
+        // while an SM has three or fewer.  6,144 columns, K = 4,096, small and large: 300 rows 418 and 446
+        // us, 1,024 rows 1,234 and 1,177; 1,536 columns, K = 1,024, 701 rows: 66 and 103.
+        const int sms = sm_count();
+        const auto blocks = [&](int bm, int bn) { return (long long)((R + bm - 1) / bm) * ((N + bn - 1) / bn); };
+        const long long per_small = (blocks(32, 64) + sms - 1) / sms, per_large = (blocks(64, 64) + sms - 1) / sms;
+        if (per_small >= 2 && blocks(64, 32) <= 2 * sms)  // two a SM, a longer stage: 200 rows of N = 1,536 41 us, not 49
+            return launch_tiles<64, 32, 4, 4, 64, 4>(x, W, y, R, N, K, st);
+        if (per_small * 106 <= per_large * (per_large <= 3 ? 260 : 200))
+            return launch_tiles<32, 64, 4, 4, 32, 4>(x, W, y, R, N, K, st);
+        return launch_tiles<64, 64, 8, 4, 32, 3>(x, W, y, R, N, K, st);
     }
     RFX_LAUNCH(gemm_f32_kernel, grid, 256, 0, (cudaStream_t)stream, x, W, y, R, N, K);
     return 0;

@@ -17,8 +17,8 @@ def i32(v):
     return torch.tensor(list(v), dtype=torch.int32, device=DEV)
 
 
-@pytest.mark.parametrize("N,K", [(31, 64), (33, 68), (130, 4), (64, 132), (300, 2052), (4100, 96)])
-@pytest.mark.parametrize("R", [1, 7, 8, 9, 32, 33, 63, 64, 65, 129, 2100])
+@pytest.mark.parametrize("N,K", [(31, 64), (33, 68), (130, 4), (64, 132), (300, 2052), (4100, 96), (4801, 132)])
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 7, 8, 9, 16, 32, 33, 63, 64, 65, 129, 300, 2100])
 def test_every_form_of_the_product_gives_the_same_bits(R, N, K):
     """Rows of a matrix whose start is off 16 bytes take the general form, one thread an element."""
     g = torch.Generator(device=DEV).manual_seed(R + N + K)
