@@ -1274,6 +1274,34 @@ def short_conv(proj: torch.Tensor, col0: int, channels: int, bias: Optional[torc
     return (out, lo) if also_bf16 else out
 
 
+# Up to this many sequences a decode step's filter, [dt | B | C] product and scan are one launch: every
+# sequence's cluster of CTAs reads all of W_x, which the three launches read once.
+MAMBA_STEP_MAX_ROWS = _env_int("REFLEX_B200_MAMBA_STEP_MAX_ROWS", 8, 0, 1 << 30)
+
+
+def mamba_step(xz: torch.Tensor, channels: int, states: int, filters_t: torch.Tensor, conv_bias, w_x: torch.Tensor,
+               w_dt: torch.Tensor, dt_bias, A: torch.Tensor, D, state: torch.Tensor, batch) -> Optional[torch.Tensor]:
+    """A decode step of a selective scan between its first and last product (one row a
+    sequence, bfloat16): `short_conv` with its state, the product of `w_x` [dt | B | C],
+    `mamba_scan`, in one launch (csrc/mamba_step.cu).  `xz` float32 rows [x | z].  Returns
+    y * silu(z), bfloat16 [R, channels]; None, with nothing done, for sizes it does not take."""
+    R, rank = xz.shape[0], w_dt.shape[1]
+    if (R > MAMBA_STEP_MAX_ROWS or w_x.dtype != torch.bfloat16 or w_dt.dtype != torch.bfloat16
+            or tuple(w_x.shape) != (rank + 2 * states, channels)):
+        return None
+    out = _new((R, channels), torch.bfloat16, xz.device)
+    st = native.lib().rfx_mamba_step(
+        _chk(xz, "xz", torch.float32), xz.shape[1], channels, states, rank, filters_t.shape[0],
+        _chk(filters_t, "filters_t", torch.float32), _chk(conv_bias, "conv_bias", torch.float32), _chk(w_x, "w_x"),
+        _chk(w_dt, "w_dt"), _chk(dt_bias, "dt_bias", torch.float32), _chk(A, "A", torch.float32),
+        _chk(D, "D", torch.float32), _chk(state, "state", torch.float32), state.stride(0),
+        _chk(batch.row_slot, "row_slot", torch.int32), R, out.data_ptr(), _stream())
+    if st == native.ERR_UNSUPPORTED:
+        return None
+    native.check(st, f"mamba_step (channels={channels}, states={states})")
+    return out
+
+
 def conv_state_update(proj: torch.Tensor, col0: int, channels: int, bias: Optional[torch.Tensor], taps: int,
                       state: torch.Tensor, batch) -> None:
     """After a step's rows have been convolved: the sequences' new last taps - 1

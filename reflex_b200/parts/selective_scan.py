@@ -90,6 +90,15 @@ class SelectiveScan:
         ops.prof_mark("qkv_gemm")
         # a row a sequence (decoding): the convolution's launch also moves the last inputs on
         single = xz.shape[0] == batch.seq_slot.numel()
+        if single and lo:
+            # a few sequences: everything up to the last product in one launch
+            y = ops.mamba_step(xz, C, N, self.filters, self.conv_bias, self.w_x, self.w_dt, self.dt_bias, self.A, self.D,
+                               state, batch)
+            if y is not None:
+                ops.prof_mark("scan")
+                out = ops.linear(y, self.o, out_dtype=torch.float32)
+                ops.prof_mark("o_proj")
+                return out
         u = ops.short_conv(xz, 0, C, None, self.filters, self.conv_bias, state if self.taps > 1 else None, batch,
                            also_bf16=lo, activation="silu", update_state=single and self.taps > 1)
         u, u_in = u if lo else (u, u)
