@@ -14,16 +14,19 @@
 //
 // A walk through the rows has one chain of dependent steps a head and leaves most SMs without
 // work; chunks cost the memory's way out and back (heads x N x P floats each) and about twice the
-// arithmetic.  A prompt of 2,048 rows: 1.2 ms walking and 0.15 ms in chunks for 32 heads of 64 x 128
-// (36 us the chunks' sums, 19 the carry, 96 the rows), 0.76 and 0.14 ms for 8 of 128 x 256 (36, 27 and
-// 74); the three kernels are bound by the tensor pipe's mma.sync rate and, in the carry, by L2.  64 rows: with 32 that traffic doubles, with 128 the products inside the chunk do and
-// a block no longer shares its SM.
+// arithmetic.  A prompt of 2,048 rows: 1.2 ms walking and 0.12 ms in chunks for 32 heads of 64 x 128
+// (30 us the chunks' sums, 19 the carry, 75 the rows), 0.76 and 0.13 ms for 8 of 128 x 256 (35, 27 and
+// 65); the carry is bound by L2, the other two by the latency of tiles and fragments on the way to
+// the tensor pipe (28 % busy).  64 rows: with 32 the memories' traffic doubles, with 128 the products
+// inside the chunk do and a block no longer shares its SM.
 //
 // A policy `Pol` gives: q, k, v rows (float32, 16-byte aligned, counts in fours), `heads`, `per`
 // (heads per q/k head), N (elements of q and k, at most 128), P (elements of v) and the functions
 // named below.  What depends on a step: sequence `seq`'s rows `first_row` .. in chunks from
 // `seg * seg_rows` on, so that a long step can go through a bounded scratch in several rounds.
 #pragma once
+
+#include <type_traits>
 
 #include "attn_mma.cuh"
 #include "common.cuh"
@@ -44,6 +47,7 @@ struct Step {
     float* scratch;  // [place][head][P][N] (+ [N] with a normaliser): a chunk's own sum, then the memory before it
     float4* aux;     // [place][head]: what the carry needs of a chunk
     float* before;   // [place][head]: the policy's running number before the chunk
+    float4* rows;    // [place][head][L][RECORDS]: the policy's records of the chunk's rows
 };
 
 // The place of chunk c (of this segment) of sequence `seq` among all: with one segment at most
@@ -67,10 +71,19 @@ __device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
 template <int THREADS>
 __device__ __forceinline__ void load_tile(float* dst, int ld, const float* src, size_t src_ld, int rows, int n, int c4,
                                           int n4) {
-    for (int e = threadIdx.x; e < rows * c4; e += THREADS) {
-        const int r = e / c4, c = e - r * c4;
-        const bool ok = r < n && c < n4;
-        attn::cp_async_16(dst + r * ld + 4 * c, ok ? src + (size_t)r * src_ld + 4 * c : src, ok);
+    if (THREADS % c4 == 0) {  // a thread keeps its column: no division a piece
+        const int c = threadIdx.x % c4, step = THREADS / c4;
+        int r = threadIdx.x / c4;
+        float* d = dst + r * ld + 4 * c;
+        const float* s = src + (size_t)r * src_ld + 4 * c;
+        const int live = c < n4 ? n : 0;
+        for (; r < rows; r += step, d += step * ld, s += (size_t)step * src_ld) attn::cp_async_16(d, r < live ? s : src, r < live);
+    } else {
+        for (int e = threadIdx.x; e < rows * c4; e += THREADS) {
+            const int r = e / c4, c = e - r * c4;
+            const bool ok = r < n && c < n4;
+            attn::cp_async_16(dst + r * ld + 4 * c, ok ? src + (size_t)r * src_ld + 4 * c : src, ok);
+        }
     }
 }
 
@@ -93,7 +106,7 @@ __global__ void __launch_bounds__(256) chunk_state_kernel(Pol pol, Step st) {
     attn::cp_async_commit();
     const size_t at = ch.place * pol.heads + h;
     if (warp == 0) {
-        const float4 a = pol.state_weights(wl, h, ch.first, ch.n, lane);
+        const float4 a = pol.state_weights(wl, p0 == 0 ? st.rows + at * L * Pol::RECORDS : nullptr, h, ch.first, ch.n, lane);
         if (p0 == 0 && lane == 0) st.aux[at] = a;
     }
     attn::cp_async_wait<0>();
@@ -208,18 +221,22 @@ __device__ __forceinline__ void two_parts(double v, float* hi, float* lo) {
     *lo = isinf(h) ? 0.0f : (float)(v - (double)h);
 }
 
-// The rows' weights of a chunk and head: w_ts = exp((g_s + e_t)) * w_s, g and e in two parts.
-struct Weights {
-    float g_hi[L], g_lo[L], e_hi[L], e_lo[L], w[L], alpha[L], extra[L];
+// What a row t brings to its results: w_ts = exp((g_s + e_t)) * w_s with e in two parts, the factor of
+// q . S, and a number for the policy's store.
+struct RowTerms {
+    float e_hi, e_lo, alpha, extra;
 };
 
 // A block a (chunk, q/k head, some of that head's items); an item is a (head, PT elements of v).
-// A warp takes sixteen rows: their products with the chunk's k, once, stay in registers; then item
-// by item the memory's tile and v's replace k's in shared memory.
+// Two warps take sixteen rows, half an item's columns each: the rows' products with the chunk's k, once,
+// stay in registers; then item by item the memory's tile and v's replace k's in shared memory.  Eight
+// warps, although two then make the same products with k: at 87 KB a block two share an SM, and four
+// warps each leave too few to cover the tiles' arrival, the exponentials and the fragments' splitting
+// (96 and 74 us for the two shapes above, now 75 and 65).
 template <class Pol>
-__global__ void __launch_bounds__(128) chunk_out_kernel(Pol pol, Step st, int items_a_block) {
+__global__ void __launch_bounds__(256, 2) chunk_out_kernel(Pol pol, Step st, int items_a_block) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ Weights wt;
+    __shared__ __align__(16) float4 rec[L * Pol::RECORDS];
     __shared__ float nv[128];
     rfx::pdl_prologue();
     const int seq = blockIdx.y;
@@ -232,35 +249,30 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(Pol pol, Step st, int it
     const int N8 = (pol.N + 7) / 8 * 8, ld = N8 + 8;
     float *Qs = sm, *Bs = sm + L * ld, *Vs = Bs + L * ld;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
-    load_tile<128>(Qs, ld, pol.q_row(ch.first, kvh * pol.per), pol.ldq, L, ch.n, N8 / 4, pol.N / 4);
-    load_tile<128>(Bs, ld, pol.k_row(ch.first, kvh * pol.per), pol.ldk, L, ch.n, N8 / 4, pol.N / 4);
+    const int rw = warp & 3, c0 = (warp >> 2) * (PT / 2);  // the warp's rows (sixteen) and columns of a tile
+    load_tile<256>(Qs, ld, pol.q_row(ch.first, kvh * pol.per), pol.ldq, L, ch.n, N8 / 4, pol.N / 4);
+    load_tile<256>(Bs, ld, pol.k_row(ch.first, kvh * pol.per), pol.ldk, L, ch.n, N8 / 4, pol.N / 4);
     attn::cp_async_commit();
     attn::cp_async_wait<0>();
     __syncthreads();
-    const float* qa = Qs + (16 * warp + g) * ld + 2 * j;
-    const int tiles = 2 * warp + 2;  // of eight rows s <= the warp's last row
+    const float* qa = Qs + (16 * rw + g) * ld + 2 * j;
+    const int tiles = 2 * rw + 2;  // of eight rows s <= the warp's last row
     float G[8][4] = {};
-    if (warp >= 2) {
+    auto scores = [&](auto& acc, auto count) {
+        constexpr int T = decltype(count)::value;
         for (int s = 0; s < N8 / 8; ++s) {
             const float2 x = *reinterpret_cast<const float2*>(qa + 8 * s);
             const float2 y = *reinterpret_cast<const float2*>(qa + 8 * ld + 8 * s);
             const Left a = left_from(x.x, y.x, x.y, y.y);
-            float2 b[8];
+            float2 b[T];
 #pragma unroll
-            for (int t = 0; t < 8; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
-            product3<8>(G, a, b);
+            for (int t = 0; t < T; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
+            product3<T>(acc, a, b);
         }
-    } else {
-        for (int s = 0; s < N8 / 8; ++s) {
-            const float2 x = *reinterpret_cast<const float2*>(qa + 8 * s);
-            const float2 y = *reinterpret_cast<const float2*>(qa + 8 * ld + 8 * s);
-            const Left a = left_from(x.x, y.x, x.y, y.y);
-            float2 b[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
-            product3<4>(*reinterpret_cast<float(*)[4][4]>(&G), a, b);
-        }
-    }
+    };
+    if (rw >= 2) scores(G, std::integral_constant<int, 8>{});
+    else scores(*reinterpret_cast<float(*)[4][4]>(&G), std::integral_constant<int, 4>{});
+    const int ra = 16 * rw + g, rb = ra + 8;
     int head = -1;
     for (int item = i0; item < i1; ++item) {
         const int h = kvh * pol.per + item / ptiles, p0 = (item % ptiles) * PT;
@@ -268,37 +280,38 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(Pol pol, Step st, int it
         const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
         const float* S = st.scratch + at * E;
         __syncthreads();  // k, or the item before, has been read by every warp
-        load_tile<128>(Bs, ld, S + (size_t)p0 * pol.N, pol.N, PT, min(PT, pol.P - p0), N8 / 4, pol.N / 4);
-        load_tile<128>(Vs, VLD, pol.v_row(ch.first, h) + p0, pol.ldv, L, ch.n, PT / 4, min(PT, pol.P - p0) / 4);
-        attn::cp_async_commit();
+        load_tile<256>(Bs, ld, S + (size_t)p0 * pol.N, pol.N, PT, min(PT, pol.P - p0), N8 / 4, pol.N / 4);
+        load_tile<256>(Vs, VLD, pol.v_row(ch.first, h) + p0, pol.ldv, L, ch.n, PT / 4, min(PT, pol.P - p0) / 4);
         if (h != head) {
-            if (warp == 0) pol.row_weights(wt, h, ch.first, ch.n, st.before[at], lane);
+            for (int i = threadIdx.x; i < L * Pol::RECORDS; i += 256)
+                attn::cp_async_16(&rec[i], st.rows + at * L * Pol::RECORDS + i, true);
             if (Pol::NORMALISER)
-                for (int n = threadIdx.x; n < pol.N; n += 128) nv[n] = S[(size_t)pol.P * pol.N + n];
+                for (int n = threadIdx.x; n < pol.N; n += 256) nv[n] = S[(size_t)pol.P * pol.N + n];
             head = h;
         }
+        attn::cp_async_commit();
+        const float before = st.before[at];
         attn::cp_async_wait<0>();
         __syncthreads();
-        const int ra = 16 * warp + g, rb = ra + 8;
-        float acc[8][4] = {};
+        float acc[4][4] = {};
         for (int s = 0; s < N8 / 8; ++s) {
             const float2 x = *reinterpret_cast<const float2*>(qa + 8 * s);
             const float2 y = *reinterpret_cast<const float2*>(qa + 8 * ld + 8 * s);
             const Left a = left_from(x.x, y.x, x.y, y.y);
-            float2 b[8];
+            float2 b[4];
 #pragma unroll
-            for (int t = 0; t < 8; ++t) b[t] = *reinterpret_cast<const float2*>(Bs + (8 * t + g) * ld + 8 * s + 2 * j);
-            product3<8>(acc, a, b);
+            for (int t = 0; t < 4; ++t)
+                b[t] = *reinterpret_cast<const float2*>(Bs + (c0 + 8 * t + g) * ld + 8 * s + 2 * j);
+            product3<4>(acc, a, b);
         }
-        const float aa = wt.alpha[ra], ab = wt.alpha[rb];
+        const RowTerms ta = pol.row_terms(rec + ra * Pol::RECORDS, before), tb = pol.row_terms(rec + rb * Pol::RECORDS, before);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            acc[t][0] *= aa;
-            acc[t][1] *= aa;
-            acc[t][2] *= ab;
-            acc[t][3] *= ab;
+        for (int t = 0; t < 4; ++t) {
+            acc[t][0] *= ta.alpha;
+            acc[t][1] *= ta.alpha;
+            acc[t][2] *= tb.alpha;
+            acc[t][3] *= tb.alpha;
         }
-        const float eah = wt.e_hi[ra], eal = wt.e_lo[ra], ebh = wt.e_hi[rb], ebl = wt.e_lo[rb];
         float sum_a = 0.0f, sum_b = 0.0f;
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
@@ -307,50 +320,51 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(Pol pol, Step st, int it
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const int s = 8 * t + 2 * j + i;
-                    const float gh = wt.g_hi[s], gl = wt.g_lo[s], w = wt.w[s];
-                    p[i] = s <= ra ? G[t][i] * (w * expf((gh + eah) + (gl + eal))) : 0.0f;
-                    p[2 + i] = s <= rb ? G[t][2 + i] * (w * expf((gh + ebh) + (gl + ebl))) : 0.0f;
+                    const float4 r = rec[s * Pol::RECORDS];
+                    const float gh = Pol::g_hi(r), gl = Pol::g_lo(r), w = Pol::weight(r);
+                    p[i] = s <= ra ? G[t][i] * (w * expf((gh + ta.e_hi) + (gl + ta.e_lo))) : 0.0f;
+                    p[2 + i] = s <= rb ? G[t][2 + i] * (w * expf((gh + tb.e_hi) + (gl + tb.e_lo))) : 0.0f;
                 }
                 if (Pol::NORMALISER) {
                     sum_a += p[0] + p[1];
                     sum_b += p[2] + p[3];
                 }
                 const Left a = left_of(p);
-                const float* v = Vs + (8 * t + 2 * j) * VLD + g;
-                float2 b[8];
+                const float* v = Vs + (8 * t + 2 * j) * VLD + c0 + g;
+                float2 b[4];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) b[c] = make_float2(v[8 * c], v[VLD + 8 * c]);
-                product3<8>(acc, a, b);
+                for (int c = 0; c < 4; ++c) b[c] = make_float2(v[8 * c], v[VLD + 8 * c]);
+                product3<4>(acc, a, b);
             }
         }
         if constexpr (Pol::NORMALISER) {
-            if (p0 == 0) {
+            if (p0 == 0 && c0 == 0) {
                 float qa_n = 0.0f, qb_n = 0.0f;
                 for (int n = j; n < pol.N; n += 4) {
                     qa_n = fmaf(Qs[ra * ld + n], nv[n], qa_n);
                     qb_n = fmaf(Qs[rb * ld + n], nv[n], qb_n);
                 }
-                sum_a = fmaf(aa, qa_n, sum_a);
-                sum_b = fmaf(ab, qb_n, sum_b);
+                sum_a = fmaf(ta.alpha, qa_n, sum_a);
+                sum_b = fmaf(tb.alpha, qb_n, sum_b);
 #pragma unroll
                 for (int o = 1; o < 4; o <<= 1) {
                     sum_a += __shfl_xor_sync(0xffffffffu, sum_a, o);
                     sum_b += __shfl_xor_sync(0xffffffffu, sum_b, o);
                 }
                 if (j == 0) {
-                    if (ra < ch.n) pol.store_sum(ch.first + ra, h, sum_a, wt.extra[ra]);
-                    if (rb < ch.n) pol.store_sum(ch.first + rb, h, sum_b, wt.extra[rb]);
+                    if (ra < ch.n) pol.store_sum(ch.first + ra, h, sum_a, ta.extra);
+                    if (rb < ch.n) pol.store_sum(ch.first + rb, h, sum_b, tb.extra);
                 }
             }
         }
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int p = p0 + 8 * t + 2 * j;
+        for (int t = 0; t < 4; ++t) {
+            const int c = c0 + 8 * t + 2 * j, p = p0 + c;
             if (p < pol.P) {
-                const float* va = Vs + ra * VLD + 8 * t + 2 * j;
-                const float* vb = Vs + rb * VLD + 8 * t + 2 * j;
-                if (ra < ch.n) pol.store_row(ch.first + ra, h, p, acc[t][0], acc[t][1], va[0], va[1]);
-                if (rb < ch.n) pol.store_row(ch.first + rb, h, p, acc[t][2], acc[t][3], vb[0], vb[1]);
+                const float2 va = *reinterpret_cast<const float2*>(Vs + ra * VLD + c);
+                const float2 vb = *reinterpret_cast<const float2*>(Vs + rb * VLD + c);
+                if (ra < ch.n) pol.store_row(ch.first + ra, h, p, acc[t][0], acc[t][1], va.x, va.y);
+                if (rb < ch.n) pol.store_row(ch.first + rb, h, p, acc[t][2], acc[t][3], vb.x, vb.y);
             }
         }
     }
@@ -362,9 +376,9 @@ inline long long places(int R, int n_seq, int seg_rows, int n_segs) {
 
 // Floats of scratch a step needs: the memories of all its chunks, up to about `budget` floats;
 // beyond that the rows go through in rounds of `*seg_rows` rows a sequence.
-inline long long scratch_floats(int R, int n_seq, int max_rows, int heads, long long E, int* seg_rows) {
+inline long long scratch_floats(int R, int n_seq, int max_rows, int heads, long long E, int records, int* seg_rows) {
     const long long budget = 64LL << 20;  // 256 MB
-    const long long one = heads * (E + 8);
+    const long long one = heads * (E + 8 + 4 * L * records);
     const int whole = (max_rows + L - 1) / L * L;
     int seg = whole;
     if ((long long)(R / L + n_seq) * one > budget) {
@@ -381,7 +395,7 @@ int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int
         cudaStream_t s) {
     const long long E = (long long)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
     int seg_rows = 0;
-    scratch_floats(R, n_seq, max_rows, pol.heads, E, &seg_rows);
+    scratch_floats(R, n_seq, max_rows, pol.heads, E, Pol::RECORDS, &seg_rows);
     Step st;
     st.seq_slot = seq_slot;
     st.seq_row0 = seq_row0;
@@ -390,15 +404,25 @@ int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int
     const long long n_places = places(R, n_seq, seg_rows, st.n_segs);
     st.scratch = scratch;
     st.aux = reinterpret_cast<float4*>(scratch + n_places * pol.heads * E);  // E is a multiple of four
-    st.before = scratch + n_places * pol.heads * (E + 4);
+    st.rows = st.aux + n_places * pol.heads;
+    st.before = reinterpret_cast<float*>(st.rows + n_places * pol.heads * L * Pol::RECORDS);
     const int N8 = (pol.N + 7) / 8 * 8, ptiles = (pol.P + PT - 1) / PT;
     const int chunks = (min(seg_rows, max_rows) + L - 1) / L;
     const size_t sm_state = (size_t)L * (VLD + N8 + 4) * sizeof(float);
     const size_t sm_out = (size_t)L * (VLD + 2 * (N8 + 8)) * sizeof(float);
     const int qk_heads = pol.heads / pol.per, items = pol.per * ptiles;
-    // as many items a block as leave two blocks an SM: the rows' products with k serve them all
+    // items a block: the rows' products with k, which serve them all, cost about as much as one item; two
+    // blocks share an SM
     int ipb = items;
-    while (ipb > 1 && (long long)chunks * n_seq * qk_heads * ((items + ipb - 1) / ipb) < 2LL * sm_count()) ipb = (ipb + 1) / 2;
+    long long least = -1;
+    for (int i = items; i >= 1; --i) {
+        const long long blocks = (long long)chunks * n_seq * qk_heads * ((items + i - 1) / i);
+        const long long cost = (blocks + 2 * sm_count() - 1) / (2 * sm_count()) * (1 + i);
+        if (least < 0 || cost < least) {
+            least = cost;
+            ipb = i;
+        }
+    }
     const int sets = (items + ipb - 1) / ipb;
     if (n_seq > 65535 || (long long)pol.heads * ptiles > 65535 || (long long)qk_heads * sets > 65535)
         return RFX_ERR_UNSUPPORTED;
@@ -409,7 +433,7 @@ int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int
     for (st.seg = 0; st.seg < st.n_segs; ++st.seg) {
         RFX_LAUNCH(chunk_state_kernel<Pol>, dim3(chunks, n_seq, pol.heads * ptiles), 256, sm_state, s, pol, st);
         RFX_LAUNCH(chunk_carry_kernel<Pol>, dim3((unsigned)((E / 4 + 127) / 128), n_seq, pol.heads), 128, 0, s, pol, st);
-        RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, n_seq, qk_heads * sets), 128, sm_out, s, pol, st, ipb);
+        RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, n_seq, qk_heads * sets), 256, sm_out, s, pol, st, ipb);
     }
     return 0;
 }

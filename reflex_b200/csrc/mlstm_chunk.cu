@@ -12,6 +12,7 @@ namespace {
 
 struct Mlstm {
     static constexpr bool NORMALISER = true;
+    static constexpr int RECORDS = 2;  // g and its running maximum, F, each in two parts
     const float *proj, *bias_i, *bias_f;
     float cap, q_scale;
     float *state, *num, *den;
@@ -41,33 +42,38 @@ struct Mlstm {
         gg[0] = (double)gi[0] - F[0];
         gg[1] = (double)gi[1] - F[1];
     }
-    __device__ __forceinline__ float4 state_weights(float* wl, int h, int first, int n, int lane) const {
+    __device__ __forceinline__ float4 state_weights(float* wl, float4* rows, int h, int first, int n, int lane) const {
         double F[2], gg[2];
         gates(h, first, n, lane, F, gg);
-        double ma = gg[0], mb = gg[1];
-        chunk::scan_max(ma, mb, lane);
-        const double G = __shfl_sync(0xffffffffu, mb, 31), all = __shfl_sync(0xffffffffu, F[1], 31);
-        wl[lane] = expf((float)(gg[0] - G));
-        wl[lane + 32] = expf((float)(gg[1] - G));
+        double M[2] = {gg[0], gg[1]};
+        chunk::scan_max(M[0], M[1], lane);
+        const double G = __shfl_sync(0xffffffffu, M[1], 31), all = __shfl_sync(0xffffffffu, F[1], 31);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = lane + 32 * i;
+            wl[r] = expf((float)(gg[i] - G));
+            if (rows) {
+                float4 a, b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                chunk::two_parts(gg[i], &a.x, &a.y);
+                chunk::two_parts(M[i], &a.z, &a.w);
+                chunk::two_parts(F[i], &b.x, &b.y);
+                rows[2 * r] = a;
+                rows[2 * r + 1] = b;
+            }
+        }
         float4 a;
         chunk::two_parts(all, &a.x, &a.y);
         chunk::two_parts(G, &a.z, &a.w);
         return a;
     }
-    __device__ __forceinline__ void row_weights(chunk::Weights& w, int h, int first, int n, float m_prev, int lane) const {
-        double F[2], gg[2];
-        gates(h, first, n, lane, F, gg);
-        double M[2] = {fmax(gg[0], (double)m_prev), fmax(gg[1], (double)m_prev)};
-        chunk::scan_max(M[0], M[1], lane);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = lane + 32 * i;
-            chunk::two_parts(gg[i], &w.g_hi[r], &w.g_lo[r]);
-            chunk::two_parts(-M[i], &w.e_hi[r], &w.e_lo[r]);
-            w.w[r] = 1.0f;
-            w.alpha[r] = expf((float)((double)m_prev - M[i]));
-            w.extra[r] = expf((float)(-(F[i] + M[i])));  // e^(-m_t)
-        }
+    static __device__ __forceinline__ float g_hi(const float4& r) { return r.x; }
+    static __device__ __forceinline__ float g_lo(const float4& r) { return r.y; }
+    static __device__ __forceinline__ float weight(const float4&) { return 1.0f; }
+    // M_t = max(m_prev, the rows' maximum so far)
+    __device__ __forceinline__ chunk::RowTerms row_terms(const float4* r, float m_prev) const {
+        const bool prev = m_prev > r->z || (m_prev == r->z && r->w < 0.0f);
+        const float hi = prev ? m_prev : r->z, lo = prev ? 0.0f : r->w;
+        return {-hi, -lo, expf((m_prev - hi) - lo), expf(-((r[1].x + hi) + (r[1].y + lo)))};
     }
     __device__ __forceinline__ float* head_state(int slot, int h) const {
         return state + ((size_t)slot * heads + h) * ((size_t)N * P + N + (P + 63) / 64);
@@ -112,7 +118,7 @@ struct Mlstm {
 // Floats of scratch rfx_mlstm_chunks needs for a step of R rows in S sequences of at most max_rows.
 extern "C" long long rfx_mlstm_chunks_floats(int R, int S, int max_rows, int heads, int dim, int vdim) {
     int seg = 0;
-    return chunk::scratch_floats(R, S, max_rows, heads, (long long)vdim * dim + dim, &seg);
+    return chunk::scratch_floats(R, S, max_rows, heads, (long long)vdim * dim + dim, Mlstm::RECORDS, &seg);
 }
 
 // As rfx_mlstm_scan.  dim in fours up to 128, vdim in fours; rows, results and `scratch` on 16 bytes.

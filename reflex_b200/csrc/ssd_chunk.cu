@@ -11,6 +11,7 @@ namespace {
 
 struct Ssd {
     static constexpr bool NORMALISER = false;
+    static constexpr int RECORDS = 1;  // running logarithm in two parts, step size, its exponential
     const float *xbc, *proj, *dt_bias, *A, *D;
     float *state, *out;
     long long state_stride, state_off;
@@ -40,28 +41,27 @@ struct Ssd {
         cb = (double)A[h] * db;
         chunk::scan_sum(ca, cb, lane);
     }
-    __device__ __forceinline__ float4 state_weights(float* wl, int h, int first, int n, int lane) const {
-        float da, db;
-        double ca, cb;
-        logs(h, first, n, lane, da, db, ca, cb);
-        const double all = __shfl_sync(0xffffffffu, cb, 31);
-        wl[lane] = da * expf((float)(all - ca));
-        wl[lane + 32] = db * expf((float)(all - cb));
-        return make_float4(expf((float)all), 0.0f, 0.0f, 0.0f);
-    }
-    __device__ __forceinline__ void row_weights(chunk::Weights& w, int h, int first, int n, float, int lane) const {
+    __device__ __forceinline__ float4 state_weights(float* wl, float4* rows, int h, int first, int n, int lane) const {
         float d[2];
         double c[2];
         logs(h, first, n, lane, d[0], d[1], c[0], c[1]);
+        const double all = __shfl_sync(0xffffffffu, c[1], 31);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = lane + 32 * i;
-            chunk::two_parts(c[i], &w.e_hi[r], &w.e_lo[r]);
-            chunk::two_parts(-c[i], &w.g_hi[r], &w.g_lo[r]);
-            w.w[r] = d[i];
-            w.alpha[r] = expf((float)c[i]);
+            wl[r] = d[i] * expf((float)(all - c[i]));
+            if (rows) {
+                float hi, lo;
+                chunk::two_parts(c[i], &hi, &lo);
+                rows[r] = make_float4(hi, lo, d[i], expf(hi));
+            }
         }
+        return make_float4(expf((float)all), 0.0f, 0.0f, 0.0f);
     }
+    static __device__ __forceinline__ float g_hi(const float4& r) { return -r.x; }
+    static __device__ __forceinline__ float g_lo(const float4& r) { return -r.y; }
+    static __device__ __forceinline__ float weight(const float4& r) { return r.z; }
+    __device__ __forceinline__ chunk::RowTerms row_terms(const float4* r, float) const { return {r->x, r->y, r->w, 0.0f}; }
     __device__ __forceinline__ float* memory(int slot, int h, int e) const {
         return state + (size_t)slot * state_stride + state_off + (size_t)h * P * N + e;
     }
@@ -86,7 +86,7 @@ struct Ssd {
 // Floats of scratch rfx_ssd_chunk needs for a step of R rows in n_seq sequences of at most max_rows.
 extern "C" long long rfx_ssd_chunk_floats(int R, int n_seq, int max_rows, int heads, int P, int N) {
     int seg = 0;
-    return chunk::scratch_floats(R, n_seq, max_rows, heads, (long long)P * N, &seg);
+    return chunk::scratch_floats(R, n_seq, max_rows, heads, (long long)P * N, Ssd::RECORDS, &seg);
 }
 
 // As rfx_ssd_scan with 32-bit results, the state [heads][P][N].  P and N in fours, N up to 128; rows and
