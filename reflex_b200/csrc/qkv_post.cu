@@ -94,15 +94,18 @@ qkv_post_wide_kernel(const TI* __restrict__ qkv, int row_stride, const float* __
                      const float* __restrict__ rope_denom, int rotary_dim,
                      const int* __restrict__ row_pos, const int* __restrict__ row_slot,
                      TO* __restrict__ q_out, TO* __restrict__ k_pages, TO* __restrict__ v_pages,
-                     PagedKV cache, int nq, int nkv_in, int dry_pass, float magnitude, int v_head0) {
-    extern __shared__ float smem[];  // cos[half], sin[half]
+                     PagedKV cache, int nq, int nkv_in, int dry_pass, float magnitude, int v_head0, int rows, int R) {
+    extern __shared__ float smem[];  // [rows] cos[half], sin[half]
     pdl_launch_dependents();
     constexpr int D = PER * LPH;
     constexpr int HPW = 32 / LPH;  // heads a warp takes at a time
     constexpr int CH = 3;          // units whose loads are in flight together
     constexpr float inv_d = 1.0f / (float)D;
-    const int r = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    // a block has `rows` rows (1, 2, 4 or 8), a row `nwarps` of its warps
+    const int nwarps = (blockDim.x >> 5) / rows, all_warps = threadIdx.x >> 5;
+    const int warp = all_warps % nwarps, lane = threadIdx.x & 31;
+    const int r_first = blockIdx.x * rows, r_in = all_warps / nwarps;
+    const int r = min(r_first + r_in, R - 1);  // (behind the last row: its warps do nothing but meet the others)
     const int half = rotary_dim / 2;
     const bool rotate = rope_denom != nullptr && half > 0;
     const int sub = lane / LPH;          // which of the unit's heads
@@ -113,7 +116,7 @@ qkv_post_wide_kernel(const TI* __restrict__ qkv, int row_stride, const float* __
     const int partner = turns ? (low ? lane + hl : lane - hl) : lane;
     // units: the query heads in groups of HPW, then the key heads, then the value heads
     const int uq = (nq + HPW - 1) / HPW, ukv = (nkv_in + HPW - 1) / HPW;
-    const int units = uq + 2 * ukv;
+    const int units = r_first + r_in < R ? uq + 2 * ukv : 0;
     const int stride = gridDim.y * nwarps;
     const int first = blockIdx.y * nwarps + warp;
 
@@ -128,10 +131,10 @@ qkv_post_wide_kernel(const TI* __restrict__ qkv, int row_stride, const float* __
     auto prepare = [&]() {
         const int pos = row_pos[r];
         const int slot = row_slot[r];
-        float* cs_tab = smem;
+        float* cs_tab = smem + r_in * rotary_dim;
         float* sn_tab = cs_tab + half;
         if (rotate) {
-            for (int i = threadIdx.x; i < half; i += blockDim.x) {
+            for (int i = warp * 32 + lane; i < half; i += nwarps * 32) {
                 const float theta = (float)pos / rope_denom[i];
                 float sv, cv;
                 row_sincos<TO>(theta, &sv, &cv);
@@ -433,10 +436,16 @@ extern "C" int rfx_qkv_post_kv(const void* qkv, int in_dt, int row_stride, const
         const int hpw = 32 / lph;
         const int units = (nq + hpw - 1) / hpw + 2 * ((nkv_in + hpw - 1) / hpw);
         const int unit_blocks = many ? 1 : (units + warps - 1) / warps;
-        dim3 grid(R, unit_blocks < 65535 ? unit_blocks : 65535);
-        const size_t smem = (size_t)rotary_dim * sizeof(float);
+        // Several rows a block where that leaves two blocks an SM: one row's tables and first loads are
+        // little to wait for with a whole block (4,000 rows of 24 heads of 128: 32.9 us with a row a
+        // block, 26.6 with two, 24.6 with four; 700 rows of 48 heads 14.3, 14.3 and 18.5).
+        int rows = 1;
+        while (many && rows < 4 && R / (2 * rows) >= 2 * sm_count()) rows *= 2;
+        dim3 grid((R + rows - 1) / rows, unit_blocks < 65535 ? unit_blocks : 65535);
+        const size_t smem = (size_t)rows * rotary_dim * sizeof(float);
 #define RFX_WIDE(TI, TO, P, L)                                                                    \
-    RFX_LAUNCH((qkv_post_wide_kernel<TI, TO, P, L>), grid, threads, smem, s, RFX_POST_ARGS(TI, TO), magnitude, v_head0)
+    RFX_LAUNCH((qkv_post_wide_kernel<TI, TO, P, L>), grid, threads, smem, s, RFX_POST_ARGS(TI, TO), magnitude, v_head0, \
+               rows, R)
 #define RFX_WIDE_32(TI, TO)  /* 32-bit input: 4 elements are 16 bytes */   \
     do {                                                                  \
         if (per == 4 && lph == 4) RFX_WIDE(TI, TO, 4, 4);                 \
