@@ -35,71 +35,104 @@ using rfx::product3;
 // (a sequence of n rows has ceil(n / 16), so no two places meet; at most R / 16 + sequences).
 __device__ __forceinline__ size_t chunk_place(int row0, int seq, int c) { return (size_t)row0 / CH + seq + c; }
 
-// A block a (chunk, query/key head): the products between the chunk's rows once, then per value
-// head of the group T, M and the decays' products.
+// A block a (chunk, query/key head): the products between the chunk's rows once, on the tensor cores, each
+// warp some of the channels; then per value head of the group (eight at a time) T, M and the decays'
+// products.  Bound by the steps' latencies with six blocks an SM.  (A thread a pair of rows instead, three
+// 16-byte reads of shared memory for eight multiply-adds, was bound by those reads: 66 us for 4,096 rows of
+// 16 heads of 128 with two value heads each; 51 with this.)
+constexpr int PREP_WARPS = CH * CH / 32, PREP_HEADS = 8;
 __global__ void __launch_bounds__(CH * CH)
 gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __restrict__ gates,
                               const int* __restrict__ seq_row0, float* __restrict__ coef, int H, int G, int d, int dv) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ float L[CH][CH + 1], gs[CH], bs[CH];
+    __shared__ float L[PREP_HEADS][CH][CH + 1], gs[PREP_HEADS][CH], bs[PREP_HEADS][CH];
     rfx::pdl_prologue();
     const int seq = blockIdx.y, kvh = blockIdx.z;
     const int row0 = seq_row0[seq], row1 = seq_row0[seq + 1];
     const int first = row0 + blockIdx.x * CH, n = min(CH, row1 - first);
     if (n <= 0) return;
-    const int C = 2 * G * d + H * dv, LD = d + 4, d4 = d / 4;
+    const int C = 2 * G * d + H * dv, d8 = (d + 7) / 8 * 8, LD = d8 + 8, c4 = d8 / 4;
     float *ks = sm, *qs = sm + CH * LD;
+    float4* part = reinterpret_cast<float4*>(sm + 2 * CH * LD);  // [warp][tile][lane]
     const int tid = threadIdx.x, i = tid / CH, j = tid % CH;
-    for (int e = tid; e < CH * d4; e += CH * CH) {
-        const int r = e / d4, c = 4 * (e - r * d4);
-        float4 k = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q = k;
-        if (r < n) {
-            const float* src = qkv + (size_t)(first + r) * C + kvh * d + c;
-            q = *reinterpret_cast<const float4*>(src);
-            k = *reinterpret_cast<const float4*>(src + G * d);
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    for (int r = warp; r < CH; r += PREP_WARPS) {  // rows and channels that are not there as zeros
+        const float* src = qkv + (size_t)(first + r) * C + kvh * d;
+        for (int c = lane; c < c4; c += 32) {
+            const bool ok = r < n && 4 * c < d;
+            attn::cp_async_16(qs + r * LD + 4 * c, ok ? src + 4 * c : qkv, ok);
+            attn::cp_async_16(ks + r * LD + 4 * c, ok ? src + G * d + 4 * c : qkv, ok);
         }
-        *reinterpret_cast<float4*>(ks + r * LD + c) = k;
-        *reinterpret_cast<float4*>(qs + r * LD + c) = q;
+    }
+    attn::cp_async_commit();
+    const int per = H / G;
+    auto load_gates = [&](int h0) {
+        for (int e = tid; e < min(PREP_HEADS, per - h0) * CH; e += CH * CH) {
+            const int hh = e / CH, r = e % CH, h = kvh * per + h0 + hh;
+            gs[hh][r] = r < n ? gates[(size_t)(first + r) * 2 * H + h] : 1.0f;
+            bs[hh][r] = r < n ? gates[(size_t)(first + r) * 2 * H + H + h] : 0.0f;
+        }
+    };
+    load_gates(0);
+    attn::cp_async_wait<0>();
+    __syncthreads();
+    float A[2][4] = {}, B[2][4] = {};  // k k^T and q k^T, columns 0..7 and 8..15
+    for (int s = warp; s < d8 / 8; s += PREP_WARPS) {
+        const float *kr = ks + g * LD + 8 * s + 2 * t4, *qr = qs + g * LD + 8 * s + 2 * t4;
+        const float2 b[2] = {*reinterpret_cast<const float2*>(kr), *reinterpret_cast<const float2*>(kr + 8 * LD)};
+        const float2 q0 = *reinterpret_cast<const float2*>(qr), q1 = *reinterpret_cast<const float2*>(qr + 8 * LD);
+        product3<2>(A, rfx::left_from(b[0].x, b[1].x, b[0].y, b[1].y), b);
+        product3<2>(B, rfx::left_from(q0.x, q1.x, q0.y, q1.y), b);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        part[(warp * 4 + t) * 32 + lane] = make_float4(A[t][0], A[t][1], A[t][2], A[t][3]);
+        part[(warp * 4 + 2 + t) * 32 + lane] = make_float4(B[t][0], B[t][1], B[t][2], B[t][3]);
     }
     __syncthreads();
     float kk = 0.0f, qk = 0.0f;
-    for (int c = 0; c < d; c += 4) {
-        const float4 kj = *reinterpret_cast<const float4*>(ks + j * LD + c);
-        const float4 ki = *reinterpret_cast<const float4*>(ks + i * LD + c);
-        const float4 qi = *reinterpret_cast<const float4*>(qs + i * LD + c);
-        kk = fmaf(ki.x, kj.x, fmaf(ki.y, kj.y, fmaf(ki.z, kj.z, fmaf(ki.w, kj.w, kk))));
-        qk = fmaf(qi.x, kj.x, fmaf(qi.y, kj.y, fmaf(qi.z, kj.z, fmaf(qi.w, kj.w, qk))));
+    {
+        const float* p = reinterpret_cast<const float*>(part) +
+                         4 * ((j / 8) * 32 + (i % 8) * 4 + (j % 8) / 2) + (i / 8) * 2 + (j & 1);
+#pragma unroll
+        for (int w = 0; w < PREP_WARPS; ++w) {
+            kk += p[w * 4 * 128];
+            qk += p[(w * 4 + 2) * 128];
+        }
     }
-    for (int h = kvh * (H / G); h < (kvh + 1) * (H / G); ++h) {
-        __syncthreads();  // L, gs and bs of the head before have been read
-        if (tid < CH) {
-            gs[tid] = tid < n ? gates[(size_t)(first + tid) * 2 * H + h] : 1.0f;
-            bs[tid] = tid < n ? gates[(size_t)(first + tid) * 2 * H + H + h] : 0.0f;
+    for (int h0 = 0; h0 < per; h0 += PREP_HEADS) {
+        const int heads = min(PREP_HEADS, per - h0);
+        if (h0) {
+            __syncthreads();  // L, gs and bs of the heads before have been read
+            load_gates(h0);
+            __syncthreads();
+        }
+        float* out = coef + (chunk_place(row0, seq, blockIdx.x) * H + kvh * per + h0) * COEF;
+        for (int hh = 0; hh < heads; ++hh) {
+            float r = 1.0f;
+            for (int l = j + 1; l <= i; ++l) r *= gs[hh][l];
+            L[hh][i][j] = j < i ? bs[hh][i] * (r * kk) : 0.0f;
+            float* o = out + (size_t)hh * COEF;
+            o[CH * TLD + i * TLD + j] = j <= i ? r * qk : 0.0f;
+            if (i == hh) {
+                float c = gs[hh][0], last = 1.0f;
+                for (int l = 1; l <= j; ++l) c *= gs[hh][l];
+                for (int l = j + 1; l < CH; ++l) last *= gs[hh][l];
+                o[2 * CH * TLD + j] = c;
+                o[2 * CH * TLD + CH + j] = last;
+                if (j == CH - 1) o[2 * CH * TLD + 2 * CH] = c;
+            }
         }
         __syncthreads();
-        float* out = coef + (chunk_place(row0, seq, blockIdx.x) * H + h) * COEF;
-        float r = 1.0f;
-        for (int l = j + 1; l <= i; ++l) r *= gs[l];
-        L[i][j] = j < i ? bs[i] * (r * kk) : 0.0f;
-        out[CH * TLD + i * TLD + j] = j <= i ? r * qk : 0.0f;
-        if (i == 0) {
-            float c = gs[0], last = 1.0f;
-            for (int l = 1; l <= j; ++l) c *= gs[l];
-            for (int l = j + 1; l < CH; ++l) last *= gs[l];
-            out[2 * CH * TLD + j] = c;
-            out[2 * CH * TLD + CH + j] = last;
-            if (j == CH - 1) out[2 * CH * TLD + 2 * CH] = c;
-        }
-        __syncthreads();
-        if (tid < CH) {  // column `tid` of T, row by row
+        if (warp < heads && lane < CH) {  // a warp a head: column `lane` of T, row by row
             float t[CH];
 #pragma unroll
             for (int a = 0; a < CH; ++a) {
-                float s = a == tid ? bs[a] : 0.0f;
+                float s = a == lane ? bs[warp][a] : 0.0f;
 #pragma unroll
-                for (int l = 0; l < a; ++l) s = fmaf(-L[a][l], t[l], s);
+                for (int l = 0; l < a; ++l) s = fmaf(-L[warp][a][l], t[l], s);
                 t[a] = s;
-                out[a * TLD + tid] = s;
+                out[(size_t)warp * COEF + a * TLD + lane] = s;
             }
         }
     }
@@ -384,9 +417,13 @@ extern "C" int rfx_gated_delta_chunk_prep(const float* qkv, const float* gates, 
                                           float* coef, int H, int G, int d, int dv, int max_rows, void* stream) {
     if (n_seq <= 0 || max_rows <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0) return RFX_ERR_BAD_ARG;
-    const size_t smem = (size_t)2 * CH * (d + 4) * sizeof(float);
-    if (d % 4 || dv % 4 || smem > 48 * 1024 || n_seq > 65535 || G > 65535) return RFX_ERR_UNSUPPORTED;
+    const size_t smem = (size_t)2 * CH * ((d + 7) / 8 * 8 + 8) * sizeof(float) + PREP_WARPS * 4 * 32 * sizeof(float4);
+    if (d % 4 || dv % 4 || (size_t)2 * CH * (d + 4) * sizeof(float) > 48 * 1024 || n_seq > 65535 || G > 65535) return RFX_ERR_UNSUPPORTED;
     dim3 grid((max_rows + CH - 1) / CH, n_seq, G);
+    if (smem + 12 * 1024 > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(gated_delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
     RFX_LAUNCH(gated_delta_chunk_prep_kernel, grid, CH * CH, smem, (cudaStream_t)stream, qkv, gates, seq_row0, coef, H,
                G, d, dv);
     return 0;
