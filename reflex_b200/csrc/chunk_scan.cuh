@@ -5,7 +5,9 @@
 //   chunk_state_kernel   what each chunk adds to the memory, from zero: sum_s W_s k_s v_s^T
 //   chunk_carry_kernel   the memory before each chunk, chunk after chunk, element by element; the
 //                        running state's start and end
-//   chunk_out_kernel     a chunk's rows: alpha_t (q_t . S) + sum_{s<=t} w_ts (q_t . k_s) v_s
+//   chunk_out_kernel     a chunk's rows: alpha_t (q_t . S) + sum_{s<=t} w_ts (q_t . k_s) v_s; the policy's
+//                        running number after a sequence's last chunk (every block of the carry reads the
+//                        number before the first one, and nothing orders those blocks)
 //
 // W, alpha and w come from the policy (which recurrence): products of decays as exponentials of
 // differences of their running logarithms.  Those are summed in 64 bits from the chunk's first row
@@ -58,13 +60,14 @@ __device__ __forceinline__ size_t place_of(const Step& s, int row0, int seq, int
 
 struct Rows {
     int first, n;  // the chunk's first row and how many it has
+    bool last;     // of its sequence's in this segment
     size_t place;
 };
 __device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
     const int row0 = s.seq_row0[seq], from = row0 + s.seg * s.seg_rows;
     const int to = min(s.seq_row0[seq + 1], from + s.seg_rows);
     const int first = from + c * L;
-    return {first, min(L, to - first), place_of(s, row0, seq, c)};
+    return {first, min(L, to - first), to - first <= L, place_of(s, row0, seq, c)};
 }
 
 // A tile of `rows` rows of 4 * c4 floats, rows from n on and columns from n4 (in fours) on zero.
@@ -187,9 +190,6 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(Pol pol, Step st) {
             }
     }
     pol.store_state(slot, h, e, S);
-    if constexpr (Pol::NORMALISER) {
-        if (e == 0) pol.store_number(slot, h, m);
-    }
 }
 
 // Inclusive sums (or maxima) over the chunk's 64 rows, lane i holding rows i and i + 32.
@@ -291,6 +291,13 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(Pol pol, Step st, int
         }
         attn::cp_async_commit();
         const float before = st.before[at];
+        if constexpr (Pol::NORMALISER) {
+            if (ch.last && p0 == 0 && threadIdx.x == 0) {
+                float m = before;
+                pol.carry(st.aux[at], m);
+                pol.store_number(st.seq_slot[seq], h, m);
+            }
+        }
         attn::cp_async_wait<0>();
         __syncthreads();
         float acc[4][4] = {};

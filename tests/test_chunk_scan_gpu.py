@@ -99,30 +99,37 @@ def mlstm_rule(q, k, v, i, f, S, n, m):
     return np.stack(num), np.stack(den), S, n, m
 
 
-@pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 256), (3, 20, 12), (2, 64, 68), (4, 100, 130 - 2)])
-@pytest.mark.parametrize("counts", [(64,), (65, 1, 127), (193,)])
-def test_mlstm_in_chunks(heads, dim, vdim, counts):
+def mlstm_case(heads, dim, vdim, counts, slots, running, forget):
+    """A step's rows and states; the slots in `running` go on from earlier rows, the others start."""
     rng = np.random.default_rng(heads + dim + sum(counts))
-    R, cap = sum(counts), 12.0
-    q_off, k_off, v_off = 0, heads * dim, 2 * heads * dim
-    i_off = v_off + heads * vdim
+    R = sum(counts)
+    i_off = heads * (2 * dim + vdim)
     f_off = i_off + heads
     ld = f_off + heads + (-(f_off + heads)) % 4
     proj = rng.standard_normal((R, ld)).astype(np.float32)
     proj[:, i_off:f_off + heads] *= 4.0  # gates that swing
-    bi, bf = rng.standard_normal(heads).astype(np.float32), (rng.standard_normal(heads) + 2).astype(np.float32)
-    floats = ops().mlstm_state_floats(dim, vdim)
-    state = np.zeros((6, heads, floats), dtype=np.float32)
-    state[3, :, :dim * vdim + dim] = rng.standard_normal((heads, dim * vdim + dim))
-    state[3, :, dim * vdim + dim:] = rng.standard_normal(heads)[:, None]  # a sequence that goes on
-    slots = [3, 0, 5][:len(counts)]
-    dev = torch.from_numpy(state.copy()).to(DEV)
+    bi, bf = rng.standard_normal(heads).astype(np.float32), (rng.standard_normal(heads) + forget).astype(np.float32)
+    state = np.zeros((max(slots) + 1, heads, ops().mlstm_state_floats(dim, vdim)), dtype=np.float32)
+    for slot in running:
+        state[slot, :, :dim * vdim + dim] = rng.standard_normal((heads, dim * vdim + dim))
+        state[slot, :, dim * vdim + dim:] = rng.standard_normal(heads)[:, None]
+    return proj, (0, heads * dim, 2 * heads * dim, i_off, f_off), bi, bf, state, Batch(counts, slots)
+
+
+def mlstm_run(case, heads, dim, vdim, cap=12.0):
+    proj, offsets, bi, bf, state, b = case
     to = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
-    b = Batch(counts, slots)
-    num, den = ops().mlstm_scan(to(proj), (q_off, k_off, v_off, i_off, f_off), to(bi), to(bf), cap, 0.25, b, dev, heads,
-                                dim, vdim, max_rows=b.max_new, exact=False)
-    for j, (n, slot) in enumerate(zip(counts, slots)):
-        rows = slice(b.row0[j], b.row0[j + 1])
+    dev = torch.from_numpy(state.copy()).to(DEV)
+    num, den = ops().mlstm_scan(to(proj), offsets, to(bi), to(bf), cap, 0.25, b, dev, heads, dim, vdim,
+                                max_rows=b.max_new, exact=False)
+    return num, den, dev
+
+
+def mlstm_check(case, got, heads, dim, vdim, cap=12.0):
+    proj, (q_off, k_off, v_off, i_off, f_off), bi, bf, state, b = case
+    num, den, dev = got
+    for j, slot in enumerate(b.seq_slot.tolist()):
+        n, rows = b.row0[j + 1] - b.row0[j], slice(b.row0[j], b.row0[j + 1])
         p = proj[rows].astype(np.float64)
         cut = lambda o, w: p[:, o:o + heads * w].reshape(n, heads, w)  # noqa: E731
         i = cap * np.tanh((p[:, i_off:i_off + heads] + bi) / cap)
@@ -134,10 +141,29 @@ def test_mlstm_in_chunks(heads, dim, vdim, counts):
         assert off(num[rows], rn.reshape(n, -1)) < TOL
         assert off(den[rows], rd) < TOL
         new = dev[slot].double().cpu().numpy()
+        assert (new[:, dim * vdim + dim:] == new[:, -1:]).all()
         scale = np.exp(new[:, -1] - m)  # the memory is relative to the number beside it
         assert np.abs(new[:, -1] - m).max() < 1e-5 * (1 + np.abs(m).max())
         assert off(torch.from_numpy(new[:, :dim * vdim] * scale[:, None]), S.reshape(heads, -1)) < TOL
         assert off(torch.from_numpy(new[:, dim * vdim:dim * vdim + dim] * scale[:, None]), nn) < TOL
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 256), (3, 20, 12), (2, 64, 68), (4, 100, 130 - 2)])
+@pytest.mark.parametrize("counts", [(64,), (65, 1, 127), (193,)])
+def test_mlstm_in_chunks(heads, dim, vdim, counts):
+    case = mlstm_case(heads, dim, vdim, counts, [3, 0, 5][:len(counts)], [3], 2.0)
+    mlstm_check(case, mlstm_run(case, heads, dim, vdim), heads, dim, vdim)
+
+
+def test_mlstm_with_more_blocks_than_the_chip_holds():
+    """Heads that remember, running states, one long sequence before short ones: blocks of a head
+    start long after others of it have ended, and still read the number the sequence came with."""
+    heads, dim, vdim = 16, 128, 256
+    case = mlstm_case(heads, dim, vdim, (450, 1, 64, 3, 65, 1, 17, 130), [3, 0, 5, 1, 7, 2, 4, 6], range(8), 5.0)
+    first = mlstm_run(case, heads, dim, vdim)
+    mlstm_check(case, first, heads, dim, vdim)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(mlstm_run(case, heads, dim, vdim), first))
 
 
 def test_a_long_step_goes_through_a_bounded_scratch():
