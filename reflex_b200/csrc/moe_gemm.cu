@@ -4,9 +4,11 @@
 // As in gemm_tc.cu the weights are the M operand of tcgen05.mma (128 weight rows a CTA, streamed by
 // TMA into an mbarrier ring) and the expert's rows its N operand: they lie side by side (moe.cu places
 // the (row, choice) pairs expert by expert), so one TMA box of 16, 32 or 64 rows from the expert's
-// first one brings them, and the rows behind them are not stored.  A gated expert ([gate rows | up
-// rows]) gives a CTA 64 gate rows and the 64 up rows that belong to them; its epilogue writes the
-// activation of the pair, so the up product's 2 ff columns never go to memory.
+// first one brings them, and the rows behind them are not stored.  (An expert that a row names several
+// times can have more rows than the step: its CTAs go over the weights again for every further box.)
+// A gated expert ([gate rows | up rows]) gives a CTA 64 gate rows and the 64 up rows that belong to
+// them; its epilogue writes the activation of the pair, so the up product's 2 ff columns never go to
+// memory.
 //
 // Memory bounds it: a CTA's ring is filled with weights before the wait on the kernel before where
 // most experts have rows (the weights do not depend on the routing; an expert without rows then drops
@@ -52,7 +54,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     constexpr int B_BYTES = BN * BK * 2, STAGE = A_BYTES + B_BYTES;
     constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], done_bar;
+    __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], done_bar, read_bar;
     __shared__ uint32_t tmem_base;
     __shared__ float ups[GATED ? BN * (BM / 2) : 1];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -67,6 +69,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             mbar_init(&empty_bar[s], 1);
         }
         mbar_init(&done_bar, 1);
+        mbar_init(&read_bar, 4);
         fence_barrier_init();
         prefetch_tensormap(&map_w);
         prefetch_tensormap(&map_x);
@@ -93,19 +96,22 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             rfx::pdl_wait();
             const int first = offsets[e], rows = offsets[e + 1] - first;
             if (rows > 0) {
-                for (int i = 0; i < nkb; ++i) {
-                    const int s = i % stages;
-                    const uint32_t ph = (i / stages) & 1;
-                    if (i >= pre) {
-                        if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
-                            atomicExch(err, 51);
-                            break;
+                bool ok = true;
+                for (int r = 0, it = 0; r < rows && ok; r += BN)
+                    for (int i = 0; i < nkb; ++i, ++it) {
+                        const int s = it % stages;
+                        const uint32_t ph = (it / stages) & 1;
+                        if (it >= pre) {
+                            if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
+                                atomicExch(err, 51);
+                                ok = false;
+                                break;
+                            }
+                            load_w(i, s);
                         }
-                        load_w(i, s);
+                        mbar_expect_tx(&full_bar[s], B_BYTES);
+                        tma_load_2d(tiles + (size_t)s * STAGE + A_BYTES, &map_x, &full_bar[s], i * BK, first + r);
                     }
-                    mbar_expect_tx(&full_bar[s], B_BYTES);
-                    tma_load_2d(tiles + (size_t)s * STAGE + A_BYTES, &map_x, &full_bar[s], i * BK, first);
-                }
             } else {
                 // nothing to do: what was brought ahead has to land before the CTA leaves
                 for (int i = 0; i < pre; ++i) mbar_arrive(&full_bar[i]);
@@ -120,32 +126,39 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (rows > 0 && elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
             bool ok = true;
-            for (int i = 0; i < nkb && ok; ++i) {
-                const int s = i % stages;
-                if (!mbar_wait(&full_bar[s], (i / stages) & 1)) {
-                    atomicExch(err, 53);
-                    ok = false;
+            for (int box = 0, it = 0; box * BN < rows && ok; ++box) {
+                if (box && !mbar_wait(&read_bar, (box - 1) & 1)) {  // the sums of the box before have been read
+                    atomicExch(err, 55);
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t a = smem_u32(tiles + (size_t)s * STAGE);
-                const uint64_t da = umma_desc_k_sw128(a), db = umma_desc_k_sw128(a + A_BYTES);
+                for (int i = 0; i < nkb; ++i, ++it) {
+                    const int s = it % stages;
+                    if (!mbar_wait(&full_bar[s], (it / stages) & 1)) {
+                        atomicExch(err, 53);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t a = smem_u32(tiles + (size_t)s * STAGE);
+                    const uint64_t da = umma_desc_k_sw128(a), db = umma_desc_k_sw128(a + A_BYTES);
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&empty_bar[s]);
+                    for (int k = 0; k < BK / 16; ++k) umma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(&empty_bar[s]);
+                }
+                if (ok) umma_commit(&done_bar);
             }
-            if (ok) umma_commit(&done_bar);
         }
         __syncwarp();
     } else {
         rfx::pdl_wait();
         const int first = offsets[e], rows = offsets[e + 1] - first;
-        if (rows > 0) {
-            const int q = warp & 3, m = q * 32 + lane;  // this warp may read TMEM lanes [32 q, 32 q + 32)
-            const bool have = mbar_wait(&done_bar, 0);
+        const int q = warp & 3, m = q * 32 + lane;  // this warp may read TMEM lanes [32 q, 32 q + 32)
+        const uint32_t base = tmem + ((uint32_t)(q * 32) << 16);
+        for (int box = 0; box * BN < rows; ++box) {  // (all boxes, also after a wait that gave up: the warps meet below)
+            const bool have = mbar_wait(&done_bar, box & 1);
             if (!have && lane == 0) atomicExch(err, 54);
             tc_fence_after_sync();
-            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16);
             if constexpr (GATED) {
                 if (q >= 2) {
 #pragma unroll 1
@@ -159,23 +172,26 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
             if (!GATED || q < 2) {
-                const int n = n0 + m;
+                const int n = n0 + m, here = rows - box * BN;
 #pragma unroll 1
                 for (int c = 0; c < BN / 16; ++c) {
                     float v[16];
                     tmem_ld_16(base + c * 16, v);
-                    if (c * 16 >= rows) break;
+                    if (c * 16 >= here) break;
                     if (n < N && have) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             const int r = c * 16 + j;
                             const float u = GATED ? ups[r * (BM / 2) + m] : 0.0f;
-                            if (r < rows) rfx::st<TO>(y, (size_t)(first + r) * N + n, activation<ACT>(v[j], u, alpha, limit));
+                            if (r < here)
+                                rfx::st<TO>(y, (size_t)(first + box * BN + r) * N + n, activation<ACT>(v[j], u, alpha, limit));
                         }
                     }
                 }
             }
             tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&read_bar);
         }
     }
     __syncthreads();
@@ -222,7 +238,8 @@ int by_rows(int max_rows, const void* x, const void* W, const int* offsets, void
 
 // y[p, :] = act(x[p, :] W_e^T) for the rows p in [offsets[e], offsets[e + 1]) of every expert e: x bfloat16
 // [n_pairs, K], W bfloat16 [E, N, K] (gated activations: [E, 2 N, K], gate rows first), offsets int32
-// [E + 1] on the device, at most max_rows <= 64 rows an expert.  act 0 none (y float32), 1 relu^2, 2 silu,
+// [E + 1] on the device.  max_rows <= 64: the most rows an expert has as a rule (more are right, at the
+// price of reading its weights again).  act 0 none (y float32), 1 relu^2, 2 silu,
 // 3 the clamped gated form with alpha and limit, 4 silu(gate) * up (y bfloat16).  K in eights, x and W on
 // 16 bytes.
 extern "C" int rfx_moe_gemm(const void* x, const void* W, const int* offsets, void* y, int n_pairs, int max_rows, int E,

@@ -27,30 +27,54 @@ def act64(kind, g, u):
     return g * torch.sigmoid(1.5 * g) * (u + 1)
 
 
+def check(x, up, down, ids, wts, kind, by_input, placed):
+    R, ff, gated = x.shape[0], down.shape[2], kind in ("glu_clamped", "swiglu")
+    got = ops().moe_experts(x, up, down, ids, wts, activation=kind, weight_input=by_input, alpha=1.5, limit=0.7,
+                            placed=placed)
+    ref = torch.zeros(x.shape, dtype=torch.float64, device=DEV)
+    for r in range(R):
+        for k in range(ids.shape[1]):
+            e, w = int(ids[r, k]), wts[r, k].double()
+            row = (x[r].float() * wts[r, k]).bfloat16().double() if by_input else x[r].double()
+            h = up[e].double() @ row
+            y = down[e].double() @ act64(kind, h[:ff], h[ff:] if gated else None)
+            ref[r] += y if by_input else w * y
+    assert ((got - ref).norm() / ref.norm()).item() < 3e-3  # 2^-9 = 2e-3 an activation, uniform: 1.1e-3 rms
+
+
+def weights(g, E, width, ff, kind):
+    gated = kind in ("glu_clamped", "swiglu")
+    up = (torch.randn((E, ff * (2 if gated else 1), width), generator=g, device=DEV) * 0.1).bfloat16()
+    return up, (torch.randn((E, width, ff), generator=g, device=DEV) * 0.1).bfloat16()
+
+
 @pytest.mark.parametrize("kind", ["relu2", "silu", "glu_clamped", "swiglu"])
 @pytest.mark.parametrize("R,E,top,width,ff", [(2, 8, 1, 64, 8), (5, 3, 2, 40, 72), (16, 16, 4, 136, 200),
                                               (17, 4, 3, 264, 128), (33, 40, 2, 128, 64), (64, 2, 2, 512, 136)])
 def test_a_few_rows_through_their_experts(R, E, top, width, ff, kind):
     g = torch.Generator(device=DEV).manual_seed(R + E)
-    gated = kind in ("glu_clamped", "swiglu")
     x = torch.randn((R, width), generator=g, device=DEV).bfloat16()
-    up = (torch.randn((E, ff * (2 if gated else 1), width), generator=g, device=DEV) * 0.1).bfloat16()
-    down = (torch.randn((E, width, ff), generator=g, device=DEV) * 0.1).bfloat16()
+    up, down = weights(g, E, width, ff, kind)
     # the first expert is never chosen where there are others enough
     scores = torch.randn((R, E), generator=g, device=DEV)
     if E > top:
         scores[:, 0] = -100.0
     ids, wts, placed = ops().moe_route(scores, None, top, place=True)
     for by_input in (False, True):
-        got = ops().moe_experts(x, up, down, ids, wts, activation=kind, weight_input=by_input, alpha=1.5, limit=0.7,
-                                placed=placed)
-        ref = torch.zeros((R, width), dtype=torch.float64, device=DEV)
-        for r in range(R):
-            for k in range(top):
-                e, w = int(ids[r, k]), wts[r, k].double()
-                row = (x[r].float() * wts[r, k]).bfloat16().double() if by_input else x[r].double()
-                h = up[e].double() @ row
-                y = down[e].double() @ act64(kind, h[:ff], h[ff:] if gated else None)
-                ref[r] += y if by_input else w * y
-        assert ((got - ref).norm() / ref.norm()).item() < 3e-3  # 2^-9 = 2e-3 an activation, uniform: 1.1e-3 rms
+        check(x, up, down, ids, wts, kind, by_input, placed)
+    ops().check_device_errors(DEV)
+
+
+@pytest.mark.parametrize("kind", ["relu2", "swiglu"])
+@pytest.mark.parametrize("R,E,top,width,ff", [(9, 3, 4, 712, 200), (20, 2, 3, 136, 72), (40, 5, 3, 264, 136),
+                                              (64, 3, 4, 64, 520)])
+def test_rows_that_name_an_expert_several_times(R, E, top, width, ff, kind):
+    """Expert 1 has R top rows or nearly so: more than the boxes of 16, 32 or 64 that R alone would ask for."""
+    g = torch.Generator(device=DEV).manual_seed(R + E)
+    x = torch.randn((R, width), generator=g, device=DEV).bfloat16()
+    up, down = weights(g, E, width, ff, kind)
+    ids = torch.ones((R, top), dtype=torch.int32, device=DEV)
+    ids[R // 2, 0] = 0
+    wts = torch.rand((R, top), generator=g, device=DEV)
+    check(x, up, down, ids, wts, kind, False, None)
     ops().check_device_errors(DEV)
