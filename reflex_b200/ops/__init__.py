@@ -1027,8 +1027,8 @@ def moe_experts(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, ids: torc
     in_scale, out_wts = (wts, None) if weight_input else (None, wts)
     if moe_grouped(x):
         # captured steps too, as long as a grouped product that needs no wait for the host is there
-        if not torch.cuda.is_current_stream_capturing() or (width % 8 == 0 and ff % 8 == 0
-                                                            and (_GROUPED_MM[0] or R <= MOE_GEMM_MAX_ROWS)):
+        if (not torch.cuda.is_current_stream_capturing() or (_GROUPED_MM[0] and width % 8 == 0 and ff % 8 == 0)
+                or _moe_gemm_takes(x, up, down)):
             rows = moe_experts_grouped(x, up, down, ids, wts, activation, weight_input, alpha, limit, placed)
             return rows if leave_sum else rows.summed()
     act = _new((R * top, ff), x.dtype, x.device)
@@ -1054,6 +1054,13 @@ MOE_GROUPED_MIN_ROWS = _env_int("REFLEX_B200_MOE_GROUPED_MIN_ROWS", 2, 1, 1 << 3
 def moe_grouped(x: torch.Tensor) -> bool:
     """Whether `moe_experts` groups these rows expert by expert (where it can)."""
     return x.dtype == torch.bfloat16 and MOE_GROUPED and x.shape[0] >= MOE_GROUPED_MIN_ROWS
+
+
+def _moe_gemm_takes(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor) -> bool:
+    """Whether this library's product of a few rows (csrc/moe_gemm.cu) takes these experts."""
+    return (x.dtype == up.dtype == down.dtype == torch.bfloat16 and x.shape[0] <= MOE_GEMM_MAX_ROWS
+            and x.shape[1] % 8 == 0 and down.shape[2] % 8 == 0 and up.shape[0] <= 65535 and up.is_contiguous()
+            and down.is_contiguous() and (up.data_ptr() | down.data_ptr()) % 16 == 0)
 
 
 def moe_experts_grouped(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, ids: torch.Tensor,
@@ -1096,16 +1103,20 @@ def moe_experts_grouped(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, i
     xg = _new((n, width), x.dtype, x.device)
     native.check(lib.rfx_moe_gather(_chk(x, "x"), place.data_ptr(), _chk(in_scale, "wts", torch.float32),
                                     xg.data_ptr(), dt_code(x.dtype), n, top, width, _stream()), "moe_gather")
-    if R <= MOE_GEMM_MAX_ROWS and width % 8 == 0 and ff % 8 == 0 and (up.data_ptr() | down.data_ptr()) % 16 == 0:
+    if _moe_gemm_takes(x, up, down):
         # a few rows: this library's kernel streams each chosen expert's weights once
         act = _new((n, ff), x.dtype, x.device)
         yg = _new((n, width), torch.float32, x.device)
         err = device_error_word(x.device).data_ptr()
         code = {"relu2": 1, "silu": 2, "glu_clamped": 3, "swiglu": 4}[activation]
         for a, w, out, rows, cols, kind in ((xg, up, act, ff, width, code), (act, down, yg, width, ff, 0)):
-            native.check(lib.rfx_moe_gemm(a.data_ptr(), _chk(w, "experts", x.dtype), offsets.data_ptr(), out.data_ptr(), n,
-                                          R, E, rows, cols, kind, float(alpha), float(limit), err, _stream()), "moe_gemm")
-        return ExpertRows(yg, place, out_wts, R, top)
+            st = lib.rfx_moe_gemm(a.data_ptr(), _chk(w, "experts"), offsets.data_ptr(), out.data_ptr(), n, R, E, rows,
+                                  cols, kind, float(alpha), float(limit), err, _stream())
+            if st == native.ERR_UNSUPPORTED:
+                break
+            native.check(st, "moe_gemm")
+        else:
+            return ExpertRows(yg, place, out_wts, R, top)
     grouped = getattr(torch, "_grouped_mm", None) if _GROUPED_MM[0] else None
     if grouped is not None and width % 8 == 0 and ff % 8 == 0:
         # the library's grouped product reads the experts' offsets on the device: no wait for the host

@@ -78,3 +78,47 @@ def test_rows_that_name_an_expert_several_times(R, E, top, width, ff, kind):
     wts = torch.rand((R, top), generator=g, device=DEV)
     check(x, up, down, ids, wts, kind, False, None)
     ops().check_device_errors(DEV)
+
+
+@pytest.mark.parametrize("why", ["off 16 bytes", "not contiguous", "refused"])
+def test_experts_the_kernel_does_not_take_go_through_the_library(why, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(7)
+    R, E, top, width, ff = 6, 4, 2, 64, 72
+    x = torch.randn((R, width), generator=g, device=DEV).bfloat16()
+    up, down = weights(g, E, width, ff, "swiglu")
+    ids, wts, placed = ops().moe_route(torch.randn((R, E), generator=g, device=DEV), None, top, place=True)
+    monkeypatch.setattr(ops(), "_GROUPED_MM", [False, False])  # one library product an expert: takes any operands
+    if why == "off 16 bytes":
+        down = torch.empty(down.numel() + 1, dtype=down.dtype, device=DEV)[1:].view(down.shape).copy_(down)
+    elif why == "not contiguous":
+        wide = torch.empty((E, 2 * ff, width + 8), dtype=up.dtype, device=DEV)
+        wide[:, :, :width] = up
+        up = wide[:, :, :width]
+    else:
+        lib = ops().native.lib()
+
+        class Refuses:
+            def __getattr__(self, name):
+                return (lambda *a: ops().native.ERR_UNSUPPORTED) if name == "rfx_moe_gemm" else getattr(lib, name)
+
+        monkeypatch.setattr(ops().native, "lib", Refuses)
+    check(x, up, down, ids, wts, "swiglu", False, placed)
+
+
+def test_a_captured_step_of_experts_off_16_bytes_waits_for_nobody(monkeypatch):
+    """Without a grouped product that takes them, a captured step is the one expert a row form."""
+    g = torch.Generator(device=DEV).manual_seed(8)
+    R, E, top, width, ff = 4, 4, 2, 64, 40
+    x = torch.randn((R, width), generator=g, device=DEV).bfloat16()
+    up, down = weights(g, E, width, ff, "silu")
+    up = torch.empty(up.numel() + 4, dtype=up.dtype, device=DEV)[4:].view(up.shape).copy_(up)
+    assert up.data_ptr() % 16 == 8
+    ids, wts = ops().moe_route(torch.randn((R, E), generator=g, device=DEV), None, top)
+    monkeypatch.setattr(ops(), "_GROUPED_MM", [False, False])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = ops().moe_experts(x, up, down, ids, wts, activation="silu")
+    graph.replay()
+    eager = ops().moe_experts(x, up, down, ids, wts, activation="silu")
+    assert ((out - eager).norm() / eager.norm()).item() < 5e-3
