@@ -1749,9 +1749,10 @@ def attention_sigmoid_mma(q, k_pages, v_pages, page_table, page_size, seq_slot, 
 
 
 def attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, seq_slot, seq_start, seq_new, seq_row0,
-                         max_new: int, nq, nkv, dim, window, scale, bias) -> torch.Tensor:
+                         max_new: int, nq, nkv, dim, window, scale, bias) -> Optional[torch.Tensor]:
     """The tcgen05/TMEM form of `attention_sigmoid_mma` for keys and values of one size, 64
-    or 128 (csrc/attention_prefill_tc.cu)."""
+    or 128 (csrc/attention_prefill_tc.cu); None for steps beyond its launches (more than 65,535
+    tiles of a sequence, as wide groups over long prompts have)."""
     out = _new(q.shape, q.dtype, q.device)
     st = native.lib().rfx_attention_sigmoid_tc(
         _chk(q, "q", torch.bfloat16), _chk(k_pages, "k_pages", torch.bfloat16), _chk(v_pages, "v_pages", torch.bfloat16),
@@ -1760,6 +1761,8 @@ def attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, seq_slot, s
         _chk(seq_new, "seq_new", torch.int32), _chk(seq_row0, "seq_row0", torch.int32), out.data_ptr(),
         seq_slot.numel(), int(max_new), q.shape[0], nq, nkv, dim, int(window or 0), float(scale),
         _chk(bias, "bias", torch.float32), device_error_word(q.device).data_ptr(), _stream())
+    if st == native.ERR_UNSUPPORTED:
+        return None
     native.check(st, f"attention_sigmoid_tc (dim={dim})")
     return out
 
@@ -1775,8 +1778,10 @@ def attention_sigmoid(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv
             and nq // nkv <= 128 and page_size == 64):
         if (dim == vdim and dim in (64, 128) and batch.max_new >= SIGMOID_TC_MIN_ROWS and k_pages.dim() == 4
                 and (q.data_ptr() | k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0):
-            return attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, batch.seq_slot, batch.seq_start,
-                                        batch.seq_new, batch.seq_row0, batch.max_new, nq, nkv, dim, window, scale, bias)
+            out = attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, batch.seq_slot, batch.seq_start,
+                                       batch.seq_new, batch.seq_row0, batch.max_new, nq, nkv, dim, window, scale, bias)
+            if out is not None:
+                return out
         return attention_sigmoid_mma(q, k_pages, v_pages, page_table, page_size, batch.seq_slot, batch.seq_start,
                                      batch.seq_new, batch.seq_row0, batch.max_new, nq, nkv, dim, vdim, window,
                                      scale, bias)
