@@ -377,7 +377,7 @@ extern "C" int rfx_gemm_f32(const float* x, const float* W, float* y, int R, int
         const long long per_small = (blocks(32, 64) + sms - 1) / sms, per_large = (blocks(64, 64) + sms - 1) / sms;
         if (per_small >= 2 && blocks(64, 32) <= 2 * sms)  // two a SM, a longer stage: 200 rows of N = 1,536 41 us, not 49
             return launch_tiles<64, 32, 4, 4, 64, 4>(x, W, y, R, N, K, st);
-        if (per_small * 106 <= per_large * (per_large <= 3 ? 260 : 200))
+        if (per_small * 106 <= per_large * (per_large <= 3 ? 260 : 200) && (R + 31) / 32 <= 65535)  // (a grid's limit)
             return launch_tiles<32, 64, 4, 4, 32, 4>(x, W, y, R, N, K, st);
         return launch_tiles<64, 64, 8, 4, 32, 3>(x, W, y, R, N, K, st);
     }

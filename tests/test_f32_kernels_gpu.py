@@ -32,6 +32,14 @@ def test_every_form_of_the_product_gives_the_same_bits(R, N, K):
     assert ((y - ref).abs().max() / ref.abs().max()).item() < 5e-7 * K ** 0.5
 
 
+def test_more_rows_than_a_grid_of_small_tiles_has():
+    R, N, K = 32 * 65535 + 33, 4, 4
+    x = torch.randn((R, K), generator=torch.Generator(device=DEV).manual_seed(1), device=DEV)
+    w = torch.randn((N, K), generator=torch.Generator(device=DEV).manual_seed(2), device=DEV)
+    apart = torch.empty(N * K + 1, device=DEV)[1:].view(N, K).copy_(w)
+    assert torch.equal(ops().linear(x, w), ops().linear(x, apart))
+
+
 class Batch:
     def __init__(self, counts, starts, slots):
         row0 = [0]
