@@ -110,7 +110,7 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
         float kk = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
 #pragma unroll
         for (int o = 1; o < 16; o <<= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
-        const float inv = 1.0f / sqrtf(kk + unit_eps);
+        const float inv = t < n ? 1.0f / sqrtf(kk + unit_eps) : 0.0f;  // (no row, no unit key, whatever unit_eps is)
         const float4 u = make_float4(k.x * inv, k.y * inv, k.z * inv, k.w * inv);
         store4(Us + t * LD + c, u);
         store4(Rs + t * LD + c, r);

@@ -200,10 +200,7 @@ def delta_rule_rows(r, k, v, w, a, S, eps):
     return np.stack(out), S
 
 
-@pytest.mark.parametrize("rate", [math.exp(-0.5), 2.0, 0.0, 2.5])  # 2.5: beyond the chunks' range, the walk
-@pytest.mark.parametrize("counts", [(32,), (33, 1, 31), (64, 0, 97), (160,)])
-def test_delta_rule_in_chunks(counts, rate, monkeypatch):
-    monkeypatch.setattr(ops(), "DELTA_CHUNK_MIN_ROWS", 1)
+def delta_case(counts, rate, eps):
     heads, d = 3, 64
     hd, R = heads * d, sum(counts)
     rng = np.random.default_rng(sum(counts))
@@ -215,7 +212,7 @@ def test_delta_rule_in_chunks(counts, rate, monkeypatch):
     dev = torch.from_numpy(state.copy()).to(DEV)
     to = lambda x: torch.from_numpy(x).to(DEV)  # noqa: E731
     b = Batch(counts, slots)
-    out = ops().delta_rule(to(proj), 0, hd, 2 * hd, 3 * hd, to(wpre), to(wb), to(ab), rate, 1e-6, dev, 4, b, heads, d,
+    out = ops().delta_rule(to(proj), 0, hd, 2 * hd, 3 * hd, to(wpre), to(wb), to(ab), rate, eps, dev, 4, b, heads, d,
                            exact=False)
     for i, (n, slot) in enumerate(zip(counts, slots)):
         if not n:
@@ -226,12 +223,25 @@ def test_delta_rule_in_chunks(counts, rate, monkeypatch):
         sig = lambda x: 1 / (1 + np.exp(-x))  # noqa: E731
         w = np.exp(-rate * sig((wpre[rows].astype(np.float64) + wb).reshape(n, heads, d)))
         ref, S = delta_rule_rows(r, k, v, w, sig(a + ab.astype(np.float64).reshape(heads, d)),
-                                 state[slot, 4:].astype(np.float64).reshape(heads, d, d), 1e-6)
+                                 state[slot, 4:].astype(np.float64).reshape(heads, d, d), eps)
         assert off(out[rows], ref.reshape(n, hd)) < TOL
         assert off(dev[slot, 4:], S.ravel()) < TOL
         assert torch.equal(dev[slot, :4].cpu(), torch.from_numpy(state[slot, :4]))
     untouched = [s for s in range(6) if s not in slots]
     assert torch.equal(dev[untouched].cpu(), torch.from_numpy(state[untouched]))
+
+
+@pytest.mark.parametrize("rate", [math.exp(-0.5), 2.0, 0.0, 2.5])  # 2.5: beyond the chunks' range, the walk
+@pytest.mark.parametrize("counts", [(32,), (33, 1, 31), (64, 0, 97), (160,)])
+def test_delta_rule_in_chunks(counts, rate, monkeypatch):
+    monkeypatch.setattr(ops(), "DELTA_CHUNK_MIN_ROWS", 1)
+    delta_case(counts, rate, 1e-6)
+
+
+def test_delta_rule_in_chunks_without_an_epsilon(monkeypatch):
+    """Rows that a last chunk does not have bring nothing: their key has no length to divide by."""
+    monkeypatch.setattr(ops(), "DELTA_CHUNK_MIN_ROWS", 1)
+    delta_case((33, 1, 31), 0.5, 0.0)
 
 
 def test_a_long_delta_step_goes_through_a_bounded_scratch():
