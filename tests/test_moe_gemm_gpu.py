@@ -27,7 +27,7 @@ def act64(kind, g, u):
     return g * torch.sigmoid(1.5 * g) * (u + 1)
 
 
-def check(x, up, down, ids, wts, kind, by_input, placed):
+def check(x, up, down, ids, wts, kind, by_input, placed, bound=3e-3):
     R, ff, gated = x.shape[0], down.shape[2], kind in ("glu_clamped", "swiglu")
     got = ops().moe_experts(x, up, down, ids, wts, activation=kind, weight_input=by_input, alpha=1.5, limit=0.7,
                             placed=placed)
@@ -39,7 +39,7 @@ def check(x, up, down, ids, wts, kind, by_input, placed):
             h = up[e].double() @ row
             y = down[e].double() @ act64(kind, h[:ff], h[ff:] if gated else None)
             ref[r] += y if by_input else w * y
-    assert ((got - ref).norm() / ref.norm()).item() < 3e-3  # 2^-9 = 2e-3 an activation, uniform: 1.1e-3 rms
+    assert ((got - ref).norm() / ref.norm()).item() < bound  # 2^-9 = 2e-3 an activation, uniform: 1.1e-3 rms
 
 
 def weights(g, E, width, ff, kind):
@@ -102,7 +102,8 @@ def test_experts_the_kernel_does_not_take_go_through_the_library(why, monkeypatc
                 return (lambda *a: ops().native.ERR_UNSUPPORTED) if name == "rfx_moe_gemm" else getattr(lib, name)
 
         monkeypatch.setattr(ops().native, "lib", Refuses)
-    check(x, up, down, ids, wts, "swiglu", False, placed)
+    # the library's up product is rounded to bfloat16 too: gate, up and activation, at most 2^-9 each
+    check(x, up, down, ids, wts, "swiglu", False, placed, bound=6e-3)
 
 
 def test_a_captured_step_of_experts_off_16_bytes_waits_for_nobody(monkeypatch):
