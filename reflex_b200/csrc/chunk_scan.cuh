@@ -24,13 +24,13 @@
 //
 // A policy `Pol` gives: q, k, v rows (float32, 16-byte aligned, counts in fours), `heads`, `per`
 // (heads per q/k head), N (elements of q and k, at most 128), P (elements of v) and the functions
-// named below.  What depends on a step: sequence `seq`'s rows `first_row` .. in chunks from
-// `seg * seg_rows` on, so that a long step can go through a bounded scratch in several rounds.
+// named below.  A long step goes through a bounded scratch in several rounds (chunk_plan.cuh).
 #pragma once
 
 #include <type_traits>
 
 #include "attn_mma.cuh"
+#include "chunk_plan.cuh"
 #include "common.cuh"
 #include "split_mma.cuh"
 
@@ -45,29 +45,23 @@ constexpr int VLD = PT + 4;  // row stride of v's tile: 2 VLD = 8 mod 32, four r
 struct Step {
     const int* seq_slot;
     const int* seq_row0;
-    int seg_rows, seg, n_segs;
+    Round round;
     float* scratch;  // [place][head][P][N] (+ [N] with a normaliser): a chunk's own sum, then the memory before it
     float4* aux;     // [place][head]: what the carry needs of a chunk
     float* before;   // [place][head]: the policy's running number before the chunk
     float4* rows;    // [place][head][L][RECORDS]: the policy's records of the chunk's rows
 };
 
-// The place of chunk c (of this segment) of sequence `seq` among all: with one segment at most
-// R / L + sequences of them, with several (seg_rows / L) x sequences.
-__device__ __forceinline__ size_t place_of(const Step& s, int row0, int seq, int c) {
-    return s.n_segs == 1 ? (size_t)row0 / L + seq + c : (size_t)seq * (s.seg_rows / L) + c;
-}
-
 struct Rows {
     int first, n;  // the chunk's first row and how many it has
-    bool last;     // of its sequence's in this segment
+    bool last;     // of its sequence's in this round
     size_t place;
 };
 __device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
-    const int row0 = s.seq_row0[seq], from = row0 + s.seg * s.seg_rows;
-    const int to = min(s.seq_row0[seq + 1], from + s.seg_rows);
+    const int row0 = s.seq_row0[seq], from = row0 + s.round.seg * s.round.seg_rows;
+    const int to = min(s.seq_row0[seq + 1], from + s.round.seg_rows);
     const int first = from + c * L;
-    return {first, min(L, to - first), to - first <= L, place_of(s, row0, seq, c)};
+    return {first, min(L, to - first), to - first <= L, place_in(s.round, L, row0, seq, c)};
 }
 
 // A tile of `rows` rows of 4 * c4 floats, rows from n on and columns from n4 (in fours) on zero.
@@ -97,7 +91,7 @@ __global__ void __launch_bounds__(256) chunk_state_kernel(Pol pol, Step st) {
     extern __shared__ __align__(16) float sm[];
     __shared__ __align__(8) float wl[L];
     rfx::pdl_prologue();
-    const int seq = blockIdx.y;
+    const int seq = st.round.seq0 + blockIdx.y;
     const Rows ch = rows_of(st, seq, blockIdx.x);
     if (ch.n <= 0) return;
     const int ptiles = (pol.P + PT - 1) / PT, h = blockIdx.z / ptiles, p0 = (blockIdx.z - h * ptiles) * PT;
@@ -155,18 +149,18 @@ template <class Pol>
 __global__ void __launch_bounds__(128) chunk_carry_kernel(Pol pol, Step st) {
     constexpr int AHEAD = 8;
     rfx::pdl_prologue();
-    const int seq = blockIdx.y, h = blockIdx.z;
+    const int seq = st.round.seq0 + blockIdx.y, h = blockIdx.z;
     const int e = 4 * (blockIdx.x * 128 + threadIdx.x);
     const int E = pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
     if (e >= E) return;
-    const int row0 = st.seq_row0[seq], from = row0 + st.seg * st.seg_rows;
-    const int rows = min(st.seq_row0[seq + 1] - from, st.seg_rows);
+    const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows;
+    const int rows = min(st.seq_row0[seq + 1] - from, st.round.seg_rows);
     const int n = (rows + L - 1) / L;
     if (rows <= 0) return;
     const int slot = st.seq_slot[seq];
     float4 S = pol.load_state(slot, h, e);
     float m = pol.load_number(slot, h);
-    const size_t at = place_of(st, row0, seq, 0) * pol.heads + h;
+    const size_t at = place_in(st.round, L, row0, seq, 0) * pol.heads + h;
     float* sc = st.scratch + at * E + e;
     const size_t step = (size_t)pol.heads * E;
     for (int c0 = 0; c0 < n; c0 += AHEAD) {
@@ -239,7 +233,7 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(Pol pol, Step st, int
     __shared__ __align__(16) float4 rec[L * Pol::RECORDS];
     __shared__ float nv[128];
     rfx::pdl_prologue();
-    const int seq = blockIdx.y;
+    const int seq = st.round.seq0 + blockIdx.y;
     const Rows ch = rows_of(st, seq, blockIdx.x);
     if (ch.n <= 0) return;
     const int ptiles = (pol.P + PT - 1) / PT, items = pol.per * ptiles;
@@ -377,44 +371,24 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(Pol pol, Step st, int
     }
 }
 
-inline long long places(int R, int n_seq, int seg_rows, int n_segs) {
-    return n_segs == 1 ? R / L + n_seq : (long long)n_seq * (seg_rows / L);
-}
-
-// Floats of scratch a step needs: the memories of all its chunks, up to about `budget` floats;
-// beyond that the rows go through in rounds of `*seg_rows` rows a sequence.
-inline long long scratch_floats(int R, int n_seq, int max_rows, int heads, long long E, int records, int* seg_rows) {
-    const long long budget = 64LL << 20;  // 256 MB
-    const long long one = heads * (E + 8 + 4 * L * records);
-    const int whole = (max_rows + L - 1) / L * L;
-    int seg = whole;
-    if ((long long)(R / L + n_seq) * one > budget) {
-        seg = (int)((budget / (one * n_seq)) * L);
-        if (seg < 4 * L) seg = 4 * L;
-        if (seg >= whole) seg = whole;
-    }
-    *seg_rows = seg;
-    return places(R, n_seq, seg, (max_rows + seg - 1) / seg) * one;
-}
+// Floats of scratch a chunk needs: its memories and what the other kernels read beside them.
+inline long long chunk_floats(int heads, long long E, int records) { return heads * (E + 8 + 4 * L * records); }
 
 template <class Pol>
 int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int R, int max_rows, float* scratch,
         cudaStream_t s) {
     const long long E = (long long)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
-    int seg_rows = 0;
-    scratch_floats(R, n_seq, max_rows, pol.heads, E, Pol::RECORDS, &seg_rows);
+    const Plan plan = plan_rounds(R, n_seq, max_rows, L, chunk_floats(pol.heads, E, Pol::RECORDS));
     Step st;
     st.seq_slot = seq_slot;
     st.seq_row0 = seq_row0;
-    st.seg_rows = seg_rows;
-    st.n_segs = (max_rows + seg_rows - 1) / seg_rows;
-    const long long n_places = places(R, n_seq, seg_rows, st.n_segs);
+    const long long n_places = plan.places;
     st.scratch = scratch;
     st.aux = reinterpret_cast<float4*>(scratch + n_places * pol.heads * E);  // E is a multiple of four
     st.rows = st.aux + n_places * pol.heads;
     st.before = reinterpret_cast<float*>(st.rows + n_places * pol.heads * L * Pol::RECORDS);
     const int N8 = (pol.N + 7) / 8 * 8, ptiles = (pol.P + PT - 1) / PT;
-    const int chunks = (min(seg_rows, max_rows) + L - 1) / L;
+    const int chunks = plan.seg_rows / L;
     const size_t sm_state = (size_t)L * (VLD + N8 + 4) * sizeof(float);
     const size_t sm_out = (size_t)L * (VLD + 2 * (N8 + 8)) * sizeof(float);
     const int qk_heads = pol.heads / pol.per, items = pol.per * ptiles;
@@ -423,7 +397,7 @@ int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int
     int ipb = items;
     long long least = -1;
     for (int i = items; i >= 1; --i) {
-        const long long blocks = (long long)chunks * n_seq * qk_heads * ((items + i - 1) / i);
+        const long long blocks = (long long)chunks * plan.group * qk_heads * ((items + i - 1) / i);
         const long long cost = (blocks + 2 * sm_count() - 1) / (2 * sm_count()) * (1 + i);
         if (least < 0 || cost < least) {
             least = cost;
@@ -437,11 +411,14 @@ int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(chunk_out_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_out);
     if (e != cudaSuccess) return (int)e;
-    for (st.seg = 0; st.seg < st.n_segs; ++st.seg) {
-        RFX_LAUNCH(chunk_state_kernel<Pol>, dim3(chunks, n_seq, pol.heads * ptiles), 256, sm_state, s, pol, st);
-        RFX_LAUNCH(chunk_carry_kernel<Pol>, dim3((unsigned)((E / 4 + 127) / 128), n_seq, pol.heads), 128, 0, s, pol, st);
-        RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, n_seq, qk_heads * sets), 256, sm_out, s, pol, st, ipb);
-    }
+    for (int seq0 = 0; seq0 < n_seq; seq0 += plan.group)
+        for (int seg = 0; seg < plan.n_segs; ++seg) {
+            const int seqs = min(plan.group, n_seq - seq0);
+            st.round = Round{plan.seg_rows, seg, seq0, plan.whole};
+            RFX_LAUNCH(chunk_state_kernel<Pol>, dim3(chunks, seqs, pol.heads * ptiles), 256, sm_state, s, pol, st);
+            RFX_LAUNCH(chunk_carry_kernel<Pol>, dim3((unsigned)((E / 4 + 127) / 128), seqs, pol.heads), 128, 0, s, pol, st);
+            RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, seqs, qk_heads * sets), 256, sm_out, s, pol, st, ipb);
+        }
     return 0;
 }
 

@@ -18,6 +18,7 @@
 // their relative precision); rates for which that leaves 32 bits' range take the row-by-row walk.
 // The memory itself stays 32-bit from chunk to chunk.
 #include "attn_mma.cuh"
+#include "chunk_plan.cuh"
 #include "common.cuh"
 #include "split_mma.cuh"
 
@@ -37,12 +38,9 @@ constexpr int STAGES = 3;
 struct Step {
     const int* seq_slot;
     const int* seq_row0;
-    int seg_rows, seg, n_segs;
+    chunk::Round round;
     float* scratch;
 };
-__device__ __forceinline__ size_t place_of(const Step& s, int row0, int seq, int c) {
-    return s.n_segs == 1 ? (size_t)row0 / L + seq + c : (size_t)seq * (s.seg_rows / L) + c;
-}
 
 __device__ __forceinline__ float sigmoid_f(float t) { return 1.0f / (1.0f + expf(-t)); }
 
@@ -85,9 +83,9 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
     float *As = Zs + L * VLD, *Bs = As + L * SLD, *Cs = Bs + L * SLD, *Es = Cs + L * SLD;
     __shared__ float wl[D];
     pdl_prologue();
-    const int seq = blockIdx.y, h = blockIdx.z;
-    const int row0 = st.seq_row0[seq], from = row0 + st.seg * st.seg_rows;
-    const int first = from + blockIdx.x * L, n = min(L, min(st.seq_row0[seq + 1], from + st.seg_rows) - first);
+    const int seq = st.round.seq0 + blockIdx.y, h = blockIdx.z;
+    const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows;
+    const int first = from + blockIdx.x * L, n = min(L, min(st.seq_row0[seq + 1], from + st.round.seg_rows) - first);
     if (n <= 0) return;
     const int hd = heads * D, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
     float* ws = Zs;  // the rows' decays, until the right sides take their place
@@ -212,7 +210,7 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
         for (int t = 0; t < L; ++t) x[t * LD] *= w;
     }
     __syncthreads();
-    float* place = st.scratch + (place_of(st, row0, seq, blockIdx.x) * heads + h) * PLACE;
+    float* place = st.scratch + (chunk::place_in(st.round, L, row0, seq, blockIdx.x) * heads + h) * PLACE;
     {   // C V - E Zl into the results, r W - E Y for the walk: sixteen rows by 32 columns a warp
         const int m0 = 16 * (warp & 1), half = (warp >> 1) & 1, n0 = 32 * (warp >> 2);
         const int ta = m0 + g, tb = ta + 8;
@@ -286,13 +284,13 @@ delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stri
     extern __shared__ __align__(16) float sm[];
     __shared__ __align__(16) float4 part[2][D / 8][32];
     pdl_prologue();
-    const int seq = blockIdx.x, h = blockIdx.y, c0 = 16 * blockIdx.z;
-    const int row0 = st.seq_row0[seq], from = row0 + st.seg * st.seg_rows;
-    const int rows = min(st.seq_row0[seq + 1] - from, st.seg_rows);
+    const int seq = st.round.seq0 + blockIdx.x, h = blockIdx.y, c0 = 16 * blockIdx.z;
+    const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows;
+    const int rows = min(st.seq_row0[seq + 1] - from, st.round.seg_rows);
     if (rows <= 0) return;
     const int chunks = (rows + L - 1) / L, hd = heads * D;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
-    const float* base = st.scratch + (place_of(st, row0, seq, 0) * heads + h) * PLACE;
+    const float* base = st.scratch + (chunk::place_in(st.round, L, row0, seq, 0) * heads + h) * PLACE;
     const size_t step = (size_t)heads * PLACE;
     auto fetch = [&](int c) {
         if (c < chunks) {
@@ -384,29 +382,15 @@ delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stri
     }
 }
 
-inline long long places(int R, int n_seq, int seg_rows, int n_segs) {
-    return n_segs == 1 ? R / L + n_seq : (long long)n_seq * (seg_rows / L);
-}
-// The factors of all chunks up to about 256 MB; beyond that the rows go through in rounds.
-inline long long scratch_floats(int R, int n_seq, int max_rows, int heads, int* seg_rows) {
-    const long long budget = 64LL << 20, one = (long long)heads * PLACE;
-    const int whole = (max_rows + L - 1) / L * L;
-    int seg = whole;
-    if ((R / L + n_seq) * one > budget) {
-        seg = (int)(budget / (one * n_seq)) * L;
-        if (seg < 8 * L) seg = 8 * L;
-        if (seg >= whole) seg = whole;
-    }
-    *seg_rows = seg;
-    return places(R, n_seq, seg, (max_rows + seg - 1) / seg) * one;
+inline chunk::Plan plan_of(int R, int n_seq, int max_rows, int heads) {
+    return chunk::plan_rounds(R, n_seq, max_rows, L, (long long)heads * PLACE);
 }
 
 }  // namespace
 
 // Floats of scratch rfx_delta_rule_chunk needs for a step of R rows in n_seq sequences of at most max_rows.
 extern "C" long long rfx_delta_rule_chunk_floats(int R, int n_seq, int max_rows, int heads) {
-    int seg = 0;
-    return scratch_floats(R, n_seq, max_rows, heads, &seg);
+    return plan_of(R, n_seq, max_rows, heads).places * heads * PLACE;
 }
 
 // As rfx_delta_rule with 32-bit results and the state [heads][value column][key channel].  d 64, rates
@@ -429,19 +413,21 @@ extern "C" int rfx_delta_rule_chunk(const float* proj, int ld, int r_off, int k_
     st.seq_slot = seq_slot;
     st.seq_row0 = seq_row0;
     st.scratch = scratch;
-    scratch_floats(R, n_seq, max_rows, heads, &st.seg_rows);
-    st.n_segs = (max_rows + st.seg_rows - 1) / st.seg_rows;
-    const int chunks = ((max_rows < st.seg_rows ? max_rows : st.seg_rows) + L - 1) / L;
+    const chunk::Plan plan = plan_of(R, n_seq, max_rows, heads);
+    const int chunks = plan.seg_rows / L;
     constexpr size_t sm_prep = PREP_FLOATS * sizeof(float), sm_walk = (size_t)STAGES * MR * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_prep);
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
     if (e != cudaSuccess) return (int)e;
-    for (st.seg = 0; st.seg < st.n_segs; ++st.seg) {
-        RFX_LAUNCH(delta_chunk_prep_kernel, dim3(chunks, n_seq, heads), 256, sm_prep, s, proj, ld, r_off, k_off, v_off,
-                   a_off, wpre, w_bias, a_bias, rate, unit_eps, st, out, heads);
-        RFX_LAUNCH(delta_chunk_walk_kernel, dim3(n_seq, heads, D / 16), 128, sm_walk, s, st, state, state_stride,
-                   state_off, out, heads);
-    }
+    for (int seq0 = 0; seq0 < n_seq; seq0 += plan.group)
+        for (int seg = 0; seg < plan.n_segs; ++seg) {
+            const int seqs = min(plan.group, n_seq - seq0);
+            st.round = chunk::Round{plan.seg_rows, seg, seq0, plan.whole};
+            RFX_LAUNCH(delta_chunk_prep_kernel, dim3(chunks, seqs, heads), 256, sm_prep, s, proj, ld, r_off, k_off, v_off,
+                       a_off, wpre, w_bias, a_bias, rate, unit_eps, st, out, heads);
+            RFX_LAUNCH(delta_chunk_walk_kernel, dim3(seqs, heads, D / 16), 128, sm_walk, s, st, state, state_stride,
+                       state_off, out, heads);
+        }
     return 0;
 }

@@ -117,8 +117,8 @@ struct Mlstm {
 
 // Floats of scratch rfx_mlstm_chunks needs for a step of R rows in S sequences of at most max_rows.
 extern "C" long long rfx_mlstm_chunks_floats(int R, int S, int max_rows, int heads, int dim, int vdim) {
-    int seg = 0;
-    return chunk::scratch_floats(R, S, max_rows, heads, (long long)vdim * dim + dim, Mlstm::RECORDS, &seg);
+    const long long one = chunk::chunk_floats(heads, (long long)vdim * dim + dim, Mlstm::RECORDS);
+    return chunk::plan_rounds(R, S, max_rows, chunk::L, one).places * one;
 }
 
 // As rfx_mlstm_scan.  dim in fours up to 128, vdim in fours; rows, results and `scratch` on 16 bytes.

@@ -85,8 +85,8 @@ struct Ssd {
 
 // Floats of scratch rfx_ssd_chunk needs for a step of R rows in n_seq sequences of at most max_rows.
 extern "C" long long rfx_ssd_chunk_floats(int R, int n_seq, int max_rows, int heads, int P, int N) {
-    int seg = 0;
-    return chunk::scratch_floats(R, n_seq, max_rows, heads, (long long)P * N, Ssd::RECORDS, &seg);
+    const long long one = chunk::chunk_floats(heads, (long long)P * N, Ssd::RECORDS);
+    return chunk::plan_rounds(R, n_seq, max_rows, chunk::L, one).places * one;
 }
 
 // As rfx_ssd_scan with 32-bit results, the state [heads][P][N].  P and N in fours, N up to 128; rows and

@@ -167,8 +167,8 @@ def test_mlstm_with_more_blocks_than_the_chip_holds():
 
 
 def test_a_long_step_goes_through_a_bounded_scratch():
-    """Memories of 64 heads of 256 x 128 for 37 chunks (310 MB) do not fit the scratch: two rounds,
-    the second going on from the state that the first one left; beside it a short sequence.  With
+    """Memories of 64 heads of 256 x 128 for 37 chunks (310 MB) do not fit the scratch: rounds of rows,
+    each going on from the state that the one before left; beside it a short sequence.  With
     decays near one a result is a sum over all rows; the walk it is compared with rounds 2,300 times,
     2300 * 2^-24 = 1.4e-4."""
     heads, groups, P, N, counts = 64, 2, 256, 128, (2300, 70)
@@ -260,3 +260,34 @@ def test_a_long_delta_step_goes_through_a_bounded_scratch():
         got.append((y, state))
     for a, b in zip(*got):  # the removal forgets what 32 rows back added: no sum over all rows here
         assert ((a - b).abs().max() / a.abs().max()).item() < TOL
+
+
+def test_many_sequences_go_through_a_bounded_scratch():
+    """121 chunks of 64 heads of 256 x 128 where the scratch holds 31, and 260 of the delta rule's of 64 heads where it
+    holds 95: rounds of sequences, the longest of them in several; against the walk, a short sum's roundings apart."""
+    heads, groups, P, N = 64, 2, 256, 128
+    counts = [120 + (i * 7) % 30 for i in range(39)] + [700]
+    g = torch.Generator(device=DEV).manual_seed(6)
+    R, inner = sum(counts), heads * P
+    xbc = torch.randn((R, inner + 2 * groups * N), generator=g, device=DEV)
+    proj = torch.randn((R, inner + heads), generator=g, device=DEV)
+    A, D = -torch.rand(heads, generator=g, device=DEV) - 0.5, torch.randn(heads, generator=g, device=DEV)
+    bias, start = torch.zeros(heads, device=DEV), torch.randn((40, heads * P * N), generator=g, device=DEV)
+    slots = [(i * 11) % 40 for i in range(40)]
+    got = []
+    for exact in (True, False):
+        state = start.clone()
+        y = ops().ssd_scan(xbc, proj, 0, inner, bias, A, D, state, 0, Batch(counts, slots), heads, P, N, groups, exact=exact)
+        got.append((y, state))
+    for a, b in zip(*got):
+        assert ((a - b).abs().max() / a.abs().max()).item() < 2 * TOL
+    hd = heads * 64
+    proj, wpre = torch.randn((R, 4 * hd), generator=g, device=DEV), torch.randn((R, hd), generator=g, device=DEV)
+    zero, got = torch.zeros(hd, device=DEV), []
+    for exact in (True, False):
+        state = start[:, :hd * 64].clone()
+        y = ops().delta_rule(proj, 0, hd, 2 * hd, 3 * hd, wpre, zero, zero, math.exp(-0.5), 1e-6, state, 0,
+                             Batch(counts, slots), heads, 64, exact=exact)
+        got.append((y, state))
+    for a, b in zip(*got):
+        assert ((a - b).abs().max() / a.abs().max()).item() < 2 * TOL
