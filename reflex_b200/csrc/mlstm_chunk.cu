@@ -1,5 +1,5 @@
-// The mLSTM matrix memory (mlstm.cu) for steps that bring a sequence many rows: 64 rows at a time
-// on the tensor cores, all chunks side by side (chunk_scan.cuh).
+// The mLSTM matrix memory (mlstm.cu) for steps that bring a sequence many rows: 64 rows at a time,
+// all chunks side by side (chunk_scan.cuh).
 //
 // With F_t the sum of the log forget gates from the chunk's first row to t, g_s = i_s - F_s and
 // M_t = max(m_prev, max_{s<=t} g_s), the walk gives m_t = F_t + M_t and
@@ -105,8 +105,9 @@ struct Mlstm {
         float* s = head_state(slot, h) + (size_t)N * P + N;
         for (int i = 0; i < (P + 63) / 64; ++i) s[i] = m;
     }
-    __device__ __forceinline__ void store_row(int r, int h, int p, float y0, float y1, float, float) const {
-        rfx::store2(num + ((size_t)r * heads + h) * P + p, y0 * q_scale, y1 * q_scale);
+    __device__ __forceinline__ void store_row(int r, int h, int p, const float4& y, const float4&) const {
+        rfx::store4(num + ((size_t)r * heads + h) * P + p,
+                    make_float4(y.x * q_scale, y.y * q_scale, y.z * q_scale, y.w * q_scale));
     }
     __device__ __forceinline__ void store_sum(int r, int h, float nq, float floor) const {
         den[(size_t)r * heads + h] = fmaxf(fabsf(nq * q_scale), floor) + 1e-6f;

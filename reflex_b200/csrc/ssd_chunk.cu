@@ -1,5 +1,5 @@
 // The state-space recurrence with one decay a head (ssd.cu) for steps that bring a sequence many
-// rows: 64 rows at a time on the tensor cores, all chunks side by side (chunk_scan.cuh).
+// rows: 64 rows at a time, all chunks side by side (chunk_scan.cuh).
 //
 //     dt = softplus(dt_pre[h] + dt_bias[h]),  S <- exp(A[h] dt) S + dt B x^T,  y = S^T C + D[h] x
 //     out = y * silu(z)
@@ -53,7 +53,8 @@ struct Ssd {
             if (rows) {
                 float hi, lo;
                 chunk::two_parts(c[i], &hi, &lo);
-                rows[r] = make_float4(hi, lo, d[i], expf(hi));
+                const float e = expf(hi);
+                rows[r] = make_float4(hi, lo, d[i], fmaf(e, lo, e));  // exp(hi + lo)
             }
         }
         return make_float4(expf((float)all), 0.0f, 0.0f, 0.0f);
@@ -73,11 +74,12 @@ struct Ssd {
     __device__ __forceinline__ void store_state(int slot, int h, int e, const float4& S) const {
         *reinterpret_cast<float4*>(memory(slot, h, e)) = S;
     }
-    __device__ __forceinline__ void store_row(int r, int h, int p, float y0, float y1, float x0, float x1) const {
-        const float2 z = *reinterpret_cast<const float2*>(proj + (size_t)r * ldp + z_off + h * P + p);
+    __device__ __forceinline__ void store_row(int r, int h, int p, const float4& y, const float4& x) const {
+        const float4 z = rfx::load4(proj + (size_t)r * ldp + z_off + h * P + p);
         const float d = D ? D[h] : 0.0f;
-        rfx::store2(out + (size_t)r * inner + h * P + p, fmaf(d, x0, y0) * (z.x / (1.0f + expf(-z.x))),
-                    fmaf(d, x1, y1) * (z.y / (1.0f + expf(-z.y))));
+        rfx::store4(out + (size_t)r * inner + h * P + p,
+                    make_float4(fmaf(d, x.x, y.x) * (z.x / (1.0f + expf(-z.x))), fmaf(d, x.y, y.y) * (z.y / (1.0f + expf(-z.y))),
+                                fmaf(d, x.z, y.z) * (z.z / (1.0f + expf(-z.z))), fmaf(d, x.w, y.w) * (z.w / (1.0f + expf(-z.w)))));
     }
 };
 

@@ -900,8 +900,8 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale:
     `max_rows`: the most rows any sequence brings; from `MLSTM_CHUNK_MIN_ROWS`
     on (and dim up to 256) the chunkwise kernel runs, else the row-by-row walk:
     the same function, rounded differently.  Without `exact`, and for dim up to 128,
-    many rows go through the kernels that take 64 at a time on the tensor cores, products
-    of 32-bit numbers split in two (csrc/mlstm_chunk.cu)."""
+    many rows go through the kernels that take 64 at a time, all chunks side by side
+    (csrc/mlstm_chunk.cu)."""
     R = proj.shape[0]
     _chk(proj, "proj", torch.float32)
     if state.shape[-1] != mlstm_state_floats(dim, vdim) or state.shape[-2] != heads:
@@ -1811,8 +1811,8 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
     `state[slot, state_off : state_off + heads * states * vdim]`.  Returns
     (S^T C + D x) * silu(z), [R, heads * vdim].  Without `exact`, from
     `SSD_CHUNK_MIN_ROWS` rows of a sequence on the kernels that take 64 rows at a time
-    run (csrc/ssd_chunk.cu: the same function, products of 32-bit numbers split for the
-    tensor cores); else, and for sizes those do not take, the row-by-row walk."""
+    run (csrc/ssd_chunk.cu: the same function, its sums in another order); else, and for
+    sizes those do not take, the row-by-row walk."""
     R = xbc.shape[0]
     inner = heads * vdim
     if xbc.shape[1] != inner + 2 * groups * states:
