@@ -18,6 +18,7 @@
 // same registers are the left operand of the next chunk's products; likewise u^T.
 #include "attn_mma.cuh"
 #include "common.cuh"
+#include "fma_tiles.cuh"
 #include "split_mma.cuh"
 
 namespace {
@@ -35,12 +36,11 @@ using rfx::product3;
 // (a sequence of n rows has ceil(n / 16), so no two places meet; at most R / 16 + sequences).
 __device__ __forceinline__ size_t chunk_place(int row0, int seq, int c) { return (size_t)row0 / CH + seq + c; }
 
-// A block a (chunk, query/key head): the products between the chunk's rows once, on the tensor cores, each
-// warp some of the channels; then per value head of the group (eight at a time) T, M and the decays'
-// products.  Bound by the steps' latencies with six blocks an SM.  (A thread a pair of rows instead, three
-// 16-byte reads of shared memory for eight multiply-adds, was bound by those reads: 66 us for 4,096 rows of
-// 16 heads of 128 with two value heads each; 51 with this.)
+// A block a (chunk, query/key head): the products between the chunk's rows once, by 32-bit multiply-adds,
+// each warp some of the channels (four by four results a lane, of [k; q] by k); then per value head of
+// the group (eight at a time) T, M and the decays' products.
 constexpr int PREP_WARPS = CH * CH / 32, PREP_HEADS = 8;
+__host__ __device__ constexpr int prep_ld(int d) { return (d + 15) / 16 * 16 + 4; }  // an odd number of 16 bytes
 __global__ void __launch_bounds__(CH * CH)
 gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __restrict__ gates,
                               const int* __restrict__ seq_row0, float* __restrict__ coef, int H, int G, int d, int dv) {
@@ -51,11 +51,11 @@ gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __rest
     const int row0 = seq_row0[seq], row1 = seq_row0[seq + 1];
     const int first = row0 + blockIdx.x * CH, n = min(CH, row1 - first);
     if (n <= 0) return;
-    const int C = 2 * G * d + H * dv, d8 = (d + 7) / 8 * 8, LD = d8 + 8, c4 = d8 / 4;
+    const int C = 2 * G * d + H * dv, LD = prep_ld(d), c4 = (LD - 4) / 4;
     float *ks = sm, *qs = sm + CH * LD;
-    float4* part = reinterpret_cast<float4*>(sm + 2 * CH * LD);  // [warp][tile][lane]
+    float4* part = reinterpret_cast<float4*>(sm + 2 * CH * LD);  // [warp][four rows][lane]
     const int tid = threadIdx.x, i = tid / CH, j = tid % CH;
-    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int warp = tid >> 5, lane = tid & 31;
     for (int r = warp; r < CH; r += PREP_WARPS) {  // rows and channels that are not there as zeros
         const float* src = qkv + (size_t)(first + r) * C + kvh * d;
         for (int c = lane; c < c4; c += 32) {
@@ -76,24 +76,15 @@ gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __rest
     load_gates(0);
     attn::cp_async_wait<0>();
     __syncthreads();
-    float A[2][4] = {}, B[2][4] = {};  // k k^T and q k^T, columns 0..7 and 8..15
-    for (int s = warp; s < d8 / 8; s += PREP_WARPS) {
-        const float *kr = ks + g * LD + 8 * s + 2 * t4, *qr = qs + g * LD + 8 * s + 2 * t4;
-        const float2 b[2] = {*reinterpret_cast<const float2*>(kr), *reinterpret_cast<const float2*>(kr + 8 * LD)};
-        const float2 q0 = *reinterpret_cast<const float2*>(qr), q1 = *reinterpret_cast<const float2*>(qr + 8 * LD);
-        product3<2>(A, rfx::left_from(b[0].x, b[1].x, b[0].y, b[1].y), b);
-        product3<2>(B, rfx::left_from(q0.x, q1.x, q0.y, q1.y), b);
-    }
+    float acc[4][4] = {};  // rows lane / 4 + 8 i of [k; q], columns lane % 4 + 4 j
+    for (int s = warp; s < c4 / 4; s += PREP_WARPS)
+        rfx::product_along<4>(acc, ks + (lane >> 2) * LD + 16 * s, 8 * LD, ks + (lane & 3) * LD + 16 * s, 4 * LD, 1);
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        part[(warp * 4 + t) * 32 + lane] = make_float4(A[t][0], A[t][1], A[t][2], A[t][3]);
-        part[(warp * 4 + 2 + t) * 32 + lane] = make_float4(B[t][0], B[t][1], B[t][2], B[t][3]);
-    }
+    for (int t = 0; t < 4; ++t) part[(warp * 4 + t) * 32 + lane] = make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]);
     __syncthreads();
     float kk = 0.0f, qk = 0.0f;
     {
-        const float* p = reinterpret_cast<const float*>(part) +
-                         4 * ((j / 8) * 32 + (i % 8) * 4 + (j % 8) / 2) + (i / 8) * 2 + (j & 1);
+        const float* p = reinterpret_cast<const float*>(part) + 4 * ((i / 8) * 32 + (i % 8) * 4 + j % 4) + j / 4;
 #pragma unroll
         for (int w = 0; w < PREP_WARPS; ++w) {
             kk += p[w * 4 * 128];
@@ -417,7 +408,7 @@ extern "C" int rfx_gated_delta_chunk_prep(const float* qkv, const float* gates, 
                                           float* coef, int H, int G, int d, int dv, int max_rows, void* stream) {
     if (n_seq <= 0 || max_rows <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0) return RFX_ERR_BAD_ARG;
-    const size_t smem = (size_t)2 * CH * ((d + 7) / 8 * 8 + 8) * sizeof(float) + PREP_WARPS * 4 * 32 * sizeof(float4);
+    const size_t smem = (size_t)2 * CH * prep_ld(d) * sizeof(float) + PREP_WARPS * 4 * 32 * sizeof(float4);
     if (d % 4 || dv % 4 || (size_t)2 * CH * (d + 4) * sizeof(float) > 48 * 1024 || n_seq > 65535 || G > 65535) return RFX_ERR_UNSUPPORTED;
     dim3 grid((max_rows + CH - 1) / CH, n_seq, G);
     if (smem + 12 * 1024 > 48 * 1024) {
