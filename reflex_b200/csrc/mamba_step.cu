@@ -181,7 +181,9 @@ __global__ void __launch_bounds__(THREADS) mamba_step_kernel(Args a) {
 template <int NPL>
 int launch(Args a, int R, cudaStream_t s) {
     auto kernel = mamba_step_kernel<NPL>;
-    // sixteen CTAs a sequence where the device places such a cluster, else eight
+    // sixteen CTAs a sequence where the device holds such a cluster for each at a time, else eight; not in two
+    // waves (width 2,048: 24.7 us for the layer with six sequences and 35.1 with eight, 29.5 and 28.9 with
+    // three launches; width 1,024: 20.0 with eight and 27.0 with sixteen, 21.3 and 22.6)
     for (int ranks = 16; ranks >= 8; ranks /= 2) {
         if (a.C % (ranks * 8 * (32 / LPC))) continue;  // slices of whole warps' channels, 16 bytes a copy
         a.keep_dt = step_smem(a.C / ranks, a.outs, a.rank, ranks, 1) <= MAX_SMEM;
@@ -189,27 +191,25 @@ int launch(Args a, int R, cudaStream_t s) {
         if (smem > MAX_SMEM) continue;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        if (ranks > 8) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-                cudaGetLastError();
-                continue;
-            }
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(1, 1, ranks);
-            cfg.blockDim = dim3(THREADS);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 1;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = ranks;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int n = 0;
-            const bool fits = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
-            cudaGetLastError();  // a refusal is an answer, not an error to carry on
-            if (!fits) continue;
+        if (ranks > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
         }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, ranks);
+        cfg.blockDim = dim3(THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = ranks;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int n = 0;  // clusters the device holds at a time
+        const bool fits = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= R;
+        cudaGetLastError();  // a refusal is an answer, not an error to carry on
+        if (!fits) continue;
         e = rfx::launch(kernel, dim3(1, R, ranks), dim3(THREADS), smem, s, ranks, a);
         return e == cudaSuccess ? 0 : (int)e;
     }
@@ -221,7 +221,8 @@ int launch(Args a, int R, cudaStream_t s) {
 // One row a sequence: xz float32 [R][ld] = [x | z | ..], filters [taps][C], w_x bfloat16 [rank + 2 N][C] (rows
 // dt, B, C), w_dt bfloat16 [C][rank], A [C][N] (negative), state [slots][stride]: the filter's last taps - 1
 // inputs, oldest first, then S [C][N]; both move on.  out bfloat16 [R][C] = y * silu(z).  N 4, 8, 16 or 32;
-// RFX_ERR_UNSUPPORTED, before anything has run, for other sizes and what is not on 16 bytes.
+// RFX_ERR_UNSUPPORTED, before anything has run, for other sizes, more sequences than the device holds clusters
+// at a time, and what is not on 16 bytes.
 extern "C" int rfx_mamba_step(const float* xz, int ld, int C, int N, int rank, int taps, const float* filters,
                               const float* conv_bias, const void* w_x, const void* w_dt, const float* dt_bias,
                               const float* A, const float* D, float* state, long long stride, const int* row_slot, int R,
