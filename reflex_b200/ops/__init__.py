@@ -1797,11 +1797,20 @@ def _most_rows(batch) -> int:
     return int(getattr(batch, "max_new", 0))
 
 
-# Rows of the longest sequence from which the chunked kernels run: their three launches and the
-# memory's way out and back cost about 30 us, the walk 0.5 us a row (one sequence, width 2048, the
-# whole mixer: 71 us walking and 79 in chunks at 48 rows, 106 and 84 at 100; eight sequences of 37
-# rows 117 and 105).
-SSD_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_SSD_CHUNK_MIN_ROWS", 80, 1, 1 << 30)
+# Rows of the longest sequence from which the chunked kernels run where a step has about 32 to 64
+# (sequence, head) pairs; twice as many with fewer, three quarters with up to 128 and half beyond: the walk's time
+# grows with the rows and, once its blocks share SMs, with the pairs, the chunks' hardly with either.
+# Measured, in chunks and walking, us at the rows around the crossing: 16 pairs 34.7 and 28.3 at 100 rows, 35.1 each
+# at 128; 32 pairs 34.9 and 33.1 at 64, 34.9 and 41.4 at 80; 64 pairs 36.4 and 38.9 at 64; 128 pairs 41 and 40 at 48;
+# 256 pairs 45 each at 32.
+SSD_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_SSD_CHUNK_MIN_ROWS", 72, 1, 1 << 30)
+
+
+def _ssd_in_chunks(most: int, rows: int, heads: int) -> bool:
+    if not most:
+        return False
+    pairs = heads * rows // most  # as many sequences as the step's rows would make of the longest
+    return most >= SSD_CHUNK_MIN_ROWS * (2.0 if pairs < 32 else 1.0 if pairs <= 64 else 0.75 if pairs <= 128 else 0.5)
 
 
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_bias: torch.Tensor, A: torch.Tensor,
@@ -1812,7 +1821,7 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
     pre-activations at `dt_off`; `A` float32 [heads], negative; the running state is
     `state[slot, state_off : state_off + heads * states * vdim]`.  Returns
     (S^T C + D x) * silu(z), [R, heads * vdim].  Without `exact`, from
-    `SSD_CHUNK_MIN_ROWS` rows of a sequence on the kernels that take 64 rows at a time
+    about `SSD_CHUNK_MIN_ROWS` rows of a sequence on the kernels that take 64 rows at a time
     run (csrc/ssd_chunk.cu: the same function, its sums in another order); else, and for
     sizes those do not take, the row-by-row walk."""
     R = xbc.shape[0]
@@ -1823,8 +1832,7 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
         raise InvalidInput("ssd_scan: z or dt do not fit into the rows of proj")
     out = _new((R, inner), out_dtype, xbc.device)
     most = _most_rows(batch)
-    chunked = most >= SSD_CHUNK_MIN_ROWS or (most >= 32 and R >= 256 and SSD_CHUNK_MIN_ROWS <= 256)
-    if (not exact and chunked and out_dtype == torch.float32 and vdim % 4 == 0
+    if (not exact and _ssd_in_chunks(most, R, heads) and out_dtype == torch.float32 and vdim % 4 == 0
             and states % 4 == 0 and states <= 128):
         S = batch.seq_slot.numel()
         scratch = _new((int(native.lib().rfx_ssd_chunk_floats(R, S, most, heads, vdim, states)),), torch.float32,
