@@ -885,9 +885,16 @@ def mlstm_state_floats(dim: int, vdim: int) -> int:
 
 
 MLSTM_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_CHUNK_MIN_ROWS", 48, 1, 1 << 30)
-# from here on the tensor-core chunks: level with the walk at 48 to 64 rows of a sequence (the whole
-# mixer at width 2048: 50 us walking and 53 in chunks at 48 rows, 76 and 54 at 100)
-MLSTM_CHUNKS_MIN_ROWS = 64
+# Rows of a sequence from which all chunks go side by side (csrc/mlstm_chunk.cu); five eighths of that where the step
+# has eight (sequence, head) pairs or fewer.  Us side by side and chunk after chunk, heads of 128 x 256: 8 pairs 30.5
+# and 31.5 at 64 rows, 32 and 41 at 80; 16 pairs 47 and 41 at 80, 47 and 51 at 100; 32 pairs 55 and 52 at 100, 55 each
+# at 128; 128 pairs 160 each at 80, 168 and 199 at 100.
+MLSTM_SIDE_BY_SIDE_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_SIDE_BY_SIDE_MIN_ROWS", 128, 1, 1 << 30)
+
+
+def _mlstm_side_by_side(most: int, rows: int, heads: int) -> bool:
+    few = heads * rows // max(1, most) <= 8
+    return most >= MLSTM_SIDE_BY_SIDE_MIN_ROWS * (0.625 if few else 1.0)
 
 
 def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale: float, batch,
@@ -900,8 +907,8 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale:
     `max_rows`: the most rows any sequence brings; from `MLSTM_CHUNK_MIN_ROWS`
     on (and dim up to 256) the chunkwise kernel runs, else the row-by-row walk:
     the same function, rounded differently.  Without `exact`, and for dim up to 128,
-    many rows go through the kernels that take 64 at a time, all chunks side by side
-    (csrc/mlstm_chunk.cu)."""
+    from `MLSTM_SIDE_BY_SIDE_MIN_ROWS` on the kernels that take 64 rows at a time, all
+    chunks side by side (csrc/mlstm_chunk.cu)."""
     R = proj.shape[0]
     _chk(proj, "proj", torch.float32)
     if state.shape[-1] != mlstm_state_floats(dim, vdim) or state.shape[-2] != heads:
@@ -910,7 +917,7 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale:
     den = _new((R, heads), torch.float32, proj.device)
     q_off, k_off, v_off, i_off, f_off = (int(o) for o in offsets)
     chunked = max_rows is not None and max_rows >= MLSTM_CHUNK_MIN_ROWS and dim <= 256
-    if chunked and not exact and max_rows >= MLSTM_CHUNKS_MIN_ROWS and dim <= 128 and dim % 4 == 0 and vdim % 4 == 0:
+    if chunked and not exact and _mlstm_side_by_side(max_rows, R, heads) and dim <= 128 and dim % 4 == 0 and vdim % 4 == 0:
         S, most = batch.seq_slot.numel(), min(int(max_rows), R)
         scratch = _new((int(native.lib().rfx_mlstm_chunks_floats(R, S, most, heads, dim, vdim)),), torch.float32,
                        proj.device)

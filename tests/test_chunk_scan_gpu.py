@@ -28,6 +28,11 @@ def i32(v):
     return torch.tensor(list(v), dtype=torch.int32, device=DEV)
 
 
+@pytest.fixture(autouse=True)
+def rules(monkeypatch):
+    monkeypatch.setattr(ops(), "MLSTM_SIDE_BY_SIDE_MIN_ROWS", ops().MLSTM_SIDE_BY_SIDE_MIN_ROWS)
+
+
 class Batch:
     def __init__(self, counts, slots):
         self.row0 = [0]
@@ -126,6 +131,7 @@ def mlstm_case(heads, dim, vdim, counts, slots, running, forget):
 
 def mlstm_run(case, heads, dim, vdim, cap=12.0):
     proj, offsets, bi, bf, state, b = case
+    ops().MLSTM_SIDE_BY_SIDE_MIN_ROWS = 1  # (the fixture below puts it back)
     to = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
     dev = torch.from_numpy(state.copy()).to(DEV)
     num, den = ops().mlstm_scan(to(proj), offsets, to(bi), to(bf), cap, 0.25, b, dev, heads, dim, vdim,
@@ -232,7 +238,7 @@ def delta_case(counts, rate, eps):
         w = np.exp(-rate * sig((wpre[rows].astype(np.float64) + wb).reshape(n, heads, d)))
         ref, S = delta_rule_rows(r, k, v, w, sig(a + ab.astype(np.float64).reshape(heads, d)),
                                  state[slot, 4:].astype(np.float64).reshape(heads, d, d), eps)
-        assert off(out[rows], ref.reshape(n, hd)) < TOL
+        assert off(out[rows], ref.reshape(n, hd)) < TOL and (rate > 1 or norm_off(out[rows], ref.reshape(n, hd)) < NORM)
         assert off(dev[slot, 4:], S.ravel()) < TOL
         assert torch.equal(dev[slot, :4].cpu(), torch.from_numpy(state[slot, :4]))
     untouched = [s for s in range(6) if s not in slots]
@@ -334,3 +340,33 @@ def test_a_row_that_is_not_finite_does_not_reach_earlier_rows(bad):
     hit[256 + 100] = True
     assert torch.equal(num2[:70], num[:70]) and torch.equal(num2[:, ~hit], num[:, ~hit]) and torch.equal(den, den2)
     assert not torch.isfinite(num2[70:, hit]).any()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_row_that_is_not_finite_does_not_reach_earlier_rows_of_the_delta_rule(bad, monkeypatch):
+    """An element of v at row 70 spoils its own column from there on; one of k or of the decay its head's results:
+    from row 70 on, and nothing of rows 64 to 69 before it in its chunk."""
+    monkeypatch.setattr(ops(), "DELTA_CHUNK_MIN_ROWS", 1)
+    heads, d, T = 2, 64, 100
+    hd, b = heads * d, Batch([T], [0])
+    g = torch.Generator(device=DEV).manual_seed(10)
+    proj, wpre = torch.randn((T, 4 * hd), generator=g, device=DEV), torch.randn((T, hd), generator=g, device=DEV)
+    zero = torch.zeros(hd, device=DEV)
+
+    def run(p, w):
+        state = torch.zeros((1, hd * d), device=DEV)
+        return ops().delta_rule(p, 0, hd, 2 * hd, 3 * hd, w, zero, zero, 0.6, 1e-6, state, 0, b, heads, d, exact=False), state
+
+    clean, clean_state = run(proj, wpre)
+    for part in ("v", "k", "decay"):
+        p, w = proj.clone(), wpre.clone()
+        if part == "decay":
+            w[70, 67] = float("nan")
+        else:
+            p[70, (2 * hd if part == "v" else hd) + 67] = bad
+        y, state = run(p, w)
+        hit = torch.zeros(hd, dtype=torch.bool, device=DEV)
+        hit[67 if part == "v" else slice(64, 128)] = True
+        assert torch.equal(y[:70], clean[:70]) and torch.equal(y[:, ~hit], clean[:, ~hit]), part
+        assert not torch.isfinite(y[71:, hit]).any(), part
+        assert torch.equal(state.view(hd, d)[~hit], clean_state.view(hd, d)[~hit]), part
