@@ -1,5 +1,5 @@
 // The generalized delta rule (delta_rule.cu) for steps that bring a sequence many rows: 32 rows at a
-// time, as products on the tensor cores of operands split in two (split_mma.cuh).  Heads of 64.
+// time, as products of 32-bit multiply-adds.  Heads of 64.
 //
 // With W_t the product of the decays from the chunk's first row to t (per key channel), z_t = S^T u_t
 // what row t removes, S0 the memory before the chunk, and
@@ -11,8 +11,12 @@
 //     S_last = (diag(W_last) - p'^T Y) S0 + (k'^T V - p'^T Zl).
 // Everything but S0 is the chunk's own: delta_chunk_prep_kernel makes the four factors for all chunks
 // side by side (C V - E Zl straight into the results), and delta_chunk_walk_kernel is left with one
-// 64 x 64 product a chunk and 16 value columns, a chain of about 0.7 us instead of 32 rows' walk of
-// 0.35 us each.
+// product of 96 x 64 with the memory a chunk, a chain of about 1.4 us instead of 32 rows' walk of 0.35 us
+// each.
+//
+// As products on the tensor cores of operands split in two parts of 11 bits both kernels were about 60 us
+// faster for 2,048 rows of 32 heads, and eleven times as far from 64 bits as the walk (1.1e-6 against
+// 9.7e-8); these are 1.3e-7 off, the state 9.8e-8 (7e-8 walking).
 //
 // The factors W_t and 1 / W_s lie within e^(rate 32) of one (their products are what counts and keep
 // their relative precision); rates for which that leaves 32 bits' range take the row-by-row walk.
@@ -20,19 +24,18 @@
 #include "attn_mma.cuh"
 #include "chunk_plan.cuh"
 #include "common.cuh"
-#include "split_mma.cuh"
+#include "fma_tiles.cuh"
 
 namespace {
 
 using namespace rfx;
 
 constexpr int L = 32, D = 64;
-constexpr int LD = D + 8;   // rows read 8 bytes a lane along the channels
-constexpr int VLD = D + 4;  // rows read down the rows
-constexpr int SLD = L + 8;  // the rows' products with one another
-// per (chunk, head): M [64][LD] and R [32][LD] in one piece, then the chunk's own sum [value][key]
+constexpr int LD = D + 4;   // an odd number of 16 bytes: eight rows side by side meet all banks
+constexpr int SLD = L + 4;  // the rows' products with one another
+// per (chunk, head): M [64][LD] and R [32][LD] in one piece, then the chunk's own sum [key][value]
 constexpr int MR = (D + L) * LD, PLACE = MR + D * D;
-constexpr int PREP_FLOATS = 4 * L * LD + 2 * L * VLD + 4 * L * SLD;  // 75 KB: three blocks an SM
+constexpr int PREP_FLOATS = 6 * L * LD + 4 * L * SLD;  // 70 KB
 constexpr int STAGES = 3;
 
 struct Step {
@@ -44,50 +47,24 @@ struct Step {
 
 __device__ __forceinline__ float sigmoid_f(float t) { return 1.0f / (1.0f + expf(-t)); }
 
-// acc [16 rows m0 ..][8 N columns n0 ..] += sign * left^T right over the chunk's rows, both read down
-// the rows (eight at a time from row 8 s on)
-template <int N>
-__device__ __forceinline__ void down_step(float (&acc)[N][4], const float* left, int lld, float sign,
-                                          const float* right, int rld, int s, int g, int j) {
-    const float* l = left + (8 * s + 2 * j) * lld + g;
-    const Left a = left_from(sign * l[0], sign * l[8], sign * l[lld], sign * l[lld + 8]);
-    const float* r = right + (8 * s + 2 * j) * rld + g;
-    float2 b[N];
-#pragma unroll
-    for (int t = 0; t < N; ++t) b[t] = make_float2(r[8 * t], r[rld + 8 * t]);
-    product3<N>(acc, a, b);
-}
-// acc += S right, S [t][s] read along s
-template <int N>
-__device__ __forceinline__ void along_step(float (&acc)[N][4], const float* S, const float* right, int rld, int s,
-                                           int g, int j) {
-    const float2 x = *reinterpret_cast<const float2*>(S + g * SLD + 8 * s + 2 * j);
-    const float2 y = *reinterpret_cast<const float2*>(S + (g + 8) * SLD + 8 * s + 2 * j);
-    const Left a = left_from(x.x, y.x, x.y, y.y);
-    const float* r = right + (8 * s + 2 * j) * rld + g;
-    float2 b[N];
-#pragma unroll
-    for (int t = 0; t < N; ++t) b[t] = make_float2(r[8 * t], r[rld + 8 * t]);
-    product3<N>(acc, a, b);
-}
-
-// A block a (chunk, head); eight warps, since what bounds it is how many warps an SM holds to issue
-// the short phases' instructions (with four warps and two blocks an SM 130 us for 2,000 rows of 32 heads).
-__global__ void __launch_bounds__(256, 3)
+// A block a (chunk, head), eight warps; two halves of them where there are two things to do.  What
+// is not finite in a row reaches that row's results and later ones alone: products between rows take
+// the rows that count, not zeros for the others.
+__global__ void __launch_bounds__(256, 2)
 delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k_off, int v_off, int a_off,
                         const float* __restrict__ wpre, const float* __restrict__ w_bias,
                         const float* __restrict__ a_bias, float rate, float unit_eps, Step st, float* __restrict__ out,
                         int heads) {
     extern __shared__ __align__(16) float sm[];
-    float *Us = sm, *Rs = Us + L * LD, *Ks = Rs + L * LD, *Ps = Ks + L * LD, *Vs = Ps + L * LD, *Zs = Vs + L * VLD;
-    float *As = Zs + L * VLD, *Bs = As + L * SLD, *Cs = Bs + L * SLD, *Es = Cs + L * SLD;
-    __shared__ float wl[D];
+    float *Us = sm, *Rs = Us + L * LD, *Ks = Rs + L * LD, *Ps = Ks + L * LD, *Vs = Ps + L * LD, *Zs = Vs + L * LD;
+    float *As = Zs + L * LD, *Bs = As + L * SLD, *Cs = Bs + L * SLD, *Es = Cs + L * SLD;
+    __shared__ __align__(16) float wl[D];
     pdl_prologue();
     const int seq = st.round.seq0 + blockIdx.y, h = blockIdx.z;
     const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows;
     const int first = from + blockIdx.x * L, n = min(L, min(st.seq_row0[seq + 1], from + st.round.seg_rows) - first);
     if (n <= 0) return;
-    const int hd = heads * D, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
+    const int hd = heads * D, tid = threadIdx.x;
     float* ws = Zs;  // the rows' decays, until the right sides take their place
 #pragma unroll
     for (int i = 0; i < L * (D / 4) / 256; ++i) {
@@ -114,8 +91,8 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
         store4(Rs + t * LD + c, r);
         store4(Ks + t * LD + c, k);
         store4(Ps + t * LD + c, make_float4(a.x * u.x, a.y * u.y, a.z * u.z, a.w * u.w));
-        store4(Vs + t * VLD + c, v);
-        store4(ws + t * VLD + c, w);
+        store4(Vs + t * LD + c, v);
+        store4(ws + t * LD + c, w);
     }
     __syncthreads();
     // the decays' products, multiplied row by row (neighbouring rows' ratios are then exact to the
@@ -128,257 +105,246 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
 #pragma unroll 8
             for (int t = 0; t < L; ++t) {
                 x[t * LD] *= W;
-                W *= ws[t * VLD + c];
+                W *= ws[t * LD + c];
             }
             wl[c] = W;
         } else if (part == 1) {
 #pragma unroll 8
             for (int t = 0; t < L; ++t) {
-                W *= ws[t * VLD + c];
+                W *= ws[t * LD + c];
                 x[t * LD] *= W;
             }
         } else {
 #pragma unroll 8
             for (int t = 0; t < L; ++t) {
-                W *= ws[t * VLD + c];
+                W *= ws[t * LD + c];
                 x[t * LD] *= 1.0f / W;
             }
         }
     }
     __syncthreads();
-    // [u; r] [k; p]^T: a warp sixteen rows of u or r by the rows of k or p
+    // [u; r] [k; p]^T, rows s <= t (r) or s < t (u) alone: a thread four rows of u or r by rows tx, tx + 16
+    // of k and p
     {
-        const int m = warp & 3, to_p = warp >> 2, m0 = 16 * (m & 1);
-        const float* left = sm + (16 * m + g) * LD + 2 * j;  // Rs follows Us
-        const float* right = Ks + to_p * L * LD;
-        float acc[4][4] = {};
-#pragma unroll 2
-        for (int s = 0; s < D / 8; ++s) {
-            const float2 x = *reinterpret_cast<const float2*>(left + 8 * s);
-            const float2 y = *reinterpret_cast<const float2*>(left + 8 * LD + 8 * s);
-            const Left a = left_from(x.x, y.x, x.y, y.y);
-            float2 b[4];
+        const int tx = tid & 15, m0 = 4 * (tid >> 4), t0 = m0 & (L - 1), own = m0 >= L;
+        const float *a = Us + m0 * LD, *b = Ks + tx * LD;  // Rs follows Us, Ps Ks
+        float* to = As + 2 * own * L * SLD + t0 * SLD + tx;  // As, Bs, Cs, Es
+        auto store = [&](int to_p, int s, const float (&v)[4]) {
+            const float sign = own && to_p ? -1.0f : 1.0f;  // E is only ever taken off
 #pragma unroll
-            for (int t = 0; t < 4; ++t) b[t] = *reinterpret_cast<const float2*>(right + (8 * t + g) * LD + 8 * s + 2 * j);
-            product3<4>(acc, a, b);
-        }
-        const int own = m >> 1, ta = m0 + g, tb = ta + 8;      // rows of r meet their own row too
-        float* to = As + (2 * own + to_p) * L * SLD;           // As, Bs, Cs, Es
-        const float sign = own && to_p ? -1.0f : 1.0f;         // E is only ever taken off
+            for (int i = 0; i < 4; ++i) to[to_p * L * SLD + i * SLD + 16 * s] = tx + 16 * s < t0 + i + own ? sign * v[i] : 0.0f;
+        };
+        if (t0 < 16) {
+            float acc[4][2] = {};
+            product_along<2>(acc, a, LD, b, L * LD, D / 16);
+            const float k[4] = {acc[0][0], acc[1][0], acc[2][0], acc[3][0]}, p[4] = {acc[0][1], acc[1][1], acc[2][1], acc[3][1]};
+            store(0, 0, k);
+            store(1, 0, p);
+        } else {
+            float acc[4][4] = {};
+            product_along<4>(acc, a, LD, b, 16 * LD, D / 16);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int s = 8 * t + 2 * j;
-            store2(to + ta * SLD + s, s < ta + own ? sign * acc[t][0] : 0.0f, s + 1 < ta + own ? sign * acc[t][1] : 0.0f);
-            store2(to + tb * SLD + s, s < tb + own ? sign * acc[t][2] : 0.0f, s + 1 < tb + own ? sign * acc[t][3] : 0.0f);
-        }
-    }
-    __syncthreads();
-    {   // A V, the right side beside u W
-        const int m0 = 16 * (warp & 1), n0 = 16 * (warp >> 1);
-        float acc[2][4] = {};
-        const int ks = m0 ? 4 : 2;
-        for (int s = 0; s < ks; ++s) along_step<2>(acc, As + m0 * SLD, Vs + n0, VLD, s, g, j);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            store2(Zs + (m0 + g) * VLD + n0 + 8 * t + 2 * j, acc[t][0], acc[t][1]);
-            store2(Zs + (m0 + g + 8) * VLD + n0 + 8 * t + 2 * j, acc[t][2], acc[t][3]);
+            for (int j = 0; j < 4; ++j) {
+                const float v[4] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j]};
+                store(j >> 1, j & 1, v);
+            }
         }
     }
     __syncthreads();
-    if (tid < 2 * D) {  // (I + B) [Zl | Y] = [A V | u W], a column a thread, in place
-        float* col = tid < D ? Zs + tid : Us + tid - D;
-        const int cld = tid < D ? VLD : LD;
+    const int u = tid & 127, tx = u & 15, ty = u >> 4;  // 4 rows (8 for a 64 x 64 result) by 4 columns
+    const bool upper = tid >= 128;
+    for (int e = tid; e < 2 * L * (D / 4); e += 256) {  // k and p to the chunk's last row
+        float* x = Ks + (e / (D / 4)) * LD + 4 * (e % (D / 4));
+        const float4 v = load4(x), w = load4(wl + 4 * (e % (D / 4)));
+        store4(x, make_float4(v.x * w.x, v.y * w.y, v.z * w.z, v.w * w.w));
+    }
+    float acc[4][4] = {};  // upper: C V - E Zl, the chunk's own results; lower: A V, the right side beside u W
+    if (upper) {
+        product_below<false>(acc, Cs + 4 * ty * SLD, SLD, Vs + 4 * tx, LD, ty);
+    } else {
+        product_below<true>(acc, As + 4 * ty * SLD, SLD, Vs + 4 * tx, LD, ty);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) store4(Zs + (4 * ty + i) * LD + 4 * tx, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+    }
+    __syncthreads();
+    // upper: the chunk's own sum [key 4 ty .., 32 + 4 ty ..][value 4 tx ..]; lower: M
+    float total[2][4][4] = {};
+    if (!upper) {  // (I + B) [Zl | Y] = [A V | u W], a column a thread, in place
+        float* col = u < D ? Zs + u : Us + u - D;
         float x[L];
 #pragma unroll
         for (int t = 0; t < L; ++t) {
-            float v = col[t * cld], v1 = 0.0f;
+            float v = col[t * LD], v1 = 0.0f;
 #pragma unroll
-            for (int l = 0; l + 1 < t; l += 2) {
-                const float2 b = *reinterpret_cast<const float2*>(Bs + t * SLD + l);
+            for (int l = 0; l + 3 < t; l += 4) {
+                const float4 b = load4(Bs + t * SLD + l);
                 v = fmaf(-b.x, x[l], v);
                 v1 = fmaf(-b.y, x[l + 1], v1);
+                v = fmaf(-b.z, x[l + 2], v);
+                v1 = fmaf(-b.w, x[l + 3], v1);
             }
-            if (t & 1) v = fmaf(-Bs[t * SLD + t - 1], x[t - 1], v);
+#pragma unroll
+            for (int l = t / 4 * 4; l < t; ++l) {
+                if (l & 1) v1 = fmaf(-Bs[t * SLD + l], x[l], v1);
+                else v = fmaf(-Bs[t * SLD + l], x[l], v);
+            }
             x[t] = v + v1;
-            col[t * cld] = x[t];
+            col[t * LD] = x[t];
         }
-    } else {  // k and p to the chunk's last row
-        const int c = tid & (D - 1);
-        const float w = wl[c];
-        float* x = (tid < 3 * D ? Ks : Ps) + c;
-#pragma unroll 8
-        for (int t = 0; t < L; ++t) x[t * LD] *= w;
+    } else {
+        product_down(total, Ks + 4 * ty, LD, L, Vs + 4 * tx, LD, L);
     }
     __syncthreads();
     float* place = st.scratch + (chunk::place_in(st.round, L, row0, seq, blockIdx.x) * heads + h) * PLACE;
-    {   // C V - E Zl into the results, r W - E Y for the walk: sixteen rows by 32 columns a warp
-        const int m0 = 16 * (warp & 1), half = (warp >> 1) & 1, n0 = 32 * (warp >> 2);
-        const int ta = m0 + g, tb = ta + 8;
-        float acc[4][4] = {};
-        if (half) {
+    // r W - E Y for the walk (lower), C V - E Zl into the results (upper)
+    if (!upper) {
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const float2 x = *reinterpret_cast<const float2*>(Rs + ta * LD + n0 + 8 * t + 2 * j);
-                const float2 y = *reinterpret_cast<const float2*>(Rs + tb * LD + n0 + 8 * t + 2 * j);
-                acc[t][0] = x.x; acc[t][1] = x.y; acc[t][2] = y.x; acc[t][3] = y.y;
-            }
-        }
-        const int ks = m0 ? 4 : 2;  // rows s <= t alone
-        if (half) {
-            for (int s = 0; s < ks; ++s) along_step<4>(acc, Es + m0 * SLD, Us + n0, LD, s, g, j);
-        } else {
-            for (int s = 0; s < ks; ++s) along_step<4>(acc, Es + m0 * SLD, Zs + n0, VLD, s, g, j);
-            for (int s = 0; s < ks; ++s) along_step<4>(acc, Cs + m0 * SLD, Vs + n0, VLD, s, g, j);
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int c = n0 + 8 * t + 2 * j;
-            if (half) {
-                store2(place + (D + ta) * LD + c, acc[t][0], acc[t][1]);
-                store2(place + (D + tb) * LD + c, acc[t][2], acc[t][3]);
-            } else {
-                if (ta < n) store2(out + (size_t)(first + ta) * hd + h * D + c, acc[t][0], acc[t][1]);
-                if (tb < n) store2(out + (size_t)(first + tb) * hd + h * D + c, acc[t][2], acc[t][3]);
-            }
+        for (int i = 0; i < 4; ++i) {
+            const float4 r = load4(Rs + (4 * ty + i) * LD + 4 * tx);
+            acc[i][0] = r.x; acc[i][1] = r.y; acc[i][2] = r.z; acc[i][3] = r.w;
         }
     }
-    {   // the chunk's own sum [value][key] and M, sixteen rows by 32 key channels a warp each
-        const int m0 = 16 * (warp & 3), n0 = 32 * (warp >> 2);
-        float acc[4][4] = {};
-#pragma unroll 1
-        for (int s = 0; s < L / 8; ++s) {
-            down_step<4>(acc, Vs + m0, VLD, 1.0f, Ks + n0, LD, s, g, j);
-            down_step<4>(acc, Zs + m0, VLD, -1.0f, Ps + n0, LD, s, g, j);
-        }
-        float* sum = place + MR + (m0 + g) * D + n0 + 2 * j;
+    product_below<false>(acc, Es + 4 * ty * SLD, SLD, (upper ? Zs : Us) + 4 * tx, LD, ty);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            store2(sum + 8 * t, acc[t][0], acc[t][1]);
-            store2(sum + 8 * D + 8 * t, acc[t][2], acc[t][3]);
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int row = m0 + g + (i & 2 ? 8 : 0), c = n0 + 8 * t + 2 * j + (i & 1);
-                acc[t][i] = row == c ? wl[c] : 0.0f;
-            }
-#pragma unroll 1
-        for (int s = 0; s < L / 8; ++s) down_step<4>(acc, Ps + m0, LD, -1.0f, Us + n0, LD, s, g, j);
-        float* M = place + (m0 + g) * LD + n0 + 2 * j;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            store2(M + 8 * t, acc[t][0], acc[t][1]);
-            store2(M + 8 * LD + 8 * t, acc[t][2], acc[t][3]);
-        }
+    for (int i = 0; i < 4; ++i) {
+        const int t = 4 * ty + i;
+        const float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        if (!upper) store4(place + (D + t) * LD + 4 * tx, v);
+        else if (t < n) store4(out + (size_t)(first + t) * hd + h * D + 4 * tx, v);
     }
+    // the chunk's own sum - p'^T Zl (upper), M = diag(W_last) - p'^T Y (lower)
+    product_down<true>(total, Ps + 4 * ty, LD, L, (upper ? Zs : Us) + 4 * tx, LD, L);
+    float* to = (upper ? place + MR : place) + 4 * tx;
+    const int ld_to = upper ? D : LD;
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int key = 32 * half + 4 * ty + i;
+            if (!upper) {
+                const float w = wl[key];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (key == 4 * tx + j) total[half][i][j] += w;
+            }
+            store4(to + key * ld_to, make_float4(total[half][i][0], total[half][i][1], total[half][i][2], total[half][i][3]));
+        }
 }
 
-// A block a (sequence, head, 16 value columns) walks the chunks.  S^T is the left operand of both
-// products, held whole (split) by each of the four warps; a warp makes sixteen key channels of the
-// next S^T and eight of the chunk's rows, and the warps exchange their parts through shared memory,
-// one barrier a chunk.  M and R of the next chunks arrive meanwhile.
-__global__ void __launch_bounds__(128)
+// A block a (sequence, head, COLS value columns) walks the chunks: [M; R] S, 96 rows by COLS columns over 64
+// key channels.  Four lanes make a tile of 4 x 4, each a quarter of the channels (four of each
+// sixteen), whose parts meet by shuffles, so that a chunk has one barrier.  (The quarters in warps of
+// their own, meeting in shared memory: no faster; a thread a row and eight columns, all channels:
+// 121 us in place of 99 for 64 chunks of 32 heads.)  M and R of the next chunks arrive meanwhile.
+// What bounds a step is the latency of its reads of shared memory.  Sixteen columns a block, eight where
+// that leaves SMs without a block: both kernels take 240 and 302 us for 2,048 rows of 32 heads with
+// eight and sixteen, 460 and 442 for 64 heads.
+constexpr int TLD = D + 16;  // sixteen floats more: two columns' sixteens meet all banks
+template <int COLS>
+__global__ void __launch_bounds__(COLS * (D + L) / 4)
 delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stride, long long state_off,
                         float* __restrict__ out, int heads) {
+    constexpr int CG = COLS / 4, THREADS = CG * (D + L);
     extern __shared__ __align__(16) float sm[];
-    __shared__ __align__(16) float4 part[2][D / 8][32];
+    __shared__ __align__(16) float Ss[2][COLS * TLD];  // S^T, column 4 c + j at row CG j + c
     pdl_prologue();
-    const int seq = st.round.seq0 + blockIdx.x, h = blockIdx.y, c0 = 16 * blockIdx.z;
+    const int seq = st.round.seq0 + blockIdx.x, h = blockIdx.y, c0 = COLS * blockIdx.z;
     const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows;
     const int rows = min(st.seq_row0[seq + 1] - from, st.round.seg_rows);
     if (rows <= 0) return;
-    const int chunks = (rows + L - 1) / L, hd = heads * D;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
+    const int chunks = (rows + L - 1) / L, hd = heads * D, tid = threadIdx.x;
+    const int quarter = tid & 3, cg = tid >> 2 & (CG - 1), first_row = 4 * (tid / COLS);  // the tile's first row
+    const int row = first_row + quarter, c = c0 + 4 * cg;  // whose results the lane ends up with, and their columns
     const float* base = st.scratch + (chunk::place_in(st.round, L, row0, seq, 0) * heads + h) * PLACE;
     const size_t step = (size_t)heads * PLACE;
-    auto fetch = [&](int c) {
-        if (c < chunks) {
-            const float* src = base + c * step;
-            float* dst = sm + (c % STAGES) * MR;
-            for (int e = tid; e < MR / 4; e += 128) attn::cp_async_16(dst + 4 * e, src + 4 * e, true);
+    int to = 0;
+    auto fetch = [&](int k) {
+        if (k < chunks) {
+            const float* src = base + k * step;
+            float* dst = sm + to * MR;
+            for (int e = tid; e < MR / 4; e += THREADS) attn::cp_async_16(dst + 4 * e, src + 4 * e, true);
         }
         attn::cp_async_commit();
+        to = to + 1 == STAGES ? 0 : to + 1;
     };
 #pragma unroll
-    for (int c = 0; c < STAGES; ++c) fetch(c);
-    float* Sg = state + (size_t)st.seq_slot[seq] * state_stride + state_off + ((size_t)h * D + c0) * D;
-    Left S[D / 8];
-#pragma unroll
-    for (int s = 0; s < D / 8; ++s) {
-        const float2 x = *reinterpret_cast<const float2*>(Sg + (size_t)g * D + 8 * s + 2 * j);
-        const float2 y = *reinterpret_cast<const float2*>(Sg + (size_t)(g + 8) * D + 8 * s + 2 * j);
-        S[s] = left_from(x.x, y.x, x.y, y.y);
+    for (int k = 0; k < STAGES; ++k) fetch(k);
+    float* Sg = state + (size_t)st.seq_slot[seq] * state_stride + state_off + (size_t)h * D * D;
+    for (int e = tid; e < COLS * D / 4; e += THREADS) {
+        const int col = e / (D / 4), k = 4 * (e % (D / 4));
+        store4(Ss[0] + (CG * (col % 4) + col / 4) * TLD + k, load4(Sg + (size_t)(c0 + col) * D + k));
     }
-    float own[2][4], next[2][4];  // the warp's tiles of S^T, and the chunk's own sum they start from
-    auto sums = [&](int c) {
-        const float* d = base + c * step + MR + (c0 + g) * D + 16 * warp + 2 * j;
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const float2 x = *reinterpret_cast<const float2*>(d + 8 * t);
-            const float2 y = *reinterpret_cast<const float2*>(d + 8 * D + 8 * t);
-            next[t][0] = x.x; next[t][1] = x.y; next[t][2] = y.x; next[t][3] = y.y;
-        }
+    float4 own = make_float4(0.0f, 0.0f, 0.0f, 0.0f), next = own;  // what the products are added to: the chunk's
+    auto ahead = [&](int k) {                                       // own sum, or its own results
+        if (row < D) next = load4(base + k * step + MR + row * D + c);
+        else if (row - D < rows - k * L) next = load4(out + (size_t)(from + k * L + row - D) * hd + h * D + c);
     };
-    sums(0);
+    ahead(0);
     attn::cp_async_wait<STAGES - 1>();
     __syncthreads();
-    for (int c = 0; c < chunks; ++c) {
-        const float* M = sm + (c % STAGES) * MR;
-        const float* R = M + D * LD;
-        const int first = from + c * L, t0 = 8 * warp + 2 * j;
-        float* o = out + (size_t)(first + t0) * hd + h * D + c0 + g;
-        const bool la = t0 < rows - c * L, lb = t0 + 1 < rows - c * L;
-        float O[4] = {};
-        if (la) {
-            O[0] = o[0];
-            O[2] = o[8];
+    int at = 0;
+    for (int k = 0; k < chunks; ++k) {
+        const float* m = sm + at * MR + first_row * LD + 4 * quarter;
+        const float* S = Ss[k & 1] + cg * TLD + 4 * quarter;
+        float* Sn = Ss[(k + 1) & 1];
+        at = at + 1 == STAGES ? 0 : at + 1;
+        own = next;
+        if (k + 1 < chunks) ahead(k + 1);
+        float acc[4][4] = {};
+#pragma unroll
+        for (int s = 0; s < D; s += 16) {
+            float4 x[4], y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = load4(m + i * LD + s);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = load4(S + CG * j * TLD + s);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[i][j] = fmaf(x[i].x, y[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(x[i].y, y[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(x[i].z, y[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(x[i].w, y[j].w, acc[i][j]);
+                }
         }
-        if (lb) {
-            O[1] = o[hd];
-            O[3] = o[hd + 8];
+        // row i's four parts to lane i of the four
+        const bool odd = quarter & 1, high = quarter & 2;
+        float half[2][4], sum[4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float give = odd ? acc[2 * i][j] : acc[2 * i + 1][j];
+                half[i][j] = (odd ? acc[2 * i + 1][j] : acc[2 * i][j]) + __shfl_xor_sync(0xffffffffu, give, 1);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float give = high ? half[0][j] : half[1][j];
+            sum[j] = (high ? half[1][j] : half[0][j]) + __shfl_xor_sync(0xffffffffu, give, 2);
         }
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) own[t][i] = next[t][i];
-        if (c + 1 < chunks) sums(c + 1);
-        float Q[1][4] = {};
-#pragma unroll
-        for (int s = 0; s < D / 8; ++s) {
-            float2 b[2], r[1];
-#pragma unroll
-            for (int t = 0; t < 2; ++t)
-                b[t] = *reinterpret_cast<const float2*>(M + (16 * warp + 8 * t + g) * LD + 8 * s + 2 * j);
-            r[0] = *reinterpret_cast<const float2*>(R + (8 * warp + g) * LD + 8 * s + 2 * j);
-            product3<2>(own, S[s], b);
-            product3<1>(Q, S[s], r);
-        }
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-            part[c & 1][2 * warp + t][lane] = make_float4(own[t][0], own[t][1], own[t][2], own[t][3]);
-        if (la) {
-            o[0] = O[0] + Q[0][0];
-            o[8] = O[2] + Q[0][2];
-        }
-        if (lb) {
-            o[hd] = O[1] + Q[0][1];
-            o[hd + 8] = O[3] + Q[0][3];
+        own.x += sum[0];
+        own.y += sum[1];
+        own.z += sum[2];
+        own.w += sum[3];
+        if (row < D) {
+            Sn[cg * TLD + row] = own.x;
+            Sn[(CG + cg) * TLD + row] = own.y;
+            Sn[(2 * CG + cg) * TLD + row] = own.z;
+            Sn[(3 * CG + cg) * TLD + row] = own.w;
+        } else if (row - D < rows - k * L) {
+            store4(out + (size_t)(from + k * L + row - D) * hd + h * D + c, own);
         }
         attn::cp_async_wait<STAGES - 2>();
-        __syncthreads();  // the parts and the next chunk's factors are there; this chunk's have been read
-        fetch(c + STAGES);
-#pragma unroll
-        for (int s = 0; s < D / 8; ++s) {
-            const float4 p = part[c & 1][s][lane];
-            S[s] = left_from(p.x, p.z, p.y, p.w);
-        }
+        __syncthreads();  // the next S and the next chunk's factors are there; this chunk's have been read
+        fetch(k + STAGES);
     }
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        float* to = Sg + (size_t)g * D + 16 * warp + 8 * t + 2 * j;
-        store2(to, own[t][0], own[t][1]);
-        store2(to + 8 * D, own[t][2], own[t][3]);
+    if (row < D) {
+        float* s = Sg + (size_t)c * D + row;
+        s[0] = own.x;
+        s[D] = own.y;
+        s[2 * D] = own.z;
+        s[3 * D] = own.w;
     }
 }
 
@@ -418,7 +384,9 @@ extern "C" int rfx_delta_rule_chunk(const float* proj, int ld, int r_off, int k_
     constexpr size_t sm_prep = PREP_FLOATS * sizeof(float), sm_walk = (size_t)STAGES * MR * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_prep);
     if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
+    const bool narrow = (long long)plan.group * heads * (D / 16) <= sm_count();
+    e = narrow ? cudaFuncSetAttribute(delta_chunk_walk_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk)
+               : cudaFuncSetAttribute(delta_chunk_walk_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
     if (e != cudaSuccess) return (int)e;
     for (int seq0 = 0; seq0 < n_seq; seq0 += plan.group)
         for (int seg = 0; seg < plan.n_segs; ++seg) {
@@ -426,8 +394,12 @@ extern "C" int rfx_delta_rule_chunk(const float* proj, int ld, int r_off, int k_
             st.round = chunk::Round{plan.seg_rows, seg, seq0, plan.whole};
             RFX_LAUNCH(delta_chunk_prep_kernel, dim3(chunks, seqs, heads), 256, sm_prep, s, proj, ld, r_off, k_off, v_off,
                        a_off, wpre, w_bias, a_bias, rate, unit_eps, st, out, heads);
-            RFX_LAUNCH(delta_chunk_walk_kernel, dim3(seqs, heads, D / 16), 128, sm_walk, s, st, state, state_stride,
-                       state_off, out, heads);
+            if (narrow)
+                RFX_LAUNCH(delta_chunk_walk_kernel<8>, dim3(seqs, heads, D / 8), 2 * (D + L), sm_walk, s, st, state,
+                           state_stride, state_off, out, heads);
+            else
+                RFX_LAUNCH(delta_chunk_walk_kernel<16>, dim3(seqs, heads, D / 16), 4 * (D + L), sm_walk, s, st, state,
+                           state_stride, state_off, out, heads);
         }
     return 0;
 }
