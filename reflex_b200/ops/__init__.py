@@ -1863,9 +1863,16 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
     return out
 
 
-# rows of the longest sequence from which the chunked kernels run (one sequence, width 2048, the whole
-# mixer: 47 us walking and 48 in chunks at 48 rows, 57 and 40 at 100)
+# Rows of the longest sequence from which the chunked kernels run where a step has up to about 64 (sequence, head)
+# pairs; four times as many beyond, where the walk fills the SMs too and a last chunk's absent rows weigh most.  In
+# chunks and walking, us: 16 pairs 18.5 and 18.1 at 48 rows; 32 pairs 24.6 and 27.6 at 64, 28 and 55 at 128; 64 pairs
+# 27 and 33 at 64; 128 pairs 33 and 34 at 64, 61 and 54 at 100, 62 and 67 at 128; 512 pairs 122 and 117 at 64, 225 and
+# 236 at 128.
 DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_DELTA_CHUNK_MIN_ROWS", 64, 1, 1 << 30)
+
+
+def _delta_in_chunks(most: int, rows: int, heads: int) -> bool:
+    return most > 0 and most >= DELTA_CHUNK_MIN_ROWS * (1 if heads * rows // most <= 64 else 4)
 
 
 def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: int, wpre: torch.Tensor,
@@ -1875,17 +1882,16 @@ def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: in
     v and the removal rate's pre-activation at their column offsets (heads * dim
     each), `wpre` float32 [R, heads * dim] the decay's; the running state is
     `state[slot, state_off : state_off + heads * dim * dim]`.  Returns S^T r,
-    float32 [R, heads * dim].  Without `exact`, from `DELTA_CHUNK_MIN_ROWS` rows of a
+    float32 [R, heads * dim].  Without `exact`, from about `DELTA_CHUNK_MIN_ROWS` rows of a
     sequence on and for heads of 64, the kernels that take 32 rows at a time run
-    (csrc/delta_rule_chunk.cu: the same function, products of 32-bit numbers split for
-    the tensor cores)."""
+    (csrc/delta_rule_chunk.cu: the same function, its sums in another order)."""
     R = proj.shape[0]
     hd = heads * dim
     if max(r_off, k_off, v_off, a_off) + hd > proj.shape[1] or tuple(wpre.shape) != (R, hd):
         raise InvalidInput("delta_rule: the columns do not fit into the rows")
     out = _new((R, hd), torch.float32, proj.device)
     most = _most_rows(batch)
-    if not exact and dim == 64 and most >= DELTA_CHUNK_MIN_ROWS:
+    if not exact and dim == 64 and _delta_in_chunks(most, R, heads):
         S = batch.seq_slot.numel()
         scratch = _new((int(native.lib().rfx_delta_rule_chunk_floats(R, S, most, heads)),), torch.float32, proj.device)
         st = native.lib().rfx_delta_rule_chunk(

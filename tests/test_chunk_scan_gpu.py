@@ -276,9 +276,10 @@ def test_a_long_delta_step_goes_through_a_bounded_scratch():
         assert ((a - b).abs().max() / a.abs().max()).item() < TOL
 
 
-def test_many_sequences_go_through_a_bounded_scratch():
+def test_many_sequences_go_through_a_bounded_scratch(monkeypatch):
     """121 chunks of 64 heads of 256 x 128 where the scratch holds 31, and 260 of the delta rule's of 64 heads where it
     holds 95: rounds of sequences, the longest of them in several; against the walk, a short sum's roundings apart."""
+    monkeypatch.setattr(ops(), "DELTA_CHUNK_MIN_ROWS", 1)
     heads, groups, P, N = 64, 2, 256, 128
     counts = [120 + (i * 7) % 30 for i in range(39)] + [700]
     g = torch.Generator(device=DEV).manual_seed(6)
