@@ -1,6 +1,6 @@
 // The plain attention (attention_plain.cu) of the true 32-bit path, 32 keys and up to sixteen queries
 // at a time: the same operations on the same numbers in the same order, so the same bits, for head
-// sizes that are a multiple of 32.
+// sizes of 32, 64, 128 and 256.
 //
 // The plain kernel's warp walks the keys one after another; every key costs it a butterfly, two
 // exponentials and two loads' latency in a chain (a query of 300 keys: 0.2 ms).  Here the queries of
@@ -23,7 +23,8 @@ using namespace rfx;
 
 constexpr int KEYS = 32, WARPS = 8, QUERIES = 2 * WARPS;
 
-// The score of a lane's key with U queries (`q` of them `step` apart): 32 chains over d / 32 elements, met as a butterfly over lanes meets them.
+// The score of a lane's key with U queries (`q` of them `step` apart): 32 chains over d / 32 elements,
+// met as a butterfly over lanes meets them.
 template <int NI, int U>
 __device__ __forceinline__ void dots(const float* k, const float* q, int step, float (&s)[U]) {
     constexpr int d = 32 * NI;

@@ -210,7 +210,8 @@ int launch(const void* x, const void* W, const int* offsets, void* y, int n_pair
         !rfx::tma::make_map_rows64(&mx, x, n_pairs, K, BN))
         return RFX_ERR_UNSUPPORTED;
     constexpr int STAGE = A_BYTES + BN * BK * 2;
-    // two CTAs an SM: about 100 KB each
+    // two CTAs an SM, about 100 KB each; gated ones for 33 to 64 rows have 16 KB of up values beside the ring and
+    // an SM to themselves
     int stages = 98 * 1024 / STAGE;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     const int nkb = (K + BK - 1) / BK;

@@ -101,7 +101,7 @@ qkv_post_wide_kernel(const TI* __restrict__ qkv, int row_stride, const float* __
     constexpr int HPW = 32 / LPH;  // heads a warp takes at a time
     constexpr int CH = 3;          // units whose loads are in flight together
     constexpr float inv_d = 1.0f / (float)D;
-    // a block has `rows` rows (1, 2, 4 or 8), a row `nwarps` of its warps
+    // a block has `rows` rows (1, 2 or 4), a row `nwarps` of its warps
     const int nwarps = (blockDim.x >> 5) / rows, all_warps = threadIdx.x >> 5;
     const int warp = all_warps % nwarps, lane = threadIdx.x & 31;
     const int r_first = blockIdx.x * rows, r_in = all_warps / nwarps;

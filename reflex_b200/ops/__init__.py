@@ -1155,6 +1155,9 @@ def moe_experts_grouped(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, i
     return ExpertRows(yg, place, out_wts, R, top)
 
 
+# The most rows the kernel takes, all of them worth it: the routed experts in one launch each and by the library's
+# grouped products, 16 experts of 3 x 2,048 x 2,048, 4 chosen: 33 and 66 us with two rows, 70 and 110 with eight, 72 and
+# 111 with 32, 91 and 112 with 64; 64 experts of 3 x 512 x 2,048, 6 chosen: 28 and 43, 48 and 76, 77 and 111, 92 and 112.
 MOE_GEMM_MAX_ROWS = _env_int("REFLEX_B200_MOE_GEMM_MAX_ROWS", 64, 0, 64)
 _GROUPED_MM = [True, True]  # whether the library's grouped product is tried, and its 32-bit output
 
@@ -1776,8 +1779,9 @@ def attention_sigmoid_tc(q, k_pages, v_pages, page_table, page_size, seq_slot, s
     return out
 
 
-# level with the mma.sync form at 24 rows of a sequence (the whole pair at width 2048: 52 us either way),
-# ahead from there on (100 rows 85 -> 80, 2,048 rows 419 -> 322)
+# From two rows of a sequence on: after 1,500 earlier positions (16 heads of 128, window 1,024) 23.2 us and 41.5 on
+# mma.sync with two rows, 24.0 and 61.9 with 24, 25.6 and 68.8 with 64; without earlier positions 4.6 and 4.2 with two
+# rows, 4.6 each with four, 5.4 and 7.2 with 24.
 SIGMOID_TC_MIN_ROWS = _env_int("REFLEX_B200_SIGMOID_TC_MIN_ROWS", 2, 1, 1 << 30)
 
 
@@ -1969,8 +1973,7 @@ def gated_delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor
         native.check(st, f"gated_delta_chunk_prep (heads={heads}, dim={dim})")
         st = native.lib().rfx_gated_delta_chunk(
             qkv.data_ptr(), coef.data_ptr(), _chk(state, "state", torch.float32), state.stride(0), int(state_off),
-            _chk(batch.seq_slot, "seq_slot", torch.int32), row0, S, out.data_ptr(), heads, kv_heads, dim, vdim,
-            device_error_word(qkv.device).data_ptr(), _stream())
+            _chk(batch.seq_slot, "seq_slot", torch.int32), row0, S, out.data_ptr(), heads, kv_heads, dim, vdim, _stream())
         native.check(st, f"gated_delta_chunk (heads={heads}, dim={dim}, vdim={vdim})")
         return out
     st = native.lib().rfx_gated_delta_scan(
