@@ -131,7 +131,7 @@ def mlstm_case(heads, dim, vdim, counts, slots, running, forget):
 
 def mlstm_run(case, heads, dim, vdim, cap=12.0):
     proj, offsets, bi, bf, state, b = case
-    ops().MLSTM_SIDE_BY_SIDE_MIN_ROWS = 1  # (the fixture below puts it back)
+    ops().MLSTM_SIDE_BY_SIDE_MIN_ROWS = 1  # (the fixture above puts it back)
     to = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
     dev = torch.from_numpy(state.copy()).to(DEV)
     num, den = ops().mlstm_scan(to(proj), offsets, to(bi), to(bf), cap, 0.25, b, dev, heads, dim, vdim,
