@@ -40,7 +40,7 @@ inline Plan plan_rounds(int R, int n_seq, int max_rows, int L, long long one) {
 struct Round {
     int seg_rows, seg, seq0, whole;
 };
-// The place of chunk c (of this round) of sequence `seq`, whose first row of the step is row0.
+// The place of chunk c (of round r) of sequence `seq`, whose first row of the step is row0.
 __device__ __forceinline__ size_t place_in(const Round& r, int L, int row0, int seq, int c) {
     return r.whole ? (size_t)row0 / L + seq + c : (size_t)(seq - r.seq0) * (r.seg_rows / L) + c;
 }

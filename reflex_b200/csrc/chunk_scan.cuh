@@ -58,7 +58,7 @@ struct Step {
 
 struct Rows {
     int first, n;  // the chunk's first row and how many it has
-    bool last;     // of its sequence's in this round
+    bool last;     // of its sequence's in the launch's round
     size_t place;
 };
 __device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
