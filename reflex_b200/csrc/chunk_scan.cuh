@@ -1,6 +1,6 @@
 // Recurrences S <- decay S + weight k v^T, y = S^T q with one decay and one weight a head and
 // row (ssd.cu, mlstm.cu) over the many rows of a prompt, 64 rows at a time and all chunks side by
-// side, as products of 32-bit multiply-adds.
+// side, as 32-bit products on the tcgen05 tensor cores (tc_split.cuh).
 //
 //   chunk_state_kernel   what each chunk adds to the memory, from zero: sum_s W_s k_s v_s^T
 //   chunk_carry_kernel   the memory before each chunk, chunk after chunk, element by element; the
@@ -16,26 +16,24 @@
 //
 // A walk through the rows has one chain of dependent steps a head and leaves most SMs without
 // work; chunks cost the memory's way out and back (heads x N x P floats each) and about twice the
-// arithmetic.  A prompt of 2,048 rows: 1.2 ms walking and 0.14 ms in chunks for 32 heads of 64 x 128
-// (42 us the chunks' sums, 20 the carry, 80 the rows), 0.76 and 0.15 ms for 8 of 128 x 256 (49, 30 and
-// 73); the carry is bound by L2, the other two issue on half of the cycles (sixteen warps an SM, shared
-// memory half busy).  64 rows: with 32 the memories' traffic doubles, with 128 the products inside the
-// chunk do and a block no longer shares its SM.
+// arithmetic.  64 rows: with 32 the memories' traffic doubles, with 128 the products inside the chunk do.
+// A prompt of 2,048 rows, us: for 32 heads of 64 x 128 21 the chunks' sums, 13 the carry, 50 the rows (1,200
+// walking), for 8 of 128 x 256 24, 18 and 50 (760).  With the products by 32-bit multiply-adds, whose reads of
+// shared memory and whose latencies bound them, 42, 12 and 76, and 49, 18 and 65.  What bounds these now is
+// the instructions that take 32-bit numbers apart and put results together (about 1,500 a warp and item, 1.7 of
+// four issued a cycle); the tensor cores are busy a fifth of the time, the carry is bound by L2.
 //
-// The same products on the tensor cores, operands split in two parts of 11 bits, took 30 + 20 + 75 and
-// 35 + 27 + 65 us, but are 3 to 15 times as far from 64 bits as the walk (1.5e-6 against 1.1e-7 for the
-// first shape's results, 3.8e-7 against 7e-8 for its state): 1.2e-7 and 7e-8 here, 1.2e-7 and 7e-8 to
-// 1.1e-7 for the second shape, whose chunkwise form on CUDA cores stands at 6e-7 and 1e-6.
+// 2-norm errors against 64 bits, the same shapes: results 1.2e-7 and 1.0e-7 (1.24e-7 and 1.2e-7 by
+// multiply-adds), states 7.1e-8 and 6.2e-8 to 1.1e-7 (7.0e-8 and 5.8e-8 to 1.1e-7).
 //
 // A policy `Pol` gives: q, k, v rows (float32, 16-byte aligned, counts in fours), `heads`, `per`
 // (heads per q/k head), N (elements of q and k, at most 128), P (elements of v) and the functions
 // named below.  A long step goes through a bounded scratch in several rounds (chunk_plan.cuh).
 #pragma once
 
-#include "attn_mma.cuh"
 #include "chunk_plan.cuh"
 #include "common.cuh"
-#include "fma_tiles.cuh"
+#include "tc_split.cuh"
 
 namespace chunk {
 
@@ -43,8 +41,10 @@ using namespace rfx;
 
 constexpr int L = 64;     // rows of a chunk
 constexpr int PT = 64;    // elements of v a block takes at a time
-constexpr int VLD = PT + 4, WLD = L + 4;  // row strides of v's tile and of the rows' weights
-constexpr int THREADS = 256;
+constexpr int STATE_THREADS = 256, WARPS = STATE_THREADS / 32, OUT_THREADS = 512;
+constexpr int OLD = 68;   // row stride of results in shared memory
+constexpr uint32_t TMEM_COLS = 256;  // two blocks share an SM
+constexpr size_t SMEM = 4 * split3::TILE + 1024;  // (aligned by the kernels)
 
 struct Step {
     const int* seq_slot;
@@ -54,6 +54,7 @@ struct Step {
     float4* aux;     // [place][head]: what the carry needs of a chunk
     float* before;   // [place][head]: the policy's running number before the chunk
     float4* rows;    // [place][head][L][RECORDS]: the policy's records of the chunk's rows
+    int* err;        // where a wait that ran out is reported
 };
 
 struct Rows {
@@ -68,81 +69,183 @@ __device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
     return {first, min(L, to - first), to - first <= L, place_in(s.round, L, row0, seq, c)};
 }
 
-// A tile of 64 rows of 4 * c4 floats, rows from n on and columns from n4 (in fours) on zero.  SPREAD: row
-// r lies at 16 (r % 4) + r / 4, so that the threads that own four neighbouring rows each read, row by
-// row, rows side by side (an odd number of 16 bytes apart: eight of them meet all banks).
-template <bool SPREAD>
-__device__ __forceinline__ void load_tile(float* dst, int ld, const float* src, size_t src_ld, int n, int c4, int n4) {
-    auto at = [&](int r) { return dst + (SPREAD ? (r & 3) * 16 + (r >> 2) : r) * ld; };
-    if (THREADS % c4 == 0) {  // a thread keeps its column: no division a piece
-        const int c = threadIdx.x % c4, step = THREADS / c4;
-        int r = threadIdx.x / c4;
-        const float* s = src + (size_t)r * src_ld + 4 * c;
-        const int live = c < n4 ? n : 0;
-        for (; r < 64; r += step, s += (size_t)step * src_ld) attn::cp_async_16(at(r) + 4 * c, r < live ? s : src, r < live);
-    } else {
-        for (int e = threadIdx.x; e < 64 * c4; e += THREADS) {
-            const int r = e / c4, c = e - r * c4;
-            const bool ok = r < n && c < n4;
-            attn::cp_async_16(at(r) + 4 * c, ok ? src + (size_t)r * src_ld + 4 * c : src, ok);
+// What both tensor-core kernels of a block hold: the barrier its products arrive at, the tensor memory, and
+// whether a wait ran out (reported; nothing waits after that, and the block ends with what is there).
+struct Core {
+    uint32_t tmem;
+    uint64_t* done;
+    uint32_t phase;  // of either barrier, in a bit each
+    bool waits;
+    int* err;
+
+    // Every thread, before a barrier of the block: its products' barriers and its tensor memory.
+    __device__ __forceinline__ void open(uint64_t* bars, uint32_t* slot, int* error) {
+        done = bars;
+        phase = 0;
+        waits = true;
+        err = error;
+        if (threadIdx.x == 0) {
+            sm100::mbar_init(done, 1);
+            sm100::mbar_init(done + 1, 1);
+            sm100::fence_barrier_init();
+        }
+        if (threadIdx.x < 32) {
+            sm100::tmem_alloc(slot, TMEM_COLS);
+            sm100::tmem_relinquish();
         }
     }
+    // Products that one thread issues once all have passed this barrier; true if any thread saw odd numbers.
+    template <class Issue>
+    __device__ __forceinline__ bool start(int bar, bool odd, Issue&& issue) {
+        split3::tiles_written();
+        const bool any = __syncthreads_or(odd);
+        if (threadIdx.x < 32) {
+            sm100::tc_fence_after_sync();
+            if (sm100::elect_one()) {
+                issue();
+                sm100::umma_commit(done + bar);
+            }
+            __syncwarp();
+        }
+        return any;
+    }
+    __device__ __forceinline__ void wait(int bar) {
+        if (waits && !sm100::mbar_wait(done + bar, phase >> bar & 1)) {
+            waits = false;
+            if (err) atomicExch(err, 42);
+        }
+        phase ^= 1u << bar;
+        sm100::tc_fence_after_sync();
+    }
+    __device__ __forceinline__ void close(uint32_t slot) {
+        sm100::tc_fence_before_sync();
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            sm100::tc_fence_after_sync();
+            sm100::tmem_dealloc(slot, TMEM_COLS);
+        }
+    }
+};
+__device__ __forceinline__ char* tiles_of(char* sm) {  // shared memory from a boundary of 1,024 bytes on
+    return sm + (-(int)sm100::smem_u32(sm) & 1023);
 }
-
-// A block a (chunk, head, PT elements of v): the chunk's own sum, [P][N].
+// A block a (chunk, q/k head, some of that head's items); an item is a (head, PT elements of v): the
+// chunk's own sums, [P][N], as k's elements (128 lanes) by v's.  k is split once, the heads' weights come from
+// a warp each; an item's product runs while the one before is stored and the next one's v is on its way.
 template <class Pol>
-__global__ void __launch_bounds__(THREADS, 2) chunk_state_kernel(Pol pol, Step st) {
-    extern __shared__ __align__(16) float sm[];
-    __shared__ float wl[L];
+__global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, Step st, int items_a_block) {
+    extern __shared__ __align__(16) char sm_raw[];
+    __shared__ float wl[WARPS][L];
+    __shared__ uint64_t bars[2];
+    __shared__ uint32_t tmem_slot;
     rfx::pdl_prologue();
     const int seq = st.round.seq0 + blockIdx.y;
     const Rows ch = rows_of(st, seq, blockIdx.x);
     if (ch.n <= 0) return;
-    const int ptiles = (pol.P + PT - 1) / PT, h = blockIdx.z / ptiles, p0 = (blockIdx.z - h * ptiles) * PT;
-    const bool wide = pol.N > 64;
-    const int ldk = wide ? 132 : 68;
-    float *Vs = sm, *Ks = sm + L * VLD;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    load_tile<false>(Vs, VLD, pol.v_row(ch.first, h) + p0, pol.ldv, ch.n, PT / 4, min(PT, pol.P - p0) / 4);
-    load_tile<false>(Ks, ldk, pol.k_row(ch.first, h), pol.ldk, ch.n, wide ? 32 : 16, pol.N / 4);
-    attn::cp_async_commit();
-    const size_t at = ch.place * pol.heads + h;
-    if (tid < 32) {
-        const float4 a = pol.state_weights(wl, p0 == 0 ? st.rows + at * L * Pol::RECORDS : nullptr, h, ch.first, ch.n, tid);
-        if (p0 == 0 && tid == 0) st.aux[at] = a;
-    }
-    attn::cp_async_wait<0>();
-    __syncthreads();
-    for (int e = tid; e < L * PT / 4; e += THREADS) {  // the weights go into v
-        float* v = Vs + (e >> 4) * VLD + 4 * (e & 15);
-        const float4 x = load4(v);
-        const float w = wl[e >> 4];
-        store4(v, make_float4(x.x * w, x.y * w, x.z * w, x.w * w));
-    }
-    __syncthreads();
+    const int ptiles = (pol.P + PT - 1) / PT, items = pol.per * ptiles;
+    const int sets = (items + items_a_block - 1) / items_a_block;
+    const int kvh = blockIdx.z / sets, i0 = (blockIdx.z - kvh * sets) * items_a_block;
+    const int i1 = min(items, i0 + items_a_block), h0 = kvh * pol.per + i0 / ptiles;
+    char *Ks = tiles_of(sm_raw), *Vs = Ks + 2 * split3::TILE;  // k's two tiles of 64 elements, v of two items
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
-    float* out = st.scratch + at * E;
-    const int p = p0 + 4 * ty;
-    if (p < pol.P) {
-        float acc[2][4][4] = {};  // [half of k's elements][element of k][of v]
-        const int rows = (ch.n + 15) / 16 * 16;
-        product_down(acc, Ks + 4 * tx, ldk, wide ? 64 : 0, Vs + 4 * ty, VLD, rows);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const int n = 64 * t + 4 * tx;
-            if (n < pol.N)
-#pragma unroll
-                for (int i = 0; i < 4; ++i)  // (P is a multiple of four)
-                    store4(out + (size_t)(p + i) * pol.N + n, make_float4(acc[t][0][i], acc[t][1][i], acc[t][2][i], acc[t][3][i]));
+    Core core;
+    core.open(bars, &tmem_slot, st.err);
+    using Own = split3::Own<STATE_THREADS>;
+    auto bring = [&](Own& v, int item) {
+        const int p0 = (item % ptiles) * PT;
+        v.load(pol.v_row(ch.first, kvh * pol.per + item / ptiles) + p0, pol.ldv, ch.n, pol.P - p0);
+    };
+    Own v, k0, k1;
+    k0.load(pol.k_row(ch.first, kvh * pol.per), pol.ldk, ch.n, pol.N);
+    k1.load(pol.k_row(ch.first, kvh * pol.per) + 64, pol.ldk, ch.n, pol.N - 64);
+    bring(v, i0);
+    {
+        const int h = h0 + warp;
+        if (h <= kvh * pol.per + (i1 - 1) / ptiles) {
+            const size_t to = ch.place * pol.heads + h;
+            const bool first = warp || i0 % ptiles == 0;  // the head's first item is this block's
+            const float4 a = pol.state_weights(wl[warp], first ? st.rows + to * L * Pol::RECORDS : nullptr, h, ch.first, ch.n, lane);
+            if (first && lane == 0) st.aux[to] = a;
         }
     }
-    if (Pol::NORMALISER && p0 == 0)
-        for (int n = tid; n < pol.N; n += THREADS) {
-            float a[4] = {};
-#pragma unroll 4
-            for (int s = 0; s < L; ++s) a[s & 3] = fmaf(wl[s], Ks[s * ldk + n], a[s & 3]);  // rows from n on: zeros
-            out[(size_t)pol.P * pol.N + n] = (a[0] + a[1]) + (a[2] + a[3]);
+    bool odd_k = k0.put(Ks);
+    odd_k |= k1.put(Ks + split3::TILE);
+    sm100::tc_fence_before_sync();
+    __syncthreads();
+    sm100::tc_fence_after_sync();
+    core.tmem = tmem_slot;
+    if (Pol::NORMALISER && i0 % ptiles == 0) {  // the head's sum of k (it is the block's only head), a thread's rows first
+        float* part = reinterpret_cast<float*>(Vs + split3::TILE);
+        float* mine = part + (tid >> 3) * 128 + Own::col();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float a = 0.0f, b = 0.0f;
+#pragma unroll
+            for (int i = 0; i < Own::ROWS; ++i) {
+                a = fmaf(wl[0][Own::row(i)], k0.x[i][j], a);
+                b = fmaf(wl[0][Own::row(i)], k1.x[i][j], b);
+            }
+            mine[j] = a;
+            mine[64 + j] = b;
         }
+        __syncthreads();
+        if (tid < pol.N) {
+            float a[4] = {};
+#pragma unroll
+            for (int i = 0; i < STATE_THREADS / 8; ++i) a[i & 3] += part[i * 128 + tid];
+            st.scratch[(ch.place * pol.heads + h0) * E + (size_t)pol.P * pol.N + tid] = (a[0] + a[1]) + (a[2] + a[3]);
+        }
+    }
+    const uint32_t k_at = sm100::smem_u32(Ks);
+    const int n = 32 * (warp & 3) + lane, half = 32 * (warp >> 2);  // the thread's element of k and 32 of v's
+    bool any_odd = false;  // in the item that is being multiplied
+    auto store = [&](int item) {
+        const int h = kvh * pol.per + item / ptiles;
+        core.wait(0);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int p0 = (item % ptiles) * PT + half + 8 * c;
+            float y[8];
+            split3::sums_of<2>(y, core.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + half + 8 * c, split3::sets<2>(L / 16));
+            if (n >= pol.N) continue;
+            if (any_odd) {  // the odd numbers' products
+                const float *k = pol.k_row(ch.first, h) + n, *x = pol.v_row(ch.first, h);
+                for (int s = 0; s < ch.n; ++s) {
+                    const float ks = k[(size_t)s * pol.ldk];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float vs = x[(size_t)s * pol.ldv + min(p0 + i, pol.P - 1)] * wl[h - h0][s];
+                        if (split3::is_odd(ks) || split3::is_odd(vs)) y[i] = fmaf(ks, vs, y[i]);
+                    }
+                }
+            }
+            float* to = st.scratch + (ch.place * pol.heads + h) * E + (size_t)p0 * pol.N + n;
+            const int left = pol.P - p0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i, to += pol.N)
+                if (i < left) *to = y[i];
+        }
+    };
+    for (int item = i0; item < i1; ++item) {
+        const int h = kvh * pol.per + item / ptiles;
+        const float* weights = wl[h - h0];
+        char* V = Vs + ((item - i0) & 1) * split3::TILE;  // (the product that read it two items ago has been waited for)
+#pragma unroll
+        for (int i = 0; i < Own::ROWS; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v.x[i][j] *= weights[Own::row(i)];
+        const bool odd = v.put(V) || odd_k;
+        if (item + 1 < i1) bring(v, item + 1);
+        if (item > i0) store(item - 1);
+        any_odd = core.start(0, odd, [&] {
+            split3::issue128<2, split3::MN_STEP, split3::MN_STEP>(core.tmem, split3::A_MN | split3::B_MN, L / 16,
+                                                                  split3::mn_major(k_at, split3::TILE),
+                                                                  split3::mn_major(sm100::smem_u32(V), split3::PART));
+        });
+    }
+    store(i1 - 1);
+    core.close(tmem_slot);
 }
 
 // Four neighbouring elements of a head's memory a thread; eight chunks' sums are fetched ahead.
@@ -215,6 +318,13 @@ __device__ __forceinline__ void two_parts(double v, float* hi, float* lo) {
     *hi = h;
     *lo = isinf(h) ? 0.0f : (float)(v - (double)h);
 }
+// e^v as exactly as expf has it, where a v rounded to 32 bits would be off by 2^-25 v
+__device__ __forceinline__ float exp_of(double v) {
+    float hi, lo;
+    two_parts(v, &hi, &lo);
+    const float e = expf(hi);
+    return fmaf(e, lo, e);
+}
 
 // What a row t brings to its results: w_ts = exp((g_s + e_t)) * w_s with e in two parts, the factor of
 // q . S, and a number for the policy's store.
@@ -222,15 +332,21 @@ struct RowTerms {
     float e_hi, e_lo, alpha, extra;
 };
 
-// A block a (chunk, q/k head, some of that head's items); an item is a (head, PT elements of v).  The
-// rows' products with the chunk's k, once, stay in registers; then head by head they become the rows'
-// weights in shared memory, and item by item the memory's tile and v's come and meet q and the weights.
-// A row never multiplies a later row's v, so what is not finite there does not reach it.
+// A block a (chunk, q/k head, some of that head's items).  The rows' products with the chunk's k, once,
+// stay in registers.  Item by item q meets the memory's tile; meanwhile head by head the products become the
+// rows' weights, which then meet v.  A warp has the weights of sixteen rows by sixteen, a thread those of a row
+// by eight; results as it has v (split3::Own).
+//
+// A row's weights of later rows are zero, and a number that is not finite is no operand of the tensor core
+// (tc_split.cuh): its products are added afterwards to the rows it may reach, so that it does not reach others.
 template <class Pol>
-__global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Pol pol, Step st, int items_a_block) {
-    extern __shared__ __align__(16) float sm[];
+__global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step st, int items_a_block) {
+    extern __shared__ __align__(16) char sm_raw[];
     __shared__ __align__(16) float4 rec[L * Pol::RECORDS];
-    __shared__ float nv[128];
+    __shared__ float early[3][48];  // the weights of rows before a sixteen, up to its first row
+    __shared__ float row_sum[Pol::NORMALISER ? 8 : 1][L];
+    __shared__ uint64_t bars[2];
+    __shared__ uint32_t tmem_slot;
     rfx::pdl_prologue();
     const int seq = st.round.seq0 + blockIdx.y;
     const Rows ch = rows_of(st, seq, blockIdx.x);
@@ -239,94 +355,230 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_out_kernel(Pol pol, Step st,
     const int sets = (items + items_a_block - 1) / items_a_block;
     const int kvh = blockIdx.z / sets, i0 = (blockIdx.z - kvh * sets) * items_a_block;
     const int i1 = min(items, i0 + items_a_block);
-    const int n16 = (pol.N + 15) / 16, ld = 16 * n16 + 4;
-    float *Qs = sm, *Bs = sm + L * ld, *Vs = Bs + L * ld, *Ws = Vs + L * VLD;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, t0 = 4 * ty;
-    load_tile<false>(Qs, ld, pol.q_row(ch.first, kvh * pol.per), pol.ldq, ch.n, 4 * n16, pol.N / 4);
-    load_tile<true>(Bs, ld, pol.k_row(ch.first, kvh * pol.per), pol.ldk, ch.n, 4 * n16, pol.N / 4);
-    attn::cp_async_commit();
-    attn::cp_async_wait<0>();
+    // q's two tiles of 64 elements; two tiles of k, then an item's two of the memory, then its weights and v;
+    // between them 32-bit results.  (The products of 64 rows are made as of 128, whose other half reads what lies
+    // behind a tile and is left where it is.)
+    char *Qs = tiles_of(sm_raw), *Bs = Qs + 2 * split3::TILE, *Ws = Bs, *Vs = Bs + split3::TILE;
+    float* res = reinterpret_cast<float*>(Bs);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int blocks = pol.N > 64 ? 2 : 1, t = 16 * (warp >> 2) + (lane & 15), sb = (warp + (warp >> 2)) & 3, s0 = 16 * sb + 8 * (lane >> 4);
+    const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
+    Core core;
+    core.open(bars, &tmem_slot, st.err);
+    const float *q = pol.q_row(ch.first, kvh * pol.per), *k = pol.k_row(ch.first, kvh * pol.per);
+    using Own = split3::Own<OUT_THREADS>;
+    bool odd_qk = false;
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+        if (b < blocks) {
+            Own x, y;
+            x.load(q + 64 * b, pol.ldq, ch.n, pol.N - 64 * b);
+            y.load(k + 64 * b, pol.ldk, ch.n, pol.N - 64 * b);
+            odd_qk |= x.put(Qs + b * split3::TILE);
+            odd_qk |= y.put(Bs + b * split3::TILE);
+        }
+    sm100::tc_fence_before_sync();
     __syncthreads();
-    const float *qa = Qs + t0 * ld, *ba = Bs + tx * ld;
-    float G[4][4] = {};  // rows t0 .. by rows 4 tx .. of k, where any of those is no later
-    if (tx <= ty) product_along<4>(G, qa, ld, ba, 16 * ld, n16);
-    int head = -1;
+    sm100::tc_fence_after_sync();
+    core.tmem = tmem_slot;
+    const uint32_t q_at = sm100::smem_u32(Qs), b_at = sm100::smem_u32(Bs);
+    // q by the two tiles at b_at
+    auto q_products = [&] {
+        split3::issue64<4, split3::K_STEP, split3::K_STEP>(core.tmem, 0, (pol.N + 15) / 16, split3::k_major(q_at), split3::k_major(b_at));
+    };
+    // the warp's lanes and sixteen columns of results: row `row`, or what its m part adds (`second`)
+    const int row = 32 * (warp & 1) + lane, c0 = 16 * (warp >> 2);
+    const bool second = warp & 2;
+    const uint32_t lanes = core.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + c0;
+    auto spread = [&](const float (&y)[8], int c) {  // for every thread to read
+        float* to = res + ((second ? L : 0) + row) * OLD + c0 + c;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) store4(to + 4 * i, make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]));
+    };
+    auto read8 = [&](float (&y)[8], const float* from) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float4 r = load4(from + 4 * i), s = load4(from + L * OLD + 4 * i);
+            y[4 * i] = r.x + s.x; y[4 * i + 1] = r.y + s.y; y[4 * i + 2] = r.z + s.z; y[4 * i + 3] = r.w + s.w;
+        }
+    };
+    odd_qk = core.start(0, odd_qk, q_products);
+    core.wait(0);
+#pragma unroll
+    for (int c = 0; c < 16; c += 8) {
+        float y[8];
+        split3::sums_of<4>(y, lanes + c, split3::sets<4>((pol.N + 15) / 16), second);
+        spread(y, c);
+    }
+    sm100::tc_fence_before_sync();
+    __syncthreads();
+    float G[8];  // row t by rows s0 .. of k
+    read8(G, res + t * OLD + s0);
+    if (odd_qk && t < ch.n)
+        for (int e = 0; e < pol.N; ++e) {
+            const float qe = q[(size_t)t * pol.ldq + e];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float ke = s0 + i <= t ? k[(size_t)(s0 + i) * pol.ldk + e] : 0.0f;
+                if (split3::is_odd(qe) || split3::is_odd(ke)) G[i] = fmaf(qe, ke, G[i]);
+            }
+        }
+    __syncthreads();  // the results have been read
+    // A weight's exponential as it is where its rows are of one sixteen, else by the later row's sixteen's first row.
+    auto weights = [&](float (&w)[8], const RowTerms& r, float before) {
+        if (16 * sb > t) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = 0.0f;
+        } else if (16 * sb + 16 > t) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 c = rec[(s0 + i) * Pol::RECORDS];
+                w[i] = s0 + i <= t ? G[i] * (Pol::weight(c) * expf((Pol::g_hi(c) + r.e_hi) + (Pol::g_lo(c) + r.e_lo))) : 0.0f;
+            }
+        } else {
+            const RowTerms f = pol.row_terms(rec + (t & ~15) * Pol::RECORDS, before);
+            const float late = expf((r.e_hi - f.e_hi) + (r.e_lo - f.e_lo));
+            const float* e = early[(t >> 4) - 1] + s0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = G[i] * (e[i] * late);
+        }
+    };
+    // a head's records, and what its weights share
+    auto begin_head = [&](int h, float before) {
+        const float4* rows = st.rows + (ch.place * pol.heads + h) * L * Pol::RECORDS;
+        if (tid < L * Pol::RECORDS) rec[tid] = rows[tid];
+        if (tid >= OUT_THREADS - 96) {  // early[i][s], s below 16 (i + 1)
+            const int e = tid - (OUT_THREADS - 96), i = e < 16 ? 0 : e < 48 ? 1 : 2, s = e - (i == 0 ? 0 : i == 1 ? 16 : 48);
+            const RowTerms r = pol.row_terms(rows + 16 * (i + 1) * Pol::RECORDS, before);
+            const float4 c = rows[s * Pol::RECORDS];
+            early[i][s] = Pol::weight(c) * expf((Pol::g_hi(c) + r.e_hi) + (Pol::g_lo(c) + r.e_lo));
+        }
+    };
+    if constexpr (!Pol::SHARED) {  // one head a block: its weights stand where the products stood
+        const float before = st.before[ch.place * pol.heads + kvh];
+        begin_head(kvh, before);
+        __syncthreads();
+        float w[8];
+        weights(w, pol.row_terms(rec + t * Pol::RECORDS, before), before);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) G[i] = w[i];
+    }
     for (int item = i0; item < i1; ++item) {
         const int h = kvh * pol.per + item / ptiles, p0 = (item % ptiles) * PT;
         const size_t at = ch.place * pol.heads + h;
-        const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
-        const float* S = st.scratch + at * E;
+        const float *S = st.scratch + at * E, *vr = pol.v_row(ch.first, h) + p0;
+        Own v, m;
+        v.load(S + (size_t)p0 * pol.N, pol.N, pol.P - p0, pol.N);
+        m.load(S + (size_t)p0 * pol.N + 64, pol.N, pol.P - p0, pol.N - 64);
         const float before = st.before[at];
-        __syncthreads();  // k, or the item before, has been read by every warp
-        if (h != head) {
-            for (int i = tid; i < L * Pol::RECORDS; i += THREADS)
-                attn::cp_async_16(&rec[i], st.rows + at * L * Pol::RECORDS + i, true);
-            if (Pol::NORMALISER)
-                for (int n = tid; n < pol.N; n += THREADS) nv[n] = S[(size_t)pol.P * pol.N + n];
-        }
-        attn::cp_async_commit();
-        load_tile<true>(Bs, ld, S + (size_t)p0 * pol.N, pol.N, min(PT, pol.P - p0), 4 * n16, pol.N / 4);
-        load_tile<false>(Vs, VLD, pol.v_row(ch.first, h) + p0, pol.ldv, ch.n, PT / 4, min(PT, pol.P - p0) / 4);
-        attn::cp_async_commit();
-        if (h != head) {
-            attn::cp_async_wait<1>();
-            __syncthreads();
-            if (tx <= ty) {
+        if constexpr (Pol::SHARED) begin_head(h, before);
+        bool odd = v.put(Bs) || odd_qk;
+        if (blocks == 2) odd |= m.put(Bs + split3::TILE);
+        odd = core.start(0, odd, q_products);
+        v.load(vr, pol.ldv, ch.n, pol.P - p0);
+        float w[8];
+        auto make_weights = [&] {
+            if constexpr (Pol::SHARED) weights(w, pol.row_terms(rec + t * Pol::RECORDS, before), before);
+            else
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const RowTerms r = pol.row_terms(rec + (t0 + i) * Pol::RECORDS, before);
-                    float w[4];
+                for (int i = 0; i < 8; ++i) w[i] = G[i];
+        };
+        make_weights();
+        if constexpr (Pol::NORMALISER) {
+            if (p0 == 0) {  // eight threads a row
+                const RowTerms terms = pol.row_terms(rec + t * Pol::RECORDS, before);
+                const float* n = S + (size_t)pol.P * pol.N;
+                float sum = 0.0f, qn = 0.0f;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float4 k = rec[(4 * tx + j) * Pol::RECORDS];
-                        w[j] = 4 * tx + j <= t0 + i
-                                   ? G[i][j] * (Pol::weight(k) * expf((Pol::g_hi(k) + r.e_hi) + (Pol::g_lo(k) + r.e_lo)))
-                                   : 0.0f;
+                for (int i = 0; i < 8; ++i) sum += w[i];
+                if (t < ch.n)
+                    for (int e = s0 / 2; e < pol.N; e += 32) {
+                        const float4 a = load4(q + (size_t)t * pol.ldq + e), b = load4(n + e);
+                        qn = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, qn))));
                     }
-                    store4(Ws + (t0 + i) * WLD + 4 * tx, make_float4(w[0], w[1], w[2], w[3]));
+                row_sum[s0 / 8][t] = fmaf(terms.alpha, qn, sum);
+                if (ch.last && tid == 0) {
+                    float m = before;
+                    pol.carry(st.aux[at], m);
+                    pol.store_number(st.seq_slot[seq], h, m);
                 }
             }
-            head = h;
         }
-        if constexpr (Pol::NORMALISER) {
-            if (ch.last && p0 == 0 && tid == 0) {
-                float m = before;
-                pol.carry(st.aux[at], m);
-                pol.store_number(st.seq_slot[seq], h, m);
+        core.wait(0);
+        {  // times alpha, and out of the way of the next products' sums (over a sum that no one else reads)
+            const float alpha = pol.row_terms(rec + row * Pol::RECORDS, before).alpha;
+#pragma unroll
+            for (int c = 0; c < 16; c += 8) {
+                float y[8];
+                split3::sums_of<4>(y, lanes + c, split3::sets<4>((pol.N + 15) / 16), second);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) y[i] *= alpha;
+                sm100::tmem_st_8(lanes + 192 + c, y);
             }
+            sm100::tmem_st_wait();
         }
-        attn::cp_async_wait<0>();
+        odd |= split3::put8(w, Ws, t, s0 / 8);
+        odd |= v.put(Vs);
+        odd = core.start(1, odd, [&] {
+            split3::issue64<4, split3::K_STEP, split3::MN_STEP>(core.tmem, split3::B_MN, L / 16, split3::k_major(sm100::smem_u32(Ws)),
+                                                                split3::mn_major(sm100::smem_u32(Vs), split3::PART));
+        });
+        if constexpr (Pol::NORMALISER)
+            if (p0 == 0 && s0 == 0 && t < ch.n) {
+                float sum = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sum += row_sum[i][t];
+                pol.store_sum(ch.first + t, h, sum, pol.row_terms(rec + t * Pol::RECORDS, before).extra);
+            }
+        core.wait(1);
+#pragma unroll
+        for (int c = 0; c < 16; c += 8) {
+            float y[8], first[8];
+            split3::sums_of<4>(y, lanes + c, split3::sets<4>(L / 16), second);
+            sm100::tmem_ld_8(lanes + 192 + c, first);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] += first[i];
+            spread(y, c);
+        }
+        const int r = Own::row(0), p = p0 + Own::col();
+        float4 gate[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) gate[i] = pol.gate(min(r, ch.n - 1) + ch.first, h, min(p + 4 * i, pol.P - 4));
+        sm100::tc_fence_before_sync();
         __syncthreads();
-        float acc[4][4] = {};
-        product_along<4>(acc, qa, ld, ba, 16 * ld, n16);
+        float y[8];
+        read8(y, res + r * OLD + Own::col());
+        __syncthreads();  // the results have been read
+        if (odd) {  // the odd numbers' products
+            make_weights();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float alpha = pol.row_terms(rec + (t0 + i) * Pol::RECORDS, before).alpha;
+            for (int i = 0; i < 8; ++i) res[t * OLD + s0 + i] = w[i];
+            __syncthreads();
+            const float alpha = pol.row_terms(rec + r * Pol::RECORDS, before).alpha;
+            if (r < ch.n)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] *= alpha;
+                for (int j = 0; j < 8; ++j) {
+                    const int c = min(p + j, pol.P - 1) - p0;
+                    float a = 0.0f, b = 0.0f;
+                    for (int e = 0; e < pol.N; ++e) {
+                        const float x = q[(size_t)r * pol.ldq + e], m = S[(size_t)(p0 + c) * pol.N + e];
+                        if (split3::is_odd(x) || split3::is_odd(m)) a = fmaf(x, m, a);
+                    }
+                    for (int s = 0; s <= r; ++s) {
+                        const float x = res[r * OLD + s], m = vr[(size_t)s * pol.ldv + c];
+                        if (split3::is_odd(x) || split3::is_odd(m)) b = fmaf(x, m, b);
+                    }
+                    y[j] += fmaf(alpha, a, b);
+                }
+            __syncthreads();
         }
-        product_below<false>(acc, Ws + t0 * WLD, WLD, Vs + 4 * tx, VLD, ty);
-        if constexpr (Pol::NORMALISER) {
-            if (p0 == 0) {  // four threads a row
-                const int t = tid >> 2, j = tid & 3;
-                const RowTerms r = pol.row_terms(rec + t * Pol::RECORDS, before);
-                float sum = 0.0f, qn = 0.0f;
-                for (int s = j; s <= t; s += 4) sum += Ws[t * WLD + s];
-                for (int n = j; n < pol.N; n += 4) qn = fmaf(Qs[t * ld + n], nv[n], qn);
-                sum = fmaf(r.alpha, qn, sum);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                if (j == 0 && t < ch.n) pol.store_sum(ch.first + t, h, sum, r.extra);
-            }
-        }
-        const int p = p0 + 4 * tx;
-        if (p < pol.P)  // (P is a multiple of four)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (t0 + i < ch.n)
-                    pol.store_row(ch.first + t0 + i, h, p, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]),
-                                  load4(Vs + (t0 + i) * VLD + 4 * tx));
+        for (int i = 0; i < 2; ++i)  // (P is a multiple of four)
+            if (r < ch.n && p + 4 * i < pol.P)
+                pol.store_row(ch.first + r, h, p + 4 * i, gate[i], make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]),
+                              make_float4(v.x[0][4 * i], v.x[0][4 * i + 1], v.x[0][4 * i + 2], v.x[0][4 * i + 3]));
     }
+    core.close(tmem_slot);
 }
 
 // Floats of scratch a chunk needs: its memories and what the other kernels read beside them.
@@ -334,12 +586,13 @@ inline long long chunk_floats(int heads, long long E, int records) { return head
 
 template <class Pol>
 int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int R, int max_rows, float* scratch,
-        cudaStream_t s) {
+        int* err, cudaStream_t s) {
     const long long E = (long long)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
     const Plan plan = plan_rounds(R, n_seq, max_rows, L, chunk_floats(pol.heads, E, Pol::RECORDS));
     Step st;
     st.seq_slot = seq_slot;
     st.seq_row0 = seq_row0;
+    st.err = err;
     const long long n_places = plan.places;
     st.scratch = scratch;
     st.aux = reinterpret_cast<float4*>(scratch + n_places * pol.heads * E);  // E is a multiple of four
@@ -347,35 +600,37 @@ int run(const Pol& pol, const int* seq_slot, const int* seq_row0, int n_seq, int
     st.before = reinterpret_cast<float*>(st.rows + n_places * pol.heads * L * Pol::RECORDS);
     const int ptiles = (pol.P + PT - 1) / PT;
     const int chunks = plan.seg_rows / L;
-    const size_t sm_state = (size_t)L * (VLD + (pol.N > 64 ? 132 : 68)) * sizeof(float);
-    const size_t sm_out = (size_t)L * (VLD + WLD + 2 * ((pol.N + 15) / 16 * 16 + 4)) * sizeof(float);
     const int qk_heads = pol.heads / pol.per, items = pol.per * ptiles;
-    // items a block: the rows' products with k, which serve them all, cost about as much as one item; two
-    // blocks share an SM
-    int ipb = items;
-    long long least = -1;
-    for (int i = items; i >= 1; --i) {
-        const long long blocks = (long long)chunks * plan.group * qk_heads * ((items + i - 1) / i);
-        const long long cost = (blocks + 2 * sm_count() - 1) / (2 * sm_count()) * (1 + i);
-        if (least < 0 || cost < least) {
-            least = cost;
-            ipb = i;
+    // items a block: k (its products with the rows) and the weights, which serve them all, cost about as much as
+    // one item; two blocks share an SM
+    auto items_a_block = [&](int most) {
+        int ipb = most;
+        long long least = -1;
+        for (int i = most; i >= 1; --i) {
+            const long long blocks = (long long)chunks * plan.group * qk_heads * ((items + i - 1) / i);
+            const long long cost = (blocks + 2 * sm_count() - 1) / (2 * sm_count()) * (1 + i);
+            if (least < 0 || cost < least) {
+                least = cost;
+                ipb = i;
+            }
         }
-    }
-    const int sets = (items + ipb - 1) / ipb;
-    if (n_seq > 65535 || (long long)pol.heads * ptiles > 65535 || (long long)qk_heads * sets > 65535)
-        return RFX_ERR_UNSUPPORTED;
-    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_state);
+        return ipb;
+    };
+    const int ipb_state = items_a_block(min(items, (WARPS - 1) * ptiles));  // (a warp a head at most)
+    const int ipb_out = items_a_block(items);
+    const int sets_state = (items + ipb_state - 1) / ipb_state, sets_out = (items + ipb_out - 1) / ipb_out;
+    if (n_seq > 65535 || (long long)pol.heads * ptiles > 65535) return RFX_ERR_UNSUPPORTED;
+    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(chunk_out_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_out);
+    e = cudaFuncSetAttribute(chunk_out_kernel<Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     if (e != cudaSuccess) return (int)e;
     for (int seq0 = 0; seq0 < n_seq; seq0 += plan.group)
         for (int seg = 0; seg < plan.n_segs; ++seg) {
             const int seqs = min(plan.group, n_seq - seq0);
             st.round = Round{plan.seg_rows, seg, seq0, plan.whole};
-            RFX_LAUNCH(chunk_state_kernel<Pol>, dim3(chunks, seqs, pol.heads * ptiles), THREADS, sm_state, s, pol, st);
+            RFX_LAUNCH(chunk_state_kernel<Pol>, dim3(chunks, seqs, qk_heads * sets_state), STATE_THREADS, SMEM, s, pol, st, ipb_state);
             RFX_LAUNCH(chunk_carry_kernel<Pol>, dim3((unsigned)((E / 4 + 127) / 128), seqs, pol.heads), 128, 0, s, pol, st);
-            RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, seqs, qk_heads * sets), THREADS, sm_out, s, pol, st, ipb);
+            RFX_LAUNCH(chunk_out_kernel<Pol>, dim3(chunks, seqs, qk_heads * sets_out), OUT_THREADS, SMEM, s, pol, st, ipb_out);
         }
     return 0;
 }

@@ -12,6 +12,7 @@ namespace {
 
 struct Mlstm {
     static constexpr bool NORMALISER = true;
+    static constexpr bool SHARED = false;  // every head has its own q and k
     static constexpr int RECORDS = 2;  // g and its running maximum, F, each in two parts
     const float *proj, *bias_i, *bias_f;
     float cap, q_scale;
@@ -51,7 +52,7 @@ struct Mlstm {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = lane + 32 * i;
-            wl[r] = expf((float)(gg[i] - G));
+            wl[r] = chunk::exp_of(gg[i] - G);
             if (rows) {
                 float4 a, b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 chunk::two_parts(gg[i], &a.x, &a.y);
@@ -92,7 +93,7 @@ struct Mlstm {
         const double F = (double)a.x + a.y, G = (double)a.z + a.w, old = m;
         m = (float)(F + fmax(old, G));
         // relative to the number as it is kept, so that its rounding is no error of the memory
-        return make_float2(expf((float)(F + old - m)), expf((float)(F + G - m)));
+        return make_float2(chunk::exp_of(F + old - m), chunk::exp_of(F + G - m));
     }
     __device__ __forceinline__ void store_state(int slot, int h, int e, const float4& S) const {
         float* s = head_state(slot, h);
@@ -105,7 +106,8 @@ struct Mlstm {
         float* s = head_state(slot, h) + (size_t)N * P + N;
         for (int i = 0; i < (P + 63) / 64; ++i) s[i] = m;
     }
-    __device__ __forceinline__ void store_row(int r, int h, int p, const float4& y, const float4&) const {
+    __device__ __forceinline__ float4 gate(int, int, int) const { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+    __device__ __forceinline__ void store_row(int r, int h, int p, const float4&, const float4& y, const float4&) const {
         rfx::store4(num + ((size_t)r * heads + h) * P + p,
                     make_float4(y.x * q_scale, y.y * q_scale, y.z * q_scale, y.w * q_scale));
     }
@@ -127,7 +129,7 @@ extern "C" long long rfx_mlstm_chunks_floats(int R, int S, int max_rows, int hea
 extern "C" int rfx_mlstm_chunks(const float* proj, int ld, int q_off, int k_off, int v_off, int i_off, int f_off,
                                 const float* bias_i, const float* bias_f, float cap, float q_scale,
                                 const int* seq_slot, const int* seq_row0, int S, int R, int max_rows, float* state,
-                                float* num, float* den, float* scratch, int heads, int dim, int vdim, void* stream) {
+                                float* num, float* den, float* scratch, int heads, int dim, int vdim, int* err, void* stream) {
     if (S <= 0 || R <= 0 || max_rows <= 0) return 0;
     if (heads <= 0 || dim <= 0 || vdim <= 0 || cap <= 0.0f) return RFX_ERR_BAD_ARG;
     if (dim % 4 || vdim % 4 || dim > 128 || ((ld | q_off | k_off | v_off) & 3) ||
@@ -135,5 +137,5 @@ extern "C" int rfx_mlstm_chunks(const float* proj, int ld, int q_off, int k_off,
         return RFX_ERR_UNSUPPORTED;
     Mlstm p{proj, bias_i, bias_f, cap, q_scale, state, num, den, q_off, k_off, v_off, i_off, f_off, heads, 1, dim,
             vdim, ld, ld, ld};
-    return chunk::run(p, seq_slot, seq_row0, S, R, max_rows, scratch, (cudaStream_t)stream);
+    return chunk::run(p, seq_slot, seq_row0, S, R, max_rows, scratch, err, (cudaStream_t)stream);
 }

@@ -11,6 +11,7 @@ namespace {
 
 struct Ssd {
     static constexpr bool NORMALISER = false;
+    static constexpr bool SHARED = true;  // several heads have the same q and k
     static constexpr int RECORDS = 1;  // running logarithm in two parts, step size, its exponential
     const float *xbc, *proj, *dt_bias, *A, *D;
     float *state, *out;
@@ -49,7 +50,7 @@ struct Ssd {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = lane + 32 * i;
-            wl[r] = d[i] * expf((float)(all - c[i]));
+            wl[r] = d[i] * chunk::exp_of(all - c[i]);
             if (rows) {
                 float hi, lo;
                 chunk::two_parts(c[i], &hi, &lo);
@@ -57,7 +58,7 @@ struct Ssd {
                 rows[r] = make_float4(hi, lo, d[i], fmaf(e, lo, e));  // exp(hi + lo)
             }
         }
-        return make_float4(expf((float)all), 0.0f, 0.0f, 0.0f);
+        return make_float4(chunk::exp_of(all), 0.0f, 0.0f, 0.0f);
     }
     static __device__ __forceinline__ float g_hi(const float4& r) { return -r.x; }
     static __device__ __forceinline__ float g_lo(const float4& r) { return -r.y; }
@@ -74,12 +75,21 @@ struct Ssd {
     __device__ __forceinline__ void store_state(int slot, int h, int e, const float4& S) const {
         *reinterpret_cast<float4*>(memory(slot, h, e)) = S;
     }
-    __device__ __forceinline__ void store_row(int r, int h, int p, const float4& y, const float4& x) const {
-        const float4 z = rfx::load4(proj + (size_t)r * ldp + z_off + h * P + p);
+    // z / (1 + e^-z); one step upon the approximate reciprocal gives all but the last bit
+    static __device__ __forceinline__ float silu(float z) {
+        const float d = 1.0f + expf(fminf(-z, 87.0f));
+        float r;
+        asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+        return z * fmaf(fmaf(-d, r, 1.0f), r, r);
+    }
+    __device__ __forceinline__ float4 gate(int r, int h, int p) const {
+        return rfx::load4(proj + (size_t)r * ldp + z_off + h * P + p);
+    }
+    __device__ __forceinline__ void store_row(int r, int h, int p, const float4& z, const float4& y, const float4& x) const {
         const float d = D ? D[h] : 0.0f;
         rfx::store4(out + (size_t)r * inner + h * P + p,
-                    make_float4(fmaf(d, x.x, y.x) * (z.x / (1.0f + expf(-z.x))), fmaf(d, x.y, y.y) * (z.y / (1.0f + expf(-z.y))),
-                                fmaf(d, x.z, y.z) * (z.z / (1.0f + expf(-z.z))), fmaf(d, x.w, y.w) * (z.w / (1.0f + expf(-z.w)))));
+                    make_float4(fmaf(d, x.x, y.x) * silu(z.x), fmaf(d, x.y, y.y) * silu(z.y), fmaf(d, x.z, y.z) * silu(z.z),
+                                fmaf(d, x.w, y.w) * silu(z.w)));
     }
 };
 
@@ -97,7 +107,7 @@ extern "C" int rfx_ssd_chunk(const float* xbc, int ldx, const float* proj, int l
                              const float* dt_bias, const float* A, const float* D, float* state,
                              long long state_stride, long long state_off, const int* seq_slot, const int* seq_row0,
                              int n_seq, int R, int max_rows, float* out, float* scratch, int heads, int P, int N,
-                             int groups, void* stream) {
+                             int groups, int* err, void* stream) {
     if (n_seq <= 0 || R <= 0 || max_rows <= 0) return 0;
     if (heads <= 0 || groups <= 0 || heads % groups || P <= 0 || N <= 0) return RFX_ERR_BAD_ARG;
     if (P % 4 || N % 4 || N > 128 || ((ldx | ldp | z_off) & 3) || ((state_stride | state_off) & 3) ||
@@ -106,5 +116,5 @@ extern "C" int rfx_ssd_chunk(const float* xbc, int ldx, const float* proj, int l
         return RFX_ERR_UNSUPPORTED;
     Ssd p{xbc, proj, dt_bias, A, D, state, out, state_stride, state_off, ldx, ldp, z_off, dt_off, heads,
           heads / groups, N, P, heads * P, groups, ldx, ldx, ldx};
-    return chunk::run(p, seq_slot, seq_row0, n_seq, R, max_rows, scratch, (cudaStream_t)stream);
+    return chunk::run(p, seq_slot, seq_row0, n_seq, R, max_rows, scratch, err, (cudaStream_t)stream);
 }

@@ -926,7 +926,7 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale:
             _chk(bias_f, "bias_f", torch.float32), float(cap), float(q_scale),
             _chk(batch.seq_slot, "seq_slot", torch.int32), _chk(batch.seq_row0, "seq_row0", torch.int32), S, R, most,
             _chk(state, "state", torch.float32), num.data_ptr(), den.data_ptr(), scratch.data_ptr(), heads, dim, vdim,
-            _stream())
+            device_error_word(proj.device).data_ptr(), _stream())
         if st != native.ERR_UNSUPPORTED:  # rows that are not on 16 bytes
             native.check(st, f"mlstm_chunks (dim={dim}, vdim={vdim})")
             return num, den
@@ -1853,7 +1853,8 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
             int(dt_off), _chk(dt_bias, "dt_bias", torch.float32), _chk(A, "A", torch.float32),
             _chk(D, "D", torch.float32), _chk(state, "state", torch.float32), state.stride(0), int(state_off),
             _chk(batch.seq_slot, "seq_slot", torch.int32), _chk(batch.seq_row0, "seq_row0", torch.int32), S, R, most,
-            out.data_ptr(), scratch.data_ptr(), heads, vdim, states, groups, _stream())
+            out.data_ptr(), scratch.data_ptr(), heads, vdim, states, groups, device_error_word(xbc.device).data_ptr(),
+            _stream())
         if st != native.ERR_UNSUPPORTED:  # rows or state that are not on 16 bytes
             native.check(st, f"ssd_chunk (heads={heads}, vdim={vdim}, states={states})")
             return out

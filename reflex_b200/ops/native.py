@@ -113,7 +113,7 @@ _SIGNATURES = {
                         c_void_p],
     "rfx_mlstm_chunks": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                         c_int, c_void_p],
+                         c_int, c_void_p, c_void_p],
     "rfx_mlstm_out": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int,
                       c_int, c_int, c_void_p],
     "rfx_moe_route": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -180,7 +180,7 @@ _SIGNATURES = {
                      c_void_p],
     "rfx_ssd_chunk": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
-                      c_int, c_int, c_void_p],
+                      c_int, c_int, c_void_p, c_void_p],
     "rfx_delta_rule": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float,
                        c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                        c_void_p],

@@ -371,3 +371,35 @@ def test_a_row_that_is_not_finite_does_not_reach_earlier_rows_of_the_delta_rule(
         assert torch.equal(y[:70], clean[:70]) and torch.equal(y[:, ~hit], clean[:, ~hit]), part
         assert not torch.isfinite(y[71:, hit]).any(), part
         assert torch.equal(state.view(hd, d)[~hit], clean_state.view(hd, d)[~hit]), part
+
+
+@pytest.mark.parametrize("huge", [3.3895e38, 3.395e38])  # bfloat16's largest number holds the first, not the second
+@pytest.mark.parametrize("N", [24, 128])
+def test_numbers_beyond_bfloat16s_range_count_as_they_are(huge, N):
+    """One element of v near the end of 32 bits' range, with k and q small enough for finite results."""
+    heads, groups, P, T = 4, 1, 64, 200
+    g = torch.Generator(device=DEV).manual_seed(5)
+    inner, b = heads * P, Batch([T], [0])
+    xbc = torch.randn((T, inner + 2 * groups * N), generator=g, device=DEV)
+    xbc[:, inner:] *= 1e-3
+    proj = torch.randn((T, inner + heads), generator=g, device=DEV)
+    A, D, bias = -torch.ones(heads, device=DEV), torch.zeros(heads, device=DEV), torch.zeros(heads, device=DEV)
+
+    def ssd(x):
+        state = torch.zeros((1, heads * P * N), device=DEV)
+        return ops().ssd_scan(x, proj, 0, inner, bias, A, D, state, 0, b, heads, P, N, groups, exact=False), state
+
+    clean, clean_state = ssd(xbc)
+    xbc[70, P + 5] = huge
+    y, state = ssd(xbc)
+    hit = torch.zeros(inner, dtype=torch.bool, device=DEV)
+    hit[P + 5] = True
+    assert torch.equal(y[:70], clean[:70]) and torch.equal(y[:, ~hit], clean[:, ~hit])
+    assert torch.equal(state.view(inner, N)[~hit], clean_state.view(inner, N)[~hit])
+    x64, p64 = xbc.double().cpu().numpy(), proj.double().cpu().numpy()
+    dt = np.log1p(np.exp(p64[:, inner:]))
+    B, C = (x64[:, o:o + N].reshape(T, 1, N).repeat(heads, 1) for o in (inner, inner + N))
+    ref, S = ssd_rule(x64[:, :inner].reshape(T, heads, P), B, C, dt, -np.ones(heads), np.zeros(heads), np.zeros((heads, P, N)))
+    z = p64[:, P + 5]
+    assert off(y[:, P + 5], ref[:, 1, 5] * z / (1 + np.exp(-z))) < TOL
+    assert off(state.view(heads, P, N)[1, 5], S[1, 5]) < TOL
