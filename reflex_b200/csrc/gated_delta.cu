@@ -114,6 +114,72 @@ gated_delta_prep_kernel(const float* __restrict__ proj, int ld, int b_off, int a
     }
 }
 
+// The same for prompts: a warp a head of ROWS neighbouring rows (heads of up to 128 elements, in fours), whose
+// inputs are all in flight at once and are loaded once, not by every row that they reach.  Memory bounds it
+// (4,096 rows of 8,192 channels, 268 MB: 102 us a warp a head of a row, 69 so; eight rows a warp 76).
+constexpr int ROWS = 4;
+template <int TAPS>
+__global__ void __launch_bounds__(PREP_THREADS)
+gated_delta_prep_rows_kernel(const float* __restrict__ proj, int ld, int b_off, int a_off,
+                             const float* __restrict__ filters, const float* __restrict__ state, long long slot_stride,
+                             const int* __restrict__ row_slot, const float* __restrict__ dt_bias,
+                             const float* __restrict__ A, float unit_eps, float q_scale, float* __restrict__ out,
+                             float* __restrict__ gates, int R, int H, int G, int d, int dv, int fast) {
+    pdl_prologue();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r0 = blockIdx.x * ROWS, n = min(ROWS, R - r0), unit = blockIdx.y * (PREP_THREADS / 32) + warp;
+    const int C = 2 * G * d + H * dv;
+    if (unit > 2 * G + H) return;
+    if (unit == 2 * G + H) {  // the two gates of every head: [decay | write rate]
+        for (int e = lane; e < n * H; e += 32) {
+            const int i = e / H, h = e - i * H;
+            const float* pr = proj + (size_t)(r0 + i) * ld;
+            float* g = gates + (size_t)(r0 + i) * 2 * H + h;
+            g[0] = expf(A[h] * softplus_f(pr[a_off + h] + dt_bias[h]));
+            g[H] = 1.0f / (1.0f + expf(-pr[b_off + h]));
+        }
+        return;
+    }
+    const int width = unit < 2 * G ? d : dv;
+    const int c = (unit < 2 * G ? unit * d : 2 * G * d + (unit - 2 * G) * dv) + 4 * lane;
+    const bool live = 4 * lane < width;
+    float4 y[ROWS], f[TAPS];
+    if (live) {
+        auto at = [&](int r) { return proj + (size_t)r * ld + c; };
+        auto tail = [&](int slot) { return state + (size_t)slot * slot_stride + c; };
+        const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+            if (i < n) y[i] = *reinterpret_cast<const float4*>(at(r0 + i));
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) f[j] = *reinterpret_cast<const float4*>(filters + (size_t)j * C + c);
+        Window<TAPS> window;
+        window.begin(row_slot, r0, C, none, at, tail);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+            if (i < n) {
+                if (i && row_slot[r0 + i] != row_slot[r0 + i - 1]) window.begin(row_slot, r0 + i, C, none, at, tail);
+                float4 t = window.step(f, y[i]);
+                if (fast) { t.x = silu_fast(t.x); t.y = silu_fast(t.y); t.z = silu_fast(t.z); t.w = silu_fast(t.w); }
+                else { t.x = silu_of(t.x); t.y = silu_of(t.y); t.z = silu_of(t.z); t.w = silu_of(t.w); }
+                y[i] = t;
+            }
+    }
+    if (unit < 2 * G) {
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            float ss = 0.0f;
+            if (live && i < n) ss = fmaf(y[i].x, y[i].x, fmaf(y[i].y, y[i].y, fmaf(y[i].z, y[i].z, fmaf(y[i].w, y[i].w, ss))));
+            const float k = (unit < G ? q_scale : 1.0f) / sqrtf(warp_sum(ss) + unit_eps);
+            if (live && i < n) { y[i].x *= k; y[i].y *= k; y[i].z *= k; y[i].w *= k; }
+        }
+    }
+    if (live)
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+            if (i < n) store4(out + (size_t)(r0 + i) * C + c, y[i]);
+}
+
 __device__ __forceinline__ void cp_async_4(void* smem, const void* gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(attn::smem_u32(smem)), "l"(gmem) : "memory");
 }
@@ -328,6 +394,17 @@ extern "C" int rfx_gated_delta_prep(const float* proj, int ld, int b_off, int a_
                      ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(filters) |
                        reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     cudaStream_t s = (cudaStream_t)stream;
+    if (by4 && !update && R >= 256 && d <= 128 && dv <= 128 && taps >= 2 && taps <= 4) {  // (fewer: too few warps)
+        dim3 rows((R + ROWS - 1) / ROWS, grid.y);
+#define RFX_ROWS(T)                                                                                                 \
+    RFX_LAUNCH(gated_delta_prep_rows_kernel<T>, rows, PREP_THREADS, 0, s, proj, ld, b_off, a_off, filters, state,   \
+               slot_stride, row_slot, dt_bias, A, unit_eps, q_scale, out, gates, R, H, G, d, dv, fast)
+        if (taps == 2) RFX_ROWS(2);
+        else if (taps == 3) RFX_ROWS(3);
+        else RFX_ROWS(4);
+#undef RFX_ROWS
+        return 0;
+    }
 #define RFX_PREP(N, T)                                                                                              \
     RFX_LAUNCH((gated_delta_prep_kernel<N, T>), grid, PREP_THREADS, 0, s, proj, ld, b_off, a_off, filters, taps, state, \
                slot_stride, row_slot, dt_bias, A, unit_eps, q_scale, out, gates, H, G, d, dv, update, fast)

@@ -85,6 +85,46 @@ short_conv_kernel(const float* __restrict__ proj, int ld, int col0, const float*
     }
 }
 
+// The same for prompts: a thread four channels of ROWS neighbouring rows, whose inputs are all in flight at
+// once.  Memory bounds it (2,048 rows of 2,560 channels, 42 MB: 27 us a row a block, each input
+// loaded by four rows, 15 so; with eight rows a thread, half the warps an SM, 18.5).
+constexpr int ROWS = 4;
+template <int TAPS>
+__global__ void __launch_bounds__(256)
+short_conv_rows_kernel(const float* __restrict__ proj, int ld, int col0, const float* __restrict__ bias,
+                       const float* __restrict__ w, const float* __restrict__ cbias, const float* __restrict__ state,
+                       size_t slot_stride, const int* __restrict__ row_slot, float* __restrict__ out,
+                       __nv_bfloat16* __restrict__ out_lo, int R, int C, int act) {
+    pdl_prologue();
+    const int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x), r0 = blockIdx.x * ROWS, n = min(ROWS, R - r0);
+    if (c >= C) return;
+    float4 now[ROWS], f[TAPS], b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), cb = b;
+    auto at = [&](int r) { return proj + (size_t)r * ld + col0 + c; };
+    auto tail = [&](int slot) { return state + (size_t)slot * slot_stride + c; };
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (i < n) now[i] = *reinterpret_cast<const float4*>(at(r0 + i));
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) f[j] = *reinterpret_cast<const float4*>(w + (size_t)j * C + c);
+    if (bias) b = *reinterpret_cast<const float4*>(bias + c);
+    if (cbias) cb = *reinterpret_cast<const float4*>(cbias + c);
+    Window<TAPS> window;
+    window.begin(row_slot, r0, C, b, at, tail);
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (i < n) {
+            const int r = r0 + i;
+            if (i && row_slot[r] != row_slot[r - 1]) window.begin(row_slot, r, C, b, at, tail);
+            float4 u = now[i];
+            if (bias) { u.x += b.x; u.y += b.y; u.z += b.z; u.w += b.w; }
+            float4 y = window.step(f, u);
+            if (cbias) { y.x += cb.x; y.y += cb.y; y.z += cb.z; y.w += cb.w; }
+            if (act == 1) { y.x = silu_of(y.x); y.y = silu_of(y.y); y.z = silu_of(y.z); y.w = silu_of(y.w); }
+            store4(out + (size_t)r * C + c, y);
+            if (out_lo) store4(out_lo + (size_t)r * C + c, y);
+        }
+}
+
 template <typename TO>
 __global__ void __launch_bounds__(256)
 conv_qkv_post_kernel(const float* __restrict__ proj, int ld, const float* __restrict__ bias,
@@ -196,6 +236,20 @@ extern "C" int rfx_short_conv_act(const float* proj, int ld, int col0, const flo
     const int by4 = C % 4 == 0 && ld % 4 == 0 && col0 % 4 == 0 && slot_stride % 4 == 0 && aligned16(proj) &&
                     aligned16(bias) && aligned16(w) && aligned16(cbias) && aligned16(state) && aligned16(out) &&
                     ((reinterpret_cast<uintptr_t>(out_lo) & 7) == 0);
+    if (by4 && !update && R >= 256 && taps >= 2 && taps <= 4) {  // (fewer rows: too few threads a row less)
+        dim3 rows((R + ROWS - 1) / ROWS, (C / 4 + 255) / 256);
+        cudaStream_t s = (cudaStream_t)stream;
+        if (rows.y <= 65535) {
+#define RFX_ROWS(T)                                                                                                  \
+    RFX_LAUNCH(short_conv_rows_kernel<T>, rows, 256, 0, s, proj, ld, col0, bias, w, cbias, state, (size_t)slot_stride, \
+               row_slot, out, (__nv_bfloat16*)out_lo, R, C, act)
+            if (taps == 2) RFX_ROWS(2);
+            else if (taps == 3) RFX_ROWS(3);
+            else RFX_ROWS(4);
+#undef RFX_ROWS
+            return 0;
+        }
+    }
     // by fours, many rows: two units a thread share the row's own work; few rows: a unit a thread,
     // so that a decode step's loads are all in flight at once
     dim3 grid(R, chunks(by4 ? C / (R >= 256 ? 8 : 4) : C, 256));

@@ -64,6 +64,42 @@ __device__ __forceinline__ float4 conv4_at(const float* __restrict__ proj, int l
     return y;
 }
 
+// Four channels through several neighbouring rows: the last TAPS - 1 inputs in registers, oldest first, so
+// that a prompt's input is loaded once and not by every row that it reaches.  `at(r)`, `tail(slot)`: where
+// row r's and a slot's four channels lie (the state's rows `C` apart).
+template <int TAPS>
+struct Window {
+    float4 u[TAPS - 1];
+    template <class At, class Tail>
+    __device__ __forceinline__ void begin(const int* __restrict__ row_slot, int r, int C, const float4& b, At&& at, Tail&& tail) {
+        const int before = rows_before(row_slot, r, TAPS - 1);
+        const float* t = tail(row_slot[r]);
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j) {
+            const int back = TAPS - 1 - j;
+            const bool here = back <= before;
+            u[j] = *reinterpret_cast<const float4*>(here ? at(r - back) : t + (size_t)(j + before) * C);
+            if (here) { u[j].x += b.x; u[j].y += b.y; u[j].z += b.z; u[j].w += b.w; }
+        }
+    }
+    // the row's results (taps summed oldest first, as conv4_at), and its input into the window
+    __device__ __forceinline__ float4 step(const float4 (&f)[TAPS], const float4& now) {
+        float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const float4 x = j < TAPS - 1 ? u[j < TAPS - 1 ? j : 0] : now;
+            y.x = fmaf(f[j].x, x.x, y.x);
+            y.y = fmaf(f[j].y, x.y, y.y);
+            y.z = fmaf(f[j].z, x.z, y.z);
+            y.w = fmaf(f[j].w, x.w, y.w);
+        }
+#pragma unroll
+        for (int j = 0; j + 1 < TAPS - 1; ++j) u[j] = u[j + 1];
+        u[TAPS - 2] = now;
+        return y;
+    }
+};
+
 // y / (1 + e^-y), 32-bit
 __device__ __forceinline__ float silu_of(float y) { return y / (1.0f + expf(-y)); }
 

@@ -1,0 +1,71 @@
+"""The elementwise kernels of prompts that take several rows, or several small parts, a thread: the same bits as the
+forms for few rows, at the edges of their groups of rows and across sequences."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+COUNTS = (1, 2, 7, 8, 9, 100, 3, 131)  # 261 rows: the last group of four rows has one
+
+
+def ops():
+    from reflex_b200 import ops as o
+
+    return o
+
+
+def i32(v):
+    return torch.tensor(list(v), dtype=torch.int32, device=DEV)
+
+
+class Batch:
+    def __init__(self, counts, slots):
+        self.row_slot = i32([s for s, c in zip(slots, counts) for _ in range(c)])
+        self.seq_slot, self.seq_new = i32(slots), i32(counts)
+
+
+def piecewise(fn, counts):
+    """fn(rows, batch) a sequence at a time: too few rows for the form under test."""
+    out, r0 = [], 0
+    for i, c in enumerate(counts):
+        out.append(fn(slice(r0, r0 + c), Batch([c], [len(counts) - 1 - i])))
+        r0 += c
+    return [torch.cat(t) for t in zip(*out)]
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("channels,col0,ld,biases,act", [(1028, 4, 1040, True, "silu"), (12, 0, 16, False, None)])
+def test_short_convolutions_of_several_rows(taps, channels, col0, ld, biases, act):
+    g = torch.Generator(device=DEV).manual_seed(taps)
+    R = lambda *s: torch.randn(s, generator=g, device=DEV)  # noqa: E731
+    n = sum(COUNTS)
+    proj, w, state = R(n, ld), R(taps, channels), R(len(COUNTS), (taps - 1) * channels + 4)
+    b, cb = (R(channels), R(channels)) if biases else (None, None)
+
+    def run(rows, batch):
+        return ops().short_conv(proj[rows], col0, channels, b, w, cb, state, batch, also_bf16=True, activation=act)
+
+    whole = run(slice(0, n), Batch(COUNTS, range(len(COUNTS) - 1, -1, -1)))
+    for x, y in zip(whole, piecewise(run, COUNTS)):
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 128, 128), (3, 1, 20, 36)])
+@pytest.mark.parametrize("exact", [True, False])
+def test_gated_delta_rows_of_prompts(taps, heads, kv_heads, dim, vdim, exact):
+    g = torch.Generator(device=DEV).manual_seed(taps)
+    R = lambda *s: torch.randn(s, generator=g, device=DEV)  # noqa: E731
+    n, C = sum(COUNTS), 2 * kv_heads * dim + heads * vdim
+    ld = C + 2 * heads + (-2 * heads) % 4
+    proj, w, state = R(n, ld), R(taps, C), R(len(COUNTS), (taps - 1) * C + 8)
+    bias, A = R(heads), -torch.rand(heads, generator=g, device=DEV)
+
+    def run(rows, batch):
+        return ops().gated_delta_prep(proj[rows], C, C + heads, w, state, batch, bias, A, 1e-6, dim ** -0.5, heads, kv_heads,
+                                      dim, vdim, exact=exact)
+
+    whole = run(slice(0, n), Batch(COUNTS, range(len(COUNTS) - 1, -1, -1)))
+    for x, y in zip(whole, piecewise(run, COUNTS)):
+        assert torch.equal(x, y)
