@@ -69,3 +69,20 @@ def test_gated_delta_rows_of_prompts(taps, heads, kv_heads, dim, vdim, exact):
     whole = run(slice(0, n), Batch(COUNTS, range(len(COUNTS) - 1, -1, -1)))
     for x, y in zip(whole, piecewise(run, COUNTS)):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("groups,size,shared", [(32, 64, False), (33, 64, True), (40, 128, True), (36, 68, False), (64, 4, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gate", [None, "sigmoid", "silu"])
+def test_norms_of_many_small_parts(groups, size, shared, dtype, gate):
+    g = torch.Generator(device=DEV).manual_seed(size)
+    R = lambda *s: torch.randn(s, generator=g, device=DEV)  # noqa: E731
+    n, C = 16384 // groups + 3, groups * size
+    x, w, z = R(n, C), R(size if shared else C), R(n, C + 12)
+
+    def run(rows):
+        kw = dict(gate=z[rows], gate_col=8, activation=gate) if gate else {}
+        return ops().group_norm_gate(x[rows], w, 1e-5, groups, dtype, **kw)
+
+    half = n // 2
+    assert torch.equal(run(slice(0, n)), torch.cat([run(slice(0, half)), run(slice(half, n))]))
