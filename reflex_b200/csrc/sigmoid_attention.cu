@@ -81,6 +81,74 @@ sig_qkv_post_kernel(const TI* __restrict__ proj, int ldp, int col0, const float*
     }
 }
 
+// The same by fours (sizes, the turned half and the strides multiples of four), `n_rows` rows a block: a row's
+// page is looked up once, its angles by as many threads as there are for all rows.  Memory bounds it (2,048
+// rows of 3,072, 38 MB: 22.7 us an element a thread and a row a block, 10 so).
+constexpr int POST_ROWS = 4;
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256)
+sig_qkv_post4_kernel(const TI* __restrict__ proj, int ldp, int col0, const float* __restrict__ denom, int rot_dims,
+                     const int* __restrict__ row_pos, const int* __restrict__ row_slot, TO* __restrict__ q_out,
+                     TO* __restrict__ k_pages, TO* __restrict__ v_pages, const int* __restrict__ page_table,
+                     int max_pages, int page_size, int nq, int nkv, int d, int dv, int writes_cache, int R, int n_rows) {
+    extern __shared__ float cs[];  // a row: [rot_dims / 2] cosines, then as many sines
+    __shared__ int pages[POST_ROWS];
+    pdl_prologue();
+    const int r0 = blockIdx.x * n_rows, n = min(n_rows, R - r0), half = rot_dims / 2;
+    if (threadIdx.x < n && writes_cache) {
+        const int r = r0 + threadIdx.x;
+        pages[threadIdx.x] = page_table[(size_t)row_slot[r] * max_pages + row_pos[r] / page_size];
+    }
+    for (int e = threadIdx.x; e < n * half; e += 256) {
+        const int k = e / half, i = e - k * half;
+        float s, c;
+        exact_sincosf((float)row_pos[r0 + k] / denom[i], &s, &c);
+        cs[k * rot_dims + i] = c;
+        cs[k * rot_dims + half + i] = s;
+    }
+    __syncthreads();
+    const int d4 = d / 4, dv4 = dv / 4, n_q = nq * d4, n_qk = n_q + (writes_cache ? nkv * d4 : 0);
+    const int units = n_qk + (writes_cache ? nkv * dv4 : 0);
+    for (int u = threadIdx.x; u < units; u += 256) {
+        const bool turns = u < n_qk;
+        const int uu = turns ? u : u - n_qk, w4 = turns ? d4 : dv4;
+        const int head = uu / w4, i = 4 * (uu - head * w4);
+        const int col = turns ? 4 * u : (nq + nkv) * d + 4 * uu;
+        const bool turned = turns && i < rot_dims, low = i < half;
+        const int f = low ? i : i - half;
+        float4 v[POST_ROWS], p[POST_ROWS];
+#pragma unroll
+        for (int k = 0; k < POST_ROWS; ++k)
+            if (k < n) {
+                const TI* row = proj + (size_t)(r0 + k) * ldp + col0 + col;
+                v[k] = load4(row);
+                if (turned) p[k] = load4(low ? row + half : row - half);
+            }
+#pragma unroll
+        for (int k = 0; k < POST_ROWS; ++k)
+            if (k < n) {
+                if (turned) {  // (u, v) -> (u cos - v sin, v cos + u sin)
+                    const float* a = cs + k * rot_dims + f;
+                    const float4 c = make_float4(a[0], a[1], a[2], a[3]);
+                    float4 s = make_float4(a[half], a[half + 1], a[half + 2], a[half + 3]);
+                    if (low) s = make_float4(-s.x, -s.y, -s.z, -s.w);
+                    v[k].x = fmaf(p[k].x, s.x, __fmul_rn(v[k].x, c.x));
+                    v[k].y = fmaf(p[k].y, s.y, __fmul_rn(v[k].y, c.y));
+                    v[k].z = fmaf(p[k].z, s.z, __fmul_rn(v[k].z, c.z));
+                    v[k].w = fmaf(p[k].w, s.w, __fmul_rn(v[k].w, c.w));
+                }
+                const int r = r0 + k;
+                if (u < n_q) {
+                    store4(q_out + (size_t)r * nq * d + 4 * u, v[k]);
+                } else {
+                    const int kvh = turns ? head - nq : head;
+                    TO* to = turns ? k_pages : v_pages;
+                    store4(to + (((size_t)pages[k] * nkv + kvh) * page_size + row_pos[r] % page_size) * (size_t)(4 * w4) + i, v[k]);
+                }
+            }
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 attention_sigmoid_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
@@ -139,6 +207,24 @@ extern "C" int rfx_sig_qkv_post(const void* proj, int in_dt, int ld, int col0, c
     if (R <= 0) return 0;
     if (rot_dims < 0 || rot_dims % 2 || rot_dims > d) return RFX_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    const bool by4 = d > 0 && dv > 0 && ((d | dv | ld | col0) & 3) == 0 && rot_dims % 8 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(q_out) |
+                       reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages)) & 15) == 0;
+    if (by4) {
+        const int n_rows = R >= 512 ? POST_ROWS : 1;  // (fewer rows: a block each, or SMs are without one)
+        const size_t smem = (size_t)n_rows * rot_dims * sizeof(float);
+        const int blocks = (R + n_rows - 1) / n_rows;
+#define RFX_GO(TI, TO)                                                                                          \
+    RFX_LAUNCH((sig_qkv_post4_kernel<TI, TO>), blocks, 256, smem, s, (const TI*)proj, ld, col0, denom, rot_dims, \
+               row_pos, row_slot, (TO*)q_out, (TO*)k_pages, (TO*)v_pages, page_table, max_pages, page_size,     \
+               nq, nkv, d, dv, writes_cache, R, n_rows)
+        if (in_dt == RFX_DT_F32 && out_dt == RFX_DT_F32) RFX_GO(float, float);
+        else if (in_dt == RFX_DT_F32 && out_dt == RFX_DT_BF16) RFX_GO(float, __nv_bfloat16);
+        else if (in_dt == RFX_DT_BF16 && out_dt == RFX_DT_BF16) RFX_GO(__nv_bfloat16, __nv_bfloat16);
+        else return RFX_ERR_BAD_ARG;
+#undef RFX_GO
+        return 0;
+    }
     const size_t smem = (size_t)rot_dims * sizeof(float);
 #define RFX_GO(TI, TO)                                                                                        \
     RFX_LAUNCH((sig_qkv_post_kernel<TI, TO>), R, 256, smem, s, (const TI*)proj, ld, col0, denom, rot_dims,   \

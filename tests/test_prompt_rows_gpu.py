@@ -86,3 +86,31 @@ def test_norms_of_many_small_parts(groups, size, shared, dtype, gate):
 
     half = n // 2
     assert torch.equal(run(slice(0, n)), torch.cat([run(slice(0, half)), run(slice(half, n))]))
+
+
+@pytest.mark.parametrize("rows", [5, 514])
+@pytest.mark.parametrize("dim,vdim,rot", [(128, 128, 64), (36, 20, 24), (64, 64, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("writes", [True, False])
+def test_rotated_rows_by_fours(rows, dim, vdim, rot, dtype, writes):
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    nq, nkv, page, col0 = 6, 2, 64, 8
+    wide = col0 + nq * dim + nkv * (dim + vdim) + 4
+    proj = torch.randn((rows, wide), generator=g, device=DEV)
+    other = torch.zeros((rows, wide + 1), device=DEV)  # an odd stride: an element a thread
+    other[:, :wide] = proj
+    pages = rows // page + 2
+    table = torch.randperm(pages, generator=g, device=DEV).to(torch.int32).view(1, -1)
+    pos, slot = i32(range(3, rows + 3)), i32([0] * rows)
+    rotation = None
+    if rot:
+        denom = 10000.0 ** (torch.arange(rot // 2, device=DEV, dtype=torch.float32) * 2 / rot)
+        rotation = type("R", (), dict(pairing="half", magnitude=1.0, denominators=denom, rotary_dim=rot))()
+    got = []
+    for p in (proj, other):
+        kp, vp = torch.zeros((pages, nkv, page, dim), device=DEV, dtype=dtype), torch.zeros((pages, nkv, page, vdim), device=DEV, dtype=dtype)
+        q = ops().sig_qkv_post(p, col0, rotation, pos, slot, kp, vp, table, page, nq, nkv, dim, vdim, writes, dtype)
+        got.append((q, kp, vp))
+    for x, y in zip(*got):
+        assert torch.equal(x, y)
+    assert got[0][0].abs().sum() > 0 and bool(got[0][2].abs().sum() > 0) == writes
