@@ -930,6 +930,14 @@ def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale:
         if st != native.ERR_UNSUPPORTED:  # rows that are not on 16 bytes
             native.check(st, f"mlstm_chunks (dim={dim}, vdim={vdim})")
             return num, den
+    if not exact and _one_row_each(batch, R):
+        st = native.lib().rfx_mlstm_step(
+            proj.data_ptr(), proj.shape[1], q_off, k_off, v_off, i_off, f_off, _chk(bias_i, "bias_i", torch.float32),
+            _chk(bias_f, "bias_f", torch.float32), float(cap), float(q_scale), _chk(batch.seq_slot, "seq_slot", torch.int32),
+            R, _chk(state, "state", torch.float32), num.data_ptr(), den.data_ptr(), heads, dim, vdim, _stream())
+        if st != native.ERR_UNSUPPORTED:  # other sizes, or not on 16 bytes
+            native.check(st, f"mlstm_step (dim={dim}, vdim={vdim})")
+            return num, den
     fn = native.lib().rfx_mlstm_chunk if chunked else native.lib().rfx_mlstm_scan
     st = fn(
         proj.data_ptr(), proj.shape[1], q_off, k_off, v_off, i_off, f_off,
@@ -1803,6 +1811,11 @@ def attention_sigmoid(q, k_pages, v_pages, page_table, page_size, batch, nq, nkv
 
 
 # ------------------------------------------- recurrences with a matrix state a head
+def _one_row_each(batch, rows: int) -> bool:
+    """A decode step: every sequence has exactly one of the step's rows, in their order."""
+    return _most_rows(batch) == 1 and rows == batch.seq_slot.numel()
+
+
 def _most_rows(batch) -> int:
     """The most rows a sequence of the step brings; 0 where the caller's batch does not say."""
     return int(getattr(batch, "max_new", 0))
@@ -1858,6 +1871,15 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
         if st != native.ERR_UNSUPPORTED:  # rows or state that are not on 16 bytes
             native.check(st, f"ssd_chunk (heads={heads}, vdim={vdim}, states={states})")
             return out
+    if not exact and out_dtype == torch.float32 and _one_row_each(batch, R):
+        st = native.lib().rfx_ssd_step(
+            _chk(xbc, "xbc", torch.float32), xbc.shape[1], _chk(proj, "proj", torch.float32), proj.shape[1], int(z_off),
+            int(dt_off), _chk(dt_bias, "dt_bias", torch.float32), _chk(A, "A", torch.float32),
+            _chk(D, "D", torch.float32), _chk(state, "state", torch.float32), state.stride(0), int(state_off),
+            _chk(batch.seq_slot, "seq_slot", torch.int32), R, out.data_ptr(), heads, vdim, states, groups, _stream())
+        if st != native.ERR_UNSUPPORTED:  # other sizes, or not on 16 bytes
+            native.check(st, f"ssd_step (heads={heads}, vdim={vdim}, states={states})")
+            return out
     st = native.lib().rfx_ssd_scan(
         _chk(xbc, "xbc", torch.float32), xbc.shape[1], _chk(proj, "proj", torch.float32), proj.shape[1], int(z_off),
         int(dt_off), _chk(dt_bias, "dt_bias", torch.float32), _chk(A, "A", torch.float32), _chk(D, "D", torch.float32),
@@ -1908,6 +1930,16 @@ def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: in
             _stream())
         if st != native.ERR_UNSUPPORTED:  # rows that are not on 16 bytes, a rate beyond 2
             native.check(st, f"delta_rule_chunk (heads={heads}, dim={dim})")
+            return out
+    if not exact and _one_row_each(batch, R):
+        st = native.lib().rfx_delta_step(
+            _chk(proj, "proj", torch.float32), proj.shape[1], int(r_off), int(k_off), int(v_off), int(a_off),
+            _chk(wpre, "wpre", torch.float32), _chk(w_bias, "w_bias", torch.float32),
+            _chk(a_bias, "a_bias", torch.float32), float(rate), float(unit_eps), _chk(state, "state", torch.float32),
+            state.stride(0), int(state_off), _chk(batch.seq_slot, "seq_slot", torch.int32), R, out.data_ptr(), heads, dim,
+            _stream())
+        if st != native.ERR_UNSUPPORTED:  # other sizes, or not on 16 bytes
+            native.check(st, f"delta_step (heads={heads}, dim={dim})")
             return out
     st = native.lib().rfx_delta_rule(
         _chk(proj, "proj", torch.float32), proj.shape[1], int(r_off), int(k_off), int(v_off), int(a_off),
@@ -1977,6 +2009,14 @@ def gated_delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor
             _chk(batch.seq_slot, "seq_slot", torch.int32), row0, S, out.data_ptr(), heads, kv_heads, dim, vdim, _stream())
         native.check(st, f"gated_delta_chunk (heads={heads}, dim={dim}, vdim={vdim})")
         return out
+    if not exact and _one_row_each(batch, R):
+        st = native.lib().rfx_gated_delta_step(
+            _chk(qkv, "qkv", torch.float32), _chk(gates, "gates", torch.float32), _chk(state, "state", torch.float32),
+            state.stride(0), int(state_off), _chk(batch.seq_slot, "seq_slot", torch.int32), R, out.data_ptr(), heads,
+            kv_heads, dim, vdim, _stream())
+        if st != native.ERR_UNSUPPORTED:  # other sizes, or not on 16 bytes
+            native.check(st, f"gated_delta_step (heads={heads}, dim={dim}, vdim={vdim})")
+            return out
     st = native.lib().rfx_gated_delta_scan(
         _chk(qkv, "qkv", torch.float32), _chk(gates, "gates", torch.float32), _chk(state, "state", torch.float32),
         state.stride(0), int(state_off), _chk(batch.seq_slot, "seq_slot", torch.int32),

@@ -114,6 +114,14 @@ _SIGNATURES = {
     "rfx_mlstm_chunks": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
                          c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                          c_int, c_void_p, c_void_p],
+    "rfx_mlstm_step": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
+                       c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "rfx_ssd_step": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                     c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "rfx_delta_step": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float,
+                       c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p],
+    "rfx_gated_delta_step": [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_int,
+                             c_int, c_int, c_int, c_void_p],
     "rfx_mlstm_out": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int,
                       c_int, c_int, c_void_p],
     "rfx_moe_route": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
