@@ -36,19 +36,20 @@ def dt_code(dtype: torch.dtype) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the current stream's handle without an object around it (a launch asks for it; 1.3 us each otherwise)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _chk(t: Optional[torch.Tensor], name: str, dtype=None) -> int:
     if t is None:
         return 0
+    if t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype == dtype):
+        return t.data_ptr()
     if not t.is_cuda:
         raise CudaError(f"{name} must live on the GPU (there is no CPU path)")
     if not t.is_contiguous():
         raise InvalidInput(f"{name} must be contiguous")
-    if dtype is not None and t.dtype != dtype:
-        raise InvalidInput(f"{name} must be {dtype}, got {t.dtype}")
-    return t.data_ptr()
+    raise InvalidInput(f"{name} must be {dtype}, got {t.dtype}")
 
 
 # ---------------------------------------------------------------- elementwise

@@ -23,7 +23,7 @@ under a replay.
 from __future__ import annotations
 
 import contextlib
-from typing import List, Optional
+from typing import Dict, List, Optional
 
 import torch
 
@@ -36,6 +36,8 @@ class _Region:
     def __init__(self, device):
         self.device = device
         self.buf: Optional[torch.Tensor] = None
+        self.size, self.base = 0, 0  # of `buf`: bytes, and how far it starts beyond a boundary of _ALIGN
+        self.typed: Dict[torch.dtype, torch.Tensor] = {}  # `buf` as numbers of a type
         self.offset = 0
         self.need = 0  # bytes this region would have needed so far (its high-water mark)
 
@@ -43,22 +45,30 @@ class _Region:
         self.offset = 0
 
     def take(self, shape, dtype) -> Optional[torch.Tensor]:
-        n = 1
-        for s in shape:
-            n *= int(s)
-        nbytes = n * _ITEM[dtype]
-        base = 0 if self.buf is None else self.buf.data_ptr() % _ALIGN  # results start on 256 bytes
-        start = (self.offset + base + _ALIGN - 1) // _ALIGN * _ALIGN - base
-        end = start + nbytes
+        shape = [int(s) for s in shape]
+        n, strides = 1, []
+        for s in reversed(shape):
+            strides.append(n)
+            n *= s
+        item = _ITEM[dtype]
+        start = (self.offset + self.base + _ALIGN - 1) // _ALIGN * _ALIGN - self.base  # results start on 256 bytes
+        end = start + n * item
         self.offset = end
         self.need = max(self.need, end)
-        if self.buf is None or end > self.buf.numel():
+        if end > self.size:
             return None
-        return self.buf[start:end].view(dtype).view(tuple(int(s) for s in shape))
+        if n == 0 or start % item:
+            return self.buf[start:end].view(dtype).view(shape)
+        whole = self.typed.get(dtype)
+        if whole is None:
+            whole = self.typed[dtype] = self.buf[: self.size // item * item].view(dtype)
+        return whole.as_strided(shape, strides[::-1], whole.storage_offset() + start // item)
 
     def settle(self) -> None:
-        if self.need > (0 if self.buf is None else self.buf.numel()):
+        if self.need > self.size:
             self.buf = torch.empty((self.need * 5 // 4 + _ALIGN,), dtype=torch.uint8, device=self.device)
+            self.size, self.base = self.buf.numel(), self.buf.data_ptr() % _ALIGN
+            self.typed = {}
 
 
 class Workspace:
