@@ -12,6 +12,9 @@
 //               keys side by side.
 //   values      the lanes over a head's elements, key after key: l = fma(l, corr, p),
 //               acc = fma(acc, corr, p * v).
+// Reads of shared memory and a tile's chain of steps bound it (9,000 cycles a tile of 32 keys with two blocks an
+// SM).  8 heads of 128 for prompts of 155, 311 and 235 rows: 50 us; 65 with the early rows' blocks first and a
+// page looked up by every copying thread for each of its rows.  24 heads, 8 prompts of 709 rows in all: 53 (65).
 #include "attn_mma.cuh"
 #include "common.cuh"
 #include "exact_math.cuh"
@@ -99,6 +102,7 @@ struct Args {
     const int *seq_slot, *seq_start, *seq_new, *seq_row0;
     float* out;
     int nq, heads, rows;  // query heads and rows a block takes
+    int seqs;
     int window, keep_first;
     float scale;
     const float *sink, *slopes;
@@ -106,18 +110,19 @@ struct Args {
 };
 
 template <int NI>
-__global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(Args A) {
+__global__ void __launch_bounds__(WARPS * 32, NI > 4 ? 1 : 2) attention_f32_kernel(Args A) {
     constexpr int d = 32 * NI, KLD = d + 4, d4 = d / 4;
     extern __shared__ __align__(16) float sm[];
     float *Qs = sm, *Ks = Qs + QUERIES * d, *Vs = Ks + 2 * KEYS * KLD;
     float2* Ws = reinterpret_cast<float2*>(Vs + 2 * KEYS * d);  // [WARPS][2][KEYS]: corr, p
     pdl_prologue();
-    const int seq = blockIdx.y, row_first = blockIdx.x * A.rows;
-    const int n_new = A.seq_new[seq];
+    const int group = A.nq / A.cache.n_kv_heads, parts = (group + A.heads - 1) / A.heads, sets = A.cache.n_kv_heads * parts;
+    // late rows have many keys, early ones few: the latest ones first
+    const int set = blockIdx.x % sets, seq = blockIdx.x / sets % A.seqs;
+    const int n_new = A.seq_new[seq], row_first = (int)((gridDim.x - 1 - blockIdx.x) / (sets * A.seqs)) * A.rows;
     if (row_first >= n_new) return;
     const int n_rows = min(A.rows, n_new - row_first);
-    const int group = A.nq / A.cache.n_kv_heads, parts = (group + A.heads - 1) / A.heads;
-    const int kvh = blockIdx.z / parts, h0 = kvh * group + (blockIdx.z - kvh * parts) * A.heads;
+    const int kvh = set / parts, h0 = kvh * group + (set - kvh * parts) * A.heads;
     const int n_heads = min(A.heads, (kvh + 1) * group - h0);
     const int slot = A.seq_slot[seq], p_first = A.seq_start[seq] + row_first, p_last = p_first + n_rows - 1;
     const int row0 = A.seq_row0[seq] + row_first;
@@ -129,11 +134,15 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(Args A) {
         ++t;
         return KEYS * t >= kept_last && KEYS * t + KEYS - 1 < lo_first ? lo_first / KEYS : t;
     };
-    auto fetch = [&](int t, int buf) {
+    // a page holds whole tiles (or not: then every row looks its place up); a tile's page is asked for a tile ahead
+    const bool whole = A.cache.page_size % KEYS == 0;
+    auto place = [&](int t) { return whole && t <= p_last / KEYS ? kv_offset(A.cache, slot, KEYS * t, kvh) : 0; };
+    auto fetch = [&](int t, int buf, size_t base) {
+#pragma unroll
         for (int e = tid; e < KEYS * d4; e += WARPS * 32) {
             const int i = e / d4, c = 4 * (e - i * d4), j = KEYS * t + i;
             const bool ok = j <= p_last && (j < kept_last || j >= lo_first);
-            const size_t at = ok ? kv_offset(A.cache, slot, j, kvh) + c : 0;
+            const size_t at = !ok ? 0 : whole ? base + i * d + c : kv_offset(A.cache, slot, j, kvh) + c;
             attn::cp_async_16(Ks + (buf * KEYS + i) * KLD + c, A.k_pages + at, ok);
             attn::cp_async_16(Vs + (buf * KEYS + i) * d + c, A.v_pages + at, ok);
         }
@@ -141,7 +150,8 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(Args A) {
     };
     const int t_end = p_last / KEYS;
     int t = next(-1);
-    fetch(t, 0);
+    fetch(t, 0, place(t));
+    size_t base = place(next(t));
     for (int e = tid; e < QUERIES * d4; e += WARPS * 32) {
         const int i = e / d4, c = 4 * (e - i * d4), r = i / A.heads, h = i - r * A.heads;
         const bool ok = r < n_rows && h < n_heads;
@@ -171,7 +181,8 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(Args A) {
     for (int buf = 0; t <= t_end; buf ^= 1) {
         const int t_next = next(t);
         if (t_next <= t_end) {
-            fetch(t_next, buf ^ 1);
+            fetch(t_next, buf ^ 1, base);
+            base = place(next(t_next));
             attn::cp_async_wait<1>();
         } else {
             attn::cp_async_wait<0>();
@@ -277,17 +288,21 @@ extern "C" int rfx_attention_f32(const float* q, const float* k_pages, const flo
         return RFX_ERR_UNSUPPORTED;
     const int group = nq / nkv;
     Args a{q, k_pages, v_pages, PagedKV{page_table, max_pages, page_size, nkv, head_dim}, seq_slot, seq_start, seq_new,
-           seq_row0, out, nq, 0, 0, window, window > 0 ? keep_first : 0, scale, sink, slopes, softcap};
+           seq_row0, out, nq, 0, 0, S, window, window > 0 ? keep_first : 0, scale, sink, slopes, softcap};
     // sixteen queries: all heads of the group that fit, then rows (a row alone: half the warps idle at worst)
     a.heads = group < QUERIES ? group : QUERIES;
     a.rows = QUERIES / a.heads;
     if (a.rows > max_new) a.rows = max_new;
     const int parts = (group + a.heads - 1) / a.heads;
-    if ((long long)nkv * parts > 65535) return RFX_ERR_UNSUPPORTED;
-    dim3 grid((max_new + a.rows - 1) / a.rows, S, nkv * parts);
+    const long long blocks = ((long long)max_new + a.rows - 1) / a.rows * S * nkv * parts;
+    if ((long long)nkv * parts > 65535 || blocks > 2147483647LL) return RFX_ERR_UNSUPPORTED;
+    dim3 grid((unsigned)blocks);
+    // few blocks: one an SM, taken longest first, ends earlier than two side by side (50 us against 60 above)
+    const bool alone = blocks <= 4LL * sm_count();
 #define RFX_GO(NI)                                                                                                 \
     do {                                                                                                           \
-        constexpr size_t smem = (QUERIES * 32 * NI + 2 * KEYS * (64 * NI + 4) + WARPS * 2 * KEYS * 2) * sizeof(float); \
+        size_t smem = (QUERIES * 32 * NI + 2 * KEYS * (64 * NI + 4) + WARPS * 2 * KEYS * 2) * sizeof(float);         \
+        if (alone && smem < 120 * 1024) smem = 120 * 1024;                                                           \
         cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
                                              (int)smem);                                                            \
         if (e != cudaSuccess) return (int)e;                                                                        \

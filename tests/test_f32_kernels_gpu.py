@@ -77,3 +77,16 @@ def test_attention_bits_are_the_plain_kernels(d, nq, nkv, window, keep_first, ex
                                 keep_first, cap)
     assert torch.isfinite(ref).all()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("page", [16, 32, 48, 96])  # 16 and 48: a tile of 32 keys lies in several pages
+def test_attention_bits_with_pages_of_other_sizes(page):
+    g = torch.Generator(device=DEV).manual_seed(page)
+    nq, nkv, d, counts, starts, slots = 4, 2, 64, (70, 1, 33), (0, 100, 45), (2, 0, 1)
+    per = 112 // page + 2
+    k, v = (torch.randn((3 * per, nkv, page, d), generator=g, device=DEV) for _ in range(2))
+    t = torch.randperm(3 * per, generator=torch.Generator().manual_seed(1)).view(3, per).to(torch.int32).to(DEV)
+    q, b = torch.randn((sum(counts), nq * d), generator=g, device=DEV), Batch(counts, starts, slots)
+    got = ops().attention_f32(q, k, v, t, page, b, nq, nkv, d, None, d ** -0.5)
+    ref = ops().attention_plain(q, k, v, t, page, b.row_pos, b.row_slot, nq, nkv, d, None, d ** -0.5)
+    assert torch.equal(got, ref)
