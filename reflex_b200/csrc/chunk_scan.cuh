@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
 
 // Four neighbouring elements of a head's memory a thread; eight chunks' sums are fetched ahead.
 template <class Pol>
-__global__ void __launch_bounds__(128) chunk_carry_kernel(Pol pol, Step st) {
+__global__ void __launch_bounds__(128, 4) chunk_carry_kernel(Pol pol, Step st) {
     constexpr int AHEAD = 8;
     rfx::pdl_prologue();
     const int seq = st.round.seq0 + blockIdx.y, h = blockIdx.z;

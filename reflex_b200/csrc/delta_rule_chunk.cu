@@ -25,6 +25,7 @@
 #include "chunk_plan.cuh"
 #include "common.cuh"
 #include "fma_tiles.cuh"
+#include "sm100.cuh"
 
 namespace {
 
@@ -235,40 +236,58 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
 // key channels.  Four lanes make a tile of 4 x 4, each a quarter of the channels (four of each
 // sixteen), whose parts meet by shuffles, so that a chunk has one barrier.  (The quarters in warps of
 // their own, meeting in shared memory: no faster; a thread a row and eight columns, all channels:
-// 121 us in place of 99 for 64 chunks of 32 heads.)  M and R of the next chunks arrive meanwhile.
-// What bounds a step is the latency of its reads of shared memory.  Sixteen columns a block, eight where
+// 121 us in place of 99 for 64 chunks of 32 heads.)  M and R of the next chunks arrive meanwhile, a
+// chunk's by one bulk copy (by all threads, 16 bytes each, a quarter of a step's time went into issuing
+// the copies).  What bounds a step is the latency of its reads of shared memory.  Four sequences of 571, 714, 428
+// and 286 rows of 32 heads: 75 us; 105 with copies by all threads and sequences in their own order.  Sixteen columns a block, eight where
 // that leaves SMs without a block: both kernels take 240 and 302 us for 2,048 rows of 32 heads with
 // eight and sixteen, 460 and 442 for 64 heads.
 constexpr int TLD = D + 16;  // sixteen floats more: two columns' sixteens meet all banks
 template <int COLS>
 __global__ void __launch_bounds__(COLS * (D + L) / 4)
 delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stride, long long state_off,
-                        float* __restrict__ out, int heads) {
+                        float* __restrict__ out, int heads, int* err) {
     constexpr int CG = COLS / 4, THREADS = CG * (D + L);
     extern __shared__ __align__(16) float sm[];
     __shared__ __align__(16) float Ss[2][COLS * TLD];  // S^T, column 4 c + j at row CG j + c
+    __shared__ uint64_t full[STAGES];
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; ++i) sm100::mbar_init(&full[i], 1);
+        sm100::fence_barrier_init();
+    }
     pdl_prologue();
-    const int seq = st.round.seq0 + blockIdx.x, h = blockIdx.y, c0 = COLS * blockIdx.z;
-    const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows;
-    const int rows = min(st.seq_row0[seq + 1] - from, st.round.seg_rows);
+    // the longest sequences' blocks first (up to 32 of them are put in order)
+    auto rows_of = [&](int s) {
+        const int from = st.seq_row0[s] + st.round.seg * st.round.seg_rows;
+        return min(st.seq_row0[s + 1] - from, st.round.seg_rows);
+    };
+    int seq = st.round.seq0 + blockIdx.z;
+    if (gridDim.z > 1 && gridDim.z <= 32) {
+        const int lane = threadIdx.x & 31, n = gridDim.z, mine = lane < n ? rows_of(st.round.seq0 + lane) : 0;
+        int longer = 0;
+        for (int i = 0; i < n; ++i) {
+            const int other = __shfl_sync(0xffffffffu, mine, i);
+            longer += other > mine || (other == mine && i < lane);
+        }
+        seq = st.round.seq0 + __ffs(__ballot_sync(0xffffffffu, lane < n && longer == blockIdx.z)) - 1;
+    }
+    const int h = blockIdx.y, c0 = COLS * blockIdx.x;
+    const int row0 = st.seq_row0[seq], from = row0 + st.round.seg * st.round.seg_rows, rows = rows_of(seq);
     if (rows <= 0) return;
     const int chunks = (rows + L - 1) / L, hd = heads * D, tid = threadIdx.x;
     const int quarter = tid & 3, cg = tid >> 2 & (CG - 1), first_row = 4 * (tid / COLS);  // the tile's first row
     const int row = first_row + quarter, c = c0 + 4 * cg;  // whose results the lane ends up with, and their columns
     const float* base = st.scratch + (chunk::place_in(st.round, L, row0, seq, 0) * heads + h) * PLACE;
     const size_t step = (size_t)heads * PLACE;
-    int to = 0;
-    auto fetch = [&](int k) {
+    // a chunk's factors lie in one piece: one copy of 26 KB, issued by one thread
+    auto fetch = [&](int k, int to) {
         if (k < chunks) {
-            const float* src = base + k * step;
-            float* dst = sm + to * MR;
-            for (int e = tid; e < MR / 4; e += THREADS) attn::cp_async_16(dst + 4 * e, src + 4 * e, true);
+            sm100::mbar_expect_tx(&full[to], MR * sizeof(float));
+            sm100::bulk_load(sm + to * MR, base + k * step, MR * sizeof(float), &full[to]);
         }
-        attn::cp_async_commit();
-        to = to + 1 == STAGES ? 0 : to + 1;
     };
-#pragma unroll
-    for (int k = 0; k < STAGES; ++k) fetch(k);
+    if (tid == 0)
+        for (int k = 0; k < STAGES; ++k) fetch(k, k);
     float* Sg = state + (size_t)st.seq_slot[seq] * state_stride + state_off + (size_t)h * D * D;
     for (int e = tid; e < COLS * D / 4; e += THREADS) {
         const int col = e / (D / 4), k = 4 * (e % (D / 4));
@@ -280,14 +299,22 @@ delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stri
         else if (row - D < rows - k * L) next = load4(out + (size_t)(from + k * L + row - D) * hd + h * D + c);
     };
     ahead(0);
-    attn::cp_async_wait<STAGES - 1>();
     __syncthreads();
-    int at = 0;
+    int at = 0, round = 0;
+    bool waits = true;  // a wait that ran out is reported, and the walk ends with whatever is there
     for (int k = 0; k < chunks; ++k) {
+        const int now = at;
+        if (waits && !sm100::mbar_wait(&full[now], round & 1)) {
+            waits = false;
+            if (err) atomicExch(err, 43);
+        }
         const float* m = sm + at * MR + first_row * LD + 4 * quarter;
         const float* S = Ss[k & 1] + cg * TLD + 4 * quarter;
         float* Sn = Ss[(k + 1) & 1];
-        at = at + 1 == STAGES ? 0 : at + 1;
+        if (++at == STAGES) {
+            at = 0;
+            ++round;
+        }
         own = next;
         if (k + 1 < chunks) ahead(k + 1);
         float acc[4][4] = {};
@@ -335,9 +362,8 @@ delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stri
         } else if (row - D < rows - k * L) {
             store4(out + (size_t)(from + k * L + row - D) * hd + h * D + c, own);
         }
-        attn::cp_async_wait<STAGES - 2>();
-        __syncthreads();  // the next S and the next chunk's factors are there; this chunk's have been read
-        fetch(k + STAGES);
+        __syncthreads();  // the next S is there; this chunk's factors have been read
+        if (tid == 0) fetch(k + STAGES, now);
     }
     if (row < D) {
         float* s = Sg + (size_t)c * D + row;
@@ -365,7 +391,7 @@ extern "C" int rfx_delta_rule_chunk(const float* proj, int ld, int r_off, int k_
                                     const float* wpre, const float* w_bias, const float* a_bias, float rate,
                                     float unit_eps, float* state, long long state_stride, long long state_off,
                                     const int* seq_slot, const int* seq_row0, int n_seq, int R, int max_rows, float* out,
-                                    float* scratch, int heads, int d, void* stream) {
+                                    float* scratch, int heads, int d, int* err, void* stream) {
     if (n_seq <= 0 || R <= 0 || max_rows <= 0) return 0;
     if (heads <= 0 || d <= 0) return RFX_ERR_BAD_ARG;
     if (d != D || !(rate >= 0.0f && rate <= 2.0f) || n_seq > 65535 || heads > 65535 ||
@@ -395,11 +421,11 @@ extern "C" int rfx_delta_rule_chunk(const float* proj, int ld, int r_off, int k_
             RFX_LAUNCH(delta_chunk_prep_kernel, dim3(chunks, seqs, heads), 256, sm_prep, s, proj, ld, r_off, k_off, v_off,
                        a_off, wpre, w_bias, a_bias, rate, unit_eps, st, out, heads);
             if (narrow)
-                RFX_LAUNCH(delta_chunk_walk_kernel<8>, dim3(seqs, heads, D / 8), 2 * (D + L), sm_walk, s, st, state,
-                           state_stride, state_off, out, heads);
+                RFX_LAUNCH(delta_chunk_walk_kernel<8>, dim3(D / 8, heads, seqs), 2 * (D + L), sm_walk, s, st, state,
+                           state_stride, state_off, out, heads, err);
             else
-                RFX_LAUNCH(delta_chunk_walk_kernel<16>, dim3(seqs, heads, D / 16), 4 * (D + L), sm_walk, s, st, state,
-                           state_stride, state_off, out, heads);
+                RFX_LAUNCH(delta_chunk_walk_kernel<16>, dim3(D / 16, heads, seqs), 4 * (D + L), sm_walk, s, st, state,
+                           state_stride, state_off, out, heads, err);
         }
     return 0;
 }

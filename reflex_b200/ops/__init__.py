@@ -1928,7 +1928,7 @@ def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: in
             _chk(a_bias, "a_bias", torch.float32), float(rate), float(unit_eps), _chk(state, "state", torch.float32),
             state.stride(0), int(state_off), _chk(batch.seq_slot, "seq_slot", torch.int32),
             _chk(batch.seq_row0, "seq_row0", torch.int32), S, R, most, out.data_ptr(), scratch.data_ptr(), heads, dim,
-            _stream())
+            device_error_word(proj.device).data_ptr(), _stream())
         if st != native.ERR_UNSUPPORTED:  # rows that are not on 16 bytes, a rate beyond 2
             native.check(st, f"delta_rule_chunk (heads={heads}, dim={dim})")
             return out

@@ -194,7 +194,7 @@ _SIGNATURES = {
                        c_void_p],
     "rfx_delta_rule_chunk": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float,
                              c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
-                             c_void_p, c_int, c_int, c_void_p],
+                             c_void_p, c_int, c_int, c_void_p, c_void_p],
     "rfx_short_conv": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong,
                        c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "rfx_conv_qkv_post": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_void_p,
