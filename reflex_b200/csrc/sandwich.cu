@@ -446,6 +446,24 @@ __global__ void scaled_sum_kernel(float* __restrict__ a, const float* __restrict
         a[i] = fmaf(sa, a[i], sb * b[i]);
 }
 
+// by fours, two of them a thread in flight (2,048 x 2,048, 50 MB: 11.3 us an element a thread, 6.7 so)
+__global__ void __launch_bounds__(256) scaled_sum4_kernel(float4* __restrict__ a, const float4* __restrict__ b, float sa, float sb, size_t n4) {
+    pdl_prologue();
+    const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
+    float4 x[2], y[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (i0 + 256 * k < n4) {
+            x[k] = a[i0 + 256 * k];
+            y[k] = b[i0 + 256 * k];
+        }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (i0 + 256 * k < n4)
+            a[i0 + 256 * k] = make_float4(fmaf(sa, x[k].x, sb * y[k].x), fmaf(sa, x[k].y, sb * y[k].y),
+                                          fmaf(sa, x[k].z, sb * y[k].z), fmaf(sa, x[k].w, sb * y[k].w));
+}
+
 inline int blocks_for(size_t n, int threads) {
     size_t b = (n + threads - 1) / threads;
     const size_t cap = (size_t)sm_count() * 8;
@@ -615,6 +633,12 @@ extern "C" int rfx_tanh_cols(const float* in, int ld, int col, void* out, int ou
 
 extern "C" int rfx_scaled_sum(float* a, const float* b, float sa, float sb, long long n, void* stream) {
     if (n <= 0) return 0;
+    const long long blocks = (n / 4 + 511) / 512;
+    if (n % 4 == 0 && blocks <= 2147483647LL && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0) {
+        RFX_LAUNCH(scaled_sum4_kernel, (int)blocks, 256, 0, (cudaStream_t)stream, reinterpret_cast<float4*>(a),
+                   reinterpret_cast<const float4*>(b), sa, sb, (size_t)n / 4);
+        return 0;
+    }
     RFX_LAUNCH(scaled_sum_kernel, blocks_for((size_t)n, 256), 256, 0, (cudaStream_t)stream, a, b, sa, sb, (size_t)n);
     return 0;
 }

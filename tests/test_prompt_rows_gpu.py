@@ -114,3 +114,11 @@ def test_rotated_rows_by_fours(rows, dim, vdim, rot, dtype, writes):
     for x, y in zip(*got):
         assert torch.equal(x, y)
     assert got[0][0].abs().sum() > 0 and bool(got[0][2].abs().sum() > 0) == writes
+
+
+@pytest.mark.parametrize("n", [4, 2048, 2052, 4100, 262147])  # the last one: an element a thread
+def test_scaled_sums_by_fours(n):
+    a, b = (torch.randn(n, generator=torch.Generator(device=DEV).manual_seed(s), device=DEV) for s in (1, 2))
+    odd = torch.empty(n + 1, device=DEV)[1:].copy_(a)  # off 16 bytes: an element a thread
+    ops().scaled_sum_(odd, b, 0.75, 0.55)
+    assert torch.equal(ops().scaled_sum_(a, b, 0.75, 0.55), odd)
