@@ -38,12 +38,12 @@ __device__ __forceinline__ size_t chunk_place(int row0, int seq, int c) { return
 
 // A block a (chunk, query/key head): the products between the chunk's rows once, by 32-bit multiply-adds,
 // each warp some of the channels (four by four results a lane, of [k; q] by k); then per value head of
-// the group (eight at a time) T, M and the decays' products.  Bound by the steps' latencies: 56 us for 4,096
+// the group (eight at a time) T, M and the decays' products.  Bound by the steps' latencies: 53 us for 4,096
 // rows of 16 heads of 128 with two value heads each.  (A thread a pair of rows, bound by its reads of shared
 // memory: 66; on the tensor cores with operands split in two 51, and the results 1.4 times as far from 64 bits.)
 constexpr int PREP_WARPS = CH * CH / 32, PREP_HEADS = 8;
 __host__ __device__ constexpr int prep_ld(int d) { return (d + 15) / 16 * 16 + 4; }  // an odd number of 16 bytes
-__global__ void __launch_bounds__(CH * CH)
+__global__ void __launch_bounds__(CH * CH, 3)
 gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __restrict__ gates,
                               const int* __restrict__ seq_row0, float* __restrict__ coef, int H, int G, int d, int dv) {
     extern __shared__ __align__(16) float sm[];
