@@ -240,8 +240,8 @@ delta_chunk_prep_kernel(const float* __restrict__ proj, int ld, int r_off, int k
 // chunk's by one bulk copy (by all threads, 16 bytes each, a quarter of a step's time went into issuing
 // the copies).  What bounds a step is the latency of its reads of shared memory.  Four sequences of 571, 714, 428
 // and 286 rows of 32 heads: 75 us; 105 with copies by all threads and sequences in their own order.  Sixteen columns a block, eight where
-// that leaves SMs without a block: both kernels take 240 and 302 us for 2,048 rows of 32 heads with
-// eight and sixteen, 460 and 442 for 64 heads.
+// that leaves SMs without a block: both kernels take 224 and 282 us for 2,048 rows of 32 heads with
+// eight and sixteen, 441 and 412 for 64 heads.
 constexpr int TLD = D + 16;  // sixteen floats more: two columns' sixteens meet all banks
 template <int COLS>
 __global__ void __launch_bounds__(COLS * (D + L) / 4)

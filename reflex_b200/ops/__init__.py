@@ -886,16 +886,17 @@ def mlstm_state_floats(dim: int, vdim: int) -> int:
 
 
 MLSTM_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_CHUNK_MIN_ROWS", 48, 1, 1 << 30)
-# Rows of a sequence from which all chunks go side by side (csrc/mlstm_chunk.cu); five eighths of that where the step
-# has eight (sequence, head) pairs or fewer.  Us side by side and chunk after chunk, heads of 128 x 256: 8 pairs 30.5
-# and 31.5 at 64 rows, 32 and 41 at 80; 16 pairs 47 and 41 at 80, 47 and 51 at 100; 32 pairs 55 and 52 at 100, 55 each
-# at 128; 128 pairs 160 each at 80, 168 and 199 at 100.
-MLSTM_SIDE_BY_SIDE_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_SIDE_BY_SIDE_MIN_ROWS", 128, 1, 1 << 30)
+# Rows of a sequence from which all chunks go side by side (csrc/mlstm_chunk.cu); three quarters of that with so few
+# or so many (sequence, head) pairs that chunk after chunk leaves SMs idle or fills them twice, 1.4 times as many
+# with about 32, which it just fills.  Us side by side and chunk after chunk (below 48 rows: walking), heads of 128 x
+# 256: 8 pairs 26.5 and 20 at 32 rows, 27.4 and 29.5 at 48; 16 pairs 32.4 and 31.7 at 64, 32 and 41 at 80; 32 pairs 47
+# and 42 at 80, 47 and 52 at 100; 64 pairs 61 and 62 at 64; 128 pairs 96 and 114 at 48.
+MLSTM_SIDE_BY_SIDE_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_SIDE_BY_SIDE_MIN_ROWS", 64, 1, 1 << 30)
 
 
 def _mlstm_side_by_side(most: int, rows: int, heads: int) -> bool:
-    few = heads * rows // max(1, most) <= 8
-    return most >= MLSTM_SIDE_BY_SIDE_MIN_ROWS * (0.625 if few else 1.0)
+    pairs = heads * rows // max(1, most)
+    return most >= MLSTM_SIDE_BY_SIDE_MIN_ROWS * (0.75 if pairs <= 8 or pairs > 96 else 1.4 if 16 < pairs < 48 else 1.0)
 
 
 def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale: float, batch,
@@ -1822,20 +1823,20 @@ def _most_rows(batch) -> int:
     return int(getattr(batch, "max_new", 0))
 
 
-# Rows of the longest sequence from which the chunked kernels run where a step has about 32 to 64
-# (sequence, head) pairs; twice as many with fewer, three quarters with up to 128 and half beyond: the walk's time
-# grows with the rows and, once its blocks share SMs, with the pairs, the chunks' hardly with either.
-# Measured, in chunks and walking, us at the rows around the crossing: 16 pairs 34.7 and 28.3 at 100 rows, 35.1 each
-# at 128; 32 pairs 34.9 and 33.1 at 64, 34.9 and 41.4 at 80; 64 pairs 36.4 and 38.9 at 64; 128 pairs 41 and 40 at 48;
-# 256 pairs 45 each at 32.
-SSD_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_SSD_CHUNK_MIN_ROWS", 72, 1, 1 << 30)
+# Rows of the longest sequence from which the chunked kernels run where a step has 32 to 64 (sequence, head)
+# pairs; more with fewer pairs, fewer with more: the walk's time grows with the rows and, once its blocks share SMs,
+# with the pairs, the chunks' hardly with either.  Measured, in chunks and walking, us at the rows around the
+# crossing: 16 pairs 20.7 and 18.1 at 64 rows, 21.2 and 23.3 at 80; 32 pairs 21.5 and 17.1 at 32, 21.9 and 26.2 at 48;
+# 64 pairs 22.7 and 20.2 at 32, 23.1 and 30.4 at 48; 128 pairs 26 and 27 at 32; 256 pairs 38 and 26 at 16, 38 and 45
+# at 32.
+SSD_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_SSD_CHUNK_MIN_ROWS", 44, 1, 1 << 30)
 
 
 def _ssd_in_chunks(most: int, rows: int, heads: int) -> bool:
     if not most:
         return False
     pairs = heads * rows // most  # as many sequences as the step's rows would make of the longest
-    return most >= SSD_CHUNK_MIN_ROWS * (2.0 if pairs < 32 else 1.0 if pairs <= 64 else 0.75 if pairs <= 128 else 0.5)
+    return most >= SSD_CHUNK_MIN_ROWS * (1.6 if pairs < 32 else 1.0 if pairs <= 64 else 0.75 if pairs <= 128 else 0.6)
 
 
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_bias: torch.Tensor, A: torch.Tensor,
@@ -1892,15 +1893,15 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_
 
 
 # Rows of the longest sequence from which the chunked kernels run where a step has up to about 64 (sequence, head)
-# pairs; four times as many beyond, where the walk fills the SMs too and a last chunk's absent rows weigh most.  In
-# chunks and walking, us: 16 pairs 18.5 and 18.1 at 48 rows; 32 pairs 24.6 and 27.6 at 64, 28 and 55 at 128; 64 pairs
-# 27 and 33 at 64; 128 pairs 33 and 34 at 64, 61 and 54 at 100, 62 and 67 at 128; 512 pairs 122 and 117 at 64, 225 and
-# 236 at 128.
-DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_DELTA_CHUNK_MIN_ROWS", 64, 1, 1 << 30)
+# pairs; 2.25 times as many beyond, where the walk fills the SMs too and a last chunk's absent rows weigh most.  In
+# chunks and walking, us: 16 pairs 18.9 and 18.1 at 48 rows, 18 and 23 at 64; 32 pairs 23.9 and 21.6 at 48, 24 and 28
+# at 64; 64 pairs 26.3 and 25.6 at 48, 26.5 and 33 at 64; 128 pairs 33 and 34 at 64, 60 and 54 at 100, 60 and 67 at
+# 128; 512 pairs 114 and 117 at 64, 209 and 188 at 100, 212 and 236 at 128.
+DELTA_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_DELTA_CHUNK_MIN_ROWS", 56, 1, 1 << 30)
 
 
 def _delta_in_chunks(most: int, rows: int, heads: int) -> bool:
-    return most > 0 and most >= DELTA_CHUNK_MIN_ROWS * (1 if heads * rows // most <= 64 else 4)
+    return most > 0 and most >= DELTA_CHUNK_MIN_ROWS * (1 if heads * rows // most <= 64 else 2.25)
 
 
 def delta_rule(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, a_off: int, wpre: torch.Tensor,
