@@ -18,7 +18,7 @@
 // work; chunks cost the memory's way out and back (heads x N x P floats each) and about twice the
 // arithmetic.  64 rows: with 32 the memories' traffic doubles, with 128 the products inside the chunk do.
 // A prompt of 2,048 rows, us: for 32 heads of 64 x 128 21 the chunks' sums, 13 the carry, 50 the rows (1,200
-// walking), for 8 of 128 x 256 24, 18 and 50 (760).  With the products by 32-bit multiply-adds, whose reads of
+// walking), for 8 of 128 x 256 24, 17 and 50 (760).  With the products by 32-bit multiply-adds, whose reads of
 // shared memory and whose latencies bound them, 42, 12 and 76, and 49, 18 and 65.  What bounds these now is
 // the instructions that take 32-bit numbers apart and put results together (about 1,500 a warp and item, 1.7 of
 // four issued a cycle); the tensor cores are busy a fifth of the time, the carry is bound by L2.
