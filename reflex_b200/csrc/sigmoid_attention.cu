@@ -211,7 +211,7 @@ extern "C" int rfx_sig_qkv_post(const void* proj, int in_dt, int ld, int col0, c
                      ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(q_out) |
                        reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages)) & 15) == 0;
     if (by4) {
-        const int n_rows = R >= 512 ? POST_ROWS : 1;  // (fewer rows: a block each, or SMs are without one)
+        const int n_rows = R >= 512 && rot_dims <= 2048 ? POST_ROWS : 1;  // (fewer rows: a block each, or SMs are without one)
         const size_t smem = (size_t)n_rows * rot_dims * sizeof(float);
         const int blocks = (R + n_rows - 1) / n_rows;
 #define RFX_GO(TI, TO)                                                                                          \
