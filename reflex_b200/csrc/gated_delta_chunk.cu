@@ -38,8 +38,8 @@ __device__ __forceinline__ size_t chunk_place(int row0, int seq, int c) { return
 
 // A block a (chunk, query/key head): the products between the chunk's rows once, by 32-bit multiply-adds,
 // each warp some of the channels (four by four results a lane, of [k; q] by k); then per value head of
-// the group (eight at a time) T, M and the decays' products.  Bound by the steps' latencies: 53 us for 4,096
-// rows of 16 heads of 128 with two value heads each.  (A thread a pair of rows, bound by its reads of shared
+// the group (eight at a time) T, M and the decays' products.  Bound by the steps' latencies: 45 us for 4,096
+// rows of 16 heads of 128 with two value heads each (53 with the decays' products by pairs of rows).  (A thread a pair of rows, bound by its reads of shared
 // memory: 66; on the tensor cores with operands split in two 51, and the results 1.4 times as far from 64 bits.)
 constexpr int PREP_WARPS = CH * CH / 32, PREP_HEADS = 8;
 __host__ __device__ constexpr int prep_ld(int d) { return (d + 15) / 16 * 16 + 4; }  // an odd number of 16 bytes
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(CH * CH, 3)
 gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __restrict__ gates,
                               const int* __restrict__ seq_row0, float* __restrict__ coef, int H, int G, int d, int dv) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ float L[PREP_HEADS][CH][CH + 1], gs[PREP_HEADS][CH], bs[PREP_HEADS][CH];
+    __shared__ float L[PREP_HEADS][CH][CH + 1], bs[PREP_HEADS][CH];  // L: the decays' products until it is made
     rfx::pdl_prologue();
     const int seq = blockIdx.y, kvh = blockIdx.z;
     const int row0 = seq_row0[seq], row1 = seq_row0[seq + 1];
@@ -68,14 +68,27 @@ gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __rest
     }
     attn::cp_async_commit();
     const int per = H / G;
-    auto load_gates = [&](int h0) {
-        for (int e = tid; e < min(PREP_HEADS, per - h0) * CH; e += CH * CH) {
-            const int hh = e / CH, r = e % CH, h = kvh * per + h0 + hh;
-            gs[hh][r] = r < n ? gates[(size_t)(first + r) * 2 * H + h] : 1.0f;
-            bs[hh][r] = r < n ? gates[(size_t)(first + r) * 2 * H + H + h] : 0.0f;
+    auto place = [&](int h) { return coef + (chunk_place(row0, seq, blockIdx.x) * H + kvh * per + h) * COEF; };
+    // A warp a head: lane j has the product of the decays after row j, down the rows, lane CH that of all
+    auto decays = [&](int h0) {
+        const int h = h0 + warp;
+        if (h >= per) return;
+        const float* src = gates + (size_t)(first + lane) * 2 * H + kvh * per + h;
+        const float g = lane < n ? src[0] : 1.0f;
+        if (lane < CH) bs[warp][lane] = lane < n ? src[H] : 0.0f;
+        float* o = place(h) + 2 * CH * TLD;
+        float r = 1.0f;
+#pragma unroll
+        for (int a = 0; a < CH; ++a) {
+            const float next = __shfl_sync(0xffffffffu, g, a);
+            if (lane == CH || a > lane) r *= next;
+            if (lane < CH) L[warp][a][lane] = r;
+            if (lane == CH) o[a] = r;
         }
+        if (lane < CH) o[CH + lane] = r;
+        if (lane == CH) o[2 * CH] = r;
     };
-    load_gates(0);
+    decays(0);
     attn::cp_async_wait<0>();
     __syncthreads();
     float acc[4][4] = {};  // rows lane / 4 + 8 i of [k; q], columns lane % 4 + 4 j
@@ -96,36 +109,26 @@ gated_delta_chunk_prep_kernel(const float* __restrict__ qkv, const float* __rest
     for (int h0 = 0; h0 < per; h0 += PREP_HEADS) {
         const int heads = min(PREP_HEADS, per - h0);
         if (h0) {
-            __syncthreads();  // L, gs and bs of the heads before have been read
-            load_gates(h0);
+            __syncthreads();  // L and bs of the heads before have been read
+            decays(h0);
             __syncthreads();
         }
-        float* out = coef + (chunk_place(row0, seq, blockIdx.x) * H + kvh * per + h0) * COEF;
+        float* out = place(h0);
         for (int hh = 0; hh < heads; ++hh) {
-            float r = 1.0f;
-            for (int l = j + 1; l <= i; ++l) r *= gs[hh][l];
+            const float r = L[hh][i][j];
             L[hh][i][j] = j < i ? bs[hh][i] * (r * kk) : 0.0f;
-            float* o = out + (size_t)hh * COEF;
-            o[CH * TLD + i * TLD + j] = j <= i ? r * qk : 0.0f;
-            if (i == hh) {
-                float c = gs[hh][0], last = 1.0f;
-                for (int l = 1; l <= j; ++l) c *= gs[hh][l];
-                for (int l = j + 1; l < CH; ++l) last *= gs[hh][l];
-                o[2 * CH * TLD + j] = c;
-                o[2 * CH * TLD + CH + j] = last;
-                if (j == CH - 1) o[2 * CH * TLD + 2 * CH] = c;
-            }
+            out[(size_t)hh * COEF + CH * TLD + i * TLD + j] = j <= i ? r * qk : 0.0f;
         }
         __syncthreads();
         if (warp < heads && lane < CH) {  // a warp a head: column `lane` of T, row by row
-            float t[CH];
+            float t[CH];  // (each row known is taken off all later ones: fifteen multiply-adds deep, not 120)
 #pragma unroll
-            for (int a = 0; a < CH; ++a) {
-                float s = a == lane ? bs[warp][a] : 0.0f;
+            for (int a = 0; a < CH; ++a) t[a] = a == lane ? bs[warp][a] : 0.0f;
 #pragma unroll
-                for (int l = 0; l < a; ++l) s = fmaf(-L[warp][a][l], t[l], s);
-                t[a] = s;
-                out[(size_t)warp * COEF + a * TLD + lane] = s;
+            for (int l = 0; l < CH; ++l) {
+                out[(size_t)warp * COEF + l * TLD + lane] = t[l];
+#pragma unroll
+                for (int a = l + 1; a < CH; ++a) t[a] = fmaf(-L[warp][a][l], t[l], t[a]);
             }
         }
     }
