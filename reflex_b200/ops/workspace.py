@@ -55,7 +55,7 @@ class _Region:
         end = start + n * item
         self.offset = end
         self.need = max(self.need, end)
-        if end > self.size:
+        if self.buf is None or end > self.size:  # (no buffer yet: nothing to give, not even an empty tensor)
             return None
         if n == 0 or start % item:
             return self.buf[start:end].view(dtype).view(shape)

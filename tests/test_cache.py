@@ -210,3 +210,16 @@ def test_workspace_regions_take_turns_and_grow_after_the_step():
     lies_in = lambda t: any(b.data_ptr() <= t.data_ptr() < b.data_ptr() + b.numel() for b in bufs)
     assert lies_in(inside) and not lies_in(own)
     assert not lies_in(wsm.new((5,), torch.float32, "cpu"))  # no step: the allocator's
+
+
+def test_an_empty_tensor_may_be_a_workspaces_first_request():
+    import torch
+
+    from reflex_b200.ops import workspace as wsm
+
+    ws = wsm.Workspace("cpu")
+    for _ in range(2):  # before and after the regions have memory
+        with wsm.use(ws):
+            assert wsm.new((0, 4), torch.float32, "cpu").shape == (0, 4)
+            wsm.new((3,), torch.float32, "cpu")
+        ws.settle()
