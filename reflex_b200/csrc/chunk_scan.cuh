@@ -78,7 +78,9 @@ struct Core {
     bool waits;
     int* err;
 
-    // Every thread, before a barrier of the block: its products' barriers and its tensor memory.
+    // Every thread, first of all: the products' barriers and the tensor memory, before the next kernels are let in
+    // (their blocks could otherwise hold columns while they wait for this grid, and a block of this grid wait for
+    // those columns); then the wait for the kernels before.
     __device__ __forceinline__ void open(uint64_t* bars, uint32_t* slot, int* error) {
         done = bars;
         phase = 0;
@@ -93,6 +95,11 @@ struct Core {
             sm100::tmem_alloc(slot, TMEM_COLS);
             sm100::tmem_relinquish();
         }
+        sm100::tc_fence_before_sync();
+        __syncthreads();
+        sm100::tc_fence_after_sync();
+        tmem = *slot;
+        rfx::pdl_prologue();
     }
     // Products that one thread issues once all have passed this barrier; true if any thread saw odd numbers.
     template <class Issue>
@@ -117,12 +124,12 @@ struct Core {
         phase ^= 1u << bar;
         sm100::tc_fence_after_sync();
     }
-    __device__ __forceinline__ void close(uint32_t slot) {
+    __device__ __forceinline__ void close() {
         sm100::tc_fence_before_sync();
         __syncthreads();
         if (threadIdx.x < 32) {
             sm100::tc_fence_after_sync();
-            sm100::tmem_dealloc(slot, TMEM_COLS);
+            sm100::tmem_dealloc(tmem, TMEM_COLS);
         }
     }
 };
@@ -138,10 +145,14 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
     __shared__ float wl[WARPS][L];
     __shared__ uint64_t bars[2];
     __shared__ uint32_t tmem_slot;
-    rfx::pdl_prologue();
+    Core core;
+    core.open(bars, &tmem_slot, st.err);
     const int seq = st.round.seq0 + blockIdx.y;
     const Rows ch = rows_of(st, seq, blockIdx.x);
-    if (ch.n <= 0) return;
+    if (ch.n <= 0) {
+        core.close();
+        return;
+    }
     const int ptiles = (pol.P + PT - 1) / PT, items = pol.per * ptiles;
     const int sets = (items + items_a_block - 1) / items_a_block;
     const int kvh = blockIdx.z / sets, i0 = (blockIdx.z - kvh * sets) * items_a_block;
@@ -149,8 +160,6 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
     char *Ks = tiles_of(sm_raw), *Vs = Ks + 2 * split3::TILE;  // k's two tiles of 64 elements, v of two items
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
-    Core core;
-    core.open(bars, &tmem_slot, st.err);
     using Own = split3::Own<STATE_THREADS>;
     auto bring = [&](Own& v, int item) {
         const int p0 = (item % ptiles) * PT;
@@ -171,10 +180,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
     }
     bool odd_k = k0.put(Ks);
     odd_k |= k1.put(Ks + split3::TILE);
-    sm100::tc_fence_before_sync();
-    __syncthreads();
-    sm100::tc_fence_after_sync();
-    core.tmem = tmem_slot;
+    __syncthreads();  // the weights are there
     if (Pol::NORMALISER && i0 % ptiles == 0) {  // the head's sum of k (it is the block's only head), a thread's rows first
         float* part = reinterpret_cast<float*>(Vs + split3::TILE);
         float* mine = part + (tid >> 3) * 128 + Own::col();
@@ -245,7 +251,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
         });
     }
     store(i1 - 1);
-    core.close(tmem_slot);
+    core.close();
 }
 
 // Four neighbouring elements of a head's memory a thread; eight chunks' sums are fetched ahead.
@@ -347,10 +353,14 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
     __shared__ float row_sum[Pol::NORMALISER ? 8 : 1][L];
     __shared__ uint64_t bars[2];
     __shared__ uint32_t tmem_slot;
-    rfx::pdl_prologue();
+    Core core;
+    core.open(bars, &tmem_slot, st.err);
     const int seq = st.round.seq0 + blockIdx.y;
     const Rows ch = rows_of(st, seq, blockIdx.x);
-    if (ch.n <= 0) return;
+    if (ch.n <= 0) {
+        core.close();
+        return;
+    }
     const int ptiles = (pol.P + PT - 1) / PT, items = pol.per * ptiles;
     const int sets = (items + items_a_block - 1) / items_a_block;
     const int kvh = blockIdx.z / sets, i0 = (blockIdx.z - kvh * sets) * items_a_block;
@@ -363,8 +373,6 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int blocks = pol.N > 64 ? 2 : 1, t = 16 * (warp >> 2) + (lane & 15), sb = (warp + (warp >> 2)) & 3, s0 = 16 * sb + 8 * (lane >> 4);
     const size_t E = (size_t)pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
-    Core core;
-    core.open(bars, &tmem_slot, st.err);
     const float *q = pol.q_row(ch.first, kvh * pol.per), *k = pol.k_row(ch.first, kvh * pol.per);
     using Own = split3::Own<OUT_THREADS>;
     bool odd_qk = false;
@@ -377,10 +385,6 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             odd_qk |= x.put(Qs + b * split3::TILE);
             odd_qk |= y.put(Bs + b * split3::TILE);
         }
-    sm100::tc_fence_before_sync();
-    __syncthreads();
-    sm100::tc_fence_after_sync();
-    core.tmem = tmem_slot;
     const uint32_t q_at = sm100::smem_u32(Qs), b_at = sm100::smem_u32(Bs);
     // q by the two tiles at b_at
     auto q_products = [&] {
@@ -578,7 +582,7 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
                 pol.store_row(ch.first + r, h, p + 4 * i, gate[i], make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]),
                               make_float4(v.x[0][4 * i], v.x[0][4 * i + 1], v.x[0][4 * i + 2], v.x[0][4 * i + 3]));
     }
-    core.close(tmem_slot);
+    core.close();
 }
 
 // Floats of scratch a chunk needs: its memories and what the other kernels read beside them.
