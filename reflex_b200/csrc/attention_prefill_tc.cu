@@ -410,7 +410,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
 #pragma unroll
             for (int c = 0; c < PAGE / 16; ++c)
                 tmem_ld_16_nowait(tmem + lane_addr + S_COL + b * PAGE + c * 16, sr + c * 16);
-            tmem_ld_wait();
+            tmem_ld_wait_16(sr);
+#pragma unroll
+            for (int c = 1; c < PAGE / 16; ++c) tmem_loaded_16(sr + c * 16);
 
             const int basej = logical(j) * PAGE;
             // every key of the page visible to every valid row of the tile: no compares
@@ -500,7 +502,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                     for (int c = 0; c < DV / 16; ++c) {
                         uint32_t o[16];
                         tmem_ld_16_nowait(tmem + lane_addr + O_COL + c * 16, o);
-                        tmem_ld_wait();
+                        tmem_ld_wait_16(o);
 #pragma unroll
                         for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
                         tmem_st_16(tmem + lane_addr + O_COL + c * 16, o);
