@@ -92,6 +92,7 @@ struct Core {
             sm100::fence_barrier_init();
         }
         if (threadIdx.x < 32) {
+            __syncwarp();
             sm100::tmem_alloc(slot, TMEM_COLS);
             sm100::tmem_relinquish();
         }
@@ -214,8 +215,8 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
             const int p0 = (item % ptiles) * PT + half + 8 * c;
             float y[8];
             split3::sums_of<2>(y, core.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + half + 8 * c, split3::sets<2>(L / 16));
-            if (n >= pol.N) continue;
-            if (any_odd) {  // the odd numbers' products
+            const bool live = n < pol.N;
+            if (live && any_odd) {  // the odd numbers' products
                 const float *k = pol.k_row(ch.first, h) + n, *x = pol.v_row(ch.first, h);
                 for (int s = 0; s < ch.n; ++s) {
                     const float ks = k[(size_t)s * pol.ldk];
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
             const int left = pol.P - p0;
 #pragma unroll
             for (int i = 0; i < 8; ++i, to += pol.N)
-                if (i < left) *to = y[i];
+                if (live && i < left) *to = y[i];
         }
     };
     for (int item = i0; item < i1; ++item) {

@@ -163,6 +163,7 @@ __device__ __forceinline__ void issue64(uint32_t to, uint32_t majors, int steps,
 template <int EVERY>
 __device__ __forceinline__ void sums_of(float (&y)[8], uint32_t at, int sets, bool second = false) {
     float x[8], z[8];
+    __syncwarp();  // (the warp's lanes load together, and what came before may have parted them)
     sm100::tmem_ld_8(at + 64 * sets, x);
     if (!second) {
         sm100::tmem_ld_8(at + 64 * sets + 64, z);
