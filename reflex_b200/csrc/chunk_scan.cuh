@@ -70,7 +70,7 @@ __device__ __forceinline__ Rows rows_of(const Step& s, int seq, int c) {
 }
 
 // What both tensor-core kernels of a block hold: the barrier its products arrive at, the tensor memory, and
-// whether a wait ran out (reported; nothing waits after that, and the block ends with what is there).
+// whether a wait ran out (reported; nothing is multiplied or waits after that, and the block ends with what is there).
 struct Core {
     uint32_t tmem;
     uint64_t* done;
@@ -109,7 +109,7 @@ struct Core {
         const bool any = __syncthreads_or(odd);
         if (threadIdx.x < 32) {
             sm100::tc_fence_after_sync();
-            if (sm100::elect_one()) {
+            if (sm100::elect_one() && waits) {
                 issue();
                 sm100::umma_commit(done + bar);
             }
@@ -121,6 +121,7 @@ struct Core {
         if (waits && !sm100::mbar_wait(done + bar, phase >> bar & 1)) {
             waits = false;
             if (err) atomicExch(err, 42);
+            sm100::mbar_wait(done + bar, phase >> bar & 1);  // as long again for what is still being multiplied
         }
         phase ^= 1u << bar;
         sm100::tc_fence_after_sync();

@@ -307,6 +307,8 @@ delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stri
         if (waits && !sm100::mbar_wait(&full[now], round & 1)) {
             waits = false;
             if (err) atomicExch(err, 43);
+            if (tid == 0)  // no copy is begun any more; those on their way get as long again each
+                for (int i = k; i < min(chunks, k + STAGES); ++i) sm100::mbar_wait(&full[i % STAGES], i / STAGES & 1);
         }
         const float* m = sm + at * MR + first_row * LD + 4 * quarter;
         const float* S = Ss[k & 1] + cg * TLD + 4 * quarter;
@@ -363,7 +365,7 @@ delta_chunk_walk_kernel(Step st, float* __restrict__ state, long long state_stri
             store4(out + (size_t)(from + k * L + row - D) * hd + h * D + c, own);
         }
         __syncthreads();  // the next S is there; this chunk's factors have been read
-        if (tid == 0) fetch(k + STAGES, now);
+        if (tid == 0 && waits) fetch(k + STAGES, now);
     }
     if (row < D) {
         float* s = Sg + (size_t)c * D + row;
