@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
         for (int c = 0; c < 4; ++c) {
             const int p0 = (item % ptiles) * PT + half + 8 * c;
             float y[8];
-            split3::sums_of<2>(y, core.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + half + 8 * c, split3::sets<2>(L / 16));
+            split3::sums_of<2>(y, core.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + half + 8 * c, L / 16);
             const bool live = n < pol.N;
             if (live && any_odd) {  // the odd numbers' products
                 const float *k = pol.k_row(ch.first, h) + n, *x = pol.v_row(ch.first, h);
@@ -247,9 +247,9 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
         if (item + 1 < i1) bring(v, item + 1);
         if (item > i0) store(item - 1);
         any_odd = core.start(0, odd, [&] {
-            split3::issue128<2, split3::MN_STEP, split3::MN_STEP>(core.tmem, split3::A_MN | split3::B_MN, L / 16,
-                                                                  split3::mn_major(k_at, split3::TILE),
-                                                                  split3::mn_major(sm100::smem_u32(V), split3::PART));
+            split3::issue<2, split3::MN_STEP, split3::MN_STEP>(core.tmem, split3::A_MN | split3::B_MN, L / 16,
+                                                               split3::mn_major(k_at, split3::TILE),
+                                                               split3::mn_major(sm100::smem_u32(V), split3::PART));
         });
     }
     store(i1 - 1);
@@ -387,35 +387,37 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             odd_qk |= x.put(Qs + b * split3::TILE);
             odd_qk |= y.put(Bs + b * split3::TILE);
         }
+    const int q_steps = (pol.N + 15) / 16;
     const uint32_t q_at = sm100::smem_u32(Qs), b_at = sm100::smem_u32(Bs);
     // q by the two tiles at b_at
     auto q_products = [&] {
-        split3::issue64<4, split3::K_STEP, split3::K_STEP>(core.tmem, 0, (pol.N + 15) / 16, split3::k_major(q_at), split3::k_major(b_at));
+        split3::issue<1, split3::K_STEP, split3::K_STEP>(core.tmem, 0, q_steps, split3::k_major(q_at), split3::k_major(b_at));
     };
-    // the warp's lanes and sixteen columns of results: row `row`, or what its m part adds (`second`)
+    // results lie in lanes 0 to 63, which two warps of four can read, sixteen columns each
+    const bool reads = !(warp & 2);
     const int row = 32 * (warp & 1) + lane, c0 = 16 * (warp >> 2);
-    const bool second = warp & 2;
     const uint32_t lanes = core.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + c0;
     auto spread = [&](const float (&y)[8], int c) {  // for every thread to read
-        float* to = res + ((second ? L : 0) + row) * OLD + c0 + c;
+        float* to = res + row * OLD + c0 + c;
 #pragma unroll
         for (int i = 0; i < 2; ++i) store4(to + 4 * i, make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]));
     };
     auto read8 = [&](float (&y)[8], const float* from) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const float4 r = load4(from + 4 * i), s = load4(from + L * OLD + 4 * i);
-            y[4 * i] = r.x + s.x; y[4 * i + 1] = r.y + s.y; y[4 * i + 2] = r.z + s.z; y[4 * i + 3] = r.w + s.w;
+            const float4 r = load4(from + 4 * i);
+            y[4 * i] = r.x; y[4 * i + 1] = r.y; y[4 * i + 2] = r.z; y[4 * i + 3] = r.w;
         }
     };
     odd_qk = core.start(0, odd_qk, q_products);
     core.wait(0);
+    if (reads)
 #pragma unroll
-    for (int c = 0; c < 16; c += 8) {
-        float y[8];
-        split3::sums_of<4>(y, lanes + c, split3::sets<4>((pol.N + 15) / 16), second);
-        spread(y, c);
-    }
+        for (int c = 0; c < 16; c += 8) {
+            float y[8];
+            split3::sums_of<1>(y, lanes + c, q_steps);
+            spread(y, c);
+        }
     sm100::tc_fence_before_sync();
     __syncthreads();
     float G[8];  // row t by rows s0 .. of k
@@ -511,12 +513,12 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             }
         }
         core.wait(0);
-        {  // times alpha, and out of the way of the next products' sums (over a sum that no one else reads)
+        if (reads) {  // times alpha, and out of the way of the next products' sums
             const float alpha = pol.row_terms(rec + row * Pol::RECORDS, before).alpha;
 #pragma unroll
             for (int c = 0; c < 16; c += 8) {
                 float y[8];
-                split3::sums_of<4>(y, lanes + c, split3::sets<4>((pol.N + 15) / 16), second);
+                split3::sums_of<1>(y, lanes + c, q_steps);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) y[i] *= alpha;
                 sm100::tmem_st_8(lanes + 192 + c, y);
@@ -526,8 +528,8 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
         odd |= split3::put8(w, Ws, t, s0 / 8);
         odd |= v.put(Vs);
         odd = core.start(1, odd, [&] {
-            split3::issue64<4, split3::K_STEP, split3::MN_STEP>(core.tmem, split3::B_MN, L / 16, split3::k_major(sm100::smem_u32(Ws)),
-                                                                split3::mn_major(sm100::smem_u32(Vs), split3::PART));
+            split3::issue<1, split3::K_STEP, split3::MN_STEP>(core.tmem, split3::B_MN, L / 16, split3::k_major(sm100::smem_u32(Ws)),
+                                                              split3::mn_major(sm100::smem_u32(Vs), split3::PART));
         });
         if constexpr (Pol::NORMALISER)
             if (p0 == 0 && s0 == 0 && t < ch.n) {
@@ -537,15 +539,18 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
                 pol.store_sum(ch.first + t, h, sum, pol.row_terms(rec + t * Pol::RECORDS, before).extra);
             }
         core.wait(1);
+        if (reads)
 #pragma unroll
-        for (int c = 0; c < 16; c += 8) {
-            float y[8], first[8];
-            split3::sums_of<4>(y, lanes + c, split3::sets<4>(L / 16), second);
-            sm100::tmem_ld_8(lanes + 192 + c, first);
+            for (int c = 0; c < 16; c += 8) {
+                float y[8];
+                uint32_t first[8];
+                split3::sums_of<1>(y, lanes + c, L / 16);
+                sm100::tmem_ld_8_nowait(lanes + 192 + c, first);
+                sm100::tmem_ld_wait_8(first);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) y[i] += first[i];
-            spread(y, c);
-        }
+                for (int i = 0; i < 8; ++i) y[i] += __uint_as_float(first[i]);
+                spread(y, c);
+            }
         const int r = Own::row(0), p = p0 + Own::col();
         float4 gate[2];
 #pragma unroll

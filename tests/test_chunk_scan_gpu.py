@@ -373,6 +373,50 @@ def test_a_row_that_is_not_finite_does_not_reach_earlier_rows_of_the_delta_rule(
         assert torch.equal(state.view(hd, d)[~hit], clean_state.view(hd, d)[~hit]), part
 
 
+def plain_ssd(x, B, C, S, A, step):
+    """Step sizes of `step` (32 and more is its own softplus) and a gate of 32 (its own silu): results and memory of the
+    chunks, and 64-bit ones by rows.  x [T, H, P], B, C [T, G, N], S [H, P, N]."""
+    (T, H, P), (G, N) = x.shape, B.shape[1:]
+    proj = torch.full((T, H * P + H), 32.0, device=DEV)
+    proj[:, H * P:] = step
+    state, zero = S.reshape(1, -1).clone(), torch.zeros(H, device=DEV)
+    xbc = torch.cat([t.reshape(T, -1) for t in (x, B, C)], 1).contiguous()
+    y = ops().ssd_scan(xbc, proj, 0, H * P, zero, A, zero, state, 0, Batch([T], [0]), H, P, N, G, exact=False)
+    up = lambda t: t.double().cpu().numpy()  # noqa: E731
+    dt = np.full((T, H), step if step >= 32 else np.log1p(np.exp(step)))
+    ref, ref_S = ssd_rule(up(x), up(B).repeat(H // G, 1), up(C).repeat(H // G, 1), dt, up(A), np.zeros(H), up(S))
+    return y.view(T, H, P), 32 * ref, state.view(H, P, N), ref_S
+
+
+@pytest.mark.parametrize("N", [16, 24, 64, 100, 128])
+@pytest.mark.parametrize("decay", [0.0, 1.0])
+def test_sums_that_32_bits_hold_are_exact(N, decay):
+    """Small whole numbers and steps of 32: without a decay all sums are whole numbers below 2^24; with one every row
+    forgets what was before it (e^-32), which leaves one product an element."""
+    H, G, P, T = 4, 2, 64, 200
+    g = torch.Generator(device=DEV).manual_seed(N)
+    whole = lambda *s: torch.randint(-3, 4, s, generator=g, device=DEV).float()  # noqa: E731
+    y, ref, state, ref_S = plain_ssd(whole(T, H, P), whole(T, G, N), whole(T, G, N), whole(H, P, N),
+                                     torch.full((H,), -decay, device=DEV), 32.0)
+    tiny = 1e-9 if decay else 0.0  # beside what e^-32 leaves of the rows before
+    assert np.abs(y.double().cpu().numpy() - ref).max() <= tiny * np.abs(ref).max()
+    assert np.abs(state.double().cpu().numpy() - ref_S).max() <= tiny * np.abs(ref_S).max()
+
+
+@pytest.mark.parametrize("N", [16, 64, 128])
+def test_sums_of_one_sign_lean_to_neither_side(N):
+    """51,200 results of either rounding: what is off on average is far less than one rounding's 2^-25 of the value, and
+    a quarter of that is allowed for what the tensor core cuts off."""
+    H, G, P, T = 4, 2, 64, 200
+    g = torch.Generator(device=DEV).manual_seed(N)
+    pos = lambda *s: torch.rand(s, generator=g, device=DEV)  # noqa: E731
+    y, ref, state, ref_S = plain_ssd(pos(T, H, P), pos(T, G, N), pos(T, G, N), pos(H, P, N),
+                                     torch.full((H,), -0.25, device=DEV), 0.5)
+    for got, want in ((y, ref), (state, ref_S)):
+        d = got.double().cpu().numpy() - want
+        assert abs(d.sum()) / want.sum() < 3e-8 and np.linalg.norm(d) / np.linalg.norm(want) < 1e-7
+
+
 @pytest.mark.parametrize("huge", [3.3895e38, 3.395e38])  # bfloat16's largest number holds the first, not the second
 @pytest.mark.parametrize("N", [24, 128])
 def test_numbers_beyond_bfloat16s_range_count_as_they_are(huge, N):
