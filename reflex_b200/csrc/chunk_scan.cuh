@@ -351,7 +351,6 @@ template <class Pol>
 __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step st, int items_a_block) {
     extern __shared__ __align__(16) char sm_raw[];
     __shared__ __align__(16) float4 rec[L * Pol::RECORDS];
-    __shared__ float early[3][48];  // the weights of rows before a sixteen, up to its first row
     __shared__ float row_sum[Pol::NORMALISER ? 8 : 1][L];
     __shared__ uint64_t bars[2];
     __shared__ uint32_t tmem_slot;
@@ -432,42 +431,28 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             }
         }
     __syncthreads();  // the results have been read
-    // A weight's exponential as it is where its rows are of one sixteen, else by the later row's sixteen's first row.
-    auto weights = [&](float (&w)[8], const RowTerms& r, float before) {
+    auto weights = [&](float (&w)[8], const RowTerms& r) {
         if (16 * sb > t) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) w[i] = 0.0f;
-        } else if (16 * sb + 16 > t) {
+        } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float4 c = rec[(s0 + i) * Pol::RECORDS];
                 w[i] = s0 + i <= t ? G[i] * (Pol::weight(c) * expf((Pol::g_hi(c) + r.e_hi) + (Pol::g_lo(c) + r.e_lo))) : 0.0f;
             }
-        } else {
-            const RowTerms f = pol.row_terms(rec + (t & ~15) * Pol::RECORDS, before);
-            const float late = expf((r.e_hi - f.e_hi) + (r.e_lo - f.e_lo));
-            const float* e = early[(t >> 4) - 1] + s0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = G[i] * (e[i] * late);
         }
     };
-    // a head's records, and what its weights share
-    auto begin_head = [&](int h, float before) {
+    auto begin_head = [&](int h) {
         const float4* rows = st.rows + (ch.place * pol.heads + h) * L * Pol::RECORDS;
         if (tid < L * Pol::RECORDS) rec[tid] = rows[tid];
-        if (tid >= OUT_THREADS - 96) {  // early[i][s], s below 16 (i + 1)
-            const int e = tid - (OUT_THREADS - 96), i = e < 16 ? 0 : e < 48 ? 1 : 2, s = e - (i == 0 ? 0 : i == 1 ? 16 : 48);
-            const RowTerms r = pol.row_terms(rows + 16 * (i + 1) * Pol::RECORDS, before);
-            const float4 c = rows[s * Pol::RECORDS];
-            early[i][s] = Pol::weight(c) * expf((Pol::g_hi(c) + r.e_hi) + (Pol::g_lo(c) + r.e_lo));
-        }
     };
     if constexpr (!Pol::SHARED) {  // one head a block: its weights stand where the products stood
         const float before = st.before[ch.place * pol.heads + kvh];
-        begin_head(kvh, before);
+        begin_head(kvh);
         __syncthreads();
         float w[8];
-        weights(w, pol.row_terms(rec + t * Pol::RECORDS, before), before);
+        weights(w, pol.row_terms(rec + t * Pol::RECORDS, before));
 #pragma unroll
         for (int i = 0; i < 8; ++i) G[i] = w[i];
     }
@@ -479,14 +464,14 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
         v.load(S + (size_t)p0 * pol.N, pol.N, pol.P - p0, pol.N);
         m.load(S + (size_t)p0 * pol.N + 64, pol.N, pol.P - p0, pol.N - 64);
         const float before = st.before[at];
-        if constexpr (Pol::SHARED) begin_head(h, before);
+        if constexpr (Pol::SHARED) begin_head(h);
         bool odd = v.put(Bs) || odd_qk;
         if (blocks == 2) odd |= m.put(Bs + split3::TILE);
         odd = core.start(0, odd, q_products);
         v.load(vr, pol.ldv, ch.n, pol.P - p0);
         float w[8];
         auto make_weights = [&] {
-            if constexpr (Pol::SHARED) weights(w, pol.row_terms(rec + t * Pol::RECORDS, before), before);
+            if constexpr (Pol::SHARED) weights(w, pol.row_terms(rec + t * Pol::RECORDS, before));
             else
 #pragma unroll
                 for (int i = 0; i < 8; ++i) w[i] = G[i];

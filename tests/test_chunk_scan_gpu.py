@@ -417,6 +417,23 @@ def test_sums_of_one_sign_lean_to_neither_side(N):
         assert abs(d.sum()) / want.sum() < 3e-8 and np.linalg.norm(d) / np.linalg.norm(want) < 1e-7
 
 
+def test_a_weight_is_one_exponential(monkeypatch):
+    """k and v of unit vectors and q of ones leave every weight on its own in the results, 32 e^(A (dt_s+1 + .. + dt_t)).
+    A rounding is off by 2.5e-8 of the value in the mean square, an exponential by a third more; two exponentials and
+    their product by 5e-8 (4.8e-8 were measured, 3.4e-8 with one)."""
+    monkeypatch.setattr(ops(), "SSD_CHUNK_MIN_ROWS", 1)
+    H, T = 16, 64
+    g = torch.Generator(device=DEV).manual_seed(3)
+    eye = torch.eye(T, device=DEV)
+    x, B, C = eye.view(T, 1, T).repeat(1, H, 1), eye.view(T, 1, T), torch.ones((T, 1, T), device=DEV)
+    A = -torch.rand(H, generator=g, device=DEV) * 8e-5 - 4e-5  # exponents down to -0.25
+    y, ref, _, _ = plain_ssd(x, B, C, torch.zeros((H, T, T), device=DEV), A, 32.0)
+    t, s = torch.meshgrid(torch.arange(T), torch.arange(T), indexing="ij")
+    apart = (t // 16 > s // 16).numpy()
+    d = (y.double().cpu().numpy() / np.where(ref, ref, 1.0) - 1.0).transpose(0, 2, 1)[apart]
+    assert np.sqrt((d * d).mean()) < 4e-8
+
+
 @pytest.mark.parametrize("huge", [3.3895e38, 3.395e38])  # bfloat16's largest number holds the first, not the second
 @pytest.mark.parametrize("N", [24, 128])
 def test_numbers_beyond_bfloat16s_range_count_as_they_are(huge, N):
