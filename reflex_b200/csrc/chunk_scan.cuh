@@ -334,6 +334,11 @@ __device__ __forceinline__ float exp_of(double v) {
     return fmaf(e, lo, e);
 }
 
+// (in a chain of eight the first numbers are rounded seven times)
+__device__ __forceinline__ float sum8(const float (&x)[8]) {
+    return ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+}
+
 // What a row t brings to its results: w_ts = exp((g_s + e_t)) * w_s with e in two parts, the factor of
 // q . S, and a number for the policy's store.
 struct RowTerms {
@@ -481,9 +486,8 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             if (p0 == 0) {  // eight threads a row
                 const RowTerms terms = pol.row_terms(rec + t * Pol::RECORDS, before);
                 const float* n = S + (size_t)pol.P * pol.N;
-                float sum = 0.0f, qn = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) sum += w[i];
+                const float sum = sum8(w);
+                float qn = 0.0f;
                 if (t < ch.n)
                     for (int e = s0 / 2; e < pol.N; e += 32) {
                         const float4 a = load4(q + (size_t)t * pol.ldq + e), b = load4(n + e);
@@ -518,9 +522,10 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
         });
         if constexpr (Pol::NORMALISER)
             if (p0 == 0 && s0 == 0 && t < ch.n) {
-                float sum = 0.0f;
+                float parts[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) sum += row_sum[i][t];
+                for (int i = 0; i < 8; ++i) parts[i] = row_sum[i][t];
+                const float sum = sum8(parts);
                 pol.store_sum(ch.first + t, h, sum, pol.row_terms(rec + t * Pol::RECORDS, before).extra);
             }
         core.wait(1);
