@@ -75,13 +75,7 @@ struct Ssd {
     __device__ __forceinline__ void store_state(int slot, int h, int e, const float4& S) const {
         *reinterpret_cast<float4*>(memory(slot, h, e)) = S;
     }
-    // z / (1 + e^-z); one step upon the approximate reciprocal gives all but the last bit
-    static __device__ __forceinline__ float silu(float z) {
-        const float d = 1.0f + expf(fminf(-z, 87.0f));
-        float r;
-        asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-        return z * fmaf(fmaf(-d, r, 1.0f), r, r);
-    }
+    static __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
     __device__ __forceinline__ float4 gate(int r, int h, int p) const {
         return rfx::load4(proj + (size_t)r * ldp + z_off + h * P + p);
     }

@@ -434,6 +434,26 @@ def test_a_weight_is_one_exponential(monkeypatch):
     assert np.sqrt((d * d).mean()) < 4e-8
 
 
+def test_gates_of_all_sizes_as_a_decode_step_has_them(monkeypatch):
+    """silu(z) from -inf to inf and where e^-z overflows: the rows of a prompt (the results before the gate are 128
+    everywhere) and as many sequences of one row, the same operations on the same numbers."""
+    monkeypatch.setattr(ops(), "SSD_CHUNK_MIN_ROWS", 2)
+    H, G, P, N, T = 4, 2, 64, 16, 64
+    z = torch.cat([torch.linspace(-120, 120, H * P - 6, device=DEV),
+                   torch.tensor([-float("inf"), float("inf"), float("nan"), -3e38, 3e38, -0.0], device=DEV)])
+    proj = torch.cat([z, torch.full((H,), 32.0, device=DEV)]).repeat(T, 1).contiguous()
+    xbc, zero = torch.ones((T, H * P + 2 * G * N), device=DEV), torch.zeros(H, device=DEV)
+    xbc[:, H * P:] = 0.5
+    forget = torch.full((H,), -64.0, device=DEV)  # e^-2048: a row has no other before it
+    pre = []
+    for counts in ((T,), (1,) * T):
+        b = Batch(counts, range(len(counts)))
+        state = torch.zeros((len(counts), H * P * N), device=DEV)
+        pre.append(ops().ssd_scan(xbc, proj, 0, H * P, zero, forget, zero, state, 0, b, H, P, N, G, exact=False))
+    assert torch.equal(pre[0].isnan(), pre[1].isnan())
+    assert torch.equal(pre[0].nan_to_num(7.0), pre[1].nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("huge", [3.3895e38, 3.395e38])  # bfloat16's largest number holds the first, not the second
 @pytest.mark.parametrize("N", [24, 128])
 def test_numbers_beyond_bfloat16s_range_count_as_they_are(huge, N):
