@@ -326,12 +326,15 @@ __device__ __forceinline__ void two_parts(double v, float* hi, float* lo) {
     *hi = h;
     *lo = isinf(h) ? 0.0f : (float)(v - (double)h);
 }
+__device__ __forceinline__ float exp_of(float hi, float lo) {
+    const float e = expf(hi);
+    return isinf(e) ? e : fmaf(e, lo, e);
+}
 // e^v as exactly as expf has it, where a v rounded to 32 bits would be off by 2^-25 v
 __device__ __forceinline__ float exp_of(double v) {
     float hi, lo;
     two_parts(v, &hi, &lo);
-    const float e = expf(hi);
-    return fmaf(e, lo, e);
+    return exp_of(hi, lo);
 }
 
 // (in a chain of eight the first numbers are rounded seven times)
@@ -502,8 +505,8 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             }
         }
         core.wait(0);
-        if (reads) {  // times alpha, and out of the way of the next products' sums
-            const float alpha = pol.row_terms(rec + row * Pol::RECORDS, before).alpha;
+        if (reads) {  // times alpha (if that is all of it), and out of the way of the next products' sums
+            const float alpha = odd ? 1.0f : pol.row_terms(rec + row * Pol::RECORDS, before).alpha;
 #pragma unroll
             for (int c = 0; c < 16; c += 8) {
                 float y[8];
@@ -514,6 +517,7 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
             }
             sm100::tmem_st_wait();
         }
+        const bool odd_q = odd;
         odd |= split3::put8(w, Ws, t, s0 / 8);
         odd |= v.put(Vs);
         odd = core.start(1, odd, [&] {
@@ -529,16 +533,23 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
                 pol.store_sum(ch.first + t, h, sum, pol.row_terms(rec + t * Pol::RECORDS, before).extra);
             }
         core.wait(1);
+        auto first8 = [&](float (&y)[8], int c) {
+            uint32_t first[8];
+            __syncwarp();
+            sm100::tmem_ld_8_nowait(lanes + 192 + c, first);
+            sm100::tmem_ld_wait_8(first);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(first[i]);
+        };
         if (reads)
 #pragma unroll
             for (int c = 0; c < 16; c += 8) {
-                float y[8];
-                uint32_t first[8];
+                float y[8], first[8];
                 split3::sums_of<1>(y, lanes + c, L / 16);
-                sm100::tmem_ld_8_nowait(lanes + 192 + c, first);
-                sm100::tmem_ld_wait_8(first);
+                first8(first, c);
+                if (!odd_q)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) y[i] += __uint_as_float(first[i]);
+                    for (int i = 0; i < 8; ++i) y[i] += first[i];
                 spread(y, c);
             }
         const int r = Own::row(0), p = p0 + Own::col();
@@ -551,25 +562,34 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) chunk_out_kernel(Pol pol, Step
         read8(y, res + r * OLD + Own::col());
         __syncthreads();  // the results have been read
         if (odd) {  // the odd numbers' products
+            float* weight = reinterpret_cast<float*>(Vs);
+            if (odd_q && reads)
+#pragma unroll 1
+                for (int c = 0; c < 16; c += 8) {
+                    float first[8];
+                    first8(first, c);
+                    spread(first, c);
+                }
             make_weights();
 #pragma unroll
-            for (int i = 0; i < 8; ++i) res[t * OLD + s0 + i] = w[i];
+            for (int i = 0; i < 8; ++i) weight[t * OLD + s0 + i] = w[i];
             __syncthreads();
-            const float alpha = pol.row_terms(rec + r * Pol::RECORDS, before).alpha;
             if (r < ch.n)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int c = min(p + j, pol.P - 1) - p0;
-                    float a = 0.0f, b = 0.0f;
-                    for (int e = 0; e < pol.N; ++e) {
-                        const float x = q[(size_t)r * pol.ldq + e], m = S[(size_t)(p0 + c) * pol.N + e];
-                        if (split3::is_odd(x) || split3::is_odd(m)) a = fmaf(x, m, a);
+                    if (odd_q) {
+                        float a = res[r * OLD + Own::col() + j];
+                        for (int e = 0; e < pol.N; ++e) {
+                            const float x = q[(size_t)r * pol.ldq + e], m = S[(size_t)(p0 + c) * pol.N + e];
+                            if (split3::is_odd(x) || split3::is_odd(m)) a = fmaf(x, m, a);
+                        }
+                        y[j] += __fmul_rn(pol.row_terms(rec + r * Pol::RECORDS, before).alpha, a);  // (rounded as without odd numbers)
                     }
                     for (int s = 0; s <= r; ++s) {
-                        const float x = res[r * OLD + s], m = vr[(size_t)s * pol.ldv + c];
-                        if (split3::is_odd(x) || split3::is_odd(m)) b = fmaf(x, m, b);
+                        const float x = weight[r * OLD + s], m = vr[(size_t)s * pol.ldv + c];
+                        if (split3::is_odd(x) || split3::is_odd(m)) y[j] = fmaf(x, m, y[j]);
                     }
-                    y[j] += fmaf(alpha, a, b);
                 }
             __syncthreads();
         }

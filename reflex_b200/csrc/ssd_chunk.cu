@@ -54,8 +54,7 @@ struct Ssd {
             if (rows) {
                 float hi, lo;
                 chunk::two_parts(c[i], &hi, &lo);
-                const float e = expf(hi);
-                rows[r] = make_float4(hi, lo, d[i], fmaf(e, lo, e));  // exp(hi + lo)
+                rows[r] = make_float4(hi, lo, d[i], chunk::exp_of(hi, lo));
             }
         }
         return make_float4(chunk::exp_of(all), 0.0f, 0.0f, 0.0f);

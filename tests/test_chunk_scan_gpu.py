@@ -454,6 +454,14 @@ def test_gates_of_all_sizes_as_a_decode_step_has_them(monkeypatch):
     assert torch.equal(pre[0].nan_to_num(7.0), pre[1].nan_to_num(7.0))
 
 
+def test_memories_that_grow_beyond_32_bits_are_infinite():
+    """e^128 a row, positive numbers throughout: infinity, as by rows, and no NaN."""
+    H, G, P, N, T = 4, 2, 64, 16, 130
+    one = lambda *s: torch.ones(s, device=DEV)  # noqa: E731
+    y, _, state, _ = plain_ssd(one(T, H, P), one(T, G, N), one(T, G, N), one(H, P, N), 4.0 * one(H), 32.0)
+    assert bool((y == math.inf).all()) and bool((state == math.inf).all())
+
+
 @pytest.mark.parametrize("huge", [3.3895e38, 3.395e38])  # bfloat16's largest number holds the first, not the second
 @pytest.mark.parametrize("N", [24, 128])
 def test_numbers_beyond_bfloat16s_range_count_as_they_are(huge, N):
