@@ -462,6 +462,36 @@ def test_memories_that_grow_beyond_32_bits_are_infinite():
     assert bool((y == math.inf).all()) and bool((state == math.inf).all())
 
 
+@pytest.mark.parametrize("N", [24, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 1e30])
+def test_numbers_no_part_holds_in_q_and_in_the_memory(N, bad):
+    """An element of q reaches its row's results in its group's heads; one of the memory that a sequence comes with its own
+    column's; all others keep their bits.  1e30 is finite and counts as it is."""
+    H, G, P, T = 4, 2, 64, 200
+    g = torch.Generator(device=DEV).manual_seed(11)
+    draw = lambda *s: torch.randn(s, generator=g, device=DEV)  # noqa: E731
+    x, B, C, S = draw(T, H, P), draw(T, G, N), draw(T, G, N), draw(H, P, N)
+    A = torch.full((H,), -0.01, device=DEV)
+    y, _, state, _ = plain_ssd(x, B, C, S, A, 0.5)
+    for where in ("q", "memory"):
+        C2, S2 = C.clone(), S.clone()
+        hit, moved = torch.zeros((T, H, P), dtype=torch.bool, device=DEV), torch.zeros((H, P, N), dtype=torch.bool, device=DEV)
+        if where == "q":
+            C2[70, 1, 3] = bad
+            hit[70, 2:] = True
+        else:
+            S2[1, 5, 7] = bad
+            hit[:, 1, 5] = True
+            moved[1, 5, 7] = True
+        y2, ref, state2, ref_S = plain_ssd(x, B, C2, S2, A, 0.5)
+        assert torch.equal(y2[~hit], y[~hit]) and torch.equal(state2[~moved], state[~moved])
+        if math.isfinite(bad):
+            for got, want in ((y2, ref), (state2, ref_S)):
+                assert off(got, want) < TOL
+        else:
+            assert not y2[hit].isfinite().any() and not state2[moved].isfinite().any()
+
+
 @pytest.mark.parametrize("huge", [3.3895e38, 3.395e38])  # bfloat16's largest number holds the first, not the second
 @pytest.mark.parametrize("N", [24, 128])
 def test_numbers_beyond_bfloat16s_range_count_as_they_are(huge, N):
