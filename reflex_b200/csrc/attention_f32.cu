@@ -274,13 +274,14 @@ __global__ void __launch_bounds__(WARPS * 32, NI > 4 ? 1 : 2) attention_f32_kern
 }  // namespace
 
 // As rfx_attention_plain with 32-bit rows, sequence by sequence (rows packed from seq_row0, positions from
-// seq_start); at most max_new rows a sequence.  head_dim 32, 64, 128 or 256, everything on 16 bytes;
+// seq_start); at most max_new rows a sequence.  `longest_blocks`: the blocks' work in blocks as long as the longest, 0
+// where the caller does not know it.  head_dim 32, 64, 128 or 256, everything on 16 bytes;
 // RFX_ERR_UNSUPPORTED otherwise.
 extern "C" int rfx_attention_f32(const float* q, const float* k_pages, const float* v_pages, const int* page_table,
                                  int max_pages, int page_size, const int* seq_slot, const int* seq_start,
                                  const int* seq_new, const int* seq_row0, float* out, int S, int max_new, int nq, int nkv,
                                  int head_dim, int window, int keep_first, float scale, const float* sink,
-                                 const float* slopes, float softcap, void* stream) {
+                                 const float* slopes, float softcap, float longest_blocks, void* stream) {
     if (S <= 0 || max_new <= 0) return 0;
     if (softcap < 0.0f || nkv <= 0 || nq % nkv != 0) return RFX_ERR_BAD_ARG;
     if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages) |
@@ -297,14 +298,20 @@ extern "C" int rfx_attention_f32(const float* q, const float* k_pages, const flo
     const long long blocks = ((long long)max_new + a.rows - 1) / a.rows * S * nkv * parts;
     if ((long long)nkv * parts > 65535 || blocks > 2147483647LL) return RFX_ERR_UNSUPPORTED;
     dim3 grid((unsigned)blocks);
-    // few blocks: one an SM, taken longest first, ends earlier than two side by side (50 us against 60 above)
-    const bool alone = blocks <= 4LL * sm_count();
+    // Two blocks an SM, or one: then a block has the SM's shared memory to itself and ends in 1/1.15 of the time.  That
+    // wins where the longest block decides, the longest ones being taken first: as long as all blocks are no more
+    // work than one as long as the longest an SM.  us with one and with two, 8 query heads and 2 others of 128, new
+    // prompts of 512 rows (0.86 of that work) 68 and 80, of 600 (1.01) 88 and 96, of 155, 311 and 235 (0.98) 55 and 66,
+    // of 700 (1.18) 121 and 113; 512 rows after 800 others (1.39) 240 and 205; where blocks are of like length, as in
+    // a decode step of 64 sequences with 8 key/value heads after 1,000 tokens, 488 and 291.
+    const bool alone = longest_blocks > 0.0f && longest_blocks <= 1.02f * sm_count();
 #define RFX_GO(NI)                                                                                                 \
     do {                                                                                                           \
-        size_t smem = (QUERIES * 32 * NI + 2 * KEYS * (64 * NI + 4) + WARPS * 2 * KEYS * 2) * sizeof(float);         \
-        if (alone && smem < 120 * 1024) smem = 120 * 1024;                                                           \
+        constexpr size_t need = (QUERIES * 32 * NI + 2 * KEYS * (64 * NI + 4) + WARPS * 2 * KEYS * 2) * sizeof(float); \
+        constexpr size_t most = need < 120 * 1024 ? 120 * 1024 : need;                                                \
+        const size_t smem = alone ? most : need;                                                                    \
         cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                             (int)smem);                                                            \
+                                             (int)most);                                                            \
         if (e != cudaSuccess) return (int)e;                                                                        \
         RFX_LAUNCH(attention_f32_kernel<NI>, grid, WARPS * 32, smem, (cudaStream_t)stream, a);                        \
         return 0;                                                                                                   \

@@ -525,6 +525,23 @@ def attention_plain(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     return out
 
 
+def _longest_blocks(batch, nq: int, nkv: int, window) -> float:
+    """The work of csrc/attention_f32.cu's blocks, in blocks as long as the longest, where they differ in length and the
+    longest go first (several blocks a sequence, no window that ends them) and the batch's host side says; else 0."""
+    counts, starts = getattr(batch, "new_counts", None), getattr(batch, "starts", None)
+    if not counts or starts is None or nkv <= 0 or nq % nkv:  # (the kernel refuses the last two)
+        return 0.0
+    group = nq // nkv
+    heads = min(group, 16)
+    rows, sets = 16 // heads, nkv * -(-group // heads)  # of a block; blocks side by side
+    if max(counts) <= rows:
+        return 0.0
+    longest = max(s + n for s, n in zip(starts, counts))
+    if window and longest > window:
+        return 0.0
+    return sets * sum(-(-n // rows) * (s + 0.5 * n) for s, n in zip(starts, counts)) / longest
+
+
 def attention_f32(q, k_pages, v_pages, page_table, page_size, batch, nq: int, nkv: int, head_dim: int, window, scale,
                   sink=None, slopes=None, keep_first: int = 0, softcap: float = 0.0) -> Optional[torch.Tensor]:
     """`attention_plain`'s 32-bit results, bit for bit, from a kernel that takes 32 keys and
@@ -541,7 +558,7 @@ def attention_f32(q, k_pages, v_pages, page_table, page_size, batch, nq: int, nk
         _chk(batch.seq_new, "seq_new", torch.int32), _chk(batch.seq_row0, "seq_row0", torch.int32), out.data_ptr(),
         batch.seq_slot.numel(), most, nq, nkv, head_dim, int(window or 0),
         int(keep_first if window else 0), float(scale), _chk(sink, "sink", torch.float32),
-        _chk(slopes, "slopes", torch.float32), float(softcap), _stream())
+        _chk(slopes, "slopes", torch.float32), float(softcap), _longest_blocks(batch, nq, nkv, window), _stream())
     if st == native.ERR_UNSUPPORTED:
         return None
     native.check(st, f"attention_f32 (head_dim={head_dim})")

@@ -45,3 +45,20 @@ def test_decode_splits_grow_with_context_and_shrink_with_batch():
         picks = [decode_splits(rows, 32, 8, pages) for rows in (1, 8, 64, 256)]
         assert picks == sorted(picks, reverse=True)
         assert all(1 <= s <= 64 and s <= pages for s in picks)
+
+
+def test_which_batches_give_the_32_bit_attention_an_sm_a_block():
+    """The work in blocks as long as the longest: half of a new prompt's blocks, nearly all of a continued one's; nothing
+    where blocks do not differ in length or the host does not say."""
+    from types import SimpleNamespace as B
+
+    from reflex_b200.ops import _longest_blocks as f
+
+    assert f(B(new_counts=[512], starts=[0]), 8, 2, None) == 128
+    assert 200 < f(B(new_counts=[512], starts=[800]), 8, 2, None) < 256
+    assert 140 < f(B(new_counts=[155, 311, 235], starts=[0, 0, 0]), 8, 2, None) < 151
+    assert f(B(new_counts=[64], starts=[0]), 40, 2, 64) == 2 * 2 * 32  # two heads' blocks of sixteen and four, a row each
+    for b, window in ((B(new_counts=[1] * 64, starts=[1000] * 64), None), (B(new_counts=[4, 4], starts=[0, 9]), None),
+                      (B(new_counts=[512], starts=[0]), 100), (B(), None), (B(new_counts=[], starts=[]), None)):
+        assert f(b, 8, 2, window) == 0
+    assert f(B(new_counts=[512], starts=[0]), 8, 3, None) == 0 and f(B(new_counts=[512], starts=[0]), 8, 0, None) == 0

@@ -90,3 +90,20 @@ def test_attention_bits_with_pages_of_other_sizes(page):
     got = ops().attention_f32(q, k, v, t, page, b, nq, nkv, d, None, d ** -0.5)
     ref = ops().attention_plain(q, k, v, t, page, b.row_pos, b.row_slot, nq, nkv, d, None, d ** -0.5)
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("counts,starts", [((300, 40), (0, 0)), ((600,), (0,)), ((33, 65), (70, 0))])
+@pytest.mark.parametrize("d", [32, 128, 256])
+def test_attention_bits_with_one_block_an_sm_and_two(counts, starts, d):
+    """The host's lengths decide how many blocks share an SM; a batch that does not say has two."""
+    g = torch.Generator(device=DEV).manual_seed(d)
+    nq, nkv, n = 8, 2, len(counts)
+    per = max(s + c for s, c in zip(starts, counts)) // 64 + 1
+    k, v = (torch.randn((n * per, nkv, 64, d), generator=g, device=DEV) for _ in range(2))
+    t = torch.arange(n * per, dtype=torch.int32, device=DEV).view(n, per)
+    q, b, got = torch.randn((sum(counts), nq * d), generator=g, device=DEV), Batch(counts, starts, range(n)), []
+    for _ in range(2):
+        got.append(ops().attention_f32(q, k, v, t, 64, b, nq, nkv, d, None, d ** -0.5))
+        b.new_counts, b.starts = list(counts), list(starts)
+    assert 0 < ops()._longest_blocks(b, nq, nkv, None)
+    assert torch.equal(*got)
