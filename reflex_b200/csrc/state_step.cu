@@ -68,7 +68,7 @@ ssd_step_kernel(const float* __restrict__ xbc, int ldx, const float* __restrict_
         s[i].z = fmaf(s[i].z, decay, b.z * dx);
         s[i].w = fmaf(s[i].w, decay, b.w * dx);
         if (live && p0 + SIDE * i < P) store4(S + (size_t)SIDE * i * N, s[i]);
-        y[i] = dot4(s[i], c);
+        y[i] = live ? dot4(s[i], c) : 0.0f;  // (an infinite x leaves NaN in lanes beyond N)
     }
 #pragma unroll
     for (int i = 0; i < COLS; ++i) y[i] = fmaf(d, x[i], lanes_sum<LANES>(y[i]));
@@ -133,7 +133,7 @@ delta_step_kernel(const float* __restrict__ proj, int ld, int r_off, int k_off, 
         s[i].z = fmaf(k.z, v[i], fmaf(w.z, s[i].z, -au.z * seen[i]));
         s[i].w = fmaf(k.w, v[i], fmaf(w.w, s[i].w, -au.w * seen[i]));
         if (live && j0 + SIDE * i < d) store4(S + (size_t)SIDE * i * d, s[i]);
-        o[i] = dot4(s[i], r);
+        o[i] = live ? dot4(s[i], r) : 0.0f;
     }
 #pragma unroll
     for (int i = 0; i < COLS; ++i) o[i] = lanes_sum<LANES>(o[i]);

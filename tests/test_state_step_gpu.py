@@ -94,3 +94,31 @@ def test_mlstm_step(heads, dim, vdim, slots):
     compare(lambda s, b, exact: ops().mlstm_scan(proj, (0, heads * dim, 2 * heads * dim, io, io + heads), bi, bf, 15.0,
                                                  dim ** -0.5, b, s, heads, dim, vdim, max_rows=b.max_new, exact=exact),
             state, slots)
+
+
+def test_infinite_values_stay_infinite_where_lanes_have_no_element():
+    """Sizes that leave lanes of a column without an element: an infinite value among positive numbers gives its own
+    results infinities, as walking does, and no NaN."""
+    g = torch.Generator(device=DEV).manual_seed(2)
+    R = lambda *s: torch.rand(s, generator=g, device=DEV)  # noqa: E731
+    heads, d, n = 2, 36, 3
+    hd, slots = heads * d, (2, 0, 1)
+
+    def bad(row, at):
+        row[:, at] = float("inf")
+        return row
+
+    def check(run, floats):
+        out = []
+        for batch, exact in ((Batch(slots), False), (Batch(slots, 2), True)):
+            state = start[:, :floats].clone()
+            out.append((run(state, batch, exact), state))
+        for a, b in zip(*out):
+            assert not a.isnan().any() and torch.equal(a.isinf(), b.isinf()) and a.isinf().any()
+
+    start = R(3, hd * d)
+    xbc, proj, one = bad(R(n, hd + 2 * d), 7), R(n, hd + heads), torch.ones(heads, device=DEV)
+    check(lambda s, b, exact: ops().ssd_scan(xbc, proj, 0, hd, one, -one, one, s, 0, b, heads, d, d, 1, exact=exact), hd * d)
+    rows, wpre, zero = bad(R(n, 4 * hd), 2 * hd + 7), R(n, hd), torch.zeros(hd, device=DEV)
+    check(lambda s, b, exact: ops().delta_rule(rows, 0, hd, 2 * hd, 3 * hd, wpre, zero, zero, 0.6, 1e-6, s, 0, b, heads, d,
+                                               exact=exact), hd * d)
