@@ -17,14 +17,14 @@
 // A walk through the rows has one chain of dependent steps a head and leaves most SMs without
 // work; chunks cost the memory's way out and back (heads x N x P floats each) and about twice the
 // arithmetic.  64 rows: with 32 the memories' traffic doubles, with 128 the products inside the chunk do.
-// A prompt of 2,048 rows, us: for 32 heads of 64 x 128 21 the chunks' sums, 13 the carry, 50 the rows (1,200
-// walking), for 8 of 128 x 256 24, 17 and 50 (760).  With the products by 32-bit multiply-adds, whose reads of
-// shared memory and whose latencies bound them, 42, 12 and 76, and 49, 18 and 65.  What bounds these now is
-// the instructions that take 32-bit numbers apart and put results together (about 1,500 a warp and item, 1.7 of
-// four issued a cycle); the tensor cores are busy a fifth of the time, the carry is bound by L2.
+// A prompt of 2,048 rows, us: for 32 heads of 64 x 128 21 the chunks' sums, 13.5 the carry, 58 the rows (1,200
+// walking), for 8 of 128 x 256 24, 17 and 57 (760).  With the products by 32-bit multiply-adds, whose reads of
+// shared memory and whose latencies bound them, 42, 12 and 76, and 49, 18 and 65.  What bounds these now is a block's
+// stages, which wait for one another: numbers taken apart, eight products a sixteen, sums out of tensor memory (1.5 of
+// four instructions issued a cycle, the tensor cores busy a quarter of the time); the carry is bound by L2.
 //
-// 2-norm errors against 64 bits, the same shapes: results 1.2e-7 and 1.0e-7 (1.24e-7 and 1.2e-7 by
-// multiply-adds), states 7.1e-8 and 6.2e-8 to 1.1e-7 (7.0e-8 and 5.8e-8 to 1.1e-7).
+// 2-norm errors against 64 bits, the same shapes, normal numbers: results 9.1e-8 and 1.07e-7 (1.36e-7 and 1.40e-7 by
+// multiply-adds), states 7.4e-8 and 1.18e-7 (9.5e-8 and 1.39e-7); other numbers in tc_split.cuh.
 //
 // A policy `Pol` gives: q, k, v rows (float32, 16-byte aligned, counts in fours), `heads`, `per`
 // (heads per q/k head), N (elements of q and k, at most 128), P (elements of v) and the functions

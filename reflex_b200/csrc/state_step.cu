@@ -4,8 +4,9 @@
 //
 // A row reads and writes its head's whole memory, 16 to 128 KB, so memory bounds the step.  The walks there
 // serve any number of rows: a warp has a column or four, and waits for the row, staged in shared memory
-// behind one or two barriers.  Here nothing is staged: a thread's share of the memory, eight or sixteen 16-byte
-// loads, is on its way at once with what it needs of the row, and a block has a head or half of one.
+// behind one or two barriers.  Here (but for the mLSTM's k and q) nothing is staged: a thread's share of the memory, up
+// to eight 16-byte loads (one to four where heads are few or small), is on its way at once with what it needs of the
+// row.  A block has 64 columns of a head, 32 or 16 where few heads leave SMs without one.
 //
 // us walking and now: state-space of 64 heads of 64 x 128, 59 sequences (247 MB) 127 and 48; mLSTM of 16 heads of
 // 128 x 256, 40 sequences (168 MB) 85 and 30; delta rule of 64 heads of 64, 40 sequences (84 MB) 59 and 19; gated
