@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 2) chunk_state_kernel(Pol pol, 
 template <class Pol>
 __global__ void __launch_bounds__(128, 4) chunk_carry_kernel(Pol pol, Step st) {
     constexpr int AHEAD = 8;
-    rfx::pdl_prologue();
+    rfx::pdl_wait();
     const int seq = st.round.seq0 + blockIdx.y, h = blockIdx.z;
     const int e = 4 * (blockIdx.x * 128 + threadIdx.x);
     const int E = pol.P * pol.N + (Pol::NORMALISER ? pol.N : 0);
@@ -295,6 +295,9 @@ __global__ void __launch_bounds__(128, 4) chunk_carry_kernel(Pol pol, Step st) {
                 S.w = fmaf(f.x, S.w, f.y * d[i].w);
             }
     }
+    // the next kernel's blocks are let in as these end: before, they crowd on the SMs that these leave free (48 rows of 32
+    // heads of 64 x 128: 29 us all three launches, 24 so)
+    rfx::pdl_launch_dependents();
     pol.store_state(slot, h, e, S);
 }
 

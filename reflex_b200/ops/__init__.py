@@ -903,17 +903,18 @@ def mlstm_state_floats(dim: int, vdim: int) -> int:
 
 
 MLSTM_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_CHUNK_MIN_ROWS", 48, 1, 1 << 30)
-# Rows of a sequence from which all chunks go side by side (csrc/mlstm_chunk.cu); three quarters of that with so many
-# (sequence, head) pairs that chunk after chunk fills the SMs twice, half as many again with about 32, which it just
-# fills.  Us side by side and chunk after chunk, heads of 128 x 256: 8 pairs 33 and 32 at 64 rows, 33.6 and 40.4 at 72;
-# 16 pairs 37.7 and 32 at 64, 38.3 and 40.6 at 72; 32 pairs 48.7 and 43.6 at 90, 48.7 and 52.3 at 100; 64 pairs 62.3
-# and 62.4 at 64, 75 and 79 at 72; 128 pairs 81 each at 32, 99 and 114 at 48.
+# Rows of a sequence from which all chunks go side by side (csrc/mlstm_chunk.cu): beyond 64 chunk after chunk takes one
+# more; three quarters of that with so few or so many (sequence, head) pairs that chunk after chunk leaves SMs idle or
+# fills them twice, half as many again with about 32, which it just fills.  Us side by side and chunk after chunk, heads
+# of 128 x 256: 8 pairs 21.5 each at 32 rows, 27.7 and 29.9 at 48; 16 pairs 32.5 and 32.1 at 64, 31.9 and 40.6 at 72; 32
+# pairs 49 and 43.4 at 90, 49 and 52.2 at 100; 64 pairs 63 and 62.5 at 64, 77 and 79 at 72; 128 pairs 81 each at 32, 100
+# and 115 at 48.
 MLSTM_SIDE_BY_SIDE_MIN_ROWS = _env_int("REFLEX_B200_MLSTM_SIDE_BY_SIDE_MIN_ROWS", 64, 1, 1 << 30)
 
 
 def _mlstm_side_by_side(most: int, rows: int, heads: int) -> bool:
     pairs = heads * rows // max(1, most)
-    return most >= MLSTM_SIDE_BY_SIDE_MIN_ROWS * (0.75 if pairs > 96 else 1.05 if pairs <= 16 else 1.52 if pairs < 48 else 1.0)
+    return most >= MLSTM_SIDE_BY_SIDE_MIN_ROWS * (0.75 if pairs <= 8 or pairs > 96 else 1.52 if 16 < pairs < 48 else 1.02)
 
 
 def mlstm_scan(proj: torch.Tensor, offsets, bias_i, bias_f, cap: float, q_scale: float, batch,
@@ -1843,8 +1844,8 @@ def _most_rows(batch) -> int:
 # Rows of the longest sequence from which the chunked kernels run where a step has about 64 (sequence, head) pairs;
 # more with fewer pairs, fewer with more: the walk's time grows with the rows and, once its blocks share SMs, with the
 # pairs, the chunks' hardly with either.  Measured, in chunks and walking, us at the rows around the crossing: 16 pairs
-# 26.8 and 23 at 80 rows, 27 and 31 at 112; 32 pairs 30 and 28.4 at 64, 29.7 and 32.3 at 71; 64 pairs 25.6 and 22.9 at
-# 33, 25.9 and 30.4 at 48; 128 pairs 31.4 and 30.7 at 33, 29.5 and 35.1 at 40; 256 pairs 40.9 and 39.9 at 27, 41 and 50
+# 24 and 22.9 at 80 rows, 24 and 26.4 at 96; 32 pairs 24.4 and 22.7 at 48, 24.7 and 25.4 at 56; 64 pairs 25.5 and 22.9 at
+# 33, 25.8 and 30.5 at 48; 128 pairs 30.6 and 30.7 at 33, 29.3 and 35 at 40; 256 pairs 41.1 and 40 at 27, 41.6 and 50
 # at 33.
 SSD_CHUNK_MIN_ROWS = _env_int("REFLEX_B200_SSD_CHUNK_MIN_ROWS", 44, 1, 1 << 30)
 
@@ -1853,8 +1854,8 @@ def _ssd_in_chunks(most: int, rows: int, heads: int) -> bool:
     if not most:
         return False
     pairs = heads * rows // most  # as many sequences as the step's rows would make of the longest
-    return most >= SSD_CHUNK_MIN_ROWS * (2.25 if pairs < 32 else 1.5 if pairs < 40 else 0.9 if pairs <= 64 else
-                                         0.8 if pairs <= 128 else 0.65)
+    return most >= SSD_CHUNK_MIN_ROWS * (2.0 if pairs < 32 else 1.25 if pairs < 40 else 0.9 if pairs <= 64 else
+                                         0.77 if pairs <= 128 else 0.65)
 
 
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, z_off: int, dt_off: int, dt_bias: torch.Tensor, A: torch.Tensor,
